@@ -11,7 +11,6 @@ namespace mat {
 __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double sub(double a, double b) { return __dadd_rn(a, -b); }
-__device__ __forceinline__ double dvd(double a, double b) { return __ddiv_rn(a, b); }
 
 // a / b where the divisor b is fixed for the run and y = RN(1 / b) was
 // formed once on the host.  Markstein's correction q' = RN(q + r y), with the
@@ -20,7 +19,7 @@ __device__ __forceinline__ double dvd(double a, double b) { return __ddiv_rn(a, 
 // returns the correctly rounded quotient (P. Markstein, "Computation of
 // elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
 // Dev. 34(1), 1990).  Five FP64 operations in place of a full division; the
-// result equals dvd(a, b) for normal operands and quotients (a zero quotient
+// result equals a / b for normal operands and quotients (a zero quotient
 // comes out +0, and non-finite operands are not carried through).
 __device__ __forceinline__ double dvd_known(double a, double b, double y)
 {
@@ -31,30 +30,238 @@ __device__ __forceinline__ double dvd_known(double a, double b, double y)
     return __fma_rn(r, y, q);
 }
 
-constexpr double kThird = 1.0 / 3.0;   // RN(1/3), the reciprocal of the divisor 3.0
+// A divisor b fixed for the run, with its reciprocal as an unevaluated sum
+// zh + zl (zh = RN(1/b), zl = RN(1/b - zh)), formed on the host.
+struct Known {
+    double b, zh, zl;
+    int two;   // RN(a zh + RN(a zl)) is RN(a / b) for every normal a
+};
+
+// The two-operation quotient of Brisebarre, Muller and Raina ("Accelerating
+// correctly rounded floating-point division when the divisor is known in
+// advance", IEEE Trans. Computers 53(8), 2004).  Scaled to [1, 2) each, with
+// B = 2^52 b and A = 2^52 a: a zh + RN(a zl) is within 2^-106 of a / b (half
+// an ulp of zl times a, plus half an ulp of a zl), and a quotient's distance
+// from a midpoint of two doubles is |D| / (B 2^53) for a >= b and
+// |D| / (B 2^54) for a < b, D = A 2^53 - (2 M + 1) B (or with 2^54) a nonzero
+// integer.  So a >= b always rounds correctly, and a < b unless |D| = 1, which
+// needs an odd B and then fixes 2 M + 1 = -D / B modulo 2^54: `two` records
+// that these two numerators come out right.
+inline Known make_known(double b)
+{
+    Known k;
+    k.b = b;
+    k.zh = 1.0 / b;
+    k.zl = 0.0;
+    k.two = 0;
+    const double m = fabs(b);
+    if (!(m > 0x1p-400 && m < 0x1p400)) return k;
+    k.zl = fma(-b, k.zh, 1.0) / b;
+    k.two = 1;
+    int e;
+    const uint64_t B = (uint64_t)ldexp(frexp(m, &e), 53);
+    if ((B & 1) == 0) return k;
+    const double bm = (double)B, zh = 1.0 / bm, zl = fma(-bm, zh, 1.0) / bm;
+    uint64_t inv = B;                                   // B^-1 mod 2^64 by Newton's iteration
+    for (int i = 0; i < 5; i++) inv *= 2 - B * inv;
+    const uint64_t mask = (1ull << 54) - 1;
+    for (int sign = 0; sign < 2; sign++) {
+        const uint64_t odd = (sign ? inv : 0 - inv) & mask;
+        const unsigned __int128 prod = (unsigned __int128)odd * B + (sign ? (unsigned __int128)0 : 1) -
+                                       (sign ? (unsigned __int128)1 : 0);
+        const uint64_t A = (uint64_t)(prod >> 54);
+        if (A < (1ull << 52) || A >= B) continue;
+        const double a = (double)A;
+        if (fma(a, zh, a * zl) != a / bm) k.two = 0;
+    }
+    return k;
+}
+
+static __device__ __noinline__ double dvd_slow(double a, double b, double y)
+{
+    return dvd_known(a, b, y);
+}
+
+// a / b correctly rounded, for normal operands and quotients (and a = 0, which
+// gives a zero), in two FP64 operations for all but rare divisors.
+__device__ __forceinline__ double dvd_const(double a, const Known &k)
+{
+    if (!k.two) return dvd_slow(a, k.b, k.zh);
+    return __fma_rn(a, k.zh, __dmul_rn(a, k.zl));
+}
+
+// a / 3: RN(1/3) = 1/3 - 2^-54/3.  a / 3 is never nearer than 2^-54/3 times
+// its binade to a midpoint (a - 3 m is a nonzero multiple of half its ulp), so
+// the two operations suffice.
+__device__ __forceinline__ double third(double a)
+{
+    return __fma_rn(a, 0x1.5555555555555p-2, __dmul_rn(a, 0x1.5555555555555p-56));
+}
+
+// Sign and order tests on the bit patterns (the FP64 pipe issues a compare at
+// the rate of a multiply): non-negative doubles order as integers.
+__device__ __forceinline__ bool is_nan(double a)
+{
+    return (__double_as_longlong(a) & 0x7fffffffffffffffLL) > 0x7ff0000000000000LL;
+}
+__device__ __forceinline__ bool is_pos(double a)   // a > 0
+{
+    const long long b = __double_as_longlong(a);
+    return b > 0 && b <= 0x7ff0000000000000LL;
+}
+__device__ __forceinline__ bool is_neg(double a)   // a < 0
+{
+    const long long b = __double_as_longlong(a);
+    return b > (long long)0x8000000000000000ULL && b <= (long long)0xfff0000000000000ULL;
+}
+__device__ __forceinline__ bool less_equal_pos(double a, double b)   // a <= b for a >= +0 or NaN, b not -0
+{
+    const long long x = __double_as_longlong(a), y = __double_as_longlong(b);
+    return x >= 0 && x <= y && y <= 0x7ff0000000000000LL;
+}
+__device__ __forceinline__ bool is_finite(double a)
+{
+    return (__double2hiint(a) & 0x7ff00000) != 0x7ff00000;
+}
+// IEEE square root and quotient in three FP64 operations.  GB300's FP64 pipe
+// runs at 1/64 of its FP32 rate and bounds the kernels that use these, while
+// the integer and FP32 pipes idle: so the seed is refined there.  The operand's
+// 52-bit significand is split into an FP32 head and tail, the approximate FP32
+// reciprocal (root) gives the result's head, and the head's residual, exact in
+// an FP32 FMA, its tail: head + tail is good to about 2^-44 and is assembled
+// into a double by integer addition (the head held in [1, 2], where the
+// double's spacing is one).  One FP64 correction with the exact
+// residual then lands within 2^-64 relative of the value before its rounding,
+// so the rounded result is at most one ulp from the correctly rounded one, and
+// the residual of that result (exact: it has at most 53 bits) decides: it is
+// kept where its magnitude is at most that of half an ulp, else moved by one.
+// A square root or quotient of doubles is never a midpoint, so this decision
+// is exact.  The compiler's operations issue eight FP64 instructions each; with
+// these, the two-operation constant quotients and the integer compares above,
+// the G2P with g_local_mu2 went from 211 to 164 FP64 instructions a particle
+// and from 417 to 327 us at 1 048 576 particles.  Zeros, negatives, non-finite values and exponents near the ends
+// of the range take the compiler's operation.
+
+// The FP32 head (in [1, 2)) and tail of a double's significand.
+__device__ __forceinline__ float sig_head(int hi, int lo, int exponent)
+{
+    return __int_as_float(((127 + exponent) << 23) | ((hi & 0xfffff) << 3) | (int)((unsigned)lo >> 29));
+}
+__device__ __forceinline__ float sig_tail(int lo, float unit)   // to 23 bits, without a conversion
+{
+    return (__int_as_float(0x3f800000 | (lo & 0x1fffffff) >> 6) - 1.0f) * unit;
+}
+// The bits of the double with a normal float's value times 2^e.
+__device__ __forceinline__ long long widen(float f, int e)
+{
+    const unsigned b = __float_as_uint(f);
+    return __double_as_longlong(__hiloint2double((int)((b >> 3) + ((unsigned)(896 + e) << 20)), (int)(b << 29)));
+}
+
+// A non-negative integer as a double, in integer arithmetic (conversions run
+// on the FP64 pipe).
+__device__ __forceinline__ double small_int(int c)
+{
+    const int z = __clz(c);
+    const unsigned m = (unsigned)c << (z & 31);
+    return __hiloint2double(c == 0 ? 0 : (int)(((1022u + 31 - z) << 20) + (m >> 11)), c == 0 ? 0 : (int)(m << 21));
+}
+
+// sqrt(2^E x).
+template <int E = 0>
+__device__ __forceinline__ double root(double x)
+{
+    if ((unsigned)__double2hiint(x) - (223u << 20) >= (1600u << 20))   // outside 2^-800 .. 2^800
+        return __dsqrt_rn(E == 0 ? x : __dmul_rn(x, E == -1 ? 0.5 : 2.0));
+    const int hi = __double2hiint(x) + (E << 20), lo = __double2loint(x);
+    if (E != 0) x = __hiloint2double(hi, lo);
+    const int e = (hi >> 20) - 1023, odd = e & 1, k = e >> 1;
+    // x = m 4^k, m = head + tail in [1, 4)
+    const float mh = sig_head(hi, lo, odd), ml = sig_tail(lo, odd ? 0x1p-22f : 0x1p-23f);
+    const float y = rsqrtf(mh);
+    const float sh = fminf(fmaxf(mh * y, 1.0f), 2.0f);
+    const float sl = 0.5f * y * (__fmaf_rn(-sh, sh, mh) + ml);
+    const long long sb = widen(sh, k) + ((long long)__float2int_rn(sl * 0x1p50f) << 2);
+    const double s0 = __longlong_as_double(sb);
+    const double h = __longlong_as_double(widen(y, -k - 1));
+    const double s = __fma_rn(__fma_rn(-s0, s0, x), h, s0);
+    const double r = __fma_rn(-s, s, x);
+    // sqrt(x) <= s + u/2 iff r <= s u, and sqrt(x) >= s - u/2 iff r > -s u
+    // (r and s u are multiples of u^2); below a power of two the gap is half
+    long long b = __double_as_longlong(s);
+    const long long su = b + ((long long)((int)(b >> 52) - 1023 - 52) << 52);
+    const long long rb = __double_as_longlong(r), mag = rb & 0x7fffffffffffffffLL;
+    if (rb >= 0) b += mag > su ? 1 : 0;
+    else b -= mag >= su - ((b & 0xfffffffffffffLL) == 0 ? (1LL << 52) : 0) ? 1 : 0;
+    return __longlong_as_double(b);
+}
+
+// 2^E a / b.
+template <int E = 0>
+__device__ __forceinline__ double quot(double a, double b)
+{
+    int ah = __double2hiint(a) & 0x7fffffff;
+    const int al = __double2loint(a);
+    const int bh = __double2hiint(b) & 0x7fffffff, bl = __double2loint(b);
+    if ((unsigned)ah - (623u << 20) >= (800u << 20) || (unsigned)bh - (623u << 20) >= (800u << 20))
+        return __ddiv_rn(E == 0 ? a : __dmul_rn(a, 2.0), b);   // outside 2^-400 .. 2^400
+    static_assert(E == 0 || E == 1, "the fallback's factor");
+    ah += E << 20;
+    const long long ab = (long long)((unsigned long long)(unsigned)ah << 32 | (unsigned)al);
+    const long long bb = __double_as_longlong(b) & 0x7fffffffffffffffLL;
+    const long long frac = 0xfffffffffffffLL;
+    // significands scaled so that the quotient's lies in [1, 2)
+    const int up = (ab & frac) < (bb & frac) ? 1 : 0;
+    const float afh = sig_head(ah, al, up), afl = sig_tail(al, up ? 0x1p-22f : 0x1p-23f);
+    const float bfh = sig_head(bh, bl, 0), bfl = sig_tail(bl, 0x1p-23f);
+    const float y = __fdividef(1.0f, bfh);
+    const float qh = fminf(fmaxf(afh * y, 1.0f), 2.0f);
+    const float ql = __fmaf_rn(-qh, bfl, __fmaf_rn(-qh, bfh, afh) + afl) * y;
+    const int eb = (bh >> 20) - 1023, eq = (ah >> 20) - 1023 - eb - up;
+    const double am = __longlong_as_double(ab), bm = __longlong_as_double(bb);
+    const double q0 = __longlong_as_double(widen(qh, eq) + ((long long)__float2int_rn(ql * 0x1p50f) << 2));
+    const double yd = __longlong_as_double(widen(y, -eb));
+    const double q = __fma_rn(__fma_rn(-bm, q0, am), yd, q0);
+    const double r = __fma_rn(-bm, q, am);
+    // |a - b q| against b times half the gap to the neighbour (the gap below a
+    // power of two is half the one above)
+    long long qb = __double_as_longlong(q);
+    const long long rb = __double_as_longlong(r), mag = rb & 0x7fffffffffffffffLL;
+    const long long above = bb + ((long long)((int)(qb >> 52) - 1023 - 53) << 52);
+    if (rb >= 0) qb += mag > above ? 1 : 0;
+    else qb -= mag > above - ((qb & frac) == 0 ? (1LL << 52) : 0) ? 1 : 0;
+    const long long sign = (__double_as_longlong(a) ^ __double_as_longlong(b)) & (long long)0x8000000000000000ULL;
+    return __longlong_as_double(qb | sign);
+}
 
 struct Elastic {
     double G, K, lambda, dt;
     double twoG;            // 2 G, exact
-    double inv_G, inv_dt;   // RN(1/G), RN(1/dt)
-    double Gdt, inv_Gdt;    // RN(G dt), RN(1 / RN(G dt))
+    double Gdt;             // RN(G dt)
+    Known kG, kdt, kGdt;    // G, dt and RN(G dt) as divisors
 };
 
 // exp(x) for the volume update v <- v exp(dt tr D), whose argument is tiny at
-// any stable time step: where |x| < 2^-9 the degree-5 Taylor polynomial about
-// 0 in Horner form (truncation below x^6 / 720 < 2^-63, under a tenth of an
-// ulp of the result, so the result lies within about half an ulp of e^x);
-// elsewhere exp().
+// any stable time step: where |x| < 2^-14 the degree-3 Taylor polynomial about
+// 0 in Horner form (truncation below x^4 / 24 < 2^-60), where |x| < 2^-9 the
+// degree-5 one (below x^6 / 720 < 2^-63), either under a tenth of an ulp of the
+// result, so the result lies within about half an ulp of e^x; elsewhere exp().
+static __device__ __noinline__ double exp_wide(double x)
+{
+    if ((__double2hiint(x) & 0x7fffffff) >= 0x3f600000) return exp(x);
+    double p = __fma_rn(x, 1.0 / 120.0, 1.0 / 24.0);
+    p = __fma_rn(p, x, 1.0 / 6.0);
+    p = __fma_rn(p, x, 0.5);
+    p = __fma_rn(p, x, 1.0);
+    return __fma_rn(p, x, 1.0);
+}
+
 __device__ __forceinline__ double exp_small(double x)
 {
-    if ((__double2hiint(x) & 0x7fffffff) < 0x3f600000) {
-        double p = __fma_rn(x, 1.0 / 120.0, 1.0 / 24.0);
-        p = __fma_rn(p, x, 1.0 / 6.0);
-        p = __fma_rn(p, x, 0.5);
-        p = __fma_rn(p, x, 1.0);
-        return __fma_rn(p, x, 1.0);
-    }
-    return exp(x);
+    if ((__double2hiint(x) & 0x7fffffff) >= 0x3f100000) return exp_wide(x);
+    double p = __fma_rn(x, 1.0 / 6.0, 0.5);
+    p = __fma_rn(p, x, 1.0);
+    return __fma_rn(p, x, 1.0);
 }
 
 // isolin calculate_stress_threaded, materialsrc/isolin.c:75-116.
@@ -75,19 +282,21 @@ __device__ __forceinline__ void isolin(const Elastic &el, double exx, double exy
     syy = add(syy, mul(el.dt, dsjyy));
 }
 
-// negative_root, g_local_mu2.c:90-99 (also g_nonlocal_mu2.c:226-235).
-__device__ __forceinline__ double negative_root(double a, double b, double c)
+// negative_root, g_local_mu2.c:90-99 (also g_nonlocal_mu2.c:226-235), with
+// a = 1: the products by 4 and 2 are exact, so they ride in an FMA and in the
+// quotient's exponent.
+__device__ __forceinline__ double negative_root(double b, double c)
 {
-    double disc = __dsqrt_rn(sub(mul(b, b), mul(mul(4.0, a), c)));
-    if (b > 0) return dvd(sub(-b, disc), mul(2.0, a));
-    return dvd(mul(2.0, c), add(-b, disc));
+    const double disc = root(__fma_rn(-4.0, c, mul(b, b)));
+    if (is_pos(b)) return mul(0.5, sub(-b, disc));
+    return quot<1>(c, sub(disc, b));
 }
 
 struct Mu2Params {
     double mu_s, mu_2, I0, grains_rho, grains_d, rho_critical, A;
-    double inv_grains_rho, inv_grains_d;   // RN(1/grains_rho), RN(1/grains_d)
-    double rho_lo, rho_hi;                 // RN(rho_critical (1 - 2^-47)), RN(rho_critical (1 + 2^-47))
-    double AAdd, inv_AAdd;                 // RN(RN(RN(A A) d) d) and its reciprocal
+    Known krho, kd, kAAdd;                 // grains_rho, grains_d and A^2 d^2 as divisors
+    double rho_lo, rho_hi;                 // RN(rho_critical (1 - 2^-47)), RN(rho_critical (1 + 2^-47)); -1 and
+                                           // infinity (no bracket) where rho_critical is not in 2^-60 .. 2^60
     double alpha_c;                        // G I0 dt / (grains_d sqrt(grains_rho))
     double GI0dt;                          // RN(RN(G I0) dt), formed on the host
 };
@@ -99,13 +308,16 @@ struct Mu2Params {
 // m > RN(v rho_hi) implies m / v > rho_critical (1 + 2^-48), hence
 // RN(m / v) > rho_critical (the roundings add at most 3 2^-53 relative, and
 // the doubles within 2^-48 of rho_critical are further than an ulp from it).
-// Only m inside the bracket, and any v that is not a normal positive number
-// above 2^-959 (or a NaN), takes the division.
+// Only m inside the bracket, and any operand that is not a normal positive
+// number above 2^-959 (or a NaN), takes the division.  Positive normal
+// products and m order as integers; the dense side is tested first.
 __device__ __forceinline__ bool below_density(double m, double v, const Mu2Params &mp)
 {
-    if (__double_as_longlong(v) > 0x0400000000000000LL && __double_as_longlong(v) < 0x7ff0000000000000LL) {
-        if (m < __dmul_rn(v, mp.rho_lo)) return true;
-        if (m > __dmul_rn(v, mp.rho_hi)) return false;
+    const long long mb = __double_as_longlong(m), vb = __double_as_longlong(v);
+    if (vb > 0x0400000000000000LL && vb < 0x7ff0000000000000LL && mb > 0x0400000000000000LL &&
+        mb < 0x7ff0000000000000LL) {
+        if (mb > __double_as_longlong(__dmul_rn(v, mp.rho_hi))) return false;
+        if (mb < __double_as_longlong(__dmul_rn(v, mp.rho_lo))) return true;
     }
     return __ddiv_rn(m, v) < mp.rho_critical;
 }
@@ -123,67 +335,56 @@ __device__ __forceinline__ void g_local_mu2(const Elastic &el, const Mu2Params &
     const double G = el.G, dt = el.dt;
     const double lambda = el.lambda;   // K - 2 G / 3, formed on the host with the same roundings
     // L (:191-199), W = skw(L), D = sym(L) (tensor.c:330-384)
-    // Exact shortcuts, bit for bit the reference's values for finite
-    // operands below DBL_MAX / 2: 0.5 (x + x) is x; W T - T W has xx entry
-    // RN(W Txy) + RN(W Txy), an exact doubling, and yy entry its negative;
-    // 0 * 2G is +0.
-    double Lxy = add(exy, wxy), Lyx = sub(exy, wxy);
-    double Wxy = mul(0.5, sub(Lxy, Lyx));
-    double Dxx = exx;
-    double Dxy = mul(0.5, add(Lxy, Lyx));
-    double Dyy = eyy;
-    double trD = add(Dxx, Dyy);
+    // Exact shortcuts, bit for bit the reference's values for normal
+    // operands below DBL_MAX / 2 (a halving or doubling commutes with a
+    // rounding): 0.5 (x + x) is x; with w2 = Lxy - Lyx = 2 Wxy, W T - T W has
+    // xx entry RN(Wxy Txy) + RN(Wxy Txy) = RN(w2 Txy), yy entry its negative,
+    // and xy entry half of RN(w2 Tyy) - RN(Txx w2), added with one rounding by
+    // an FMA; with d2 = Lxy + Lyx = 2 Dxy, Dxy 2G is d2 G; 0 * 2G is +0.
+    const double Lxy = add(exy, wxy), Lyx = sub(exy, wxy);
+    const double w2 = sub(Lxy, Lyx), d2 = add(Lxy, Lyx);
+    const double trD = add(exx, eyy);
     // Jaumann term JS = W T - T W (:209-212)
-    const double wt = mul(Wxy, Txy);
-    double JSxx = add(wt, wt);
-    double JSxy = add(mul(Wxy, Tyy), -mul(Txx, Wxy));
-    double JSyy = -JSxx;
+    const double JSxx = mul(w2, Txy);
+    const double JSxy2 = sub(mul(w2, Tyy), mul(Txx, w2));
     // trial stress (:215-222)
     const double twoG = el.twoG;
-    double lt = mul(lambda, trD);
-    double Txx_tr = add(mul(add(add(mul(Dxx, twoG), lt), JSxx), dt), Txx);
-    double Txy_tr = add(mul(add(mul(Dxy, twoG), JSxy), dt), Txy);
-    double Tyy_tr = add(mul(add(add(mul(Dyy, twoG), lt), JSyy), dt), Tyy);
-    double Tzz_tr = add(mul(add(0.0, lt), dt), Tzz);
+    const double lt = mul(lambda, trD);
+    const double Txx_tr = add(mul(add(add(mul(exx, twoG), lt), JSxx), dt), Txx);
+    const double Txy_tr = add(mul(__fma_rn(0.5, JSxy2, mul(d2, G)), dt), Txy);
+    const double Tyy_tr = add(mul(sub(add(mul(eyy, twoG), lt), JSxx), dt), Tyy);
+    const double Tzz_tr = add(mul(lt, dt), Tzz);
     // decompose and contract (:225-228; tensor.c:205-224, :422-437)
-    double p_tr = dvd_known(add(add(Txx_tr, Tyy_tr), Tzz_tr), 3.0, kThird);
-    double T0xx = sub(Txx_tr, p_tr), T0xy = Txy_tr, T0yy = sub(Tyy_tr, p_tr), T0zz = sub(Tzz_tr, p_tr);
-    double tt = add(add(add(add(mul(T0xx, T0xx), mul(T0xy, T0xy)), mul(T0xy, T0xy)), mul(T0yy, T0yy)),
-                    mul(T0zz, T0zz));
-    double tau_tr = __dsqrt_rn(mul(0.5, tt));
+    double p_tr = third(add(add(Txx_tr, Tyy_tr), Tzz_tr));
+    const double T0xx = sub(Txx_tr, p_tr), T0xy = Txy_tr, T0yy = sub(Tyy_tr, p_tr), T0zz = sub(Tzz_tr, p_tr);
+    const double xy2 = mul(T0xy, T0xy);
+    const double tt = add(add(add(add(mul(T0xx, T0xx), xy2), xy2), mul(T0yy, T0yy)), mul(T0zz, T0zz));
+    const double tau_tr = root<-1>(tt);
     p_tr = -p_tr;
 
     const bool density_flag = below_density(m, v, mp);
     double nup_tau;
-    if (density_flag || p_tr <= 0) {
+    if (density_flag || !(is_pos(p_tr) || is_nan(p_tr))) {
         nup_tau = 0;
         Txx = 0; Txy = 0; Tyy = 0; Tzz = 0;
-    } else if (p_tr > 0) {
-        double S0 = mul(mp.mu_s, p_tr);
-        if (tau_tr <= S0 && isfinite(tau_tr)) {
+    } else if (is_pos(p_tr)) {
+        const double S0 = mul(mp.mu_s, p_tr);
+        if (less_equal_pos(tau_tr, S0)) {
             // tau_tau = tau_tr, scale factor 1: (tau_tr - tau_tau) / G / dt
             // is +0 and T0 * 1 is T0 exactly, so neither is formed
-            nup_tau = 0;
+            nup_tau = is_finite(tau_tr) ? 0.0 : mul(sub(tau_tr, tau_tr), dt);
             Txx = sub(T0xx, p_tr);
             Txy = T0xy;
             Tyy = sub(T0yy, p_tr);
             Tzz = sub(T0zz, p_tr);
         } else {
-            double tau_tau, scale_factor;
-            if (tau_tr <= S0) {
-                tau_tau = tau_tr;
-                scale_factor = 1.0;
-            } else {
-                double S2 = mul(mp.mu_2, p_tr);
-                double alpha = dvd_known(mul(mp.GI0dt,
-                                             __dsqrt_rn(dvd_known(p_tr, mp.grains_rho, mp.inv_grains_rho))),
-                                         mp.grains_d, mp.inv_grains_d);
-                double B = -add(add(S2, tau_tr), alpha);
-                double H = add(mul(S2, tau_tr), mul(S0, alpha));
-                tau_tau = negative_root(1.0, B, H);
-                scale_factor = dvd(tau_tau, tau_tr);
-            }
-            nup_tau = dvd_known(dvd_known(sub(tau_tr, tau_tau), G, el.inv_G), dt, el.inv_dt);
+            const double S2 = mul(mp.mu_2, p_tr);
+            const double alpha = dvd_const(mul(mp.GI0dt, root(dvd_const(p_tr, mp.krho))), mp.kd);
+            const double B = -add(add(S2, tau_tr), alpha);
+            const double H = add(mul(S2, tau_tr), mul(S0, alpha));
+            const double tau_tau = negative_root(B, H);
+            const double scale_factor = quot(tau_tau, tau_tr);
+            nup_tau = dvd_const(dvd_const(sub(tau_tr, tau_tau), el.kG), el.kdt);
             Txx = sub(mul(T0xx, scale_factor), p_tr);
             Txy = mul(T0xy, scale_factor);
             Tyy = sub(mul(T0yy, scale_factor), p_tr);
@@ -235,7 +436,7 @@ __device__ __forceinline__ void plane_return(const Elastic &el, const ReturnPara
     double p_tr, t0zz = 0, szz_tr = 0;
     if (TRIAL3D) {
         szz_tr = add(szz, mul(mul(dt, lambda), trD));
-        p_tr = dvd(-add(add(sxx_tr, syy_tr), szz_tr), 3.0);
+        p_tr = third(-add(add(sxx_tr, syy_tr), szz_tr));
     } else {
         p_tr = mul(-0.5, add(sxx_tr, syy_tr));
     }
@@ -245,13 +446,13 @@ __device__ __forceinline__ void plane_return(const Elastic &el, const ReturnPara
         t0zz = add(szz_tr, p_tr);
         tt = add(tt, mul(t0zz, t0zz));
     }
-    double tau_tr = __dsqrt_rn(mul(0.5, tt));
+    double tau_tr = root(mul(0.5, tt));
 
-    const bool density_flag = dvd(m, v) < rp.rho_critical;
+    const bool density_flag = quot(m, v) < rp.rho_critical;
     double nup_tau;
     if (density_flag || p_tr <= 0) {
-        nup_tau = dvd(tau_tr, mul(G, dt));
-        if (BETA) beta = dvd(-p_tr, mul(K, dt));
+        nup_tau = dvd_const(tau_tr, el.kGdt);
+        if (BETA) beta = quot(-p_tr, mul(K, dt));
         sxx = 0; sxy = 0; syy = 0;
         if (TRIAL3D) szz = 0;
     } else if (p_tr > 0) {
@@ -262,16 +463,16 @@ __device__ __forceinline__ void plane_return(const Elastic &el, const ReturnPara
             scale_factor = 1.0;
         } else if (MU_I) {
             double S2 = mul(rp.mu_2, p_tr);
-            double alpha = dvd(mul(mul(mul(G, rp.I0), dt), __dsqrt_rn(dvd(p_tr, rp.grains_rho))), rp.grains_d);
+            double alpha = quot(mul(mul(mul(G, rp.I0), dt), root(quot(p_tr, rp.grains_rho))), rp.grains_d);
             double B = -add(add(S2, tau_tr), alpha);
             double H = add(mul(S2, tau_tr), mul(S0, alpha));
-            tau_tau = negative_root(1.0, B, H);
-            scale_factor = dvd(tau_tau, tau_tr);
+            tau_tau = negative_root(B, H);
+            scale_factor = quot(tau_tau, tau_tr);
         } else {
             tau_tau = S0;
-            scale_factor = dvd(tau_tau, tau_tr);
+            scale_factor = quot(tau_tau, tau_tr);
         }
-        nup_tau = dvd(dvd(sub(tau_tr, tau_tau), G), dt);
+        nup_tau = dvd_const(dvd_const(sub(tau_tr, tau_tau), el.kG), el.kdt);
         if (BETA) beta = 0;
         sxx = sub(mul(scale_factor, t0xx), p_tr);
         sxy = mul(scale_factor, t0xy);
@@ -293,8 +494,8 @@ __device__ __forceinline__ void g_local_mu2_reverse(const Elastic &el, const Mu2
                                                     double &sxy, double &syy, double &beta, double &gammap,
                                                     double &gammadotp)
 {
-    const double G = el.G, K = el.K, dt = el.dt, c = 0;
-    const double lambda = sub(K, dvd(mul(2.0, G), 3.0));
+    const double K = el.K, dt = el.dt, c = 0;
+    const double lambda = el.lambda;
     const double twoG = el.twoG;
     double p_t = mul(-0.5, add(sxx, syy));
     double trD = add(exx, eyy);
@@ -310,24 +511,24 @@ __device__ __forceinline__ void g_local_mu2_reverse(const Elastic &el, const Mu2
     double syy_tr = add(syy, mul(dt, dsjyy));
     double p_tr = mul(-0.5, add(sxx_tr, syy_tr));
     double t0xx = add(sxx_tr, p_tr), t0xy = sxy_tr, t0yy = add(syy_tr, p_tr);
-    double tau_tr = __dsqrt_rn(mul(0.5, add(add(mul(t0xx, t0xx), mul(mul(2.0, t0xy), t0xy)), mul(t0yy, t0yy))));
-    double inum = mul(mul(gammadotp, mp.grains_d), __dsqrt_rn(mp.grains_rho));
+    double tau_tr = root<-1>((add(add(mul(t0xx, t0xx), mul(mul(2.0, t0xy), t0xy)), mul(t0yy, t0yy))));
+    double inum = mul(mul(gammadotp, mp.grains_d), root(mp.grains_rho));
     double mu_t;
     if (p_t <= 0) {
         mu_t = mp.mu_2;
     } else {
-        inum = dvd(inum, __dsqrt_rn(p_t));
+        inum = quot(inum, root(p_t));
         if (inum <= 0) mu_t = mp.mu_s;
-        else mu_t = add(mp.mu_s, dvd(sub(mp.mu_2, mp.mu_s), add(dvd(mp.I0, inum), 1.0)));
+        else mu_t = add(mp.mu_s, quot(sub(mp.mu_2, mp.mu_s), add(quot(mp.I0, inum), 1.0)));
     }
     double tau_tau = mul(mu_t, add(p_tr, c));
     double f = sub(tau_tr, tau_tau);
-    const bool density_flag = dvd(m, v) < mp.rho_critical;
-    const double pmin = dvd(-c, mu_t);
+    const bool density_flag = quot(m, v) < mp.rho_critical;
+    const double pmin = quot(-c, mu_t);
     double nup_tau;
     if (density_flag) {
-        nup_tau = dvd(tau_tr, mul(G, dt));
-        beta = dvd(-p_tr, mul(K, dt));
+        nup_tau = dvd_const(tau_tr, el.kGdt);
+        beta = quot(-p_tr, mul(K, dt));
         sxx = 0; sxy = 0; syy = 0;
     } else if (f < 0) {
         nup_tau = 0;
@@ -336,15 +537,15 @@ __device__ __forceinline__ void g_local_mu2_reverse(const Elastic &el, const Mu2
         sxy = t0xy;
         syy = sub(t0yy, p_tr);
     } else if (f >= 0 && p_tr > pmin) {
-        nup_tau = dvd(dvd(f, G), dt);
+        nup_tau = dvd_const(dvd_const(f, el.kG), el.kdt);
         beta = 0;
-        double scale_factor = dvd(tau_tau, tau_tr);
+        double scale_factor = quot(tau_tau, tau_tr);
         sxx = sub(mul(scale_factor, t0xx), p_tr);
         sxy = mul(scale_factor, t0xy);
         syy = sub(mul(scale_factor, t0yy), p_tr);
     } else if (p_tr <= pmin) {
-        nup_tau = dvd(tau_tr, mul(G, dt));
-        beta = dvd(sub(dvd(c, mu_t), p_tr), mul(K, dt));
+        nup_tau = dvd_const(tau_tr, el.kGdt);
+        beta = quot(sub(quot(c, mu_t), p_tr), mul(K, dt));
         sxx = 0; sxy = 0; syy = 0;
     } else {
         nup_tau = 0;   // NaN: the reference prints the particle and keeps s
@@ -358,9 +559,9 @@ __device__ __forceinline__ double mu_from_gammadot(double gammadot, double p, do
                                                    double mu_2, double inum_0)
 {
     if (p <= 0) return mu_2;
-    double inum = dvd(mul(dsqrtrhos, gammadot), __dsqrt_rn(p));
+    double inum = quot(mul(dsqrtrhos, gammadot), root(p));
     if (inum <= 0) return mu_s;
-    return add(mu_s, dvd(sub(mu_2, mu_s), add(dvd(inum_0, inum), 1.0)));
+    return add(mu_s, quot(sub(mu_2, mu_s), add(quot(inum_0, inum), 1.0)));
 }
 
 // g_local_mu2_ext, first phase (g_local_mu2_ext.c:214-230): the local
@@ -373,9 +574,9 @@ __device__ __forceinline__ void ext_local_fluidity(const Mu2Params &mp, double s
     if (gammadotp == 0) {
         gflocal = 0;
     } else {
-        mu_t = mu_from_gammadot(gammadotp, p_t, mul(mp.grains_d, __dsqrt_rn(mp.grains_rho)), mp.mu_s, mp.mu_2,
+        mu_t = mu_from_gammadot(gammadotp, p_t, mul(mp.grains_d, root(mp.grains_rho)), mp.mu_s, mp.mu_2,
                                 mp.I0);
-        gflocal = dvd(gammadotp, mu_t);
+        gflocal = quot(gammadotp, mu_t);
     }
 }
 
@@ -387,10 +588,10 @@ __device__ __forceinline__ void ext_stress(const Elastic &el, const Mu2Params &m
                                            double &sxy, double &syy, double &mu_t, double &beta, double &gammap,
                                            double &gammadotp)
 {
-    const double G = el.G, K = el.K, dt = el.dt, c = 1e-2;
+    const double K = el.K, dt = el.dt, c = 1e-2;
     double p_t = mul(-0.5, add(sxx, syy));
-    const double Ep = dvd(E, sub(1.0, mul(nu, nu)));
-    const double Gp = dvd(E, mul(2.0, add(1.0, nu)));
+    const double Ep = quot(E, sub(1.0, mul(nu, nu)));
+    const double Gp = quot(E, mul(2.0, add(1.0, nu)));
     double dsjxx = mul(mul(dt, Ep), add(exx, mul(nu, eyy)));
     double dsjxy = mul(mul(dt, Gp), exy);
     double dsjyy = mul(mul(dt, Ep), add(eyy, mul(nu, exx)));
@@ -401,16 +602,16 @@ __device__ __forceinline__ void ext_stress(const Elastic &el, const Mu2Params &m
     double sxx_tr = add(sxx, dsjxx), sxy_tr = add(sxy, dsjxy), syy_tr = add(syy, dsjyy);
     double p_tr = mul(-0.5, add(sxx_tr, syy_tr));
     double t0xx = add(sxx_tr, p_tr), t0xy = sxy_tr, t0yy = add(syy_tr, p_tr);
-    double tau_tr = __dsqrt_rn(mul(0.5, add(add(mul(t0xx, t0xx), mul(mul(2.0, t0xy), t0xy)), mul(t0yy, t0yy))));
-    mu_t = mu_from_gammadot(gammadotp, p_t, mul(mp.grains_d, __dsqrt_rn(mp.grains_rho)), mp.mu_s, mp.mu_2, mp.I0);
+    double tau_tr = root<-1>((add(add(mul(t0xx, t0xx), mul(mul(2.0, t0xy), t0xy)), mul(t0yy, t0yy))));
+    mu_t = mu_from_gammadot(gammadotp, p_t, mul(mp.grains_d, root(mp.grains_rho)), mp.mu_s, mp.mu_2, mp.I0);
     double tau_tau = mul(mu_t, add(p_tr, c));
     double f = sub(tau_tr, tau_tau);
-    const bool density_flag = dvd(m, v) < mp.rho_critical;
-    const double pmin = dvd(-c, mu_t);   // -c / mu_t, the reference's -c/mu_t
+    const bool density_flag = quot(m, v) < mp.rho_critical;
+    const double pmin = quot(-c, mu_t);   // -c / mu_t, the reference's -c/mu_t
     double nup_tau;
     if (density_flag) {
-        nup_tau = dvd(tau_tr, mul(G, dt));
-        beta = dvd(-p_tr, mul(K, dt));
+        nup_tau = dvd_const(tau_tr, el.kGdt);
+        beta = quot(-p_tr, mul(K, dt));
         sxx = 0; sxy = 0; syy = 0;
     } else if (f < 0) {
         nup_tau = 0;
@@ -419,15 +620,15 @@ __device__ __forceinline__ void ext_stress(const Elastic &el, const Mu2Params &m
         sxy = t0xy;
         syy = sub(t0yy, p_tr);
     } else if (f >= 0 && p_tr > pmin) {
-        nup_tau = dvd(sub(tau_tr, tau_tau), mul(G, dt));
+        nup_tau = dvd_const(sub(tau_tr, tau_tau), el.kGdt);
         beta = 0;
-        double scale_factor = dvd(tau_tau, tau_tr);
+        double scale_factor = quot(tau_tau, tau_tr);
         sxx = sub(mul(scale_factor, t0xx), p_tr);
         sxy = mul(scale_factor, t0xy);
         syy = sub(mul(scale_factor, t0yy), p_tr);
     } else if (p_tr <= pmin) {
-        nup_tau = dvd(tau_tr, mul(G, dt));
-        beta = dvd(sub(dvd(c, mu_t), p_tr), mul(K, dt));
+        nup_tau = dvd_const(tau_tr, el.kGdt);
+        beta = quot(sub(quot(c, mu_t), p_tr), mul(K, dt));
         sxx = 0; sxy = 0; syy = 0;
     } else {
         nup_tau = 0;   // NaN: the reference prints the particle and keeps s
@@ -444,7 +645,7 @@ __device__ __forceinline__ void nonlocal_mu2_trial(const Elastic &el, double exx
                                                    double &t0xy, double &t0yy, double &tau_tr)
 {
     const double dt = el.dt;
-    const double lambda = el.lambda;   // sub(K, dvd(mul(2, G), 3)), formed on the host with the same roundings
+    const double lambda = el.lambda;   // sub(K, quot(mul(2, G), 3)), formed on the host with the same roundings
     const double twoG = el.twoG;
     double trD = add(exx, eyy);
     double dsjxx = add(mul(lambda, trD), mul(twoG, exx));
@@ -461,7 +662,7 @@ __device__ __forceinline__ void nonlocal_mu2_trial(const Elastic &el, double exx
     t0xx = add(sxx_tr, p_tr);
     t0xy = sxy_tr;
     t0yy = add(syy_tr, p_tr);
-    tau_tr = __dsqrt_rn(mul(0.5, add(add(mul(t0xx, t0xx), mul(mul(2.0, t0xy), t0xy)), mul(t0yy, t0yy))));
+    tau_tr = root<-1>((add(add(mul(t0xx, t0xx), mul(mul(2.0, t0xy), t0xy)), mul(t0yy, t0yy))));
 }
 
 // calculate_bulk_granular_fluidity, g_nonlocal_mu2.c:238-321, for one
@@ -479,25 +680,26 @@ __device__ __forceinline__ void nonlocal_mu2_bulk(const Elastic &el, const Mu2Pa
                                                   double v, double p_tr, double tau_tr, double &dense,
                                                   double &gf_local, double &xisq_inv)
 {
-    dense = (below_density(m, v, mp) || p_tr < 0) ? 0.0 : 1.0;
-    if (dense == 0 || p_tr <= 0) {
+    const bool is_dense = !(below_density(m, v, mp) || is_neg(p_tr));
+    dense = is_dense ? 1.0 : 0.0;
+    if (!is_dense || !(is_pos(p_tr) || is_nan(p_tr))) {
         gf_local = 0;
         xisq_inv = 0;
-    } else if (p_tr > 0) {
+    } else if (is_pos(p_tr)) {
         double tau_tau;
         double S0 = mul(mp.mu_s, p_tr);
-        if (tau_tr <= S0) {
+        if (less_equal_pos(tau_tr, S0)) {
             tau_tau = tau_tr;
             gf_local = 0;
         } else {
             double S2 = mul(mp.mu_2, p_tr);
-            double alpha = mul(mp.alpha_c, __dsqrt_rn(p_tr));
+            double alpha = mul(mp.alpha_c, root(p_tr));
             double B = add(add(S2, tau_tr), alpha);
             double H = add(mul(S2, tau_tr), mul(S0, alpha));
-            tau_tau = dvd(add(H, H), add(B, __dsqrt_rn(sub(mul(B, B), mul(4.0, H)))));
-            gf_local = dvd(mul(p_tr, sub(tau_tr, tau_tau)), mul(el.Gdt, tau_tau));
+            tau_tau = quot<1>(H, add(B, root(__fma_rn(-4.0, H, mul(B, B)))));
+            gf_local = quot(mul(p_tr, sub(tau_tr, tau_tau)), mul(el.Gdt, tau_tau));
         }
-        xisq_inv = dvd_known(fabs(sub(dvd(tau_tau, p_tr), mp.mu_s)), mp.AAdd, mp.inv_AAdd);
+        xisq_inv = dvd_const(fabs(sub(quot(tau_tau, p_tr), mp.mu_s)), mp.kAAdd);
     } else {
         gf_local = 0;
         xisq_inv = 0;
@@ -523,12 +725,12 @@ __device__ __forceinline__ void nonlocal_mu2_stress(const Elastic &el, double gf
         nup_tau = 0;
         sxx = 0; sxy = 0; syy = 0;
     } else if (p_tr > 0) {
-        double scale_factor = dvd(p_tr, add(mul(el.Gdt, gf), p_tr));
+        double scale_factor = quot(p_tr, add(mul(el.Gdt, gf), p_tr));
         double tau_tau = mul(tau_tr, scale_factor);
         // ((tau - tau_tau) / G) / dt as one quotient by G dt (the fluidity
         // comes from an iterative solve, so this value is not bit-exact
         // with the reference's anyway)
-        nup_tau = dvd_known(sub(tau_tr, tau_tau), el.Gdt, el.inv_Gdt);
+        nup_tau = dvd_const(sub(tau_tr, tau_tau), el.kGdt);
         sxx = sub(mul(scale_factor, t0xx), p_tr);
         sxy = mul(scale_factor, t0xy);
         syy = sub(mul(scale_factor, t0yy), p_tr);
@@ -552,13 +754,13 @@ __device__ __forceinline__ void nonlocal_bulk(const NonlocalParams &np, double s
     const double p_cap = 1e-2;
     double p_t = mul(-0.5, add(sxx, syy));
     double a = add(sxx, p_t), b = sxy, c = add(syy, p_t);
-    double tau_t = __dsqrt_rn(mul(0.5, add(add(mul(a, a), mul(mul(2.0, b), b)), mul(c, c))));
+    double tau_t = root<-1>((add(add(mul(a, a), mul(mul(2.0, b), b)), mul(c, c))));
     if (p_t < p_cap) p_t = p_cap;
     double S0 = mul(p_t, np.mu_s);
-    eta = mul(mul(np.B, np.grains_d), __dsqrt_rn(mul(p_t, np.grains_rho)));
-    xisq_inv = dvd(fabs(sub(dvd(tau_t, p_t), np.mu_s)),
+    eta = mul(mul(np.B, np.grains_d), root(mul(p_t, np.grains_rho)));
+    xisq_inv = quot(fabs(sub(quot(tau_t, p_t), np.mu_s)),
                    mul(mul(mul(np.grains_d, np.grains_d), np.A), np.A));
-    gf_bulk = (tau_t > S0) ? mul(dvd(p_t, eta), sub(1.0, dvd(S0, tau_t))) : 0.0;
+    gf_bulk = (tau_t > S0) ? mul(quot(p_t, eta), sub(1.0, quot(S0, tau_t))) : 0.0;
 }
 
 // Explicit stress update of g_nonlocal.c:154-298 (every particle).
@@ -568,8 +770,8 @@ __device__ __forceinline__ void nonlocal_stress(const NonlocalParams &np, double
                                                 double &syy, double &gammap)
 {
     const double EMOD = np.E, NUMOD = np.nu, c = np.cohesion;
-    const double cA = dvd(EMOD, sub(1.0, mul(NUMOD, NUMOD)));
-    const double cB = dvd(EMOD, mul(2.0, add(1.0, NUMOD)));
+    const double cA = quot(EMOD, sub(1.0, mul(NUMOD, NUMOD)));
+    const double cB = quot(EMOD, mul(2.0, add(1.0, NUMOD)));
     double p_t = mul(-0.5, add(sxx, syy));
     double a = add(sxx, p_t), b = sxy, cc = add(syy, p_t);
     double tau_t;
@@ -582,22 +784,22 @@ __device__ __forceinline__ void nonlocal_stress(const NonlocalParams &np, double
     dsjyy = add(dsjyy, jw);
     double p_tr = mul(-0.5, add(add(sxx, dsjxx), add(syy, dsjyy)));
     if (p_tr < c) {
-        sxx = dvd(mul(0.5, c), np.mu_s);
+        sxx = quot(mul(0.5, c), np.mu_s);
         sxy = 0;
-        syy = dvd(mul(0.5, c), np.mu_s);
+        syy = quot(mul(0.5, c), np.mu_s);
         return;
     }
-    tau_t = __dsqrt_rn(mul(0.5, add(add(mul(a, a), mul(mul(2.0, b), b)), mul(cc, cc))));
-    const double r = __dsqrt_rn(0.5);
-    double Npxx = dvd(mul(r, a), tau_t);
-    double Npxy = dvd(mul(r, b), tau_t);
-    double Npyy = dvd(mul(r, cc), tau_t);
+    tau_t = root<-1>((add(add(mul(a, a), mul(mul(2.0, b), b)), mul(cc, cc))));
+    const double r = root(0.5);
+    double Npxx = quot(mul(r, a), tau_t);
+    double Npxy = quot(mul(r, b), tau_t);
+    double Npyy = quot(mul(r, cc), tau_t);
     double dxx0 = mul(0.5, sub(exx, eyy)), dxy0 = exy, dyy0 = mul(0.5, sub(eyy, exx));
-    double gammadot = __dsqrt_rn(mul(2.0, add(add(mul(dxx0, dxx0), mul(mul(2.0, dxy0), dxy0)),
+    double gammadot = root(mul(2.0, add(add(mul(dxx0, dxx0), mul(mul(2.0, dxy0), dxy0)),
                                               mul(dyy0, dyy0))));
     double nup_tau, dpxx, dpxy, dpyy;
     if (p_t > c && gf > 0) {
-        nup_tau = dvd(mul(gf, tau_t), p_t);
+        nup_tau = quot(mul(gf, tau_t), p_t);
         if (nup_tau < 0) nup_tau = 0;
         if (nup_tau > gammadot) nup_tau = gammadot;
         dpxx = mul(mul(r, nup_tau), Npxx);

@@ -20,6 +20,8 @@
 // Shape functions (tent / grad_tent, interpolate.c:23-65) are recomputed in
 // registers from the start-of-step position wherever they are needed.  No
 // floating-point atomics are used; every sum has a fixed order.
+#include <math.h>
+
 #include "mpmg_fp64_common.cuh"
 #include "mpmg_internal.cuh"
 #include "mpmg_materials.cuh"
@@ -110,7 +112,7 @@ __global__ void __launch_bounds__(128) p2g_cells_kernel(
     if (k0 == k1) return;
     mpmg_order_segment(slots, perm, nullptr, k0, k1);   // ascending particle index, as the reference's lists
     const int ci = e % g.Ex, cj = e / g.Ex;
-    const double cx = ci, cy = cj;   // the element's column and row (element.c:10-19)
+    const double cx = mat::small_int(ci), cy = mat::small_int(cj);   // the element's column and row (element.c:10-19)
     // moments [A, X, Y, Z] of m, m vx, m vy; stress-term moments
     double mm[4] = {0, 0, 0, 0}, mx[4] = {0, 0, 0, 0}, my[4] = {0, 0, 0, 0};
     double P0 = 0, Py0 = 0, P1 = 0, Px1 = 0, Py1 = 0, P2 = 0, Px2 = 0;
@@ -217,7 +219,7 @@ __global__ void __launch_bounds__(256) grid_kernel(
     if (m > MPMG_TOL) {
         // one division: the four quotients by m differ from IEEE division
         // by at most an ulp
-        const double inv_m = 1.0 / m;
+        const double inv_m = mat::quot(1.0, m);
         ax = fx * inv_m;
         ay = fy * inv_m;
         mx += dt * fx;
@@ -323,8 +325,8 @@ __global__ void __launch_bounds__(256) g2p_kernel(G2PArgs A)
         xl = A.xl_out[i];
         yl = A.yl_out[i];
     } else {
-        xl = mpmg_local_coord_fma(A.x[i], (double)ci, g.inv_h);
-        yl = mpmg_local_coord_fma(A.y[i], (double)cj, g.inv_h);
+        xl = mpmg_local_coord_fma(A.x[i], mat::small_int(ci), g.inv_h);
+        yl = mpmg_local_coord_fma(A.y[i], mat::small_int(cj), g.inv_h);
     }
     const ShapeFns f = shape(xl, yl, g.inv_h);
     const double dt = A.dt;
@@ -346,14 +348,12 @@ __global__ void __launch_bounds__(256) g2p_kernel(G2PArgs A)
             dux += f.s[a] * nvx[a];
             duy += f.s[a] * nvy[a];
         }
-        A.vx[i] += dt * xtt;
-        A.vy[i] += dt * ytt;
-        dux *= dt;
-        duy *= dt;
-        A.x[i] += dux;
-        A.y[i] += duy;
-        A.ux[i] += dux;
-        A.uy[i] += duy;
+        A.vx[i] = fma(dt, xtt, A.vx[i]);
+        A.vy[i] = fma(dt, ytt, A.vy[i]);
+        A.x[i] = fma(dt, dux, A.x[i]);
+        A.y[i] = fma(dt, duy, A.y[i]);
+        A.ux[i] = fma(dt, dux, A.ux[i]);
+        A.uy[i] = fma(dt, duy, A.uy[i]);
         if (A.ax != nullptr) {
             A.ax[i] = xtt;
             A.ay[i] = ytt;
@@ -498,7 +498,7 @@ __global__ void __launch_bounds__(256) ext_stress_kernel(G2PArgs A, const double
     double mu_t = A.st0[i], gdp = A.st10[i];
     const double Ad = A.mu2.A, d = A.mu2.grains_d;
     gf = mat::mul(mat::mul(mat::mul(mat::mul(mat::mul(Ad, Ad), d), d), mu_t), gf);
-    if (mu_t > A.mu2.mu_s) gdp = mat::sub(gdp, mat::dvd(gf, fabs(mat::sub(mu_t, A.mu2.mu_s))));
+    if (mu_t > A.mu2.mu_s) gdp = mat::sub(gdp, mat::quot(gf, fabs(mat::sub(mu_t, A.mu2.mu_s))));
     if (gdp < 0) gdp = 0;
     A.st3[i] = gf;
     double sxx = A.sxx[i], sxy = A.sxy[i], syy = A.syy[i], beta = A.st5[i], gp = A.st9[i];
@@ -631,10 +631,10 @@ G2PArgs make_g2p_args(mpmg_ctx *ctx)
     A.el.K = ctx->K;
     A.el.lambda = ctx->lambda;
     A.el.dt = c.dt;
-    A.el.inv_G = 1.0 / ctx->G;
-    A.el.inv_dt = 1.0 / c.dt;
     A.el.Gdt = ctx->G * c.dt;
-    A.el.inv_Gdt = 1.0 / A.el.Gdt;
+    A.el.kG = mat::make_known(ctx->G);
+    A.el.kdt = mat::make_known(c.dt);
+    A.el.kGdt = mat::make_known(A.el.Gdt);
     A.mu2.mu_s = c.mp[MPMG_MP_MU_S];
     A.mu2.mu_2 = c.mp[MPMG_MP_MU_2];
     A.mu2.I0 = c.mp[MPMG_MP_I0];
@@ -642,12 +642,12 @@ G2PArgs make_g2p_args(mpmg_ctx *ctx)
     A.mu2.grains_d = c.mp[MPMG_MP_GRAINS_D];
     A.mu2.rho_critical = c.mp[MPMG_MP_RHO_CRITICAL];
     A.mu2.A = c.mp[MPMG_MP_A];
-    A.mu2.inv_grains_rho = 1.0 / A.mu2.grains_rho;
-    A.mu2.inv_grains_d = 1.0 / A.mu2.grains_d;
-    A.mu2.rho_lo = A.mu2.rho_critical * (1.0 - 0x1p-47);
-    A.mu2.rho_hi = A.mu2.rho_critical * (1.0 + 0x1p-47);
-    A.mu2.AAdd = ((A.mu2.A * A.mu2.A) * A.mu2.grains_d) * A.mu2.grains_d;
-    A.mu2.inv_AAdd = 1.0 / A.mu2.AAdd;
+    A.mu2.krho = mat::make_known(A.mu2.grains_rho);
+    A.mu2.kd = mat::make_known(A.mu2.grains_d);
+    const bool bracket = A.mu2.rho_critical >= 0x1p-60 && A.mu2.rho_critical <= 0x1p60;
+    A.mu2.rho_lo = bracket ? A.mu2.rho_critical * (1.0 - 0x1p-47) : -1.0;
+    A.mu2.rho_hi = bracket ? A.mu2.rho_critical * (1.0 + 0x1p-47) : (double)INFINITY;
+    A.mu2.kAAdd = mat::make_known(((A.mu2.A * A.mu2.A) * A.mu2.grains_d) * A.mu2.grains_d);
     A.mu2.alpha_c = (((ctx->G * A.mu2.I0) * c.dt) / A.mu2.grains_d) / sqrt(A.mu2.grains_rho);
     A.mu2.GI0dt = (ctx->G * A.mu2.I0) * c.dt;
     A.nl.E = c.mp[MPMG_MP_E];
