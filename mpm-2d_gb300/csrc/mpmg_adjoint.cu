@@ -877,6 +877,7 @@ int load_state(mpmg_ctx *ctx, const double *in, const int *active, const int *el
     }
     MPMG_CHECK(cudaMemcpyAsync(ctx->d_params, params, sizeof(StepParams), cudaMemcpyDeviceToDevice, s));
     MPMG_CHECK(cudaGetLastError());
+    ctx->row.ready = false;   // the positions and the element map changed
     return MPMG_OK;
 }
 
@@ -1036,7 +1037,9 @@ int mpmg_adj_backward(mpmg_ctx *ctx, const double *dl_dx, const double *dl_dy, d
         if (rc != MPMG_OK) return rc;
         for (int k = 0; k < len; k++) {
             if ((rc = save_state(ctx, t->seg_state + (size_t)k * kStateFields * n)) != MPMG_OK) return rc;
+            if ((rc = mpmg_fp64_ready(ctx)) != MPMG_OK) return rc;
             if ((rc = mpmg_launch_step(ctx)) != MPMG_OK) return rc;
+            if ((rc = mpmg_fp64_sort(ctx)) != MPMG_OK) return rc;
             const int m = (int)(n > ne + 1 ? (n > nn ? n : nn) : (ne + 1 > nn ? ne + 1 : nn));
             save_step_kernel<<<blocks_for(m, 256), 256, 0, s>>>(
                 (int)n, (int)ne, (int)nn, ctx->in_element, ctx->active, ctx->perm, ctx->cell_start, ctx->node_m,
@@ -1070,7 +1073,7 @@ int mpmg_adj_backward(mpmg_ctx *ctx, const double *dl_dx, const double *dl_dy, d
                 adj_nl_rhs_kernel<<<blocks_for(ne, 128), 128, 0, s>>>(S);
                 ctx->launches += 2;
                 MPMG_CHECK(cudaGetLastError());
-                rc = mpmg_solve_fluidity_system(ctx, t->seg_ek + (size_t)k * 10 * ne, t->rhs, S.nodes, S.cell_start,
+                rc = mpmg_solve_fluidity_system(ctx, t->seg_ek + (size_t)k * 10 * ne, t->rhs, S.nodes, nullptr, S.cell_start,
                                                 t->lam, true);
                 if (rc != MPMG_OK) return rc;
             }

@@ -102,6 +102,36 @@ int alloc_step_record(mpmg_ctx *ctx, int count)
     return MPMG_OK;
 }
 
+// The element rows of the FP64 step: a row holds at least twice the mean
+// count of the filled elements (a power of two, 16 to 64), since a flow packs
+// elements unevenly; what a row cannot hold goes to the overflow list.
+int alloc_rows(mpmg_ctx *ctx, const int *emap, size_t n)
+{
+    RowBins &r = ctx->row;
+    std::vector<bool> seen(ctx->ne, false);
+    size_t filled = 0, inside = 0;
+    for (size_t i = 0; i < n; i++) {
+        if (emap[i] < 0) continue;
+        inside++;
+        if (!seen[emap[i]]) {
+            seen[emap[i]] = true;
+            filled++;
+        }
+    }
+    r.cap = 16;
+    while (r.cap < 64 && filled > 0 && (size_t)r.cap * filled < 2 * inside) r.cap *= 2;
+    r.cur = 0;
+    r.ready = false;
+    int rc = dalloc(&r.over_n, 3);
+    if (rc == MPMG_OK) rc = dalloc(&r.over_list, n);
+    for (int b = 0; b < 2 && rc == MPMG_OK; b++) {
+        rc = dalloc(&r.count[b], ctx->ne);
+        if (rc == MPMG_OK) rc = dalloc(&r.rows[b], ctx->ne * (size_t)r.cap);
+        if (rc == MPMG_OK) rc = dalloc(&r.over[b], n);
+    }
+    return rc;
+}
+
 // The step parameters and the status word of a read-back step record: the
 // parameters go to ctx->h_params, device-side errors to their status codes.
 int take_record(mpmg_ctx *ctx, const unsigned char *rec)
@@ -391,6 +421,15 @@ int mpmg_destroy(mpmg_ctx *ctx)
         if (ctx->ring_ev[k]) cudaEventDestroy(ctx->ring_ev[k]);
     }
     if (ctx->rring_h) cudaFreeHost(ctx->rring_h);
+    for (int b = 0; b < 2; b++) {
+        cudaFree(ctx->row.count[b]);
+        cudaFree(ctx->row.rows[b]);
+        cudaFree(ctx->row.over[b]);
+    }
+    cudaFree(ctx->row.over_n);
+    cudaFree(ctx->row.over_list);
+    cudaFree(ctx->elem_coef);
+    cudaFree(ctx->sort_keys);
     mpmg_bin_free(ctx);
     mpmg_nonlocal_free(ctx);
     mpmg_mixed_free(ctx);
@@ -567,6 +606,8 @@ int mpmg_create(const mpmg_config *cfg, size_t n, const double *m, const double 
         rc = MPMG_ERR_CUDA;
         goto fail;
     }
+    if (cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, ctx->dev) != cudaSuccess || ctx->sms < 1)
+        ctx->sms = 1;
     for (int k = 0; k < 2 * PH_COUNT; k++) {
         if (cudaEventCreate(&ctx->ev[k]) != cudaSuccess) {
             rc = MPMG_ERR_CUDA;
@@ -625,7 +666,7 @@ int mpmg_create(const mpmg_config *cfg, size_t n, const double *m, const double 
             for (double **p : tn) TRY(dalloc(p, ctx->nn));
         }
         TRY(alloc_step_record(ctx, 1));
-        TRY(mpmg_bin_init(ctx));
+        TRY(dalloc(&ctx->elem_coef, 16 * ctx->ne));
         if (nonlocal) TRY(mpmg_nonlocal_init(ctx));
         if (cfg->material == MPMG_G_NONLOCAL_MU2) TRY(dalloc(&ctx->nl_trial, 5 * n));
 
@@ -675,10 +716,12 @@ int mpmg_create(const mpmg_config *cfg, size_t n, const double *m, const double 
             emap[i] = e;
             act[i] = e < 0 ? 0 : 1;
         }
+        rc = alloc_rows(ctx, emap, n);
         cudaError_t ce = cudaMemcpy(ctx->in_element, emap, n * sizeof(int), cudaMemcpyHostToDevice);
         if (ce == cudaSuccess) ce = cudaMemcpy(ctx->active, act, n * sizeof(int), cudaMemcpyHostToDevice);
         delete[] emap;
         delete[] act;
+        if (rc != MPMG_OK) goto fail;
         if (ce != cudaSuccess) {
             rc = mpmg_cuda_status(ce, "initial element map upload");
             goto fail;
@@ -894,9 +937,9 @@ int launch_one_step(mpmg_ctx *ctx)
     return MPMG_OK;
 }
 
-int parity(const mpmg_ctx *ctx)
+int &parity(mpmg_ctx *ctx)
 {
-    return ctx->mixed ? ctx->mixed->cur : 0;
+    return ctx->mixed ? ctx->mixed->cur : ctx->row.cur;
 }
 
 // Captures `steps` consecutive steps (starting at the current buffer parity)
@@ -911,7 +954,7 @@ int capture_steps(mpmg_ctx *ctx, int steps, cudaGraphExec_t *out, long *launches
     for (int k = 0; k < steps && rc == MPMG_OK; k++) rc = launch_one_step(ctx);
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
-    if (ctx->mixed) ctx->mixed->cur = p0;
+    parity(ctx) = p0;
     *launches = ctx->launches - l0;
     ctx->launches = l0;
     if (rc != MPMG_OK) {
@@ -959,7 +1002,7 @@ int step_with_graphs(mpmg_ctx *ctx, int nsteps)
         MPMG_CHECK(cudaGraphLaunch(*g, ctx->stream));
         ctx->launches += *gl;
         const int done = chunk ? chunk_steps : 1;
-        if (ctx->mixed && (done & 1)) ctx->mixed->cur ^= 1;
+        if (done & 1) parity(ctx) ^= 1;
         nsteps -= done;
     }
     return MPMG_OK;
@@ -1083,6 +1126,10 @@ int mpmg_step(mpmg_ctx *ctx, int nsteps)
 {
     if (ctx == nullptr || nsteps < 0) return MPMG_ERR_INVALID;
     MPMG_CHECK(cudaSetDevice(ctx->dev));
+    if (!ctx->mixed && nsteps > 0) {
+        const int rc = mpmg_fp64_ready(ctx);
+        if (rc != MPMG_OK) return rc;
+    }
     if (graphs_apply(ctx)) return step_with_graphs(ctx, nsteps);
     for (int k = 0; k < nsteps; k++) {
         for (int ph = 0; ph < PH_COUNT; ph++) ctx->phase_used[ph] = 0;
@@ -1172,6 +1219,7 @@ int mpmg_set_field(mpmg_ctx *ctx, const char *name, const double *host_in)
     if (f.count > 0)
         MPMG_CHECK(cudaMemcpyAsync(f.ptr, host_in, f.count * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
     MPMG_CHECK(cudaStreamSynchronize(ctx->stream));
+    if (f.ptr == ctx->x || f.ptr == ctx->y) ctx->row.ready = false;
     return MPMG_OK;
 }
 
@@ -1207,6 +1255,7 @@ int mpmg_set_map(mpmg_ctx *ctx, const int *in_element, const int *active)
         MPMG_CHECK(cudaMemcpy(ctx->in_element, in_element, ctx->np * sizeof(int), cudaMemcpyHostToDevice));
         MPMG_CHECK(cudaMemcpy(ctx->active, active, ctx->np * sizeof(int), cudaMemcpyHostToDevice));
     }
+    ctx->row.ready = false;
     return MPMG_OK;
 }
 
@@ -1214,6 +1263,12 @@ int mpmg_get_sort(mpmg_ctx *ctx, int *sorted_keys, int *perm, int *cell_start)
 {
     if (ctx == nullptr) return MPMG_ERR_INVALID;
     MPMG_CHECK(cudaSetDevice(ctx->dev));
+    if (!ctx->mixed) {
+        // the FP64 step bins into element rows; the sort is formed here from
+        // the last step's element map
+        const int rc = mpmg_fp64_sort(ctx);
+        if (rc != MPMG_OK) return rc;
+    }
     MPMG_CHECK(cudaStreamSynchronize(ctx->stream));
     if (sorted_keys && ctx->np) {
         if (ctx->mixed) {

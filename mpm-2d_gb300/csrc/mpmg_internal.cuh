@@ -104,6 +104,38 @@ struct BinScratch {
     int tiles;
 };
 
+// Element rows of the FP64 step (mpmg_step.cu): each element has a row of
+// `cap` slots for its particles' indices, filled in any order with a counter
+// per element; what does not fit goes to an overflow list of (element, index)
+// pairs.  Two buffers: while a step works on buffer `cur`, its G2P already
+// bins the moved particles into the other one for the next step.  `ready`
+// says that buffer cur holds the current positions' elements; setting x, y or
+// the element map from outside clears it, and the next step then bins first.
+struct RowBins {
+    int cap;
+    uint32_t *count[2];    // ne
+    uint32_t *rows[2];     // ne x cap
+    uint2 *over[2];        // n
+    uint32_t *over_n;      // entries in over[0], over[1]; then the cursor of over_list
+    uint32_t *over_list;   // n: the ordered lists of elements with more than cap particles
+    int cur;
+    bool ready;
+};
+
+// Device view of the rows one step works on.  list(e, cnt) is element e's
+// ordered particle list once the P2G has written it back (ordered rows).
+struct RowView {
+    const uint32_t *count;
+    uint32_t *rows;
+    uint32_t *over_list;
+    int cap;
+    __device__ __forceinline__ const uint32_t *list(int e, int cnt) const
+    {
+        uint32_t *row = rows + (size_t)e * cap;
+        return cnt <= cap ? row : over_list + row[0];
+    }
+};
+
 struct mpmg_ctx {
     mpmg_config cfg;
     int dev;
@@ -123,6 +155,13 @@ struct mpmg_ctx {
     double *ax, *ay, *exx, *exy, *eyy, *wxy, *xl, *yl;  // transients (store_transients)
     int *in_element;
     int *active;
+
+    // FP64 form: element rows, and per element the bilinear coefficients of
+    // the nodal acceleration and velocity (16 doubles, mpmg_step.cu).
+    RowBins row;
+    double *elem_coef;
+    uint32_t *sort_keys;   // input of mpmg_fp64_sort
+    int sms;
 
     // Cell sort.
     uint32_t *keys;        // element key per particle (num_elements for inactive)
@@ -235,7 +274,13 @@ size_t mpmg_sort_scratch_words(size_t n, int key_bits, int *num_tiles_out);
 int mpmg_sort_run(const uint32_t *keys, const uint32_t *vals, int n, int ne, int key_bits,
                   const SortScratch &sc, uint32_t *sorted_keys, uint32_t *perm, int *cell_start,
                   cudaStream_t s);
-int mpmg_launch_step(mpmg_ctx *ctx);             // one full step
+int mpmg_launch_step(mpmg_ctx *ctx);             // one full FP64 step
+// FP64 form: the element rows of the current positions, where they are not
+// ready (a no-op otherwise); the steps' launches assume them.
+int mpmg_fp64_ready(mpmg_ctx *ctx);
+// FP64 form: the stable cell sort of the last step's element map (sorted_keys,
+// perm, cell_start), which no local step needs.
+int mpmg_fp64_sort(mpmg_ctx *ctx);
 int mpmg_bin_init(mpmg_ctx *ctx);
 void mpmg_bin_free(mpmg_ctx *ctx);
 // Stand-alone count of keys[n] (<= ne) into the bins.
@@ -250,8 +295,10 @@ int mpmg_nonlocal_init(mpmg_ctx *ctx);
 void mpmg_nonlocal_free(mpmg_ctx *ctx);
 int mpmg_launch_fluidity(mpmg_ctx *ctx);         // nonlocal: assembly, solve, stress
 int mpmg_launch_solve(mpmg_ctx *ctx);            // nonlocal: the fluidity PCG alone
+// Elements that hold particles: counts[e] != 0, or where counts is null
+// cell_start[e] != cell_start[e + 1].
 int mpmg_solve_fluidity_system(mpmg_ctx *ctx, const double *elem_k, const double *elem_f, const double *node_m,
-                               const int *cell_start, double *x, bool zero_start);
+                               const uint32_t *counts, const int *cell_start, double *x, bool zero_start);
 int mpmg_launch_material_only(mpmg_ctx *ctx);
 int mpmg_mixed_init(mpmg_ctx *ctx, const double *m, const double *v, const double *x, const double *y,
                     const double *vx, const double *vy, const double *sxx, const double *sxy,
@@ -340,31 +387,18 @@ __device__ __forceinline__ int mpmg_which_element_fast(double xp, double yp, dou
     return fx + fy * Ex;
 }
 
-// Local coordinates in the element with bottom-left node at (xn, yn), with
-// the reference's snap to +-1 within 1e-10 (particle.c:14-30).
-// |xl| > 1 is tested on the bit pattern (positive doubles order as
-// integers), so that the common case costs no FP64 compare.
-__device__ __forceinline__ double mpmg_local_coord(double xp, double xn, double inv_h)
-{
-    double xl = (xp - xn) * inv_h;
-    if ((__double_as_longlong(xl) & 0x7fffffffffffffffLL) > 0x3ff0000000000000LL) {
-        double sg = copysign(1.0, xl);
-        if (((sg * xl) - 1.0) < MPMG_TOL) xl = sg;
-    }
-    return xl;
-}
-
-// The same with xl = x / h - c in one FMA from the element's column (or row)
-// c (one FP64 operation in place of three; xl differs from (x - c h) / h by
-// a few ulps of x / h, about 1e-14 on a 512-element grid).
+// Local coordinate xl = x / h - c in the element of column (or row) c, in one
+// FMA (it differs from (x - c h) / h by a few ulps of x / h, about 1e-14 on a
+// 512-element grid), with the reference's snap to +-1 within 1e-10
+// (particle.c:14-30).  |xl| - 1 is exact below 2, so |xl| - 1 < 1e-10 holds
+// for the 450359 doubles above 1 (1e-10 2^52 = 450359.96): an integer test,
+// where the compiler would run the FP64 form predicated off in every thread.
 __device__ __forceinline__ double mpmg_local_coord_fma(double xp, double c, double inv_h)
 {
-    double xl = fma(xp, inv_h, -c);
-    if ((__double_as_longlong(xl) & 0x7fffffffffffffffLL) > 0x3ff0000000000000LL) {
-        double sg = copysign(1.0, xl);
-        if (((sg * xl) - 1.0) < MPMG_TOL) xl = sg;
-    }
-    return xl;
+    const double xl = fma(xp, inv_h, -c);
+    const long long b = __double_as_longlong(xl), one = 0x3ff0000000000000LL;
+    const unsigned long long d = (unsigned long long)((b & 0x7fffffffffffffffLL) - one);
+    return d - 1 < 450359ull ? __longlong_as_double((b & (long long)0x8000000000000000ULL) | one) : xl;
 }
 
 // Counts one key into the bins (see BinScratch): bins[key] for keys inside

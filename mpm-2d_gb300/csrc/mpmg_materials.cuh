@@ -34,6 +34,7 @@ __device__ __forceinline__ double dvd_known(double a, double b, double y)
 // zh + zl (zh = RN(1/b), zl = RN(1/b - zh)), formed on the host.
 struct Known {
     double b, zh, zl;
+    double nz;   // -0 (see Unit)
     int two;   // RN(a zh + RN(a zl)) is RN(a / b) for every normal a
 };
 
@@ -53,6 +54,7 @@ inline Known make_known(double b)
     k.b = b;
     k.zh = 1.0 / b;
     k.zl = 0.0;
+    k.nz = -0.0;
     k.two = 0;
     const double m = fabs(b);
     if (!(m > 0x1p-400 && m < 0x1p400)) return k;
@@ -87,15 +89,7 @@ static __device__ __noinline__ double dvd_slow(double a, double b, double y)
 __device__ __forceinline__ double dvd_const(double a, const Known &k)
 {
     if (!k.two) return dvd_slow(a, k.b, k.zh);
-    return __fma_rn(a, k.zh, __dmul_rn(a, k.zl));
-}
-
-// a / 3: RN(1/3) = 1/3 - 2^-54/3.  a / 3 is never nearer than 2^-54/3 times
-// its binade to a midpoint (a - 3 m is a nonzero multiple of half its ulp), so
-// the two operations suffice.
-__device__ __forceinline__ double third(double a)
-{
-    return __fma_rn(a, 0x1.5555555555555p-2, __dmul_rn(a, 0x1.5555555555555p-56));
+    return __fma_rn(a, k.zh, __fma_rn(a, k.zl, k.nz));
 }
 
 // Sign and order tests on the bit patterns (the FP64 pipe issues a compare at
@@ -234,12 +228,50 @@ __device__ __forceinline__ double quot(double a, double b)
     return __longlong_as_double(qb | sign);
 }
 
-struct Elastic {
+// Products, sums and constants for the FP64 pipe.  On GB300 a DFMA whose three
+// operands are registers occupies a sub-partition's FP64 unit for 64.5 cycles;
+// DADD, DMUL and any operand from the constant bank or an immediate cost 76.6,
+// a compare 95.5 (measured, one to eight warps).  So the hot kernels form
+// a b as a b + (-0) and a + b as a 1 + b (the same results bit for bit), and
+// keep 1, -0 and every other constant in shared memory, from where they load
+// into registers; as literals or kernel parameters the compiler would fold
+// them back.
+struct Unit {
+    double one, nz;         // 1, -0
+    __device__ __forceinline__ double mul(double a, double b) const { return __fma_rn(a, b, nz); }
+    __device__ __forceinline__ double add(double a, double b) const { return __fma_rn(a, one, b); }
+    __device__ __forceinline__ double sub(double a, double b) const { return __fma_rn(a, one, -b); }
+};
+
+struct Elastic : Unit {
     double G, K, lambda, dt;
     double twoG;            // 2 G, exact
     double Gdt;             // RN(G dt)
-    Known kG, kdt, kGdt;    // G, dt and RN(G dt) as divisors
+    double half, two, sixth, mfour;   // 1/2, 2, RN(1/6), -4
+    Known k3, kG, kdt, kGdt;     // 3, G, dt and RN(G dt) as divisors
 };
+
+inline Elastic make_elastic(double G, double K, double lambda, double dt)
+{
+    Elastic el;
+    el.one = 1.0;
+    el.nz = -0.0;
+    el.G = G;
+    el.K = K;
+    el.lambda = lambda;
+    el.dt = dt;
+    el.twoG = 2.0 * G;
+    el.Gdt = G * dt;
+    el.half = 0.5;
+    el.two = 2.0;
+    el.sixth = 1.0 / 6.0;
+    el.mfour = -4.0;
+    el.k3 = make_known(3.0);
+    el.kG = make_known(G);
+    el.kdt = make_known(dt);
+    el.kGdt = make_known(el.Gdt);
+    return el;
+}
 
 // exp(x) for the volume update v <- v exp(dt tr D), whose argument is tiny at
 // any stable time step: where |x| < 2^-14 the degree-3 Taylor polynomial about
@@ -256,27 +288,30 @@ static __device__ __noinline__ double exp_wide(double x)
     return __fma_rn(p, x, 1.0);
 }
 
-__device__ __forceinline__ double exp_small(double x)
+__device__ __forceinline__ double exp_small(double x, double one = 1.0, double half = 0.5, double sixth = 1.0 / 6.0)
 {
     if ((__double2hiint(x) & 0x7fffffff) >= 0x3f100000) return exp_wide(x);
-    double p = __fma_rn(x, 1.0 / 6.0, 0.5);
-    p = __fma_rn(p, x, 1.0);
-    return __fma_rn(p, x, 1.0);
+    double p = __fma_rn(x, sixth, half);
+    p = __fma_rn(p, x, one);
+    return __fma_rn(p, x, one);
 }
 
 // isolin calculate_stress_threaded, materialsrc/isolin.c:75-116.
 __device__ __forceinline__ void isolin(const Elastic &el, double exx, double exy, double eyy,
                                        double wxy, double &sxx, double &sxy, double &syy)
 {
+    const auto mul = [&](double a, double b) { return el.mul(a, b); };
+    const auto add = [&](double a, double b) { return el.add(a, b); };
+    const auto sub = [&](double a, double b) { return el.sub(a, b); };
     const double twoG = el.twoG;
     double trD = add(exx, eyy);
     double dsjxx = add(mul(el.lambda, trD), mul(twoG, exx));
     double dsjxy = mul(twoG, exy);
     double dsjyy = add(mul(el.lambda, trD), mul(twoG, eyy));
-    double w2s = mul(mul(2.0, wxy), sxy);
-    dsjxx = add(dsjxx, w2s);
+    const double ws = mul(wxy, sxy);   // 2 ws rides in the FMAs: the doubling is exact
+    dsjxx = __fma_rn(el.two, ws, dsjxx);
     dsjxy = sub(dsjxy, mul(wxy, sub(sxx, syy)));
-    dsjyy = sub(dsjyy, w2s);
+    dsjyy = __fma_rn(-el.two, ws, dsjyy);
     sxx = add(sxx, mul(el.dt, dsjxx));
     sxy = add(sxy, mul(el.dt, dsjxy));
     syy = add(syy, mul(el.dt, dsjyy));
@@ -285,11 +320,11 @@ __device__ __forceinline__ void isolin(const Elastic &el, double exx, double exy
 // negative_root, g_local_mu2.c:90-99 (also g_nonlocal_mu2.c:226-235), with
 // a = 1: the products by 4 and 2 are exact, so they ride in an FMA and in the
 // quotient's exponent.
-__device__ __forceinline__ double negative_root(double b, double c)
+__device__ __forceinline__ double negative_root(const Elastic &el, double b, double c)
 {
-    const double disc = root(__fma_rn(-4.0, c, mul(b, b)));
-    if (is_pos(b)) return mul(0.5, sub(-b, disc));
-    return quot<1>(c, sub(disc, b));
+    const double disc = root(__fma_rn(el.mfour, c, el.mul(b, b)));
+    if (is_pos(b)) return el.mul(el.half, el.sub(-b, disc));
+    return quot<1>(c, el.sub(disc, b));
 }
 
 struct Mu2Params {
@@ -311,13 +346,13 @@ struct Mu2Params {
 // Only m inside the bracket, and any operand that is not a normal positive
 // number above 2^-959 (or a NaN), takes the division.  Positive normal
 // products and m order as integers; the dense side is tested first.
-__device__ __forceinline__ bool below_density(double m, double v, const Mu2Params &mp)
+__device__ __forceinline__ bool below_density(const Unit &u, double m, double v, const Mu2Params &mp)
 {
     const long long mb = __double_as_longlong(m), vb = __double_as_longlong(v);
     if (vb > 0x0400000000000000LL && vb < 0x7ff0000000000000LL && mb > 0x0400000000000000LL &&
         mb < 0x7ff0000000000000LL) {
-        if (mb > __double_as_longlong(__dmul_rn(v, mp.rho_hi))) return false;
-        if (mb < __double_as_longlong(__dmul_rn(v, mp.rho_lo))) return true;
+        if (mb > __double_as_longlong(u.mul(v, mp.rho_hi))) return false;
+        if (mb < __double_as_longlong(u.mul(v, mp.rho_lo))) return true;
     }
     return __ddiv_rn(m, v) < mp.rho_critical;
 }
@@ -332,6 +367,9 @@ __device__ __forceinline__ void g_local_mu2(const Elastic &el, const Mu2Params &
                                             double wxy, double &Txx, double &Txy, double &Tyy,
                                             double &Tzz, double &gammap, double &gammadotp)
 {
+    const auto mul = [&](double a, double b) { return el.mul(a, b); };
+    const auto add = [&](double a, double b) { return el.add(a, b); };
+    const auto sub = [&](double a, double b) { return el.sub(a, b); };
     const double G = el.G, dt = el.dt;
     const double lambda = el.lambda;   // K - 2 G / 3, formed on the host with the same roundings
     // L (:191-199), W = skw(L), D = sym(L) (tensor.c:330-384)
@@ -351,18 +389,18 @@ __device__ __forceinline__ void g_local_mu2(const Elastic &el, const Mu2Params &
     const double twoG = el.twoG;
     const double lt = mul(lambda, trD);
     const double Txx_tr = add(mul(add(add(mul(exx, twoG), lt), JSxx), dt), Txx);
-    const double Txy_tr = add(mul(__fma_rn(0.5, JSxy2, mul(d2, G)), dt), Txy);
+    const double Txy_tr = add(mul(__fma_rn(el.half, JSxy2, mul(d2, G)), dt), Txy);
     const double Tyy_tr = add(mul(sub(add(mul(eyy, twoG), lt), JSxx), dt), Tyy);
     const double Tzz_tr = add(mul(lt, dt), Tzz);
     // decompose and contract (:225-228; tensor.c:205-224, :422-437)
-    double p_tr = third(add(add(Txx_tr, Tyy_tr), Tzz_tr));
+    double p_tr = dvd_const(add(add(Txx_tr, Tyy_tr), Tzz_tr), el.k3);
     const double T0xx = sub(Txx_tr, p_tr), T0xy = Txy_tr, T0yy = sub(Tyy_tr, p_tr), T0zz = sub(Tzz_tr, p_tr);
     const double xy2 = mul(T0xy, T0xy);
     const double tt = add(add(add(add(mul(T0xx, T0xx), xy2), xy2), mul(T0yy, T0yy)), mul(T0zz, T0zz));
     const double tau_tr = root<-1>(tt);
     p_tr = -p_tr;
 
-    const bool density_flag = below_density(m, v, mp);
+    const bool density_flag = below_density(el, m, v, mp);
     double nup_tau;
     if (density_flag || !(is_pos(p_tr) || is_nan(p_tr))) {
         nup_tau = 0;
@@ -382,7 +420,7 @@ __device__ __forceinline__ void g_local_mu2(const Elastic &el, const Mu2Params &
             const double alpha = dvd_const(mul(mp.GI0dt, root(dvd_const(p_tr, mp.krho))), mp.kd);
             const double B = -add(add(S2, tau_tr), alpha);
             const double H = add(mul(S2, tau_tr), mul(S0, alpha));
-            const double tau_tau = negative_root(B, H);
+            const double tau_tau = negative_root(el, B, H);
             const double scale_factor = quot(tau_tau, tau_tr);
             nup_tau = dvd_const(dvd_const(sub(tau_tr, tau_tau), el.kG), el.kdt);
             Txx = sub(mul(T0xx, scale_factor), p_tr);
@@ -419,6 +457,9 @@ __device__ __forceinline__ void plane_return(const Elastic &el, const ReturnPara
                                              double &sxy, double &syy, double &szz, double &beta,
                                              double &gammap, double &gammadotp)
 {
+    const auto mul = [&](double a, double b) { return el.mul(a, b); };
+    const auto add = [&](double a, double b) { return el.add(a, b); };
+    const auto sub = [&](double a, double b) { return el.sub(a, b); };
     const double G = el.G, K = el.K, dt = el.dt;
     const double lambda = el.lambda;   // K - 2 G / 3, formed on the host with the same roundings
     const double twoG = el.twoG;
@@ -426,27 +467,27 @@ __device__ __forceinline__ void plane_return(const Elastic &el, const ReturnPara
     double dsjxx = add(mul(lambda, trD), mul(twoG, exx));
     double dsjxy = mul(twoG, exy);
     double dsjyy = add(mul(lambda, trD), mul(twoG, eyy));
-    double w2s = mul(mul(2.0, wxy), sxy);
-    dsjxx = add(dsjxx, w2s);
+    const double ws = mul(wxy, sxy);   // 2 ws rides in the FMAs: the doubling is exact
+    dsjxx = __fma_rn(el.two, ws, dsjxx);
     dsjxy = sub(dsjxy, mul(wxy, sub(sxx, syy)));
-    dsjyy = sub(dsjyy, w2s);
+    dsjyy = __fma_rn(-el.two, ws, dsjyy);
     double sxx_tr = add(sxx, mul(dt, dsjxx));
     double sxy_tr = add(sxy, mul(dt, dsjxy));
     double syy_tr = add(syy, mul(dt, dsjyy));
     double p_tr, t0zz = 0, szz_tr = 0;
     if (TRIAL3D) {
         szz_tr = add(szz, mul(mul(dt, lambda), trD));
-        p_tr = third(-add(add(sxx_tr, syy_tr), szz_tr));
+        p_tr = dvd_const(-add(add(sxx_tr, syy_tr), szz_tr), el.k3);
     } else {
-        p_tr = mul(-0.5, add(sxx_tr, syy_tr));
+        p_tr = -mul(el.half, add(sxx_tr, syy_tr));
     }
     double t0xx = add(sxx_tr, p_tr), t0xy = sxy_tr, t0yy = add(syy_tr, p_tr);
-    double tt = add(add(mul(t0xx, t0xx), mul(mul(2.0, t0xy), t0xy)), mul(t0yy, t0yy));
+    double tt = add(__fma_rn(el.two, mul(t0xy, t0xy), mul(t0xx, t0xx)), mul(t0yy, t0yy));
     if (TRIAL3D) {
         t0zz = add(szz_tr, p_tr);
         tt = add(tt, mul(t0zz, t0zz));
     }
-    double tau_tr = root(mul(0.5, tt));
+    double tau_tr = root<-1>(tt);
 
     const bool density_flag = quot(m, v) < rp.rho_critical;
     double nup_tau;
@@ -466,7 +507,7 @@ __device__ __forceinline__ void plane_return(const Elastic &el, const ReturnPara
             double alpha = quot(mul(mul(mul(G, rp.I0), dt), root(quot(p_tr, rp.grains_rho))), rp.grains_d);
             double B = -add(add(S2, tau_tr), alpha);
             double H = add(mul(S2, tau_tr), mul(S0, alpha));
-            tau_tau = negative_root(B, H);
+            tau_tau = negative_root(el, B, H);
             scale_factor = quot(tau_tau, tau_tr);
         } else {
             tau_tau = S0;
@@ -494,24 +535,27 @@ __device__ __forceinline__ void g_local_mu2_reverse(const Elastic &el, const Mu2
                                                     double &sxy, double &syy, double &beta, double &gammap,
                                                     double &gammadotp)
 {
+    const auto mul = [&](double a, double b) { return el.mul(a, b); };
+    const auto add = [&](double a, double b) { return el.add(a, b); };
+    const auto sub = [&](double a, double b) { return el.sub(a, b); };
     const double K = el.K, dt = el.dt, c = 0;
     const double lambda = el.lambda;
     const double twoG = el.twoG;
-    double p_t = mul(-0.5, add(sxx, syy));
+    double p_t = -mul(el.half, add(sxx, syy));
     double trD = add(exx, eyy);
     double dsjxx = add(mul(lambda, trD), mul(twoG, exx));
     double dsjxy = mul(twoG, exy);
     double dsjyy = add(mul(lambda, trD), mul(twoG, eyy));
-    double w2s = mul(mul(2.0, wxy), sxy);
-    dsjxx = sub(dsjxx, w2s);
+    const double ws = mul(wxy, sxy);   // 2 ws rides in the FMAs: the doubling is exact
+    dsjxx = __fma_rn(-el.two, ws, dsjxx);
     dsjxy = add(dsjxy, mul(wxy, sub(sxx, syy)));
-    dsjyy = add(dsjyy, w2s);
+    dsjyy = __fma_rn(el.two, ws, dsjyy);
     double sxx_tr = add(sxx, mul(dt, dsjxx));
     double sxy_tr = add(sxy, mul(dt, dsjxy));
     double syy_tr = add(syy, mul(dt, dsjyy));
-    double p_tr = mul(-0.5, add(sxx_tr, syy_tr));
+    double p_tr = -mul(el.half, add(sxx_tr, syy_tr));
     double t0xx = add(sxx_tr, p_tr), t0xy = sxy_tr, t0yy = add(syy_tr, p_tr);
-    double tau_tr = root<-1>((add(add(mul(t0xx, t0xx), mul(mul(2.0, t0xy), t0xy)), mul(t0yy, t0yy))));
+    double tau_tr = root<-1>((add(__fma_rn(el.two, mul(t0xy, t0xy), mul(t0xx, t0xx)), mul(t0yy, t0yy))));
     double inum = mul(mul(gammadotp, mp.grains_d), root(mp.grains_rho));
     double mu_t;
     if (p_t <= 0) {
@@ -588,21 +632,24 @@ __device__ __forceinline__ void ext_stress(const Elastic &el, const Mu2Params &m
                                            double &sxy, double &syy, double &mu_t, double &beta, double &gammap,
                                            double &gammadotp)
 {
+    const auto mul = [&](double a, double b) { return el.mul(a, b); };
+    const auto add = [&](double a, double b) { return el.add(a, b); };
+    const auto sub = [&](double a, double b) { return el.sub(a, b); };
     const double K = el.K, dt = el.dt, c = 1e-2;
-    double p_t = mul(-0.5, add(sxx, syy));
-    const double Ep = quot(E, sub(1.0, mul(nu, nu)));
-    const double Gp = quot(E, mul(2.0, add(1.0, nu)));
+    double p_t = -mul(el.half, add(sxx, syy));
+    const double Ep = quot(E, sub(el.one, mul(nu, nu)));
+    const double Gp = quot(E, mul(el.two, add(el.one, nu)));
     double dsjxx = mul(mul(dt, Ep), add(exx, mul(nu, eyy)));
     double dsjxy = mul(mul(dt, Gp), exy);
     double dsjyy = mul(mul(dt, Ep), add(eyy, mul(nu, exx)));
-    double w2 = mul(mul(mul(2.0, dt), wxy), sxy);
+    double w2 = mul(mul(mul(el.two, dt), wxy), sxy);
     dsjxx = sub(dsjxx, w2);
     dsjxy = add(dsjxy, mul(mul(dt, wxy), sub(sxx, syy)));
     dsjyy = add(dsjyy, w2);
     double sxx_tr = add(sxx, dsjxx), sxy_tr = add(sxy, dsjxy), syy_tr = add(syy, dsjyy);
-    double p_tr = mul(-0.5, add(sxx_tr, syy_tr));
+    double p_tr = -mul(el.half, add(sxx_tr, syy_tr));
     double t0xx = add(sxx_tr, p_tr), t0xy = sxy_tr, t0yy = add(syy_tr, p_tr);
-    double tau_tr = root<-1>((add(add(mul(t0xx, t0xx), mul(mul(2.0, t0xy), t0xy)), mul(t0yy, t0yy))));
+    double tau_tr = root<-1>((add(__fma_rn(el.two, mul(t0xy, t0xy), mul(t0xx, t0xx)), mul(t0yy, t0yy))));
     mu_t = mu_from_gammadot(gammadotp, p_t, mul(mp.grains_d, root(mp.grains_rho)), mp.mu_s, mp.mu_2, mp.I0);
     double tau_tau = mul(mu_t, add(p_tr, c));
     double f = sub(tau_tr, tau_tau);
@@ -644,6 +691,9 @@ __device__ __forceinline__ void nonlocal_mu2_trial(const Elastic &el, double exx
                                                    double syy, double &p_tr, double &t0xx,
                                                    double &t0xy, double &t0yy, double &tau_tr)
 {
+    const auto mul = [&](double a, double b) { return el.mul(a, b); };
+    const auto add = [&](double a, double b) { return el.add(a, b); };
+    const auto sub = [&](double a, double b) { return el.sub(a, b); };
     const double dt = el.dt;
     const double lambda = el.lambda;   // sub(K, quot(mul(2, G), 3)), formed on the host with the same roundings
     const double twoG = el.twoG;
@@ -651,18 +701,18 @@ __device__ __forceinline__ void nonlocal_mu2_trial(const Elastic &el, double exx
     double dsjxx = add(mul(lambda, trD), mul(twoG, exx));
     double dsjxy = mul(twoG, exy);
     double dsjyy = add(mul(lambda, trD), mul(twoG, eyy));
-    double w2s = mul(mul(2.0, wxy), sxy);
-    dsjxx = add(dsjxx, w2s);
+    const double ws = mul(wxy, sxy);   // 2 ws rides in the FMAs: the doubling is exact
+    dsjxx = __fma_rn(el.two, ws, dsjxx);
     dsjxy = sub(dsjxy, mul(wxy, sub(sxx, syy)));
-    dsjyy = sub(dsjyy, w2s);
+    dsjyy = __fma_rn(-el.two, ws, dsjyy);
     double sxx_tr = add(sxx, mul(dt, dsjxx));
     double sxy_tr = add(sxy, mul(dt, dsjxy));
     double syy_tr = add(syy, mul(dt, dsjyy));
-    p_tr = mul(-0.5, add(sxx_tr, syy_tr));
+    p_tr = -mul(el.half, add(sxx_tr, syy_tr));
     t0xx = add(sxx_tr, p_tr);
     t0xy = sxy_tr;
     t0yy = add(syy_tr, p_tr);
-    tau_tr = root<-1>((add(add(mul(t0xx, t0xx), mul(mul(2.0, t0xy), t0xy)), mul(t0yy, t0yy))));
+    tau_tr = root<-1>((add(__fma_rn(el.two, mul(t0xy, t0xy), mul(t0xx, t0xx)), mul(t0yy, t0yy))));
 }
 
 // calculate_bulk_granular_fluidity, g_nonlocal_mu2.c:238-321, for one
@@ -680,7 +730,10 @@ __device__ __forceinline__ void nonlocal_mu2_bulk(const Elastic &el, const Mu2Pa
                                                   double v, double p_tr, double tau_tr, double &dense,
                                                   double &gf_local, double &xisq_inv)
 {
-    const bool is_dense = !(below_density(m, v, mp) || is_neg(p_tr));
+    const auto mul = [&](double a, double b) { return el.mul(a, b); };
+    const auto add = [&](double a, double b) { return el.add(a, b); };
+    const auto sub = [&](double a, double b) { return el.sub(a, b); };
+    const bool is_dense = !(below_density(el, m, v, mp) || is_neg(p_tr));
     dense = is_dense ? 1.0 : 0.0;
     if (!is_dense || !(is_pos(p_tr) || is_nan(p_tr))) {
         gf_local = 0;
@@ -696,7 +749,7 @@ __device__ __forceinline__ void nonlocal_mu2_bulk(const Elastic &el, const Mu2Pa
             double alpha = mul(mp.alpha_c, root(p_tr));
             double B = add(add(S2, tau_tr), alpha);
             double H = add(mul(S2, tau_tr), mul(S0, alpha));
-            tau_tau = quot<1>(H, add(B, root(__fma_rn(-4.0, H, mul(B, B)))));
+            tau_tau = quot<1>(H, add(B, root(__fma_rn(el.mfour, H, mul(B, B)))));
             gf_local = quot(mul(p_tr, sub(tau_tr, tau_tau)), mul(el.Gdt, tau_tau));
         }
         xisq_inv = dvd_const(fabs(sub(quot(tau_tau, p_tr), mp.mu_s)), mp.kAAdd);
@@ -718,6 +771,9 @@ __device__ __forceinline__ void nonlocal_mu2_stress(const Elastic &el, double gf
                                                     double tau_tr, double &sxx, double &sxy,
                                                     double &syy, double &gammap, double &gammadotp)
 {
+    const auto mul = [&](double a, double b) { return el.mul(a, b); };
+    const auto add = [&](double a, double b) { return el.add(a, b); };
+    const auto sub = [&](double a, double b) { return el.sub(a, b); };
     const double dt = el.dt;
     const double p_tr = p_d;
     double nup_tau;

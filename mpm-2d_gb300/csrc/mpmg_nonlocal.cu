@@ -97,23 +97,23 @@ __global__ void nonlocal_bulk_kernel(int n, mat::NonlocalParams np, const double
 // them once, instead of per particle.  The kernel is bound by the FP64 pipe
 // (1/64 of the FP32 rate on GB300); the mass part stays per particle.
 __global__ void __launch_bounds__(128) assemble_kernel(
-    int ne, int Ex, double inv_h, int dense_only, const int *__restrict__ cell_start,
-    const uint32_t *__restrict__ perm, const double *__restrict__ xl, const double *__restrict__ yl,
+    int ne, int Ex, double inv_h, int dense_only, RowView rv, const double *__restrict__ xl, const double *__restrict__ yl,
     const double *__restrict__ v, const double *__restrict__ dense, const double *__restrict__ gfl,
     const double *__restrict__ xisq, double *__restrict__ elem_k, double *__restrict__ elem_f)
 {
     int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= ne) return;
-    const int k0 = cell_start[e], k1 = cell_start[e + 1];
-    if (k0 == k1) return;
+    const int cnt = (int)rv.count[e];
+    if (cnt == 0) return;
+    const uint32_t *list = rv.list(e, cnt);
     double K[10], F[4];
 #pragma unroll
     for (int k = 0; k < 10; k++) K[k] = 0;
 #pragma unroll
     for (int k = 0; k < 4; k++) F[k] = 0;
     double m0 = 0, ma = 0, maa = 0, mb = 0, mbb = 0;
-    for (int k = k0; k < k1; k++) {
-        const int i = (int)perm[k];
+    for (int k = 0; k < cnt; k++) {
+        const int i = (int)list[k];
         if (dense_only && dense[i] == 0) continue;
         const double a = xl[i], b = yl[i];
         const double ox = 1 - a, oy = 1 - b;
@@ -167,6 +167,7 @@ struct SolveArgs {
     double tol;          // relative residual
     int maxit;
     const double *node_m;
+    const uint32_t *counts;   // particles an element, or null (cell_start tells)
     const int *cell_start;
     const double *elem_k, *elem_f;
     double *x, *r, *p, *q, *dinv;
@@ -286,7 +287,7 @@ __device__ __forceinline__ void build_row(const SolveArgs &S, int i, int j, doub
         const int ci = i + qx[q], cj = j + qy[q];
         if (ci < 0 || cj < 0 || ci >= S.Ex || cj >= S.Ey) continue;
         const int e = cj * S.Ex + ci;
-        if (S.cell_start[e] == S.cell_start[e + 1]) continue;
+        if (S.counts != nullptr ? S.counts[e] == 0 : S.cell_start[e] == S.cell_start[e + 1]) continue;
 #pragma unroll
         for (int b = 0; b < 4; b++) {
             const int di = qx[q] + bx[b], dj = qy[q] + by[b];
@@ -2361,7 +2362,7 @@ void mpmg_nonlocal_free(mpmg_ctx *ctx)
 // forward step solves for the nodal fluidity; the adjoint step solves the
 // same symmetric system for the adjoint of the fluidity.
 int mpmg_solve_fluidity_system(mpmg_ctx *ctx, const double *elem_k, const double *elem_f, const double *node_m,
-                               const int *cell_start, double *x, bool zero_start)
+                               const uint32_t *counts, const int *cell_start, double *x, bool zero_start)
 {
     cudaStream_t s = ctx->stream;
     const mpmg_config &c = ctx->cfg;
@@ -2377,6 +2378,7 @@ int mpmg_solve_fluidity_system(mpmg_ctx *ctx, const double *elem_k, const double
     S.tol = c.solver_tol;
     S.maxit = c.solver_maxit;
     S.node_m = node_m;
+    S.counts = counts;
     S.cell_start = cell_start;
     S.elem_k = elem_k;
     S.elem_f = elem_f;
@@ -2421,7 +2423,9 @@ int mpmg_solve_fluidity_system(mpmg_ctx *ctx, const double *elem_k, const double
 // ctx->elem_f): the nodal fluidity lands in ctx->node_gf.
 int mpmg_launch_solve(mpmg_ctx *ctx)
 {
-    return mpmg_solve_fluidity_system(ctx, ctx->elem_k, ctx->elem_f, ctx->node_m, ctx->cell_start, ctx->node_gf,
+    return mpmg_solve_fluidity_system(ctx, ctx->elem_k, ctx->elem_f, ctx->node_m,
+                                      ctx->mixed ? (const uint32_t *)nullptr : ctx->row.count[ctx->row.cur],
+                                      ctx->cell_start, ctx->node_gf,
                                       !ctx->cfg.solver_warm_start);
 }
 
@@ -2446,24 +2450,18 @@ int mpmg_launch_fluidity(mpmg_ctx *ctx)
         ctx->launches += 1;
     }
     const double *xisq = mu2 ? ctx->state[6] : ctx->state[10];
-    assemble_kernel<<<blocks_for(ne, 128), 128, 0, s>>>(ne, ctx->Ex, ctx->inv_h, mu2 ? 1 : 0, ctx->cell_start,
-                                                        ctx->perm, ctx->xl, ctx->yl, ctx->v, ctx->state[0],
+    assemble_kernel<<<blocks_for(ne, 128), 128, 0, s>>>(ne, ctx->Ex, ctx->inv_h, mu2 ? 1 : 0,
+                                                        RowView{ctx->row.count[ctx->row.cur],
+                                                                ctx->row.rows[ctx->row.cur], ctx->row.over_list,
+                                                                ctx->row.cap},
+                                                        ctx->xl, ctx->yl, ctx->v, ctx->state[0],
                                                         ctx->state[5], xisq, ctx->elem_k, ctx->elem_f);
     ctx->launches += 1;
 
     int rc = mpmg_launch_solve(ctx);
     if (rc != MPMG_OK) return rc;
 
-    mat::Elastic el;
-    el.G = ctx->G;
-    el.twoG = 2.0 * ctx->G;
-    el.K = ctx->K;
-    el.lambda = ctx->lambda;
-    el.dt = c.dt;
-    el.Gdt = ctx->G * c.dt;
-    el.kG = mat::make_known(ctx->G);
-    el.kdt = mat::make_known(c.dt);
-    el.kGdt = mat::make_known(el.Gdt);
+    const mat::Elastic el = mat::make_elastic(ctx->G, ctx->K, ctx->lambda, c.dt);
     if (mu2) {
         fluidity_stress_kernel<true, false><<<blocks_for(n, 256), 256, 0, s>>>(
             n, c.Nx, ctx->Ex, el, np, ctx->d_params, ctx->active, ctx->in_element, ctx->xl, ctx->yl,

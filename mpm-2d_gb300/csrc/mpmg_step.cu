@@ -2,20 +2,27 @@
 // libmpm/process_usl.c:465-592, plus the driver's time_varying_loads tail,
 // src/main.c:975 and libmpm/loading.c:34-54).
 //
-//   keys      element of every particle (WHICH_ELEMENT4, :43-44 and :631-674);
-//             advances t and the gravity scalar in the device StepParams
-//   bin       stable counting sort of (element, particle) -> per-element
-//             particle segments (find_filled_elements, :677-723; mpmg_bin.cu)
-//   p2g       one thread per element sums its particles' contributions to
-//             its four corners (map_to_grid_explicit_split, :812-910)
+//   rows      each element's particle indices, in a row of the element's own
+//             (find_filled_elements, :677-723).  The G2P bins every particle it
+//             moves for the next step (WHICH_ELEMENT4, :43-44 and :631-674), so
+//             a step needs no pass of its own for it; keys_kernel does it where
+//             positions came from outside (the first step, a set field)
+//   p2g       one thread (or two) per element puts its row in particle order
+//             and sums the contributions to its four corners
+//             (map_to_grid_explicit_split, :812-910); advances t and the
+//             gravity scalar in the device StepParams
 //   grid      one thread per node adds the four adjacent elements' corner
 //             sums in colour order 0..3, applies the box / square-silo
 //             conditions and the nodal update (bc_momentum, bc_force,
-//             move_grid_split :596-625)
+//             move_grid_split :596-625); then one per element forms the
+//             bilinear coefficients of the nodal acceleration and velocity
 //   g2p       one thread per particle: velocity and position update, strain
 //             rate, volume and the material law (move_particles :914-957,
 //             calculate_strainrate :764-808, update_densities :961-970,
-//             calculate_stress_threaded)
+//             calculate_stress_threaded), and the next step's rows
+//
+// The kernels are launched with programmatic dependent launch: each waits for
+// the one before it at its start and lets the next one launch.
 //
 // Shape functions (tent / grad_tent, interpolate.c:23-65) are recomputed in
 // registers from the start-of-step position wherever they are needed.  No
@@ -37,15 +44,109 @@ using fp64::make_geom;
 using fp64::shape;
 
 // ---------------------------------------------------------------------------
-// keys
+// rows
 
-__global__ void __launch_bounds__(256) keys_kernel(GridGeom g, float inv_hf, int n, const double *__restrict__ x,
-                                                   const double *__restrict__ y, int *__restrict__ in_element,
-                                                   int *__restrict__ active, uint32_t *__restrict__ keys,
-                                                   uint32_t sentinel, uint32_t *__restrict__ bins, StepParams *sp,
-                                                   double dt, int gravity_mode, double gravity_const)
+struct RowsOut {
+    uint32_t *count, *rows, *over_n;
+    uint2 *over;
+    int cap;
+};
+
+// Adds particle i to element key's row (every lane of the warp calls it; valid
+// marks lanes with a particle inside the grid).  Runs of equal keys in
+// consecutive lanes share one atomic.
+__device__ __forceinline__ void bin_particle(const RowsOut &R, int i, uint32_t key, bool valid)
 {
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t k = valid ? key : 0xffffffffu;
+    const uint32_t prev = __shfl_up_sync(0xffffffffu, k, 1);
+    const bool start = valid && (lane == 0 || prev != k);
+    const uint32_t starts = __ballot_sync(0xffffffffu, start);
+    const uint32_t invalid = ~__ballot_sync(0xffffffffu, valid);
+    uint32_t base = 0;
+    if (start) {
+        const uint32_t above = lane == 31 ? 0u : (starts | invalid) & (0xfffffffeu << lane);
+        const int end = above ? __ffs(above) - 1 : 32;
+        base = atomicAdd(&R.count[key], (uint32_t)(end - lane));
+    }
+    const uint32_t below = starts & (0xffffffffu >> (31 - lane));
+    const int leader = below ? 31 - __clz(below) : lane;
+    base = __shfl_sync(0xffffffffu, base, leader);
+    if (!valid) return;
+    const uint32_t slot = base + (uint32_t)(lane - leader);
+    if (slot < (uint32_t)R.cap) R.rows[(size_t)key * R.cap + slot] = (uint32_t)i;
+    else R.over[atomicAdd(R.over_n, 1u)] = make_uint2(key, (uint32_t)i);
+}
+
+// The rows of the current positions, where no G2P has left them: keys[i] is
+// the element, or the sentinel for a particle that is inactive or outside.
+__global__ void __launch_bounds__(256) keys_kernel(GridGeom g, float inv_hf, int n, const double *__restrict__ x,
+                                                   const double *__restrict__ y, const int *__restrict__ active,
+                                                   uint32_t *__restrict__ keys, uint32_t sentinel, RowsOut R)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t key = sentinel;
+    if (i < n) {
+        if (active[i]) {
+            const int e = mpmg_which_element_fast(x[i], y[i], g.h, g.inv_h, inv_hf, g.xmax, g.ymax,
+                                                  __double_as_longlong(g.xmax), __double_as_longlong(g.ymax), g.Ex,
+                                                  g.Ey);
+            if (e >= 0) key = (uint32_t)e;
+        }
+        keys[i] = key;
+    }
+    bin_particle(R, i, key, key != sentinel);
+}
+
+// ---------------------------------------------------------------------------
+// p2g: per-element corner sums over the element's row, in particle order.
+//
+// The corner weights are bilinear in the local coordinates (x, y):
+// N = {(1-x)(1-y), x(1-y), xy, (1-x)y}, dN/dx h = {-(1-y), 1-y, y, -y},
+// dN/dy h = {-(1-x), -x, x, 1-x}.  So the element's four corner sums of a
+// particle quantity q follow from four moments, A = sum q, X = sum x q,
+// Y = sum y q, Z = sum xy q:  corners A - X - Y + Z, X - Z, Z, Y - Z; and the
+// eight internal-force sums from seven moments of the stress terms.  The
+// particle loop costs 26 FP64 operations; 1 / h of the gradients and the body
+// force are applied once per node (grid_kernel).
+//
+// The loop is bound by the FP64 pipe, where an instruction costs a sub-partition
+// 64 cycles whatever the number of active lanes: a warp costs its fullest
+// element's count.  So a block sorts its elements by count (each warp then
+// holds equal counts, and empty elements share warps that do nothing), and the
+// sorted warps rotate with the block index, so that no sub-partition gets the
+// full ones of every block.  SPLIT = 2 gives the two halves of an element's
+// moments to two threads in different warps, which shortens the serial chain
+// where the grid is too small to fill the chip.
+
+template <int EB, int SPLIT>
+__global__ void __launch_bounds__(EB * SPLIT) p2g_cells_kernel(
+    GridGeom g, int ne, int n, RowView rv, uint32_t *__restrict__ count_next, const uint32_t *__restrict__ over_n,
+    uint32_t *__restrict__ over_n_next, const uint2 *__restrict__ over, uint32_t *__restrict__ over_cursor,
+    int keep_order, const double *__restrict__ x, const double *__restrict__ y, const double *__restrict__ m,
+    const double *__restrict__ vx, const double *__restrict__ vy, const double *__restrict__ v,
+    const double *__restrict__ sxx, const double *__restrict__ sxy, const double *__restrict__ syy, StepParams *sp,
+    double dt, int gravity_mode, double gravity_const, double *__restrict__ cell_sums)
+{
+    constexpr int NB = 17;                 // count classes 0..15 and 16 or more
+    constexpr int kStage = 16;             // staged row entries an element
+    extern __shared__ __align__(16) unsigned char p2g_smem[];
+    uint32_t *sh_idx = reinterpret_cast<uint32_t *>(p2g_smem);         // [kStage][EB]
+    double *sh_sum = reinterpret_cast<double *>(p2g_smem);             // [20][EB], after the index stage
+    __shared__ int sh_bin[NB];
+    __shared__ int sh_order[EB], sh_count[EB];
+    __shared__ uint32_t sh_base[EB];
+    __shared__ double sh_const[3];         // constants as registers (mat::Unit)
+    if (threadIdx.x == 0) {
+        sh_const[0] = 1.0;
+        sh_const[1] = -0.0;
+        sh_const[2] = g.inv_h;
+    }
+    mpmg_pdl_wait();
+    mpmg_pdl_trigger();
+    const int tid = threadIdx.x;
+    const int e0 = blockIdx.x * EB;
+    if (blockIdx.x == 0 && tid == 0) {
         // time_varying_loads (loading.c:34-54) of the previous step's tail, or
         // initial_loads (loading.c:21-30) before the first step; then t += dt
         // (process_usl.c:522).
@@ -63,196 +164,374 @@ __global__ void __launch_bounds__(256) keys_kernel(GridGeom g, float inv_hf, int
         sp->gravity = grav;
         sp->t = t + dt;
         sp->step_count += 1;
+        *over_n_next = 0;
     }
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t key = sentinel;
-    if (i < n) {
-        if (active[i]) {
-            int e = mpmg_which_element_fast(x[i], y[i], g.h, g.inv_h, inv_hf, g.xmax, g.ymax,
-                                            __double_as_longlong(g.xmax), __double_as_longlong(g.ymax), g.Ex,
-                                            g.Ey);
-            in_element[i] = e;
-            if (e < 0) {
-                active[i] = 0;   // process_usl.c:660-666: outside the grid for good
-            } else {
-                key = (uint32_t)e;
-            }
+    if (tid < NB) sh_bin[tid] = 0;
+    int cnt0 = 0;
+    if (tid < EB && e0 + tid < ne) {
+        cnt0 = (int)rv.count[e0 + tid];
+        count_next[e0 + tid] = 0;
+    }
+    if (__syncthreads_count(cnt0) == 0) return;
+    // elements by descending count
+    int cls = 0, at = 0;
+    if (tid < EB) {
+        cls = NB - 1 - min(cnt0, NB - 1);
+        at = atomicAdd(&sh_bin[cls], 1);
+        sh_count[tid] = cnt0;
+    }
+    __syncthreads();
+    if (tid < 32) {
+        int c = tid < NB ? sh_bin[tid] : 0, incl = c;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, incl, d);
+            if (tid >= d) incl += u;
         }
-        keys[i] = key;
+        if (tid < NB) sh_bin[tid] = incl - c;
     }
-    mpmg_bin_count(key, i < n, sentinel, (uint32_t)i >> 5, bins);
-}
-
-// ---------------------------------------------------------------------------
-// p2g: per-element corner sums over the element's particle segment.
-//
-// The corner weights are bilinear in the local coordinates (x, y):
-// N = {(1-x)(1-y), x(1-y), xy, (1-x)y}, dN/dx h = {-(1-y), 1-y, y, -y},
-// dN/dy h = {-(1-x), -x, x, 1-x}.  So the element's four corner sums of a
-// particle quantity q follow from four moments, A = sum q, X = sum x q,
-// Y = sum y q, Z = sum xy q:  corners A - X - Y + Z, X - Z, Z, Y - Z; and the
-// eight internal-force sums from seven moments of the stress terms.  The
-// particle loop then costs 29 FP64 operations instead of about 60 (GB300
-// issues FP64 at 1/64 of the FP32 rate, and this loop is bound by it); the
-// body force (m g per corner), the 1/h of the gradients and the corners are
-// formed once per element.  The roundings differ from per-corner sums by a
-// few ulps of the element's totals.
-
-__global__ void __launch_bounds__(128) p2g_cells_kernel(
-    GridGeom g, int ne, const int *__restrict__ cell_start, const uint32_t *__restrict__ slots,
-    uint32_t *__restrict__ perm,
-    const double *__restrict__ x, const double *__restrict__ y, const double *__restrict__ m,
-    const double *__restrict__ vx, const double *__restrict__ vy, const double *__restrict__ v,
-    const double *__restrict__ sxx, const double *__restrict__ sxy, const double *__restrict__ syy,
-    const StepParams *__restrict__ sp, double *__restrict__ cell_sums)
-{
-    int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= ne) return;
-    const int k0 = cell_start[e], k1 = cell_start[e + 1];
-    if (k0 == k1) return;
-    mpmg_order_segment(slots, perm, nullptr, k0, k1);   // ascending particle index, as the reference's lists
+    __syncthreads();
+    if (tid < EB) sh_order[sh_bin[cls] + at] = tid;
+    __syncthreads();
+    // this thread's element and half: sorted warps rotated by the block index
+    constexpr int WB = EB / 32;            // warps an element set
+    const int half = SPLIT == 2 ? tid / EB : 0;
+    const int warp = (tid % EB) / 32;
+    const int le = sh_order[((warp + (int)blockIdx.x) % WB) * 32 + (tid & 31)];
+    const int cnt = sh_count[le], e = e0 + le;
+    const uint32_t *list = nullptr;        // a long element's list in global memory
+    if (half == 0 && cnt > 0) {
+        uint32_t *row = rv.rows + (size_t)e * rv.cap;
+        if (cnt <= kStage && cnt <= rv.cap) {
+            // ascending particle index, as the reference's lists (insertion
+            // sort of a handful of entries in this thread's shared column)
+            uint32_t *col = sh_idx + le;
+            uint4 r4[kStage / 4];              // all of the row's loads in flight
+#pragma unroll
+            for (int j = 0; j < kStage / 4; j++)
+                if (4 * j < cnt) r4[j] = reinterpret_cast<const uint4 *>(row)[j];
+#pragma unroll
+            for (int j = 0; j < kStage; j++) {
+                if (j >= cnt) break;
+                const uint4 v4 = r4[j / 4];
+                const uint32_t q = j % 4 == 0 ? v4.x : j % 4 == 1 ? v4.y : j % 4 == 2 ? v4.z : v4.w;
+                int t = j - 1;
+                while (t >= 0 && col[t * EB] > q) {
+                    col[(t + 1) * EB] = col[t * EB];
+                    t--;
+                }
+                col[(t + 1) * EB] = q;
+            }
+            if (keep_order)
+                for (int j = 0; j < cnt; j++) row[j] = col[j * EB];
+        } else if (cnt <= rv.cap) {
+            for (int j = 1; j < cnt; j++) {
+                const uint32_t q = row[j];
+                int t = j - 1;
+                while (t >= 0 && row[t] > q) {
+                    row[t + 1] = row[t];
+                    t--;
+                }
+                row[t + 1] = q;
+            }
+        } else {
+            // more particles than the row holds: the row and the element's
+            // entries of the overflow list, ordered in over_list
+            const uint32_t base = atomicAdd(over_cursor, (uint32_t)cnt);
+            uint32_t *lst = rv.over_list + base;
+            int have = 0;
+            const int total = (int)*over_n;
+            for (int j = 0; j < rv.cap + total; j++) {
+                uint32_t q;
+                if (j < rv.cap) {
+                    q = row[j];
+                } else {
+                    const uint2 o = over[j - rv.cap];
+                    if (o.x != (uint32_t)e) continue;
+                    q = o.y;
+                }
+                int t = have - 1;
+                while (t >= 0 && lst[t] > q) {
+                    lst[t + 1] = lst[t];
+                    t--;
+                }
+                lst[t + 1] = q;
+                have++;
+            }
+            row[0] = base;
+            sh_base[le] = base;
+        }
+    }
+    if (SPLIT == 2) __syncthreads();
+    if (cnt > kStage || cnt > rv.cap)
+        list = cnt <= rv.cap ? rv.rows + (size_t)e * rv.cap : rv.over_list + sh_base[le];
     const int ci = e % g.Ex, cj = e / g.Ex;
     const double cx = mat::small_int(ci), cy = mat::small_int(cj);   // the element's column and row (element.c:10-19)
     // moments [A, X, Y, Z] of m, m vx, m vy; stress-term moments
     double mm[4] = {0, 0, 0, 0}, mx[4] = {0, 0, 0, 0}, my[4] = {0, 0, 0, 0};
     double P0 = 0, Py0 = 0, P1 = 0, Px1 = 0, Py1 = 0, P2 = 0, Px2 = 0;
-    for (int k = k0; k < k1; k++) {
-        const int i = (int)perm[k];
-        const double xl = mpmg_local_coord_fma(x[i], cx, g.inv_h);
-        const double yl = mpmg_local_coord_fma(y[i], cy, g.inv_h);
-        const double xy = xl * yl;
-        const double pm = m[i];
-        const double pmx = vx[i] * pm, pmy = vy[i] * pm;
-        const double vol = v[i];
-        const double s0 = -sxx[i] * vol, s1 = -sxy[i] * vol, s2 = -syy[i] * vol;
-        mm[0] += pm;
-        mm[1] = fma(xl, pm, mm[1]);
-        mm[2] = fma(yl, pm, mm[2]);
-        mm[3] = fma(xy, pm, mm[3]);
-        mx[0] += pmx;
-        mx[1] = fma(xl, pmx, mx[1]);
-        mx[2] = fma(yl, pmx, mx[2]);
-        mx[3] = fma(xy, pmx, mx[3]);
-        my[0] += pmy;
-        my[1] = fma(xl, pmy, my[1]);
-        my[2] = fma(yl, pmy, my[2]);
-        my[3] = fma(xy, pmy, my[3]);
-        P0 += s0;
-        Py0 = fma(yl, s0, Py0);
-        P1 += s1;
-        Px1 = fma(xl, s1, Px1);
-        Py1 = fma(yl, s1, Py1);
-        P2 += s2;
-        Px2 = fma(xl, s2, Px2);
+    const bool do_a = SPLIT == 1 || half == 0, do_b = SPLIT == 1 || half == 1;
+    const mat::Unit u{sh_const[0], sh_const[1]};
+    const double inv_h = sh_const[2];
+    // the next particle's loads are in flight during this one's arithmetic
+    double nx = 0, ny = 0, nm = 0, nvx = 0, nvy = 0, nv = 0, n0 = 0, n1 = 0, n2 = 0;
+    auto fetch = [&](int k) {
+        const int i = (int)(list ? list[k] : sh_idx[k * EB + le]);
+        nx = x[i];
+        ny = y[i];
+        nm = m[i];
+        if (do_a) nvx = vx[i];
+        if (do_b) {
+            nvy = vy[i];
+            nv = v[i];
+            n0 = sxx[i];
+            n1 = sxy[i];
+            n2 = syy[i];
+        }
+    };
+    if (cnt > 0) fetch(0);
+    for (int k = 0; k < cnt; k++) {
+        const double px = nx, py = ny, pm = nm, pvx = nvx, pvy = nvy, vol = nv, t0 = n0, t1 = n1, t2 = n2;
+        if (k + 1 < cnt) fetch(k + 1);
+        const double xl = mpmg_local_coord_fma(px, cx, inv_h);
+        const double yl = mpmg_local_coord_fma(py, cy, inv_h);
+        const double xy = u.mul(xl, yl);
+        if (do_a) {
+            const double pmx = u.mul(pvx, pm);
+            mm[0] = u.add(pm, mm[0]);
+            mm[1] = fma(xl, pm, mm[1]);
+            mm[2] = fma(yl, pm, mm[2]);
+            mm[3] = fma(xy, pm, mm[3]);
+            mx[0] = u.add(pmx, mx[0]);
+            mx[1] = fma(xl, pmx, mx[1]);
+            mx[2] = fma(yl, pmx, mx[2]);
+            mx[3] = fma(xy, pmx, mx[3]);
+        }
+        if (do_b) {
+            const double pmy = u.mul(pvy, pm);
+            const double vlx = u.mul(vol, xl), vly = u.mul(vol, yl);
+            my[0] = u.add(pmy, my[0]);
+            my[1] = fma(xl, pmy, my[1]);
+            my[2] = fma(yl, pmy, my[2]);
+            my[3] = fma(xy, pmy, my[3]);
+            P0 = fma(t0, vol, P0);
+            Py0 = fma(t0, vly, Py0);
+            P1 = fma(t1, vol, P1);
+            Px1 = fma(t1, vlx, Px1);
+            Py1 = fma(t1, vly, Py1);
+            P2 = fma(t2, vol, P2);
+            Px2 = fma(t2, vlx, Px2);
+        }
     }
-    // corners BL, BR, TR, TL (process_usl.c:140-143)
-    double cm[4], cmx[4], cmy[4];
-    cm[0] = (mm[0] - mm[1]) - (mm[2] - mm[3]);
-    cm[1] = mm[1] - mm[3];
-    cm[2] = mm[3];
-    cm[3] = mm[2] - mm[3];
-    cmx[0] = (mx[0] - mx[1]) - (mx[2] - mx[3]);
-    cmx[1] = mx[1] - mx[3];
-    cmx[2] = mx[3];
-    cmx[3] = mx[2] - mx[3];
-    cmy[0] = (my[0] - my[1]) - (my[2] - my[3]);
-    cmy[1] = my[1] - my[3];
-    cmy[2] = my[3];
-    cmy[3] = my[2] - my[3];
-    const double ih = g.inv_h;
-    const double a0 = P0 - Py0, a1 = P1 - Px1, b1 = P1 - Py1, b2 = P2 - Px2;
-    double cfx[4], cfy[4];
-    cfx[0] = -(a0 + a1) * ih;
-    cfx[1] = (a0 - Px1) * ih;
-    cfx[2] = (Py0 + Px1) * ih;
-    cfx[3] = (a1 - Py0) * ih;
-    // body force bx is zero (loading.c:48); by = g acts on each corner's mass
-    const double grav = sp->gravity;
-    cfy[0] = fma(grav, cm[0], -(b1 + b2) * ih);
-    cfy[1] = fma(grav, cm[1], (b1 - Px2) * ih);
-    cfy[2] = fma(grav, cm[2], (Py1 + Px2) * ih);
-    cfy[3] = fma(grav, cm[3], (b2 - Py1) * ih);
-#pragma unroll
-    for (int c = 0; c < 4; c++) {
-        cell_sums[(size_t)(c * 5 + 0) * ne + e] = cm[c];
-        cell_sums[(size_t)(c * 5 + 1) * ne + e] = cmx[c];
-        cell_sums[(size_t)(c * 5 + 2) * ne + e] = cmy[c];
-        cell_sums[(size_t)(c * 5 + 3) * ne + e] = cfx[c];
-        cell_sums[(size_t)(c * 5 + 4) * ne + e] = cfy[c];
+    // corners BL, BR, TR, TL (process_usl.c:140-143); the sums leave through
+    // shared memory so that their stores are coalesced in element order
+    __syncthreads();
+    if (do_a && cnt > 0) {
+        const double dm = u.sub(mm[2], mm[3]), dx = u.sub(mx[2], mx[3]);
+        sh_sum[0 * EB + le] = u.sub(u.sub(mm[0], mm[1]), dm);
+        sh_sum[5 * EB + le] = u.sub(mm[1], mm[3]);
+        sh_sum[10 * EB + le] = mm[3];
+        sh_sum[15 * EB + le] = dm;
+        sh_sum[1 * EB + le] = u.sub(u.sub(mx[0], mx[1]), dx);
+        sh_sum[6 * EB + le] = u.sub(mx[1], mx[3]);
+        sh_sum[11 * EB + le] = mx[3];
+        sh_sum[16 * EB + le] = dx;
+    }
+    if (do_b && cnt > 0) {
+        const double dy = u.sub(my[2], my[3]);
+        sh_sum[2 * EB + le] = u.sub(u.sub(my[0], my[1]), dy);
+        sh_sum[7 * EB + le] = u.sub(my[1], my[3]);
+        sh_sum[12 * EB + le] = my[3];
+        sh_sum[17 * EB + le] = dy;
+        // h times the internal force, -V T grad N
+        const double a0 = u.sub(P0, Py0), a1 = u.sub(P1, Px1), b1 = u.sub(P1, Py1), b2 = u.sub(P2, Px2);
+        sh_sum[3 * EB + le] = u.add(a0, a1);
+        sh_sum[8 * EB + le] = u.sub(Px1, a0);
+        sh_sum[13 * EB + le] = -u.add(Py0, Px1);
+        sh_sum[18 * EB + le] = u.sub(Py0, a1);
+        sh_sum[4 * EB + le] = u.add(b1, b2);
+        sh_sum[9 * EB + le] = u.sub(Px2, b1);
+        sh_sum[14 * EB + le] = -u.add(Py1, Px2);
+        sh_sum[19 * EB + le] = u.sub(Py1, b2);
+    }
+    __syncthreads();
+    for (int q = tid; q < 20 * EB; q += EB * SPLIT) {
+        const int f = q / EB, l = q % EB;
+        if (sh_count[l] > 0) cell_sums[(size_t)f * ne + e0 + l] = sh_sum[q];
     }
 }
 
-// ---------------------------------------------------------------------------
-// grid: finish P2G per node, boundary conditions, nodal update.
+template <int EB>
+constexpr size_t p2g_smem_bytes()
+{
+    return sizeof(double) * 20 * EB > sizeof(uint32_t) * 16 * EB ? sizeof(double) * 20 * EB : sizeof(uint32_t) * 16 * EB;
+}
 
-__global__ void __launch_bounds__(256) grid_kernel(
-    GridGeom g, BcParams bc, int ne, const int *__restrict__ cell_start,
+// ---------------------------------------------------------------------------
+// grid: finish P2G per node, boundary conditions, nodal update; then per
+// element the bilinear coefficients of the nodal fields.
+//
+// A block of 32 x TY threads finishes a tile of 32 x TY nodes (tiles share one
+// column and row of nodes, computed by both to the same bits and stored by
+// one) and then the elements between them.  With node values q0..q3
+// (BL, BR, TR, TL) the field on the element is
+// c0 + c1 x + c2 y + c3 xy, c0 = q0, c1 = q1 - q0, c2 = q3 - q0,
+// c3 = (q2 - q3) - c1: four FP64 operations per element and field here save
+// the G2P about six per particle, and an element's sixteen doubles are one
+// 128-byte line for its gathers instead of sixteen loads from eight lines.
+// TY = 16 recomputes 10 % of the nodes; TY = 4 (39 %) where the grid is too
+// small to give every SM a tall tile, so that its chain is spread out.
+
+constexpr int kGridTX = 32;
+
+template <int TY>
+__global__ void __launch_bounds__(kGridTX * TY) grid_kernel(
+    GridGeom g, BcParams bc, int ne, int tiles_x, const uint32_t *__restrict__ count,
     const double *__restrict__ cell_sums, const StepParams *__restrict__ sp, double dt,
     double *__restrict__ node_m, double *__restrict__ node_ax, double *__restrict__ node_ay,
     double *__restrict__ node_vx, double *__restrict__ node_vy, double *__restrict__ node_mx,
-    double *__restrict__ node_my, double *__restrict__ node_fx, double *__restrict__ node_fy)
+    double *__restrict__ node_my, double *__restrict__ node_fx, double *__restrict__ node_fy,
+    double2 *__restrict__ coef, uint32_t *__restrict__ over_cursor)
 {
-    const int nn = g.Nx * g.Ny;
-    int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= nn) return;
-    const int i = n % g.Nx, j = n / g.Nx;
-    double sum[5] = {0, 0, 0, 0, 0};
+    __shared__ double sh[4][TY][kGridTX];
+    __shared__ double sh_const[4];         // constants as registers (mat::Unit)
+    if (threadIdx.x == 0) {
+        sh_const[0] = 1.0;
+        sh_const[1] = -0.0;
+        sh_const[2] = g.inv_h;
+        sh_const[3] = dt;
+    }
+    const int tx = threadIdx.x % kGridTX, ty = threadIdx.x / kGridTX;
+    const int i = (int)(blockIdx.x % tiles_x) * (kGridTX - 1) + tx, j = (int)(blockIdx.x / tiles_x) * (TY - 1) + ty;
+    const bool node = i < g.Nx && j < g.Ny;
     // Colour c = 2 * (row % 2) + (col % 2) (process_usl.c:158); the four
     // elements around a node have the four colours, summed in order 0..3.
+    // The counts are the previous step's work: read before the wait.
+    const double *src[4];
+    bool filled = false;                   // the element whose BL node this is holds particles
+    if (node) {
 #pragma unroll
-    for (int c = 0; c < 4; c++) {
-        int ci = ((i & 1) == (c & 1)) ? i : i - 1;
-        int cj = ((j & 1) == (c >> 1)) ? j : j - 1;
-        if (ci < 0 || cj < 0 || ci >= g.Ex || cj >= g.Ey) continue;
-        int e = cj * g.Ex + ci;
-        if (cell_start[e] == cell_start[e + 1]) continue;
-        int corner = (ci == i) ? ((cj == j) ? 0 : 3) : ((cj == j) ? 1 : 2);
-#pragma unroll
-        for (int f = 0; f < 5; f++) sum[f] += cell_sums[(size_t)(corner * 5 + f) * ne + e];
+        for (int c = 0; c < 4; c++) {
+            src[c] = nullptr;
+            const int ci = ((i & 1) == (c & 1)) ? i : i - 1;
+            const int cj = ((j & 1) == (c >> 1)) ? j : j - 1;
+            if (ci < 0 || cj < 0 || ci >= g.Ex || cj >= g.Ey) continue;
+            const int e = cj * g.Ex + ci;
+            if (count[e] == 0) continue;
+            const int corner = (ci == i) ? ((cj == j) ? 0 : 3) : ((cj == j) ? 1 : 2);
+            if (corner == 0) filled = true;
+            src[c] = cell_sums + (size_t)(corner * 5) * ne + e;
+        }
     }
-    double m = sum[0], mx = sum[1], my = sum[2], fx = sum[3], fy = sum[4];
-    bool bx, by;
-    bc_mask(bc, g, i, j, sp->t, bx, by);
-    if (bx) { mx = 0; fx = 0; }
-    if (by) { my = 0; fy = 0; }
+    mpmg_pdl_wait();
+    mpmg_pdl_trigger();
+    __syncthreads();
+    const mat::Unit u{sh_const[0], sh_const[1]};
+    if (blockIdx.x == 0 && threadIdx.x == 0) *over_cursor = 0;   // the P2G is done with it
     double ax = 0, ay = 0, vxn = 0, vyn = 0;
-    if (m > MPMG_TOL) {
-        // one division: the four quotients by m differ from IEEE division
-        // by at most an ulp
-        const double inv_m = mat::quot(1.0, m);
-        ax = fx * inv_m;
-        ay = fy * inv_m;
-        mx += dt * fx;
-        my += dt * fy;
-        vxn = mx * inv_m;
-        vyn = my * inv_m;
+    if (node) {
+        double sum[5] = {0, 0, 0, 0, 0};
+        if (src[0] && src[1] && src[2] && src[3]) {
+#pragma unroll
+            for (int f = 0; f < 5; f++) {
+                const size_t o = (size_t)f * ne;
+                sum[f] = u.add(u.add(u.add(src[0][o], src[1][o]), src[2][o]), src[3][o]);
+            }
+        } else {
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                if (src[c] == nullptr) continue;
+#pragma unroll
+                for (int f = 0; f < 5; f++) sum[f] = u.add(sum[f], src[c][(size_t)f * ne]);
+            }
+        }
+        const double m = sum[0];
+        double mx = sum[1], my = sum[2];
+        // body force bx is zero (loading.c:48); by = g acts on the node's mass
+        const double inv_h = sh_const[2], dtr = sh_const[3];
+        double fx = u.mul(sum[3], inv_h), fy = fma(sp->gravity, m, u.mul(sum[4], inv_h));
+        bool bx, by;
+        bc_mask(bc, g, i, j, sp->t, bx, by);
+        if (bx) { mx = 0; fx = 0; }
+        if (by) { my = 0; fy = 0; }
+        // m > MPMG_TOL on the bit patterns
+        if (__double_as_longlong(m) > __double_as_longlong(MPMG_TOL) && !mat::is_nan(m)) {
+            // one division: the four quotients by m differ from IEEE division
+            // by at most an ulp
+            const double inv_m = mat::quot(u.one, m);
+            ax = u.mul(fx, inv_m);
+            ay = u.mul(fy, inv_m);
+            mx = fma(dtr, fx, mx);
+            my = fma(dtr, fy, my);
+            vxn = u.mul(mx, inv_m);
+            vyn = u.mul(my, inv_m);
+        }
+        if ((tx < kGridTX - 1 || i == g.Nx - 1) && (ty < TY - 1 || j == g.Ny - 1)) {
+            const int n = j * g.Nx + i;
+            node_m[n] = m;
+            node_ax[n] = ax;
+            node_ay[n] = ay;
+            node_vx[n] = vxn;
+            node_vy[n] = vyn;
+            if (node_mx != nullptr) {
+                node_mx[n] = mx;
+                node_my[n] = my;
+                node_fx[n] = fx;
+                node_fy[n] = fy;
+            }
+        }
     }
-    node_m[n] = m;
-    node_ax[n] = ax;
-    node_ay[n] = ay;
-    node_vx[n] = vxn;
-    node_vy[n] = vyn;
-    if (node_mx != nullptr) {
-        node_mx[n] = mx;
-        node_my[n] = my;
-        node_fx[n] = fx;
-        node_fy[n] = fy;
+    sh[0][ty][tx] = ax;
+    sh[1][ty][tx] = ay;
+    sh[2][ty][tx] = vxn;
+    sh[3][ty][tx] = vyn;
+    __syncthreads();
+    if (filled && tx < kGridTX - 1 && ty < TY - 1) {
+        double2 *out = coef + (size_t)(j * g.Ex + i) * 8;
+#pragma unroll
+        for (int f = 0; f < 4; f++) {
+            const double q0 = sh[f][ty][tx], q1 = sh[f][ty][tx + 1], q2 = sh[f][ty + 1][tx + 1], q3 = sh[f][ty + 1][tx];
+            const double c1 = u.sub(q1, q0);
+            out[2 * f] = make_double2(q0, c1);
+            out[2 * f + 1] = make_double2(u.sub(q3, q0), u.sub(u.sub(q2, q3), c1));
+        }
     }
+}
+
+template <int TY>
+cudaError_t launch_grid(mpmg_ctx *ctx, const GridGeom &g)
+{
+    const int tiles_x = (g.Nx + kGridTX - 2) / (kGridTX - 1), tiles_y = (g.Ny + TY - 2) / (TY - 1);
+    return mpmg_launch_pdl(true, grid_kernel<TY>, dim3(tiles_x * tiles_y), dim3(kGridTX * TY), 0, ctx->stream, g,
+                           make_bc(ctx), (int)ctx->ne, tiles_x, (const uint32_t *)ctx->row.count[ctx->row.cur],
+                           (const double *)ctx->cell_sums, (const StepParams *)ctx->d_params, ctx->cfg.dt,
+                           ctx->node_m, ctx->node_ax, ctx->node_ay, ctx->node_vx, ctx->node_vy, ctx->node_mx,
+                           ctx->node_my, ctx->node_fx, ctx->node_fy, (double2 *)ctx->elem_coef, ctx->row.over_n + 2);
 }
 
 // ---------------------------------------------------------------------------
 // g2p + material
 
+// The arithmetic's constants, copied to shared memory (mat::Unit).
+struct G2PConst {
+    mat::Elastic el;
+    mat::Mu2Params mu2;
+    double inv_h, half_inv_h;
+};
+
 struct G2PArgs {
     GridGeom g;
     int n;
-    double dt;
-    mat::Elastic el;
-    mat::Mu2Params mu2;
+    G2PConst k;
     mat::NonlocalParams nl;
-    const int *in_element;
-    const int *active;
-    const double *node_ax, *node_ay, *node_vx, *node_vy;
+    uint32_t *keys;        // element of this step in, of the next step out (sentinel: none)
+    uint32_t sentinel;
+    float inv_hf;
+    RowsOut next;          // the next step's rows
+    int *in_element;
+    int *active;
+    const double2 *coef;   // element coefficients (grid_kernel)
+    const double *node_vx, *node_vy;
     double *x, *y, *vx, *vy, *ux, *uy, *v, *m;
     double *sxx, *sxy, *syy, *Tzz;
     double *st0, *st1, *st3, *st4, *st5, *st6, *st9, *st10;
@@ -268,23 +547,63 @@ struct G2PArgs {
 // then the strain phase with the nodal velocities of that second projection.
 enum { G2P_FULL = 0, G2P_MOVE = 1, G2P_STRAIN = 2 };
 
+// A particle's state in registers, loaded before the kernel waits for the grid
+// update (all of it is the previous step's work, or the move phase's).
+struct Particle {
+    double x, y, vx, vy, ux, uy, v, m, sxx, sxy, syy, Tzz, st1, st5, st9, st10, st0, xl, yl;
+};
+
+template <int MATERIAL, int PHASE>
+__device__ __forceinline__ Particle load_particle(const G2PArgs &A, int i)
+{
+    Particle p = {};
+    p.x = A.x[i];
+    p.y = A.y[i];
+    if (PHASE != G2P_STRAIN) {
+        p.vx = A.vx[i];
+        p.vy = A.vy[i];
+        p.ux = A.ux[i];
+        p.uy = A.uy[i];
+    } else {
+        // the start-of-step local coordinates the move phase kept
+        p.xl = A.xl_out[i];
+        p.yl = A.yl_out[i];
+    }
+    if (PHASE == G2P_MOVE) return p;
+    p.v = A.v[i];
+    if (MATERIAL != MPMG_G_NONLOCAL) {
+        p.sxx = A.sxx[i];
+        p.sxy = A.sxy[i];
+        p.syy = A.syy[i];
+    }
+    if (MATERIAL != MPMG_ISOLIN && MATERIAL != MPMG_G_NONLOCAL) p.m = A.m[i];
+    if (MATERIAL == MPMG_G_LOCAL_MU2) p.Tzz = A.Tzz[i];
+    if (MATERIAL == MPMG_DP_RI_MT || MATERIAL == MPMG_G_LOCAL_MU2_PLANE_STRAIN) p.st1 = A.st1[i];
+    if (MATERIAL == MPMG_G_LOCAL_MU2_PLANE_STRAIN || MATERIAL == MPMG_G_LOCAL_MU2_TRUE_2D ||
+        MATERIAL == MPMG_G_LOCAL_MU2_REVERSE)
+        p.st5 = A.st5[i];
+    if (MATERIAL != MPMG_ISOLIN && MATERIAL != MPMG_G_NONLOCAL && MATERIAL != MPMG_G_NONLOCAL_MU2 &&
+        MATERIAL != MPMG_G_LOCAL_MU2_EXT)
+        p.st9 = A.st9[i];
+    if (MATERIAL == MPMG_G_LOCAL_MU2_REVERSE || MATERIAL == MPMG_G_LOCAL_MU2_EXT) p.st10 = A.st10[i];
+    if (MATERIAL == MPMG_G_LOCAL_MU2_EXT) p.st0 = A.st0[i];
+    return p;
+}
+
 // The in-plane local returns on particle i (mat::plane_return): szz in
 // state[1] (dp_ri_mt.c:27, g_local_mu2_plane_strain.c:43), beta in state[5],
 // gammap in state[9], gammadotp in state[10].
 template <int MATERIAL>
-__device__ __forceinline__ void plane_return_particle(const G2PArgs &A, int i, double vol, double exx,
-                                                      double exy, double eyy, double wxy)
+__device__ __forceinline__ void plane_return_particle(const G2PArgs &A, const G2PConst &C, int i, const Particle &p,
+                                                      double vol, double exx, double exy, double eyy, double wxy)
 {
     constexpr bool trial3d = MATERIAL != MPMG_G_LOCAL_MU2_TRUE_2D;
     constexpr bool mu_i = MATERIAL != MPMG_DP_RI_MT;
     constexpr bool beta = MATERIAL != MPMG_DP_RI_MT;
-    const mat::ReturnParams rp = {A.mu2.mu_s, A.mu2.mu_2, A.mu2.I0, A.mu2.grains_rho, A.mu2.grains_d,
-                                  A.mu2.rho_critical};
-    double sxx = A.sxx[i], sxy = A.sxy[i], syy = A.syy[i];
-    double szz = trial3d ? A.st1[i] : 0.0, b = beta ? A.st5[i] : 0.0;
-    double gp = A.st9[i], gdp;
-    mat::plane_return<trial3d, mu_i, beta>(A.el, rp, A.m[i], vol, exx, exy, eyy, wxy, sxx, sxy, syy, szz, b,
-                                           gp, gdp);
+    const mat::ReturnParams rp = {C.mu2.mu_s, C.mu2.mu_2, C.mu2.I0, C.mu2.grains_rho, C.mu2.grains_d,
+                                  C.mu2.rho_critical};
+    double sxx = p.sxx, sxy = p.sxy, syy = p.syy, szz = p.st1, b = p.st5, gp = p.st9, gdp;
+    mat::plane_return<trial3d, mu_i, beta>(C.el, rp, p.m, vol, exx, exy, eyy, wxy, sxx, sxy, syy, szz, b, gp, gdp);
     A.sxx[i] = sxx;
     A.sxy[i] = sxy;
     A.syy[i] = syy;
@@ -296,11 +615,11 @@ __device__ __forceinline__ void plane_return_particle(const G2PArgs &A, int i, d
 
 // g_local_mu2_reverse on particle i: beta in state[5], gammap in state[9],
 // gammadotp in state[10] (g_local_mu2_reverse.c:57-64).
-__device__ __forceinline__ void reverse_particle(const G2PArgs &A, int i, double vol, double exx, double exy,
-                                                 double eyy, double wxy)
+__device__ __forceinline__ void reverse_particle(const G2PArgs &A, const G2PConst &C, int i, const Particle &p,
+                                                 double vol, double exx, double exy, double eyy, double wxy)
 {
-    double sxx = A.sxx[i], sxy = A.sxy[i], syy = A.syy[i], b = A.st5[i], gp = A.st9[i], gdp = A.st10[i];
-    mat::g_local_mu2_reverse(A.el, A.mu2, A.m[i], vol, exx, exy, eyy, wxy, sxx, sxy, syy, b, gp, gdp);
+    double sxx = p.sxx, sxy = p.sxy, syy = p.syy, b = p.st5, gp = p.st9, gdp = p.st10;
+    mat::g_local_mu2_reverse(C.el, C.mu2, p.m, vol, exx, exy, eyy, wxy, sxx, sxy, syy, b, gp, gdp);
     A.sxx[i] = sxx;
     A.sxy[i] = sxy;
     A.syy[i] = syy;
@@ -309,51 +628,86 @@ __device__ __forceinline__ void reverse_particle(const G2PArgs &A, int i, double
     A.st10[i] = gdp;
 }
 
-template <int MATERIAL, int PHASE>
-__global__ void __launch_bounds__(256) g2p_kernel(G2PArgs A)
+__device__ __forceinline__ void isolin_particle(const G2PArgs &A, const G2PConst &C, int i, const Particle &p,
+                                                double exx, double exy, double eyy, double wxy)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= A.n || !A.active[i]) return;
-    const GridGeom &g = A.g;
-    const int e = A.in_element[i];
-    const int ci = e % g.Ex, cj = e / g.Ex;
-    const int n0 = cj * g.Nx + ci;
-    const int nd[4] = {n0, n0 + 1, n0 + 1 + g.Nx, n0 + g.Nx};
-    double xl, yl;
-    if (PHASE == G2P_STRAIN) {
-        // the start-of-step local coordinates the move phase kept
-        xl = A.xl_out[i];
-        yl = A.yl_out[i];
-    } else {
-        xl = mpmg_local_coord_fma(A.x[i], mat::small_int(ci), g.inv_h);
-        yl = mpmg_local_coord_fma(A.y[i], mat::small_int(cj), g.inv_h);
-    }
-    const ShapeFns f = shape(xl, yl, g.inv_h);
-    const double dt = A.dt;
+    double sxx = p.sxx, sxy = p.sxy, syy = p.syy;
+    mat::isolin(C.el, exx, exy, eyy, wxy, sxx, sxy, syy);
+    A.sxx[i] = sxx;
+    A.sxy[i] = sxy;
+    A.syy[i] = syy;
+}
 
-    double nvx[4], nvy[4];
-#pragma unroll
-    for (int a = 0; a < 4; a++) {
-        nvx[a] = A.node_vx[nd[a]];
-        nvy[a] = A.node_vy[nd[a]];
-    }
-    if (PHASE != G2P_STRAIN) {
-        // move_particles_explicit_usl_split (process_usl.c:914-957); light
-        // nodes (m <= 1e-10) carry zero acceleration and velocity.
-        double xtt = 0, ytt = 0, dux = 0, duy = 0;
+__device__ __forceinline__ void mu2_particle(const G2PArgs &A, const G2PConst &C, int i, const Particle &p, double vol,
+                                             double exx, double exy, double eyy, double wxy)
+{
+    double Txx = p.sxx, Txy = p.sxy, Tyy = p.syy, Tzz = p.Tzz, gp = p.st9, gdp;
+    mat::g_local_mu2(C.el, C.mu2, p.m, vol, exx, exy, eyy, wxy, Txx, Txy, Tyy, Tzz, gp, gdp);
+    A.sxx[i] = Txx;
+    A.sxy[i] = Txy;
+    A.syy[i] = Tyy;
+    A.Tzz[i] = Tzz;
+    A.st9[i] = gp;
+    A.st10[i] = gdp;
+}
+
+// A field on an element from its coefficients: value at (x, y), and h times
+// its gradient.
+struct Field {
+    double val, gx, gy;
+};
+__device__ __forceinline__ Field field_at(double2 c01, double2 c23, double x, double y)
+{
+    Field f;
+    f.gy = fma(x, c23.y, c23.x);
+    f.val = fma(y, f.gy, fma(x, c01.y, c01.x));
+    f.gx = fma(y, c23.y, c01.y);
+    return f;
+}
+
+// One particle inside the grid, element e at the step's start; p.x, p.y leave
+// as the moved position.
+template <int MATERIAL, int PHASE>
+__device__ __forceinline__ void g2p_particle(const G2PArgs &A, const G2PConst &C, int i, int e, Particle &p)
+{
+    const GridGeom &g = A.g;
+    const mat::Unit &u = C.el;
+    const int cj = e / g.Ex, ci = e - cj * g.Ex;
+    const double dt = C.el.dt, inv_h = C.inv_h;
+    Field vx, vy;
+    if (PHASE == G2P_STRAIN) {
+        // the nodal velocities of the second projection: h grad N is
+        // ((-oy, -ox), (oy, -x), (y, x), (-y, ox)), grouped by node differences
+        const int n0 = cj * g.Nx + ci;
+        const int nd[4] = {n0, n0 + 1, n0 + 1 + g.Nx, n0 + g.Nx};
+        double nvx[4], nvy[4];
 #pragma unroll
         for (int a = 0; a < 4; a++) {
-            xtt += f.s[a] * A.node_ax[nd[a]];
-            ytt += f.s[a] * A.node_ay[nd[a]];
-            dux += f.s[a] * nvx[a];
-            duy += f.s[a] * nvy[a];
+            nvx[a] = A.node_vx[nd[a]];
+            nvy[a] = A.node_vy[nd[a]];
         }
-        A.vx[i] = fma(dt, xtt, A.vx[i]);
-        A.vy[i] = fma(dt, ytt, A.vy[i]);
-        A.x[i] = fma(dt, dux, A.x[i]);
-        A.y[i] = fma(dt, duy, A.y[i]);
-        A.ux[i] = fma(dt, dux, A.ux[i]);
-        A.uy[i] = fma(dt, duy, A.uy[i]);
+        const double ox = u.sub(u.one, p.xl), oy = u.sub(u.one, p.yl);
+        vx.gx = fma(oy, u.sub(nvx[1], nvx[0]), u.mul(p.yl, u.sub(nvx[2], nvx[3])));
+        vy.gx = fma(oy, u.sub(nvy[1], nvy[0]), u.mul(p.yl, u.sub(nvy[2], nvy[3])));
+        vx.gy = fma(ox, u.sub(nvx[3], nvx[0]), u.mul(p.xl, u.sub(nvx[2], nvx[1])));
+        vy.gy = fma(ox, u.sub(nvy[3], nvy[0]), u.mul(p.xl, u.sub(nvy[2], nvy[1])));
+    } else {
+        const double xl = mpmg_local_coord_fma(p.x, mat::small_int(ci), inv_h);
+        const double yl = mpmg_local_coord_fma(p.y, mat::small_int(cj), inv_h);
+        const double2 *c = A.coef + (size_t)e * 8;
+        vx = field_at(c[4], c[5], xl, yl);
+        vy = field_at(c[6], c[7], xl, yl);
+        // move_particles_explicit_usl_split (process_usl.c:914-957); light
+        // nodes (m <= 1e-10) carry zero acceleration and velocity.
+        const double xtt = field_at(c[0], c[1], xl, yl).val, ytt = field_at(c[2], c[3], xl, yl).val;
+        p.x = fma(dt, vx.val, p.x);
+        p.y = fma(dt, vy.val, p.y);
+        A.vx[i] = fma(dt, xtt, p.vx);
+        A.vy[i] = fma(dt, ytt, p.vy);
+        A.x[i] = p.x;
+        A.y[i] = p.y;
+        A.ux[i] = fma(dt, vx.val, p.ux);
+        A.uy[i] = fma(dt, vy.val, p.uy);
         if (A.ax != nullptr) {
             A.ax[i] = xtt;
             A.ay[i] = ytt;
@@ -365,21 +719,12 @@ __global__ void __launch_bounds__(256) g2p_kernel(G2PArgs A)
         if (PHASE == G2P_MOVE) return;
     }
     // calculate_strainrate_split (process_usl.c:796-803): the sums of
-    // grad N_a v_a, with h grad N = ((-oy, -ox), (oy, -a), (b, a), (-b, ox))
-    // (a, b the local coordinates), grouped by node differences and scaled
-    // by 1 / h once (the same sums in fewer FP64 operations, the pipe that
-    // bounds this kernel)
-    const double ox = 1 - xl, oy = 1 - yl;
-    const double sxv = fma(oy, nvx[1] - nvx[0], yl * (nvx[2] - nvx[3]));   // h sum gx vx
-    const double syv = fma(oy, nvy[1] - nvy[0], yl * (nvy[2] - nvy[3]));   // h sum gx vy
-    const double txv = fma(ox, nvx[3] - nvx[0], xl * (nvx[2] - nvx[1]));   // h sum gy vx
-    const double tyv = fma(ox, nvy[3] - nvy[0], xl * (nvy[2] - nvy[1]));   // h sum gy vy
-    const double exx = sxv * g.inv_h, eyy = tyv * g.inv_h;
-    const double half_inv_h = 0.5 * g.inv_h;
-    const double exy = half_inv_h * (txv + syv);
-    const double wxy = half_inv_h * (txv - syv);
+    // grad N_a v_a, scaled by 1 / h once
+    const double exx = u.mul(vx.gx, inv_h), eyy = u.mul(vy.gy, inv_h);
+    const double exy = u.mul(C.half_inv_h, u.add(vx.gy, vy.gx));
+    const double wxy = u.mul(C.half_inv_h, u.sub(vx.gy, vy.gx));
     // update_particle_densities_split (process_usl.c:961-970)
-    double vol = A.v[i] * mat::exp_small(dt * (exx + eyy));
+    const double vol = u.mul(p.v, mat::exp_small(u.mul(dt, u.add(exx, eyy)), u.one, C.el.half, C.el.sixth));
     A.v[i] = vol;
     if (A.exx != nullptr) {
         A.exx[i] = exx;
@@ -389,37 +734,24 @@ __global__ void __launch_bounds__(256) g2p_kernel(G2PArgs A)
     }
 
     if (MATERIAL == MPMG_ISOLIN) {
-        double sxx = A.sxx[i], sxy = A.sxy[i], syy = A.syy[i];
-        mat::isolin(A.el, exx, exy, eyy, wxy, sxx, sxy, syy);
-        A.sxx[i] = sxx;
-        A.sxy[i] = sxy;
-        A.syy[i] = syy;
+        isolin_particle(A, C, i, p, exx, exy, eyy, wxy);
     } else if (MATERIAL == MPMG_G_LOCAL_MU2) {
-        double Txx = A.sxx[i], Txy = A.sxy[i], Tyy = A.syy[i], Tzz = A.Tzz[i];
-        double gp = A.st9[i], gdp;
-        mat::g_local_mu2(A.el, A.mu2, A.m[i], vol, exx, exy, eyy, wxy, Txx, Txy, Tyy, Tzz, gp, gdp);
-        A.sxx[i] = Txx;
-        A.sxy[i] = Txy;
-        A.syy[i] = Tyy;
-        A.Tzz[i] = Tzz;
-        A.st9[i] = gp;
-        A.st10[i] = gdp;
+        mu2_particle(A, C, i, p, vol, exx, exy, eyy, wxy);
     } else if (MATERIAL == MPMG_DP_RI_MT || MATERIAL == MPMG_G_LOCAL_MU2_PLANE_STRAIN ||
                MATERIAL == MPMG_G_LOCAL_MU2_TRUE_2D) {
-        plane_return_particle<MATERIAL>(A, i, vol, exx, exy, eyy, wxy);
+        plane_return_particle<MATERIAL>(A, C, i, p, vol, exx, exy, eyy, wxy);
     } else if (MATERIAL == MPMG_G_LOCAL_MU2_REVERSE) {
-        reverse_particle(A, i, vol, exx, exy, eyy, wxy);
+        reverse_particle(A, C, i, p, vol, exx, exy, eyy, wxy);
     } else if (MATERIAL == MPMG_G_LOCAL_MU2_EXT) {
         // first phase only; the stress waits for the nodal Laplacian
-        double mu_t = A.st0[i], gfl;
-        mat::ext_local_fluidity(A.mu2, A.sxx[i], A.syy[i], A.st10[i], mu_t, gfl);
+        double mu_t = p.st0, gfl;
+        mat::ext_local_fluidity(C.mu2, p.sxx, p.syy, p.st10, mu_t, gfl);
         A.st0[i] = mu_t;
         A.st4[i] = gfl;
     } else if (MATERIAL == MPMG_G_NONLOCAL_MU2) {
         double p_tr, t0xx, t0xy, t0yy, tau_tr, dense, gfl, xisq;
-        mat::nonlocal_mu2_trial(A.el, exx, exy, eyy, wxy, A.sxx[i], A.sxy[i], A.syy[i], p_tr, t0xx, t0xy,
-                                t0yy, tau_tr);
-        mat::nonlocal_mu2_bulk(A.el, A.mu2, A.m[i], vol, p_tr, tau_tr, dense, gfl, xisq);
+        mat::nonlocal_mu2_trial(C.el, exx, exy, eyy, wxy, p.sxx, p.sxy, p.syy, p_tr, t0xx, t0xy, t0yy, tau_tr);
+        mat::nonlocal_mu2_bulk(C.el, C.mu2, p.m, vol, p_tr, tau_tr, dense, gfl, xisq);
         A.st0[i] = dense;
         A.st5[i] = gfl;
         A.st6[i] = xisq;
@@ -434,20 +766,63 @@ __global__ void __launch_bounds__(256) g2p_kernel(G2PArgs A)
     // fluidity phase (g_nonlocal.c:306-352).
 }
 
+// Copies the constants to shared memory (the caller synchronises).
+__device__ __forceinline__ void stage_const(G2PConst &C, const G2PConst &param)
+{
+    static_assert(sizeof(G2PConst) % 8 == 0, "copied as 64-bit words");
+    const unsigned long long *src = reinterpret_cast<const unsigned long long *>(&param);
+    unsigned long long *dst = reinterpret_cast<unsigned long long *>(&C);
+    for (int k = threadIdx.x; k < (int)(sizeof(G2PConst) / 8); k += blockDim.x) dst[k] = src[k];
+}
+
+// The block's size is the launch's (g2p_threads).  Every thread stays to the
+// end: the binning is a warp's work.
+template <int MATERIAL, int PHASE>
+__global__ void __launch_bounds__(128) g2p_kernel(const __grid_constant__ G2PArgs A)
+{
+    __shared__ G2PConst C;
+    stage_const(C, A.k);
+    const GridGeom &g = A.g;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t key = i < A.n ? A.keys[i] : A.sentinel;
+    Particle p;
+    if (key != A.sentinel) p = load_particle<MATERIAL, PHASE>(A, i);
+    __syncthreads();
+    mpmg_pdl_wait();
+    mpmg_pdl_trigger();
+    uint32_t next = A.sentinel;
+    if (key != A.sentinel) {
+        if (PHASE != G2P_STRAIN) A.in_element[i] = (int)key;
+        g2p_particle<MATERIAL, PHASE>(A, C, i, (int)key, p);
+        if (PHASE != G2P_MOVE) {
+            const int e = mpmg_which_element_fast(p.x, p.y, g.h, g.inv_h, A.inv_hf, g.xmax, g.ymax,
+                                                  __double_as_longlong(g.xmax), __double_as_longlong(g.ymax), g.Ex,
+                                                  g.Ey);
+            if (e >= 0) next = (uint32_t)e;
+            A.keys[i] = next;
+        }
+    } else if (PHASE != G2P_STRAIN && i < A.n && A.active[i]) {
+        A.active[i] = 0;       // process_usl.c:660-666: outside the grid for good
+        A.in_element[i] = -1;
+    }
+    if (PHASE != G2P_MOVE) bin_particle(A.next, i, next, next != A.sentinel);
+}
+
 // g_local_mu2_ext's second phase (g_local_mu2_ext.c:232-265): per element,
 // each particle's -v gflocal |grad N_j|^2 summed per corner in the binned
 // order of the step, with the start-of-step shape-function gradients.
 __global__ void __launch_bounds__(128) ext_cells_kernel(
-    int ne, double inv_h, const int *__restrict__ cell_start, const uint32_t *__restrict__ perm,
+    int ne, double inv_h, RowView rv,
     const double *__restrict__ xl, const double *__restrict__ yl, const double *__restrict__ v,
     const double *__restrict__ gflocal, double *__restrict__ cell_sums)
 {
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= ne) return;
-    const int k0 = cell_start[e], k1 = cell_start[e + 1];
+    const int cnt = (int)rv.count[e];
+    const uint32_t *list = rv.list(e, cnt);
     double acc[4] = {0, 0, 0, 0};
-    for (int k = k0; k < k1; k++) {
-        const int i = (int)perm[k];
+    for (int k = 0; k < cnt; k++) {
+        const int i = (int)list[k];
         const ShapeFns f = shape(xl[i], yl[i], inv_h);
         const double q = mat::mul(-v[i], gflocal[i]);
 #pragma unroll
@@ -483,8 +858,10 @@ __global__ void __launch_bounds__(256) ext_nodes_kernel(GridGeom g, int ne, cons
 
 // g_local_mu2_ext's gf and gammadotp correction (g_local_mu2_ext.c:268-290)
 // and the stress (mat::ext_stress).
-__global__ void __launch_bounds__(256) ext_stress_kernel(G2PArgs A, const double *__restrict__ d2)
+__global__ void __launch_bounds__(256) ext_stress_kernel(const __grid_constant__ G2PArgs A,
+                                                         const double *__restrict__ d2)
 {
+    const G2PConst &C = A.k;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= A.n || !A.active[i]) return;
     const GridGeom &g = A.g;
@@ -496,13 +873,13 @@ __global__ void __launch_bounds__(256) ext_stress_kernel(G2PArgs A, const double
 #pragma unroll
     for (int a = 0; a < 4; a++) gf = mat::add(gf, mat::mul(0.25, d2[nd[a]]));
     double mu_t = A.st0[i], gdp = A.st10[i];
-    const double Ad = A.mu2.A, d = A.mu2.grains_d;
+    const double Ad = C.mu2.A, d = C.mu2.grains_d;
     gf = mat::mul(mat::mul(mat::mul(mat::mul(mat::mul(Ad, Ad), d), d), mu_t), gf);
-    if (mu_t > A.mu2.mu_s) gdp = mat::sub(gdp, mat::quot(gf, fabs(mat::sub(mu_t, A.mu2.mu_s))));
+    if (mu_t > C.mu2.mu_s) gdp = mat::sub(gdp, mat::quot(gf, fabs(mat::sub(mu_t, C.mu2.mu_s))));
     if (gdp < 0) gdp = 0;
     A.st3[i] = gf;
     double sxx = A.sxx[i], sxy = A.sxy[i], syy = A.syy[i], beta = A.st5[i], gp = A.st9[i];
-    mat::ext_stress(A.el, A.mu2, A.nl.E, A.nl.nu, A.m[i], A.v[i], A.exx[i], A.exy[i], A.eyy[i], A.wxy[i], sxx, sxy,
+    mat::ext_stress(C.el, C.mu2, A.nl.E, A.nl.nu, A.m[i], A.v[i], A.exx[i], A.exy[i], A.eyy[i], A.wxy[i], sxx, sxy,
                     syy, mu_t, beta, gp, gdp);
     A.sxx[i] = sxx;
     A.sxy[i] = sxy;
@@ -515,34 +892,42 @@ __global__ void __launch_bounds__(256) ext_stress_kernel(G2PArgs A, const double
 
 // MUSL's second projection (process_usl.c:424-431): per element, the moved
 // particles' mass and momentum with their start-of-step shape functions, in
-// the binned order of the step (perm is already ordered by the P2G).
+// the step's particle order, from the same moments as the P2G.
 __global__ void __launch_bounds__(128) p2g_momentum_kernel(
-    int ne, double inv_h, const int *__restrict__ cell_start, const uint32_t *__restrict__ perm,
-    const double *__restrict__ xl, const double *__restrict__ yl, const double *__restrict__ m,
+    int ne, RowView rv, const double *__restrict__ xl, const double *__restrict__ yl, const double *__restrict__ m,
     const double *__restrict__ vx, const double *__restrict__ vy, double *__restrict__ cell_sums)
 {
+    mpmg_pdl_wait();
+    mpmg_pdl_trigger();
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= ne) return;
-    const int k0 = cell_start[e], k1 = cell_start[e + 1];
-    if (k0 == k1) return;
-    double acc[4][3];
+    const int cnt = (int)rv.count[e];
+    if (cnt == 0) return;
+    const uint32_t *list = rv.list(e, cnt);
+    double q[3][4];
 #pragma unroll
-    for (int a = 0; a < 4; a++) acc[a][0] = acc[a][1] = acc[a][2] = 0.0;
-    for (int k = k0; k < k1; k++) {
-        const int i = (int)perm[k];
-        const ShapeFns f = shape(xl[i], yl[i], inv_h);
-        const double pm = m[i], pmx = vx[i] * pm, pmy = vy[i] * pm;
+    for (int f = 0; f < 3; f++)
 #pragma unroll
-        for (int a = 0; a < 4; a++) {
-            acc[a][0] += f.s[a] * pm;
-            acc[a][1] += f.s[a] * pmx;
-            acc[a][2] += f.s[a] * pmy;
+        for (int a = 0; a < 4; a++) q[f][a] = 0.0;
+    for (int k = 0; k < cnt; k++) {
+        const int i = (int)list[k];
+        const double a = xl[i], b = yl[i], ab = a * b;
+        const double pm = m[i], p[3] = {pm, vx[i] * pm, vy[i] * pm};
+#pragma unroll
+        for (int f = 0; f < 3; f++) {
+            q[f][0] += p[f];
+            q[f][1] = fma(a, p[f], q[f][1]);
+            q[f][2] = fma(b, p[f], q[f][2]);
+            q[f][3] = fma(ab, p[f], q[f][3]);
         }
     }
 #pragma unroll
-    for (int a = 0; a < 4; a++)
-#pragma unroll
-        for (int q = 0; q < 3; q++) cell_sums[(size_t)(a * 3 + q) * ne + e] = acc[a][q];
+    for (int f = 0; f < 3; f++) {
+        cell_sums[(size_t)(0 * 3 + f) * ne + e] = (q[f][0] - q[f][1]) - (q[f][2] - q[f][3]);
+        cell_sums[(size_t)(1 * 3 + f) * ne + e] = q[f][1] - q[f][3];
+        cell_sums[(size_t)(2 * 3 + f) * ne + e] = q[f][3];
+        cell_sums[(size_t)(3 * 3 + f) * ne + e] = q[f][2] - q[f][3];
+    }
 }
 
 // MUSL nodal velocities of the second projection (process_usl.c:433-447):
@@ -550,10 +935,12 @@ __global__ void __launch_bounds__(128) p2g_momentum_kernel(
 // momenta only after forming v, so the boundary conditions do not reach v;
 // the zeroed momenta are what it keeps in the nodes (node_mx, node_my).
 __global__ void __launch_bounds__(256) node_velocity_kernel(
-    GridGeom g, BcParams bc, int ne, const int *__restrict__ cell_start, const double *__restrict__ cell_sums,
+    GridGeom g, BcParams bc, int ne, const uint32_t *__restrict__ count, const double *__restrict__ cell_sums,
     const StepParams *__restrict__ sp, double *__restrict__ node_m, double *__restrict__ node_vx,
     double *__restrict__ node_vy, double *__restrict__ node_mx, double *__restrict__ node_my)
 {
+    mpmg_pdl_wait();
+    mpmg_pdl_trigger();
     const int nn = g.Nx * g.Ny;
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= nn) return;
@@ -565,7 +952,7 @@ __global__ void __launch_bounds__(256) node_velocity_kernel(
         const int cj = ((j & 1) == (c >> 1)) ? j : j - 1;
         if (ci < 0 || cj < 0 || ci >= g.Ex || cj >= g.Ey) continue;
         const int e = cj * g.Ex + ci;
-        if (cell_start[e] == cell_start[e + 1]) continue;
+        if (count[e] == 0) continue;
         const int corner = (ci == i) ? ((cj == j) ? 0 : 3) : ((cj == j) ? 1 : 2);
 #pragma unroll
         for (int q = 0; q < 3; q++) sum[q] += cell_sums[(size_t)(corner * 3 + q) * ne + e];
@@ -573,8 +960,8 @@ __global__ void __launch_bounds__(256) node_velocity_kernel(
     const double m = sum[0];
     double vxn = 0, vyn = 0;
     if (m > MPMG_TOL) {
-        vxn = sum[1] / m;
-        vyn = sum[2] / m;
+        vxn = mat::quot(sum[1], m);
+        vyn = mat::quot(sum[2], m);
     }
     node_m[n] = m;
     node_vx[n] = vxn;
@@ -587,36 +974,59 @@ __global__ void __launch_bounds__(256) node_velocity_kernel(
     }
 }
 
-__global__ void material_only_kernel(G2PArgs A, int material)
+__global__ void material_only_kernel(const __grid_constant__ G2PArgs A, int material)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= A.n || !A.active[i]) return;
-    double exx = A.exx[i], exy = A.exy[i], eyy = A.eyy[i], wxy = A.wxy[i];
+    const G2PConst &C = A.k;
+    const double exx = A.exx[i], exy = A.exy[i], eyy = A.eyy[i], wxy = A.wxy[i], vol = A.v[i];
     if (material == MPMG_ISOLIN) {
-        double sxx = A.sxx[i], sxy = A.sxy[i], syy = A.syy[i];
-        mat::isolin(A.el, exx, exy, eyy, wxy, sxx, sxy, syy);
-        A.sxx[i] = sxx;
-        A.sxy[i] = sxy;
-        A.syy[i] = syy;
+        isolin_particle(A, C, i, load_particle<MPMG_ISOLIN, G2P_FULL>(A, i), exx, exy, eyy, wxy);
     } else if (material == MPMG_DP_RI_MT) {
-        plane_return_particle<MPMG_DP_RI_MT>(A, i, A.v[i], exx, exy, eyy, wxy);
+        plane_return_particle<MPMG_DP_RI_MT>(A, C, i, load_particle<MPMG_DP_RI_MT, G2P_FULL>(A, i), vol, exx, exy,
+                                             eyy, wxy);
     } else if (material == MPMG_G_LOCAL_MU2_PLANE_STRAIN) {
-        plane_return_particle<MPMG_G_LOCAL_MU2_PLANE_STRAIN>(A, i, A.v[i], exx, exy, eyy, wxy);
+        plane_return_particle<MPMG_G_LOCAL_MU2_PLANE_STRAIN>(
+            A, C, i, load_particle<MPMG_G_LOCAL_MU2_PLANE_STRAIN, G2P_FULL>(A, i), vol, exx, exy, eyy, wxy);
     } else if (material == MPMG_G_LOCAL_MU2_TRUE_2D) {
-        plane_return_particle<MPMG_G_LOCAL_MU2_TRUE_2D>(A, i, A.v[i], exx, exy, eyy, wxy);
+        plane_return_particle<MPMG_G_LOCAL_MU2_TRUE_2D>(
+            A, C, i, load_particle<MPMG_G_LOCAL_MU2_TRUE_2D, G2P_FULL>(A, i), vol, exx, exy, eyy, wxy);
     } else if (material == MPMG_G_LOCAL_MU2_REVERSE) {
-        reverse_particle(A, i, A.v[i], exx, exy, eyy, wxy);
+        reverse_particle(A, C, i, load_particle<MPMG_G_LOCAL_MU2_REVERSE, G2P_FULL>(A, i), vol, exx, exy, eyy, wxy);
     } else {
-        double Txx = A.sxx[i], Txy = A.sxy[i], Tyy = A.syy[i], Tzz = A.Tzz[i];
-        double gp = A.st9[i], gdp;
-        mat::g_local_mu2(A.el, A.mu2, A.m[i], A.v[i], exx, exy, eyy, wxy, Txx, Txy, Tyy, Tzz, gp, gdp);
-        A.sxx[i] = Txx;
-        A.sxy[i] = Txy;
-        A.syy[i] = Tyy;
-        A.Tzz[i] = Tzz;
-        A.st9[i] = gp;
-        A.st10[i] = gdp;
+        mu2_particle(A, C, i, load_particle<MPMG_G_LOCAL_MU2, G2P_FULL>(A, i), vol, exx, exy, eyy, wxy);
     }
+}
+
+// The key each particle's last element map gives (mpmg_fp64_sort).
+__global__ void __launch_bounds__(256) map_keys_kernel(int n, const int *__restrict__ in_element,
+                                                       const int *__restrict__ active, uint32_t sentinel,
+                                                       uint32_t *__restrict__ keys)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) keys[i] = active[i] ? (uint32_t)in_element[i] : sentinel;
+}
+
+__global__ void __launch_bounds__(128) order_kernel(int ne, const int *__restrict__ cell_start,
+                                                    const uint32_t *__restrict__ slots, uint32_t *__restrict__ perm)
+{
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e < ne) mpmg_order_segment(slots, perm, nullptr, cell_start[e], cell_start[e + 1]);
+}
+
+// Up to this many particles the P2G gives an element two threads.
+constexpr size_t kP2GSplitMax = 100000;
+
+RowsOut rows_out(const mpmg_ctx *ctx, int b)
+{
+    const RowBins &r = ctx->row;
+    return RowsOut{r.count[b], r.rows[b], r.over_n + b, r.over[b], r.cap};
+}
+
+RowView row_view(const mpmg_ctx *ctx)
+{
+    const RowBins &r = ctx->row;
+    return RowView{r.count[r.cur], r.rows[r.cur], r.over_list, r.cap};
 }
 
 G2PArgs make_g2p_args(mpmg_ctx *ctx)
@@ -625,31 +1035,24 @@ G2PArgs make_g2p_args(mpmg_ctx *ctx)
     const mpmg_config &c = ctx->cfg;
     A.g = make_geom(ctx);
     A.n = (int)ctx->np;
-    A.dt = c.dt;
-    A.el.G = ctx->G;
-    A.el.twoG = 2.0 * ctx->G;
-    A.el.K = ctx->K;
-    A.el.lambda = ctx->lambda;
-    A.el.dt = c.dt;
-    A.el.Gdt = ctx->G * c.dt;
-    A.el.kG = mat::make_known(ctx->G);
-    A.el.kdt = mat::make_known(c.dt);
-    A.el.kGdt = mat::make_known(A.el.Gdt);
-    A.mu2.mu_s = c.mp[MPMG_MP_MU_S];
-    A.mu2.mu_2 = c.mp[MPMG_MP_MU_2];
-    A.mu2.I0 = c.mp[MPMG_MP_I0];
-    A.mu2.grains_rho = c.mp[MPMG_MP_GRAINS_RHO];
-    A.mu2.grains_d = c.mp[MPMG_MP_GRAINS_D];
-    A.mu2.rho_critical = c.mp[MPMG_MP_RHO_CRITICAL];
-    A.mu2.A = c.mp[MPMG_MP_A];
-    A.mu2.krho = mat::make_known(A.mu2.grains_rho);
-    A.mu2.kd = mat::make_known(A.mu2.grains_d);
-    const bool bracket = A.mu2.rho_critical >= 0x1p-60 && A.mu2.rho_critical <= 0x1p60;
-    A.mu2.rho_lo = bracket ? A.mu2.rho_critical * (1.0 - 0x1p-47) : -1.0;
-    A.mu2.rho_hi = bracket ? A.mu2.rho_critical * (1.0 + 0x1p-47) : (double)INFINITY;
-    A.mu2.kAAdd = mat::make_known(((A.mu2.A * A.mu2.A) * A.mu2.grains_d) * A.mu2.grains_d);
-    A.mu2.alpha_c = (((ctx->G * A.mu2.I0) * c.dt) / A.mu2.grains_d) / sqrt(A.mu2.grains_rho);
-    A.mu2.GI0dt = (ctx->G * A.mu2.I0) * c.dt;
+    A.k.el = mat::make_elastic(ctx->G, ctx->K, ctx->lambda, c.dt);
+    A.k.inv_h = ctx->inv_h;
+    A.k.half_inv_h = 0.5 * ctx->inv_h;
+    A.k.mu2.mu_s = c.mp[MPMG_MP_MU_S];
+    A.k.mu2.mu_2 = c.mp[MPMG_MP_MU_2];
+    A.k.mu2.I0 = c.mp[MPMG_MP_I0];
+    A.k.mu2.grains_rho = c.mp[MPMG_MP_GRAINS_RHO];
+    A.k.mu2.grains_d = c.mp[MPMG_MP_GRAINS_D];
+    A.k.mu2.rho_critical = c.mp[MPMG_MP_RHO_CRITICAL];
+    A.k.mu2.A = c.mp[MPMG_MP_A];
+    A.k.mu2.krho = mat::make_known(A.k.mu2.grains_rho);
+    A.k.mu2.kd = mat::make_known(A.k.mu2.grains_d);
+    const bool bracket = A.k.mu2.rho_critical >= 0x1p-60 && A.k.mu2.rho_critical <= 0x1p60;
+    A.k.mu2.rho_lo = bracket ? A.k.mu2.rho_critical * (1.0 - 0x1p-47) : -1.0;
+    A.k.mu2.rho_hi = bracket ? A.k.mu2.rho_critical * (1.0 + 0x1p-47) : (double)INFINITY;
+    A.k.mu2.kAAdd = mat::make_known(((A.k.mu2.A * A.k.mu2.A) * A.k.mu2.grains_d) * A.k.mu2.grains_d);
+    A.k.mu2.alpha_c = (((ctx->G * A.k.mu2.I0) * c.dt) / A.k.mu2.grains_d) / sqrt(A.k.mu2.grains_rho);
+    A.k.mu2.GI0dt = (ctx->G * A.k.mu2.I0) * c.dt;
     A.nl.E = c.mp[MPMG_MP_E];
     A.nl.nu = c.mp[MPMG_MP_NU];
     A.nl.mu_s = c.mp[MPMG_MP_MU_S];
@@ -658,10 +1061,13 @@ G2PArgs make_g2p_args(mpmg_ctx *ctx)
     A.nl.A = c.mp[MPMG_MP_A];
     A.nl.grains_d = c.mp[MPMG_MP_GRAINS_D];
     A.nl.cohesion = c.mp[MPMG_MP_COHESION];
+    A.keys = ctx->keys;
+    A.sentinel = (uint32_t)ctx->ne;
+    A.inv_hf = (float)ctx->inv_h;
+    A.next = rows_out(ctx, 1 - ctx->row.cur);
     A.in_element = ctx->in_element;
     A.active = ctx->active;
-    A.node_ax = ctx->node_ax;
-    A.node_ay = ctx->node_ay;
+    A.coef = (const double2 *)ctx->elem_coef;
     A.node_vx = ctx->node_vx;
     A.node_vy = ctx->node_vy;
     A.x = ctx->x; A.y = ctx->y; A.vx = ctx->vx; A.vy = ctx->vy; A.ux = ctx->ux; A.uy = ctx->uy;
@@ -684,6 +1090,73 @@ inline int blocks_for(size_t n, int threads)
 
 }  // namespace
 
+// Threads of a G2P block: one warp where every warp can have a sub-partition
+// to itself or nearly so (a 256-thread block would leave most SMs idle), 128
+// beyond that.
+static int g2p_threads(const mpmg_ctx *ctx)
+{
+    return ctx->np <= (size_t)ctx->sms * 4 * 32 * 2 ? 32 : 128;
+}
+
+template <int MATERIAL, int PHASE>
+static cudaError_t launch_g2p(mpmg_ctx *ctx, const G2PArgs &A)
+{
+    const int t = g2p_threads(ctx);
+    ctx->launches += 1;
+    return mpmg_launch_pdl(true, g2p_kernel<MATERIAL, PHASE>, dim3(blocks_for(ctx->np, t)), dim3(t), 0, ctx->stream, A);
+}
+
+template <int EB, int SPLIT>
+static cudaError_t launch_p2g(mpmg_ctx *ctx, const GridGeom &g, bool keep_order)
+{
+    const mpmg_config &c = ctx->cfg;
+    RowBins &r = ctx->row;
+    const int ne = (int)ctx->ne;
+    ctx->launches += 1;
+    return mpmg_launch_pdl(true, p2g_cells_kernel<EB, SPLIT>, dim3(blocks_for(ne, EB)), dim3(EB * SPLIT),
+                           p2g_smem_bytes<EB>(), ctx->stream, g, ne, (int)ctx->np, row_view(ctx), r.count[1 - r.cur],
+                           (const uint32_t *)(r.over_n + r.cur), r.over_n + (1 - r.cur), (const uint2 *)r.over[r.cur],
+                           r.over_n + 2, keep_order ? 1 : 0, (const double *)ctx->x, (const double *)ctx->y,
+                           (const double *)ctx->m, (const double *)ctx->vx, (const double *)ctx->vy,
+                           (const double *)ctx->v, (const double *)ctx->sxx, (const double *)ctx->sxy,
+                           (const double *)ctx->syy, ctx->d_params, c.dt, c.gravity_mode, c.gravity, ctx->cell_sums);
+}
+
+int mpmg_fp64_ready(mpmg_ctx *ctx)
+{
+    RowBins &r = ctx->row;
+    if (r.ready) return MPMG_OK;
+    cudaStream_t s = ctx->stream;
+    const int n = (int)ctx->np;
+    MPMG_CHECK(cudaMemsetAsync(r.count[r.cur], 0, ctx->ne * sizeof(uint32_t), s));
+    MPMG_CHECK(cudaMemsetAsync(r.over_n, 0, 3 * sizeof(uint32_t), s));
+    keys_kernel<<<blocks_for(n, 256), 256, 0, s>>>(make_geom(ctx), (float)ctx->inv_h, n, ctx->x, ctx->y, ctx->active,
+                                                   ctx->keys, (uint32_t)ctx->ne, rows_out(ctx, r.cur));
+    ctx->launches += 1;
+    MPMG_CHECK(cudaGetLastError());
+    r.ready = true;
+    return MPMG_OK;
+}
+
+int mpmg_fp64_sort(mpmg_ctx *ctx)
+{
+    const int n = (int)ctx->np, ne = (int)ctx->ne;
+    cudaStream_t s = ctx->stream;
+    if (ctx->bin.counts == nullptr) {
+        int rc = mpmg_bin_init(ctx);
+        if (rc != MPMG_OK) return rc;
+        MPMG_CHECK(cudaMalloc(&ctx->sort_keys, (ctx->np ? ctx->np : 1) * sizeof(uint32_t)));
+    }
+    map_keys_kernel<<<blocks_for(n, 256), 256, 0, s>>>(n, ctx->in_element, ctx->active, (uint32_t)ne, ctx->sort_keys);
+    int rc = mpmg_bin_count(ctx, ctx->sort_keys);
+    if (rc == MPMG_OK) rc = mpmg_bin_scan_scatter(ctx, ctx->sort_keys, ctx->sorted_keys);
+    if (rc != MPMG_OK) return rc;
+    order_kernel<<<blocks_for(ne, 128), 128, 0, s>>>(ne, ctx->cell_start, ctx->bin.slots, ctx->perm);
+    ctx->launches += 2;
+    MPMG_CHECK(cudaGetLastError());
+    return MPMG_OK;
+}
+
 int mpmg_launch_step(mpmg_ctx *ctx)
 {
     cudaStream_t s = ctx->stream;
@@ -692,108 +1165,80 @@ int mpmg_launch_step(mpmg_ctx *ctx)
     const int n = (int)ctx->np;
     const int ne = (int)ctx->ne;
     const int nn = (int)ctx->nn;
-
-    mpmg_phase_begin(ctx, PH_KEYS);
-    keys_kernel<<<blocks_for(n, 256), 256, 0, s>>>(g, (float)ctx->inv_h, n, ctx->x, ctx->y, ctx->in_element,
-                                                   ctx->active,
-                                                   ctx->keys, (uint32_t)ne, ctx->bin.counts, ctx->d_params,
-                                                   c.dt, c.gravity_mode, c.gravity);
-    ctx->launches += 1;
-    mpmg_phase_end(ctx, PH_KEYS);
-
-    mpmg_phase_begin(ctx, PH_SORT);
-    int rc = mpmg_bin_scan_scatter(ctx, ctx->keys, ctx->sorted_keys);
-    if (rc != MPMG_OK) return rc;
-    mpmg_phase_end(ctx, PH_SORT);
+    const bool nonlocal = c.material == MPMG_G_NONLOCAL_MU2 || c.material == MPMG_G_NONLOCAL ||
+                          c.material == MPMG_G_NONLOCAL_AVG;
+    const bool musl = c.scheme == MPMG_SCHEME_MUSL;
 
     mpmg_phase_begin(ctx, PH_P2G);
-    p2g_cells_kernel<<<blocks_for(ne, 128), 128, 0, s>>>(
-        g, ne, ctx->cell_start, ctx->bin.slots, ctx->perm, ctx->x, ctx->y, ctx->m, ctx->vx, ctx->vy, ctx->v, ctx->sxx,
-        ctx->sxy, ctx->syy, ctx->d_params, ctx->cell_sums);
-    ctx->launches += 1;
+    // later phases of these read the ordered rows
+    const bool keep_order = nonlocal || musl || c.material == MPMG_G_LOCAL_MU2_EXT;
+    MPMG_CHECK((ctx->np <= kP2GSplitMax ? launch_p2g<64, 2>(ctx, g, keep_order)
+                                        : launch_p2g<128, 1>(ctx, g, keep_order)));
     mpmg_phase_end(ctx, PH_P2G);
 
     mpmg_phase_begin(ctx, PH_GRID);
-    grid_kernel<<<blocks_for(nn, 256), 256, 0, s>>>(
-        g, make_bc(ctx), ne, ctx->cell_start, ctx->cell_sums, ctx->d_params, c.dt, ctx->node_m,
-        ctx->node_ax, ctx->node_ay, ctx->node_vx, ctx->node_vy, ctx->node_mx, ctx->node_my,
-        ctx->node_fx, ctx->node_fy);
+    // a tall tile for every SM, or flat ones
+    MPMG_CHECK(ctx->nn >= (size_t)ctx->sms * 31 * 15 ? launch_grid<16>(ctx, g) : launch_grid<4>(ctx, g));
     ctx->launches += 1;
     mpmg_phase_end(ctx, PH_GRID);
 
     mpmg_phase_begin(ctx, PH_G2P);
     G2PArgs A = make_g2p_args(ctx);
-    if (c.scheme == MPMG_SCHEME_MUSL) {
+    if (musl) {
         // move, second projection of the moved momentum, then strain
         // the move phase does not depend on the material
-        g2p_kernel<MPMG_ISOLIN, G2P_MOVE><<<blocks_for(n, 256), 256, 0, s>>>(A);
-        p2g_momentum_kernel<<<blocks_for(ne, 128), 128, 0, s>>>(ne, ctx->inv_h, ctx->cell_start, ctx->perm, ctx->xl,
-                                                                ctx->yl, ctx->m, ctx->vx, ctx->vy, ctx->cell_sums);
-        node_velocity_kernel<<<blocks_for(nn, 256), 256, 0, s>>>(g, make_bc(ctx), ne, ctx->cell_start,
-                                                                 ctx->cell_sums, ctx->d_params, ctx->node_m,
-                                                                 ctx->node_vx, ctx->node_vy, ctx->node_mx,
-                                                                 ctx->node_my);
+        MPMG_CHECK((launch_g2p<MPMG_ISOLIN, G2P_MOVE>(ctx, A)));
+        MPMG_CHECK(mpmg_launch_pdl(true, p2g_momentum_kernel, dim3(blocks_for(ne, 128)), dim3(128), 0, s, ne,
+                                   row_view(ctx), (const double *)ctx->xl, (const double *)ctx->yl,
+                                   (const double *)ctx->m, (const double *)ctx->vx, (const double *)ctx->vy,
+                                   ctx->cell_sums));
+        MPMG_CHECK(mpmg_launch_pdl(true, node_velocity_kernel, dim3(blocks_for(nn, 256)), dim3(256), 0, s, g,
+                                   make_bc(ctx), ne, (const uint32_t *)ctx->row.count[ctx->row.cur],
+                                   (const double *)ctx->cell_sums, (const StepParams *)ctx->d_params, ctx->node_m,
+                                   ctx->node_vx, ctx->node_vy, ctx->node_mx, ctx->node_my));
+        ctx->launches += 2;
         switch (c.material) {
-        case MPMG_ISOLIN: g2p_kernel<MPMG_ISOLIN, G2P_STRAIN><<<blocks_for(n, 256), 256, 0, s>>>(A); break;
-        case MPMG_DP_RI_MT: g2p_kernel<MPMG_DP_RI_MT, G2P_STRAIN><<<blocks_for(n, 256), 256, 0, s>>>(A); break;
+        case MPMG_ISOLIN: MPMG_CHECK((launch_g2p<MPMG_ISOLIN, G2P_STRAIN>(ctx, A))); break;
+        case MPMG_DP_RI_MT: MPMG_CHECK((launch_g2p<MPMG_DP_RI_MT, G2P_STRAIN>(ctx, A))); break;
         case MPMG_G_LOCAL_MU2_PLANE_STRAIN:
-            g2p_kernel<MPMG_G_LOCAL_MU2_PLANE_STRAIN, G2P_STRAIN><<<blocks_for(n, 256), 256, 0, s>>>(A);
+            MPMG_CHECK((launch_g2p<MPMG_G_LOCAL_MU2_PLANE_STRAIN, G2P_STRAIN>(ctx, A)));
             break;
-        case MPMG_G_LOCAL_MU2_TRUE_2D:
-            g2p_kernel<MPMG_G_LOCAL_MU2_TRUE_2D, G2P_STRAIN><<<blocks_for(n, 256), 256, 0, s>>>(A);
-            break;
-        case MPMG_G_LOCAL_MU2_REVERSE:
-            g2p_kernel<MPMG_G_LOCAL_MU2_REVERSE, G2P_STRAIN><<<blocks_for(n, 256), 256, 0, s>>>(A);
-            break;
-        default: g2p_kernel<MPMG_G_LOCAL_MU2, G2P_STRAIN><<<blocks_for(n, 256), 256, 0, s>>>(A); break;
+        case MPMG_G_LOCAL_MU2_TRUE_2D: MPMG_CHECK((launch_g2p<MPMG_G_LOCAL_MU2_TRUE_2D, G2P_STRAIN>(ctx, A))); break;
+        case MPMG_G_LOCAL_MU2_REVERSE: MPMG_CHECK((launch_g2p<MPMG_G_LOCAL_MU2_REVERSE, G2P_STRAIN>(ctx, A))); break;
+        default: MPMG_CHECK((launch_g2p<MPMG_G_LOCAL_MU2, G2P_STRAIN>(ctx, A))); break;
         }
-        ctx->launches += 4;
     } else {
         switch (c.material) {
-        case MPMG_ISOLIN:
-            g2p_kernel<MPMG_ISOLIN, G2P_FULL><<<blocks_for(n, 256), 256, 0, s>>>(A);
-            break;
-        case MPMG_G_LOCAL_MU2:
-            g2p_kernel<MPMG_G_LOCAL_MU2, G2P_FULL><<<blocks_for(n, 256), 256, 0, s>>>(A);
-            break;
-        case MPMG_DP_RI_MT:
-            g2p_kernel<MPMG_DP_RI_MT, G2P_FULL><<<blocks_for(n, 256), 256, 0, s>>>(A);
-            break;
+        case MPMG_ISOLIN: MPMG_CHECK((launch_g2p<MPMG_ISOLIN, G2P_FULL>(ctx, A))); break;
+        case MPMG_G_LOCAL_MU2: MPMG_CHECK((launch_g2p<MPMG_G_LOCAL_MU2, G2P_FULL>(ctx, A))); break;
+        case MPMG_DP_RI_MT: MPMG_CHECK((launch_g2p<MPMG_DP_RI_MT, G2P_FULL>(ctx, A))); break;
         case MPMG_G_LOCAL_MU2_PLANE_STRAIN:
-            g2p_kernel<MPMG_G_LOCAL_MU2_PLANE_STRAIN, G2P_FULL><<<blocks_for(n, 256), 256, 0, s>>>(A);
+            MPMG_CHECK((launch_g2p<MPMG_G_LOCAL_MU2_PLANE_STRAIN, G2P_FULL>(ctx, A)));
             break;
-        case MPMG_G_LOCAL_MU2_TRUE_2D:
-            g2p_kernel<MPMG_G_LOCAL_MU2_TRUE_2D, G2P_FULL><<<blocks_for(n, 256), 256, 0, s>>>(A);
-            break;
-        case MPMG_G_LOCAL_MU2_REVERSE:
-            g2p_kernel<MPMG_G_LOCAL_MU2_REVERSE, G2P_FULL><<<blocks_for(n, 256), 256, 0, s>>>(A);
-            break;
+        case MPMG_G_LOCAL_MU2_TRUE_2D: MPMG_CHECK((launch_g2p<MPMG_G_LOCAL_MU2_TRUE_2D, G2P_FULL>(ctx, A))); break;
+        case MPMG_G_LOCAL_MU2_REVERSE: MPMG_CHECK((launch_g2p<MPMG_G_LOCAL_MU2_REVERSE, G2P_FULL>(ctx, A))); break;
         case MPMG_G_LOCAL_MU2_EXT:
-            g2p_kernel<MPMG_G_LOCAL_MU2_EXT, G2P_FULL><<<blocks_for(n, 256), 256, 0, s>>>(A);
-            ext_cells_kernel<<<blocks_for(ne, 128), 128, 0, s>>>(ne, ctx->inv_h, ctx->cell_start, ctx->perm, ctx->xl,
-                                                                ctx->yl, ctx->v, ctx->state[4], ctx->cell_sums);
+            MPMG_CHECK((launch_g2p<MPMG_G_LOCAL_MU2_EXT, G2P_FULL>(ctx, A)));
+            ext_cells_kernel<<<blocks_for(ne, 128), 128, 0, s>>>(ne, ctx->inv_h, row_view(ctx), ctx->xl, ctx->yl,
+                                                                ctx->v, ctx->state[4], ctx->cell_sums);
             ext_nodes_kernel<<<blocks_for(nn, 256), 256, 0, s>>>(g, ne, ctx->cell_sums, ctx->node_gf);
             ext_stress_kernel<<<blocks_for(n, 256), 256, 0, s>>>(A, ctx->node_gf);
             ctx->launches += 3;
             break;
-        case MPMG_G_NONLOCAL_MU2:
-            g2p_kernel<MPMG_G_NONLOCAL_MU2, G2P_FULL><<<blocks_for(n, 256), 256, 0, s>>>(A);
-            break;
-        default:
-            g2p_kernel<MPMG_G_NONLOCAL, G2P_FULL><<<blocks_for(n, 256), 256, 0, s>>>(A);
-            break;
+        case MPMG_G_NONLOCAL_MU2: MPMG_CHECK((launch_g2p<MPMG_G_NONLOCAL_MU2, G2P_FULL>(ctx, A))); break;
+        default: MPMG_CHECK((launch_g2p<MPMG_G_NONLOCAL, G2P_FULL>(ctx, A))); break;
         }
-        ctx->launches += 1;
     }
     mpmg_phase_end(ctx, PH_G2P);
     MPMG_CHECK(cudaGetLastError());
 
-    if (c.material == MPMG_G_NONLOCAL_MU2 || c.material == MPMG_G_NONLOCAL || c.material == MPMG_G_NONLOCAL_AVG) {
+    if (nonlocal) {
         mpmg_phase_begin(ctx, PH_FLUIDITY);
-        rc = mpmg_launch_fluidity(ctx);
+        const int rc = mpmg_launch_fluidity(ctx);
         if (rc != MPMG_OK) return rc;
         mpmg_phase_end(ctx, PH_FLUIDITY);
     }
+    ctx->row.cur = 1 - ctx->row.cur;
     return MPMG_OK;
 }
 

@@ -1,5 +1,5 @@
 // Test-only kernels: the library's FP64 square root and quotients
-// (mat::root, mat::quot, mat::dvd_const, mat::third) against the IEEE
+// (mat::root, mat::quot, mat::dvd_const) against the IEEE
 // operations, on random operands, on operands whose result lies next to a
 // midpoint of two doubles or to a power of two, and on the ends of the range.
 // Built by tests/test_gpu_root.py with nvcc into a temporary shared library.
@@ -34,7 +34,7 @@ __device__ double operand(uint64_t r, int kind, int span)
     return bits(e | (r & frac));
 }
 
-enum { ROOT = 0, QUOT = 1, CONST = 2, THIRD = 3 };
+enum { ROOT = 0, QUOT = 1, CONST = 2 };
 
 __global__ void check_kernel(int op, int kind, int span, mat::Known k, long long n, uint64_t seed,
                              unsigned long long *bad, double *example)
@@ -72,8 +72,8 @@ __global__ void check_kernel(int op, int kind, int span, mat::Known k, long long
                 a = __fma_rn(k.b, 0.5 * u, __dmul_rn(k.b, c));
                 a = bits((uint64_t)__double_as_longlong(a) + (r0 % 5) - 2);
             }
-            got = op == CONST ? mat::dvd_const(a, k) : mat::third(a);
-            want = __ddiv_rn(a, op == CONST ? k.b : 3.0);
+            got = mat::dvd_const(a, k);
+            want = __ddiv_rn(a, k.b);
         }
         const bool same = __double_as_longlong(got) == __double_as_longlong(want) || (isnan(got) && isnan(want));
         if (!same && atomicAdd(bad, 1ull) == 0) {
