@@ -122,12 +122,16 @@ int alloc_rows(mpmg_ctx *ctx, const int *emap, size_t n)
     while (r.cap < 64 && filled > 0 && (size_t)r.cap * filled < 2 * inside) r.cap *= 2;
     r.cur = 0;
     r.ready = false;
-    int rc = dalloc(&r.over_n, 3);
+    r.filled0 = filled;
+    int rc = dalloc(&r.n_over, 5);
+    r.n_filled = r.n_over + 2;
+    r.cursor = r.n_over + 4;
     if (rc == MPMG_OK) rc = dalloc(&r.over_list, n);
     for (int b = 0; b < 2 && rc == MPMG_OK; b++) {
         rc = dalloc(&r.count[b], ctx->ne);
         if (rc == MPMG_OK) rc = dalloc(&r.rows[b], ctx->ne * (size_t)r.cap);
         if (rc == MPMG_OK) rc = dalloc(&r.over[b], n);
+        if (rc == MPMG_OK) rc = dalloc(&r.filled[b], std::min(ctx->ne, n));
     }
     return rc;
 }
@@ -425,8 +429,9 @@ int mpmg_destroy(mpmg_ctx *ctx)
         cudaFree(ctx->row.count[b]);
         cudaFree(ctx->row.rows[b]);
         cudaFree(ctx->row.over[b]);
+        cudaFree(ctx->row.filled[b]);
     }
-    cudaFree(ctx->row.over_n);
+    cudaFree(ctx->row.n_over);   // the counters, one block
     cudaFree(ctx->row.over_list);
     cudaFree(ctx->elem_coef);
     cudaFree(ctx->sort_keys);

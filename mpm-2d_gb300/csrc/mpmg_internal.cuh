@@ -107,7 +107,8 @@ struct BinScratch {
 // Element rows of the FP64 step (mpmg_step.cu): each element has a row of
 // `cap` slots for its particles' indices, filled in any order with a counter
 // per element; what does not fit goes to an overflow list of (element, index)
-// pairs.  Two buffers: while a step works on buffer `cur`, its G2P already
+// pairs.  A list names the elements that hold particles, in any order.  Two
+// buffers: while a step works on buffer `cur`, its G2P already
 // bins the moved particles into the other one for the next step.  `ready`
 // says that buffer cur holds the current positions' elements; setting x, y or
 // the element map from outside clears it, and the next step then bins first.
@@ -116,7 +117,11 @@ struct RowBins {
     uint32_t *count[2];    // ne
     uint32_t *rows[2];     // ne x cap
     uint2 *over[2];        // n
-    uint32_t *over_n;      // entries in over[0], over[1]; then the cursor of over_list
+    uint32_t *filled[2];   // min(ne, n): the elements with particles
+    uint32_t *n_over;      // entries in over[0], over[1]
+    uint32_t *n_filled;    // entries in filled[0], filled[1]
+    uint32_t *cursor;      // entries taken from over_list
+    size_t filled0;        // filled elements of the initial positions
     uint32_t *over_list;   // n: the ordered lists of elements with more than cap particles
     int cur;
     bool ready;

@@ -22,7 +22,12 @@
 //             calculate_stress_threaded), and the next step's rows
 //
 // The kernels are launched with programmatic dependent launch: each waits for
-// the one before it at its start and lets the next one launch.
+// the one before it at its start, and lets the next one launch at its end, or
+// right after that wait where every kernel is at most a warp an SM (`early`):
+// there the next one's launch overlaps this one's work (block of 4096
+// particles: 15.7 against 17.3 us a step), while in larger grids blocks that
+// launch beside working ones are placed unevenly (125 k particles: 97 against
+// 76 us).
 //
 // Shape functions (tent / grad_tent, interpolate.c:23-65) are recomputed in
 // registers from the start-of-step position wherever they are needed.  No
@@ -43,11 +48,17 @@ using fp64::make_bc;
 using fp64::make_geom;
 using fp64::shape;
 
+// Whether the step's kernels let their successors launch early (see above).
+inline int early_launch(const mpmg_ctx *ctx)
+{
+    return ctx->np <= (size_t)ctx->sms * 32;
+}
+
 // ---------------------------------------------------------------------------
 // rows
 
 struct RowsOut {
-    uint32_t *count, *rows, *over_n;
+    uint32_t *count, *rows, *filled, *n_filled, *n_over;
     uint2 *over;
     int cap;
 };
@@ -71,11 +82,19 @@ __device__ __forceinline__ void bin_particle(const RowsOut &R, int i, uint32_t k
     }
     const uint32_t below = starts & (0xffffffffu >> (31 - lane));
     const int leader = below ? 31 - __clz(below) : lane;
+    // the first particle of an element puts it on the list
+    const uint32_t firsts = __ballot_sync(0xffffffffu, start && base == 0);
+    if (firsts) {
+        uint32_t at = 0;
+        if (lane == 0) at = atomicAdd(R.n_filled, (uint32_t)__popc(firsts));
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if (start && base == 0) R.filled[at + __popc(firsts & ((1u << lane) - 1u))] = key;
+    }
     base = __shfl_sync(0xffffffffu, base, leader);
     if (!valid) return;
     const uint32_t slot = base + (uint32_t)(lane - leader);
     if (slot < (uint32_t)R.cap) R.rows[(size_t)key * R.cap + slot] = (uint32_t)i;
-    else R.over[atomicAdd(R.over_n, 1u)] = make_uint2(key, (uint32_t)i);
+    else R.over[atomicAdd(R.n_over, 1u)] = make_uint2(key, (uint32_t)i);
 }
 
 // The rows of the current positions, where no G2P has left them: keys[i] is
@@ -112,40 +131,45 @@ __global__ void __launch_bounds__(256) keys_kernel(GridGeom g, float inv_hf, int
 //
 // The loop is bound by the FP64 pipe, where an instruction costs a sub-partition
 // 64 cycles whatever the number of active lanes: a warp costs its fullest
-// element's count.  So a block sorts its elements by count (each warp then
-// holds equal counts, and empty elements share warps that do nothing), and the
-// sorted warps rotate with the block index, so that no sub-partition gets the
+// element's count.  So a block takes EB of the filled elements from the list
+// (empty ones cost nothing, and a sparse grid's work spreads over all SMs),
+// sorts them by count, so that each warp holds about equal counts, and rotates
+// the sorted warps with the block index, so that no sub-partition gets the
 // full ones of every block.  SPLIT = 2 gives the two halves of an element's
 // moments to two threads in different warps, which shortens the serial chain
-// where the grid is too small to fill the chip.
+// where there are too few elements to fill the chip.  The sums are stored per
+// element: 4 corners x (m, mx, my, h fx), then 4 x h fy.
+
+constexpr int kCell = 20;                  // doubles an element
 
 template <int EB, int SPLIT>
 __global__ void __launch_bounds__(EB * SPLIT) p2g_cells_kernel(
-    GridGeom g, int ne, int n, RowView rv, uint32_t *__restrict__ count_next, const uint32_t *__restrict__ over_n,
-    uint32_t *__restrict__ over_n_next, const uint2 *__restrict__ over, uint32_t *__restrict__ over_cursor,
-    int keep_order, const double *__restrict__ x, const double *__restrict__ y, const double *__restrict__ m,
+    GridGeom g, RowView rv, const uint32_t *__restrict__ filled, const uint32_t *__restrict__ n_filled,
+    const uint32_t *__restrict__ n_over, const uint2 *__restrict__ over, uint32_t *__restrict__ cursor,
+    int keep_order, int early, const double *__restrict__ x, const double *__restrict__ y,
+    const double *__restrict__ m,
     const double *__restrict__ vx, const double *__restrict__ vy, const double *__restrict__ v,
     const double *__restrict__ sxx, const double *__restrict__ sxy, const double *__restrict__ syy, StepParams *sp,
     double dt, int gravity_mode, double gravity_const, double *__restrict__ cell_sums)
 {
     constexpr int NB = 17;                 // count classes 0..15 and 16 or more
     constexpr int kStage = 16;             // staged row entries an element
-    extern __shared__ __align__(16) unsigned char p2g_smem[];
-    uint32_t *sh_idx = reinterpret_cast<uint32_t *>(p2g_smem);         // [kStage][EB]
-    double *sh_sum = reinterpret_cast<double *>(p2g_smem);             // [20][EB], after the index stage
+    constexpr int kSumStride = kCell + 1;
+    __shared__ double sh_sum[EB * kSumStride];
+    __shared__ uint32_t sh_idx[kStage * EB];
     __shared__ int sh_bin[NB];
-    __shared__ int sh_order[EB], sh_count[EB];
+    __shared__ int sh_order[EB], sh_count[EB], sh_elem[EB];
     __shared__ uint32_t sh_base[EB];
     __shared__ double sh_const[3];         // constants as registers (mat::Unit)
-    if (threadIdx.x == 0) {
+    const int tid = threadIdx.x;
+    if (tid == 0) {
         sh_const[0] = 1.0;
         sh_const[1] = -0.0;
         sh_const[2] = g.inv_h;
     }
+    if (tid < NB) sh_bin[tid] = 0;
     mpmg_pdl_wait();
-    mpmg_pdl_trigger();
-    const int tid = threadIdx.x;
-    const int e0 = blockIdx.x * EB;
+    if (early) mpmg_pdl_trigger();
     if (blockIdx.x == 0 && tid == 0) {
         // time_varying_loads (loading.c:34-54) of the previous step's tail, or
         // initial_loads (loading.c:21-30) before the first step; then t += dt
@@ -164,41 +188,42 @@ __global__ void __launch_bounds__(EB * SPLIT) p2g_cells_kernel(
         sp->gravity = grav;
         sp->t = t + dt;
         sp->step_count += 1;
-        *over_n_next = 0;
     }
-    if (tid < NB) sh_bin[tid] = 0;
-    int cnt0 = 0;
-    if (tid < EB && e0 + tid < ne) {
-        cnt0 = (int)rv.count[e0 + tid];
-        count_next[e0 + tid] = 0;
-    }
-    if (__syncthreads_count(cnt0) == 0) return;
-    // elements by descending count
-    int cls = 0, at = 0;
+    const int total = (int)*n_filled;
+    const int first = blockIdx.x * EB;
+    if (first >= total) return;
+    int le = tid % EB;
     if (tid < EB) {
-        cls = NB - 1 - min(cnt0, NB - 1);
-        at = atomicAdd(&sh_bin[cls], 1);
-        sh_count[tid] = cnt0;
+        const int e0 = first + tid < total ? (int)filled[first + tid] : -1;
+        sh_elem[tid] = e0;
+        sh_count[tid] = e0 >= 0 ? (int)rv.count[e0] : 0;
     }
     __syncthreads();
-    if (tid < 32) {
-        int c = tid < NB ? sh_bin[tid] : 0, incl = c;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const int u = __shfl_up_sync(0xffffffffu, incl, d);
-            if (tid >= d) incl += u;
-        }
-        if (tid < NB) sh_bin[tid] = incl - c;
-    }
-    __syncthreads();
-    if (tid < EB) sh_order[sh_bin[cls] + at] = tid;
-    __syncthreads();
-    // this thread's element and half: sorted warps rotated by the block index
     constexpr int WB = EB / 32;            // warps an element set
     const int half = SPLIT == 2 ? tid / EB : 0;
-    const int warp = (tid % EB) / 32;
-    const int le = sh_order[((warp + (int)blockIdx.x) % WB) * 32 + (tid & 31)];
-    const int cnt = sh_count[le], e = e0 + le;
+    if (WB > 1) {
+        // elements by descending count; this thread's: sorted warps rotated
+        int cls = 0, at = 0;
+        if (tid < EB) {
+            cls = NB - 1 - min(sh_count[tid], NB - 1);
+            at = atomicAdd(&sh_bin[cls], 1);
+        }
+        __syncthreads();
+        if (tid < 32) {
+            int c = tid < NB ? sh_bin[tid] : 0, incl = c;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int w = __shfl_up_sync(0xffffffffu, incl, d);
+                if (tid >= d) incl += w;
+            }
+            if (tid < NB) sh_bin[tid] = incl - c;
+        }
+        __syncthreads();
+        if (tid < EB) sh_order[sh_bin[cls] + at] = tid;
+        __syncthreads();
+        le = sh_order[(((tid % EB) / 32 + (int)blockIdx.x) % WB) * 32 + (tid & 31)];
+    }
+    const int cnt = sh_count[le], e = sh_elem[le];
     const uint32_t *list = nullptr;        // a long element's list in global memory
     if (half == 0 && cnt > 0) {
         uint32_t *row = rv.rows + (size_t)e * rv.cap;
@@ -237,11 +262,11 @@ __global__ void __launch_bounds__(EB * SPLIT) p2g_cells_kernel(
         } else {
             // more particles than the row holds: the row and the element's
             // entries of the overflow list, ordered in over_list
-            const uint32_t base = atomicAdd(over_cursor, (uint32_t)cnt);
+            const uint32_t base = atomicAdd(cursor, (uint32_t)cnt);
             uint32_t *lst = rv.over_list + base;
             int have = 0;
-            const int total = (int)*over_n;
-            for (int j = 0; j < rv.cap + total; j++) {
+            const int extra = (int)*n_over;
+            for (int j = 0; j < rv.cap + extra; j++) {
                 uint32_t q;
                 if (j < rv.cap) {
                     q = row[j];
@@ -323,48 +348,44 @@ __global__ void __launch_bounds__(EB * SPLIT) p2g_cells_kernel(
             Px2 = fma(t2, vlx, Px2);
         }
     }
-    // corners BL, BR, TR, TL (process_usl.c:140-143); the sums leave through
-    // shared memory so that their stores are coalesced in element order
-    __syncthreads();
+    // corners BL, BR, TR, TL (process_usl.c:140-143); an element's sums leave
+    // as one run through shared memory
+    double *out = sh_sum + le * kSumStride;
     if (do_a && cnt > 0) {
         const double dm = u.sub(mm[2], mm[3]), dx = u.sub(mx[2], mx[3]);
-        sh_sum[0 * EB + le] = u.sub(u.sub(mm[0], mm[1]), dm);
-        sh_sum[5 * EB + le] = u.sub(mm[1], mm[3]);
-        sh_sum[10 * EB + le] = mm[3];
-        sh_sum[15 * EB + le] = dm;
-        sh_sum[1 * EB + le] = u.sub(u.sub(mx[0], mx[1]), dx);
-        sh_sum[6 * EB + le] = u.sub(mx[1], mx[3]);
-        sh_sum[11 * EB + le] = mx[3];
-        sh_sum[16 * EB + le] = dx;
+        out[0] = u.sub(u.sub(mm[0], mm[1]), dm);
+        out[4] = u.sub(mm[1], mm[3]);
+        out[8] = mm[3];
+        out[12] = dm;
+        out[1] = u.sub(u.sub(mx[0], mx[1]), dx);
+        out[5] = u.sub(mx[1], mx[3]);
+        out[9] = mx[3];
+        out[13] = dx;
     }
     if (do_b && cnt > 0) {
         const double dy = u.sub(my[2], my[3]);
-        sh_sum[2 * EB + le] = u.sub(u.sub(my[0], my[1]), dy);
-        sh_sum[7 * EB + le] = u.sub(my[1], my[3]);
-        sh_sum[12 * EB + le] = my[3];
-        sh_sum[17 * EB + le] = dy;
+        out[2] = u.sub(u.sub(my[0], my[1]), dy);
+        out[6] = u.sub(my[1], my[3]);
+        out[10] = my[3];
+        out[14] = dy;
         // h times the internal force, -V T grad N
         const double a0 = u.sub(P0, Py0), a1 = u.sub(P1, Px1), b1 = u.sub(P1, Py1), b2 = u.sub(P2, Px2);
-        sh_sum[3 * EB + le] = u.add(a0, a1);
-        sh_sum[8 * EB + le] = u.sub(Px1, a0);
-        sh_sum[13 * EB + le] = -u.add(Py0, Px1);
-        sh_sum[18 * EB + le] = u.sub(Py0, a1);
-        sh_sum[4 * EB + le] = u.add(b1, b2);
-        sh_sum[9 * EB + le] = u.sub(Px2, b1);
-        sh_sum[14 * EB + le] = -u.add(Py1, Px2);
-        sh_sum[19 * EB + le] = u.sub(Py1, b2);
+        out[3] = u.add(a0, a1);
+        out[7] = u.sub(Px1, a0);
+        out[11] = -u.add(Py0, Px1);
+        out[15] = u.sub(Py0, a1);
+        out[16] = u.add(b1, b2);
+        out[17] = u.sub(Px2, b1);
+        out[18] = -u.add(Py1, Px2);
+        out[19] = u.sub(Py1, b2);
     }
     __syncthreads();
-    for (int q = tid; q < 20 * EB; q += EB * SPLIT) {
-        const int f = q / EB, l = q % EB;
-        if (sh_count[l] > 0) cell_sums[(size_t)f * ne + e0 + l] = sh_sum[q];
+    const int here = min(EB, total - first);
+    for (int q = tid; q < kCell * here; q += EB * SPLIT) {
+        const int l = q / kCell, f = q - l * kCell;
+        cell_sums[(size_t)sh_elem[l] * kCell + f] = sh_sum[l * kSumStride + f];
     }
-}
-
-template <int EB>
-constexpr size_t p2g_smem_bytes()
-{
-    return sizeof(double) * 20 * EB > sizeof(uint32_t) * 16 * EB ? sizeof(double) * 20 * EB : sizeof(uint32_t) * 16 * EB;
+    mpmg_pdl_trigger();
 }
 
 // ---------------------------------------------------------------------------
@@ -384,14 +405,22 @@ constexpr size_t p2g_smem_bytes()
 
 constexpr int kGridTX = 32;
 
+// The corner (BL, BR, TR, TL) that node (i, j) is of its colour-c element.
+__device__ __forceinline__ int c_corner(int c, int i, int j)
+{
+    const bool right = (i & 1) == (c & 1), up = (j & 1) == (c >> 1);   // the element lies right of, above the node
+    return right ? (up ? 0 : 3) : (up ? 1 : 2);
+}
+
 template <int TY>
 __global__ void __launch_bounds__(kGridTX * TY) grid_kernel(
-    GridGeom g, BcParams bc, int ne, int tiles_x, const uint32_t *__restrict__ count,
+    GridGeom g, BcParams bc, int tiles_x, const uint32_t *__restrict__ count, uint32_t *__restrict__ count_next,
+    uint32_t *__restrict__ n_over_next, uint32_t *__restrict__ n_filled_next, uint32_t *__restrict__ cursor,
     const double *__restrict__ cell_sums, const StepParams *__restrict__ sp, double dt,
     double *__restrict__ node_m, double *__restrict__ node_ax, double *__restrict__ node_ay,
     double *__restrict__ node_vx, double *__restrict__ node_vy, double *__restrict__ node_mx,
     double *__restrict__ node_my, double *__restrict__ node_fx, double *__restrict__ node_fy,
-    double2 *__restrict__ coef, uint32_t *__restrict__ over_cursor)
+    double2 *__restrict__ coef, int early)
 {
     __shared__ double sh[4][TY][kGridTX];
     __shared__ double sh_const[4];         // constants as registers (mat::Unit)
@@ -418,38 +447,59 @@ __global__ void __launch_bounds__(kGridTX * TY) grid_kernel(
             if (ci < 0 || cj < 0 || ci >= g.Ex || cj >= g.Ey) continue;
             const int e = cj * g.Ex + ci;
             if (count[e] == 0) continue;
-            const int corner = (ci == i) ? ((cj == j) ? 0 : 3) : ((cj == j) ? 1 : 2);
+            const int corner = c_corner(c, i, j);
             if (corner == 0) filled = true;
-            src[c] = cell_sums + (size_t)(corner * 5) * ne + e;
+            src[c] = cell_sums + (size_t)e * kCell + corner * 4;
         }
     }
+    const bool own = node && (tx < kGridTX - 1 || i == g.Nx - 1) && (ty < TY - 1 || j == g.Ny - 1);
     mpmg_pdl_wait();
-    mpmg_pdl_trigger();
+    if (early) mpmg_pdl_trigger();
     __syncthreads();
     const mat::Unit u{sh_const[0], sh_const[1]};
-    if (blockIdx.x == 0 && threadIdx.x == 0) *over_cursor = 0;   // the P2G is done with it
+    // the next step's rows start empty (the G2P fills them)
+    if (own && i < g.Ex && j < g.Ey) count_next[j * g.Ex + i] = 0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *n_over_next = *n_filled_next = *cursor = 0;
     double ax = 0, ay = 0, vxn = 0, vyn = 0;
-    if (node) {
+    double m = 0, mx = 0, my = 0, fx = 0, fy = 0;
+    if (node && (src[0] || src[1] || src[2] || src[3])) {
         double sum[5] = {0, 0, 0, 0, 0};
-        if (src[0] && src[1] && src[2] && src[3]) {
+        // a corner's m, mx, my, h fx as two loads, and its h fy (16 - 3 corner
+        // doubles further on)
+        double2 q0[4], q1[4];
+        double q2[4];
 #pragma unroll
-            for (int f = 0; f < 5; f++) {
-                const size_t o = (size_t)f * ne;
-                sum[f] = u.add(u.add(u.add(src[0][o], src[1][o]), src[2][o]), src[3][o]);
-            }
+        for (int c = 0; c < 4; c++) {
+            if (src[c] == nullptr) continue;
+            q0[c] = *reinterpret_cast<const double2 *>(src[c]);
+            q1[c] = *reinterpret_cast<const double2 *>(src[c] + 2);
+            const int corner = c_corner(c, i, j);
+            q2[c] = src[c][16 - 3 * corner];
+        }
+        if (src[0] && src[1] && src[2] && src[3]) {
+            sum[0] = u.add(u.add(u.add(q0[0].x, q0[1].x), q0[2].x), q0[3].x);
+            sum[1] = u.add(u.add(u.add(q0[0].y, q0[1].y), q0[2].y), q0[3].y);
+            sum[2] = u.add(u.add(u.add(q1[0].x, q1[1].x), q1[2].x), q1[3].x);
+            sum[3] = u.add(u.add(u.add(q1[0].y, q1[1].y), q1[2].y), q1[3].y);
+            sum[4] = u.add(u.add(u.add(q2[0], q2[1]), q2[2]), q2[3]);
         } else {
 #pragma unroll
             for (int c = 0; c < 4; c++) {
                 if (src[c] == nullptr) continue;
-#pragma unroll
-                for (int f = 0; f < 5; f++) sum[f] = u.add(sum[f], src[c][(size_t)f * ne]);
+                sum[0] = u.add(sum[0], q0[c].x);
+                sum[1] = u.add(sum[1], q0[c].y);
+                sum[2] = u.add(sum[2], q1[c].x);
+                sum[3] = u.add(sum[3], q1[c].y);
+                sum[4] = u.add(sum[4], q2[c]);
             }
         }
-        const double m = sum[0];
-        double mx = sum[1], my = sum[2];
+        m = sum[0];
+        mx = sum[1];
+        my = sum[2];
         // body force bx is zero (loading.c:48); by = g acts on the node's mass
         const double inv_h = sh_const[2], dtr = sh_const[3];
-        double fx = u.mul(sum[3], inv_h), fy = fma(sp->gravity, m, u.mul(sum[4], inv_h));
+        fx = u.mul(sum[3], inv_h);
+        fy = fma(sp->gravity, m, u.mul(sum[4], inv_h));
         bool bx, by;
         bc_mask(bc, g, i, j, sp->t, bx, by);
         if (bx) { mx = 0; fx = 0; }
@@ -466,19 +516,19 @@ __global__ void __launch_bounds__(kGridTX * TY) grid_kernel(
             vxn = u.mul(mx, inv_m);
             vyn = u.mul(my, inv_m);
         }
-        if ((tx < kGridTX - 1 || i == g.Nx - 1) && (ty < TY - 1 || j == g.Ny - 1)) {
-            const int n = j * g.Nx + i;
-            node_m[n] = m;
-            node_ax[n] = ax;
-            node_ay[n] = ay;
-            node_vx[n] = vxn;
-            node_vy[n] = vyn;
-            if (node_mx != nullptr) {
-                node_mx[n] = mx;
-                node_my[n] = my;
-                node_fx[n] = fx;
-                node_fy[n] = fy;
-            }
+    }
+    if (own) {
+        const int n = j * g.Nx + i;
+        node_m[n] = m;
+        node_ax[n] = ax;
+        node_ay[n] = ay;
+        node_vx[n] = vxn;
+        node_vy[n] = vyn;
+        if (node_mx != nullptr) {
+            node_mx[n] = mx;
+            node_my[n] = my;
+            node_fx[n] = fx;
+            node_fy[n] = fy;
         }
     }
     sh[0][ty][tx] = ax;
@@ -496,17 +546,20 @@ __global__ void __launch_bounds__(kGridTX * TY) grid_kernel(
             out[2 * f + 1] = make_double2(u.sub(q3, q0), u.sub(u.sub(q2, q3), c1));
         }
     }
+    mpmg_pdl_trigger();
 }
 
 template <int TY>
 cudaError_t launch_grid(mpmg_ctx *ctx, const GridGeom &g)
 {
+    const RowBins &r = ctx->row;
     const int tiles_x = (g.Nx + kGridTX - 2) / (kGridTX - 1), tiles_y = (g.Ny + TY - 2) / (TY - 1);
     return mpmg_launch_pdl(true, grid_kernel<TY>, dim3(tiles_x * tiles_y), dim3(kGridTX * TY), 0, ctx->stream, g,
-                           make_bc(ctx), (int)ctx->ne, tiles_x, (const uint32_t *)ctx->row.count[ctx->row.cur],
-                           (const double *)ctx->cell_sums, (const StepParams *)ctx->d_params, ctx->cfg.dt,
+                           make_bc(ctx), tiles_x, (const uint32_t *)r.count[r.cur], r.count[1 - r.cur],
+                           r.n_over + (1 - r.cur), r.n_filled + (1 - r.cur), r.cursor, (const double *)ctx->cell_sums,
+                           (const StepParams *)ctx->d_params, ctx->cfg.dt,
                            ctx->node_m, ctx->node_ax, ctx->node_ay, ctx->node_vx, ctx->node_vy, ctx->node_mx,
-                           ctx->node_my, ctx->node_fx, ctx->node_fy, (double2 *)ctx->elem_coef, ctx->row.over_n + 2);
+                           ctx->node_my, ctx->node_fx, ctx->node_fy, (double2 *)ctx->elem_coef, early_launch(ctx));
 }
 
 // ---------------------------------------------------------------------------
@@ -522,6 +575,7 @@ struct G2PConst {
 struct G2PArgs {
     GridGeom g;
     int n;
+    int early;
     G2PConst k;
     mat::NonlocalParams nl;
     uint32_t *keys;        // element of this step in, of the next step out (sentinel: none)
@@ -789,7 +843,7 @@ __global__ void __launch_bounds__(128) g2p_kernel(const __grid_constant__ G2PArg
     if (key != A.sentinel) p = load_particle<MATERIAL, PHASE>(A, i);
     __syncthreads();
     mpmg_pdl_wait();
-    mpmg_pdl_trigger();
+    if (A.early) mpmg_pdl_trigger();
     uint32_t next = A.sentinel;
     if (key != A.sentinel) {
         if (PHASE != G2P_STRAIN) A.in_element[i] = (int)key;
@@ -806,6 +860,7 @@ __global__ void __launch_bounds__(128) g2p_kernel(const __grid_constant__ G2PArg
         A.in_element[i] = -1;
     }
     if (PHASE != G2P_MOVE) bin_particle(A.next, i, next, next != A.sentinel);
+    mpmg_pdl_trigger();
 }
 
 // g_local_mu2_ext's second phase (g_local_mu2_ext.c:232-265): per element,
@@ -1014,13 +1069,10 @@ __global__ void __launch_bounds__(128) order_kernel(int ne, const int *__restric
     if (e < ne) mpmg_order_segment(slots, perm, nullptr, cell_start[e], cell_start[e + 1]);
 }
 
-// Up to this many particles the P2G gives an element two threads.
-constexpr size_t kP2GSplitMax = 100000;
-
 RowsOut rows_out(const mpmg_ctx *ctx, int b)
 {
     const RowBins &r = ctx->row;
-    return RowsOut{r.count[b], r.rows[b], r.over_n + b, r.over[b], r.cap};
+    return RowsOut{r.count[b], r.rows[b], r.filled[b], r.n_filled + b, r.n_over + b, r.over[b], r.cap};
 }
 
 RowView row_view(const mpmg_ctx *ctx)
@@ -1035,6 +1087,7 @@ G2PArgs make_g2p_args(mpmg_ctx *ctx)
     const mpmg_config &c = ctx->cfg;
     A.g = make_geom(ctx);
     A.n = (int)ctx->np;
+    A.early = early_launch(ctx);
     A.k.el = mat::make_elastic(ctx->G, ctx->K, ctx->lambda, c.dt);
     A.k.inv_h = ctx->inv_h;
     A.k.half_inv_h = 0.5 * ctx->inv_h;
@@ -1111,15 +1164,17 @@ static cudaError_t launch_p2g(mpmg_ctx *ctx, const GridGeom &g, bool keep_order)
 {
     const mpmg_config &c = ctx->cfg;
     RowBins &r = ctx->row;
-    const int ne = (int)ctx->ne;
     ctx->launches += 1;
-    return mpmg_launch_pdl(true, p2g_cells_kernel<EB, SPLIT>, dim3(blocks_for(ne, EB)), dim3(EB * SPLIT),
-                           p2g_smem_bytes<EB>(), ctx->stream, g, ne, (int)ctx->np, row_view(ctx), r.count[1 - r.cur],
-                           (const uint32_t *)(r.over_n + r.cur), r.over_n + (1 - r.cur), (const uint2 *)r.over[r.cur],
-                           r.over_n + 2, keep_order ? 1 : 0, (const double *)ctx->x, (const double *)ctx->y,
-                           (const double *)ctx->m, (const double *)ctx->vx, (const double *)ctx->vy,
-                           (const double *)ctx->v, (const double *)ctx->sxx, (const double *)ctx->sxy,
-                           (const double *)ctx->syy, ctx->d_params, c.dt, c.gravity_mode, c.gravity, ctx->cell_sums);
+    // blocks for the most elements that can be filled; the rest leave at once
+    const size_t most = ctx->np < ctx->ne ? ctx->np : ctx->ne;
+    return mpmg_launch_pdl(true, p2g_cells_kernel<EB, SPLIT>, dim3(blocks_for(most, EB)), dim3(EB * SPLIT), 0,
+                           ctx->stream, g, row_view(ctx), (const uint32_t *)r.filled[r.cur],
+                           (const uint32_t *)(r.n_filled + r.cur), (const uint32_t *)(r.n_over + r.cur),
+                           (const uint2 *)r.over[r.cur], r.cursor, keep_order ? 1 : 0, early_launch(ctx),
+                           (const double *)ctx->x, (const double *)ctx->y, (const double *)ctx->m, (const double *)ctx->vx,
+                           (const double *)ctx->vy, (const double *)ctx->v, (const double *)ctx->sxx,
+                           (const double *)ctx->sxy, (const double *)ctx->syy, ctx->d_params, c.dt, c.gravity_mode,
+                           c.gravity, ctx->cell_sums);
 }
 
 int mpmg_fp64_ready(mpmg_ctx *ctx)
@@ -1129,7 +1184,7 @@ int mpmg_fp64_ready(mpmg_ctx *ctx)
     cudaStream_t s = ctx->stream;
     const int n = (int)ctx->np;
     MPMG_CHECK(cudaMemsetAsync(r.count[r.cur], 0, ctx->ne * sizeof(uint32_t), s));
-    MPMG_CHECK(cudaMemsetAsync(r.over_n, 0, 3 * sizeof(uint32_t), s));
+    MPMG_CHECK(cudaMemsetAsync(r.n_over, 0, 5 * sizeof(uint32_t), s));
     keys_kernel<<<blocks_for(n, 256), 256, 0, s>>>(make_geom(ctx), (float)ctx->inv_h, n, ctx->x, ctx->y, ctx->active,
                                                    ctx->keys, (uint32_t)ctx->ne, rows_out(ctx, r.cur));
     ctx->launches += 1;
@@ -1172,8 +1227,10 @@ int mpmg_launch_step(mpmg_ctx *ctx)
     mpmg_phase_begin(ctx, PH_P2G);
     // later phases of these read the ordered rows
     const bool keep_order = nonlocal || musl || c.material == MPMG_G_LOCAL_MU2_EXT;
-    MPMG_CHECK((ctx->np <= kP2GSplitMax ? launch_p2g<64, 2>(ctx, g, keep_order)
-                                        : launch_p2g<128, 1>(ctx, g, keep_order)));
+    // two threads an element in single-warp sets, where that leaves every
+    // sub-partition at most one warp
+    MPMG_CHECK((ctx->row.filled0 <= (size_t)ctx->sms * 4 * 16 ? launch_p2g<32, 2>(ctx, g, keep_order)
+                                                              : launch_p2g<128, 1>(ctx, g, keep_order)));
     mpmg_phase_end(ctx, PH_P2G);
 
     mpmg_phase_begin(ctx, PH_GRID);
