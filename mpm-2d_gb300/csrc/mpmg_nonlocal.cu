@@ -25,6 +25,7 @@
 // start at node g of the global pools and its per-block arrays at float sm
 // of a block's shared memory.
 constexpr int kMgMaxLevels = 16;
+constexpr int kMgDegree = 3;             // Chebyshev steps at level 0, down and up
 
 struct MgLevel {
     int Nx, Ny, nn, C;
@@ -50,6 +51,8 @@ struct MgPlan {
     float *rsum;           // [total]: row sums
     float *l1inv;          // [total]: inverse absolute row sums (0: not an unknown)
     unsigned long long *z1, *res, *zf;   // [total] tagged words each
+    unsigned long long *zs;              // [2 (kMgDegree - 1)][level 0's nodes] tagged words: the
+                                         // smoothing steps before the last, down then up
     unsigned int *tag;     // tag counter
 };
 
@@ -948,10 +951,16 @@ inline size_t pcg_tile_smem(int C, int Nx)
 // singular) therefore survives FP32 coarsening.
 //
 // Preconditioner: one V(1,1) cycle in FP32 on r / |r|.
-//   * On each level, one l1-Jacobi step (Baker, Falgout, Kolev and Yang,
-//     2011).  D_l1 is each row's absolute sum, so the smoother converges
+//   * On each coarse level, one l1-Jacobi step (Baker, Falgout, Kolev and
+//     Yang, 2011).  D_l1 is each row's absolute sum, so the smoother converges
 //     without an eigenvalue estimate.  The step size is the Chebyshev step
 //     for the interval [0.3, 1] of D_l1^-1 A.
+//   * On level 0, three Chebyshev steps for [0.1, 1].  A flow's xi^-2 varies
+//     by orders of magnitude from node to node, and what a bilinear coarse
+//     space leaves over is level 0's to smooth: on silos 20 to 200 steps into
+//     a flow one step took 15 to 22 iterations, two 9 to 11, three 6 to 8,
+//     while more smoothing or W-cycles on the coarse levels changed nothing.
+//     A step costs one more exchange between blocks, down and up.
 //   * Then the residual and its restriction.
 //   * At the coarsest level, an exact solve: an FP64 inverse formed every
 //     solve.
@@ -995,6 +1004,16 @@ constexpr int kMgLocal = kMgTrips * kMgThreads;   // levels this small are held 
 constexpr int kMgCoarse = 9;           // nodes of the coarsest level at most (3 x 3)
 // one smoothing step: the Chebyshev step for [0.3, 1], 1 / 0.65
 constexpr float kMgOmega = 1.0f / 0.65f;
+// The Chebyshev recurrence for [lo, hi] of D_l1^-1 A at level 0: step 0 is
+// p = D r / theta; step k is p = a_k p + b_k D r; x += p after each.
+constexpr float kChebLo = 0.1f, kChebHi = 1.0f;
+constexpr float kChebTheta = 0.5f * (kChebHi + kChebLo), kChebDelta = 0.5f * (kChebHi - kChebLo);
+constexpr float cheb_rho(int k)
+{
+    return k == 0 ? kChebDelta / kChebTheta : 1.0f / (2.0f * kChebTheta / kChebDelta - cheb_rho(k - 1));
+}
+constexpr float cheb_a(int k) { return k == 0 ? 0.0f : cheb_rho(k) * cheb_rho(k - 1); }
+constexpr float cheb_b(int k) { return k == 0 ? 1.0f / kChebTheta : 2.0f * cheb_rho(k) / kChebDelta; }
 // polls of one wait before it gives up (a poll is one L2 round trip, about
 // a microsecond: a few seconds in all)
 constexpr long long kMgPollLimit = 1ll << 22;
@@ -1288,32 +1307,23 @@ __device__ __noinline__ void mg_galerkin_row(const MgPlan &P, int c, int I, int 
 }
 
 // Sum of four values over the block in a fixed order, returned to every
-// thread (warp 0 adds; scratch holds 4 * blockDim.x + 4 doubles).
-__device__ __forceinline__ void mg_sum4(double v[4], double *scratch)
+// thread: warp c adds value c (lane l the threads l, l + 32, ..., then a
+// shuffle tree), so the four chains run on the four sub-partitions' FP64 units
+// side by side (one warp adding all four took 3.2 us an iteration).  scratch
+// holds 4 * blockDim.x + 4 doubles.
+__device__ __forceinline__ void mg_sum4(const mat::Unit &u, double v[4], double *scratch)
 {
     const int nt = blockDim.x;
 #pragma unroll
     for (int c = 0; c < 4; c++) scratch[c * nt + threadIdx.x] = v[c];
     __syncthreads();
-    if (threadIdx.x < 32) {
-        const int lane = threadIdx.x;
-        double a[4][2];
+    if (threadIdx.x < 128) {
+        const int lane = threadIdx.x & 31, c = threadIdx.x >> 5;
+        double a = scratch[c * nt + lane];
+        for (int t = lane + 32; t < nt; t += 32) a = u.add(a, scratch[c * nt + t]);
 #pragma unroll
-        for (int c = 0; c < 4; c++) a[c][0] = a[c][1] = 0;
-        for (int t = lane; t < nt; t += 64) {
-#pragma unroll
-            for (int c = 0; c < 4; c++) {
-                a[c][0] += scratch[c * nt + t];
-                if (t + 32 < nt) a[c][1] += scratch[c * nt + t + 32];
-            }
-        }
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
-            double x = a[c][0] + a[c][1];
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) x += __shfl_down_sync(0xffffffffu, x, off);
-            if (lane == 0) scratch[4 * nt + c] = x;
-        }
+        for (int off = 16; off > 0; off >>= 1) a = u.add(a, __shfl_down_sync(0xffffffffu, a, off));
+        if (lane == 0) scratch[4 * nt + c] = a;
     }
     __syncthreads();
 #pragma unroll
@@ -1321,36 +1331,41 @@ __device__ __forceinline__ void mg_sum4(double v[4], double *scratch)
     __syncthreads();
 }
 
-// The four per-block partials summed over all blocks in one fixed order by
-// warp 0; every block computes the same totals.
-__device__ __forceinline__ void mg_totals4(const double *partials, int nblocks, double v[4], double *scratch,
-                                           int slots = 4)
+// The four per-block partials summed over all blocks in one fixed order, value
+// c by warp c; every block computes the same totals.
+__device__ __forceinline__ void mg_totals4(const mat::Unit &u, const double *partials, int nblocks, double v[4],
+                                           double *scratch, int slots = 4)
 {
     const int nt = blockDim.x;
-    if (threadIdx.x < 32) {
-        const int lane = threadIdx.x;
+    if (threadIdx.x < 128) {
+        const int lane = threadIdx.x & 31, c = threadIdx.x >> 5;
         constexpr int kMax = 8;     // blocks <= 32 * kMax
-        double x[4] = {0, 0, 0, 0};
+        double p[kMax], x = 0;
 #pragma unroll
         for (int q = 0; q < kMax; q++) {
             const int t = lane + 32 * q;
-            if (t < nblocks) {
-#pragma unroll
-                for (int c = 0; c < 4; c++)
-                    if (c < slots) x[c] += __ldcg(partials + (size_t)c * nblocks + t);
-            }
+            p[q] = c < slots && t < nblocks ? __ldcg(partials + (size_t)c * nblocks + t) : 0.0;
         }
 #pragma unroll
-        for (int c = 0; c < 4; c++) {
+        for (int q = 0; q < kMax; q++)
+            if (32 * q < nblocks) x = u.add(x, p[q]);
 #pragma unroll
-            for (int off = 16; off > 0; off >>= 1) x[c] += __shfl_down_sync(0xffffffffu, x[c], off);
-            if (lane == 0) scratch[4 * nt + c] = x[c];
-        }
+        for (int off = 16; off > 0; off >>= 1) x = u.add(x, __shfl_down_sync(0xffffffffu, x, off));
+        if (lane == 0) scratch[4 * nt + c] = x;
     }
     __syncthreads();
 #pragma unroll
     for (int c = 0; c < 4; c++) v[c] = scratch[4 * nt + c];
     __syncthreads();
+}
+
+// An FP32 value (subnormals as zero) as a double, in integer arithmetic: the
+// conversion instruction runs on the FP64 pipe.
+__device__ __forceinline__ double mg_wide(float f)
+{
+    const unsigned b = __float_as_uint(f), m = b & 0x7fffffffu;
+    if (m < 0x00800000u) return 0.0;
+    return __hiloint2double((int)((b & 0x80000000u) | ((m >> 3) + (896u << 20))), (int)(b << 29));
 }
 
 // The phases of a level spread over the blocks.  Block b owns the nodes
@@ -1364,8 +1379,8 @@ __device__ __forceinline__ void mg_totals4(const double *partials, int nblocks, 
 
 // Residual phase of level l: res = b - A z1, kept in shared memory and
 // published.
-__device__ __forceinline__ void mg_residual(const MgPlan &P, float *sm, int l, const MgShared &S, unsigned tag,
-                                            int *status)
+__device__ __forceinline__ void mg_residual(const MgPlan &P, float *sm, int l, const MgShared &S,
+                                            const unsigned long long *words, unsigned tag, int *status)
 {
     const MgLevel &lv = P.lv[l];
     int n0, cnt;
@@ -1374,7 +1389,7 @@ __device__ __forceinline__ void mg_residual(const MgPlan &P, float *sm, int l, c
     const int H = lv.Nx + 1;
     float *ze = sm + P.sm_vec;          // z1 at nodes n0 - H .. n0 + cnt + H
     for (int k = threadIdx.x; k < cnt; k += kMgThreads) ze[H + k] = S.z1[k];
-    mg_stage(P.z1 + lv.g, lv.nn, n0 - H, n0, ze, n0 + cnt, n0 + cnt + H, ze + H + cnt, tag, status);
+    mg_stage(words, lv.nn, n0 - H, n0, ze, n0 + cnt, n0 + cnt + H, ze + H + cnt, tag, status);
     for (int k = threadIdx.x; k < cnt; k += kMgThreads) {
         const int n = n0 + k;
         const float *z = ze + H + k;
@@ -1386,6 +1401,48 @@ __device__ __forceinline__ void mg_residual(const MgPlan &P, float *sm, int l, c
         mg_st(P.res + lv.g + n, r, tag);
     }
     __syncthreads();
+}
+
+// Words of level 0's smoothing step k (0 .. kMgDegree - 1) on the way down or
+// up: the last one down are the z1 words, the last one up the zf words.
+__device__ __forceinline__ unsigned long long *mg_step_words(const MgPlan &P, int k, bool up)
+{
+    if (k == kMgDegree - 1) return up ? P.zf : P.z1;
+    return P.zs + (size_t)(k + (up ? kMgDegree - 1 : 0)) * P.lv[0].nn;
+}
+
+// Level 0's Chebyshev steps 1 .. kMgDegree - 1 on z (S.z1 down, zown up),
+// whose step 0 is published and whose last correction is p: each stages the
+// halo of the step before, forms r = b - A z and steps.
+__device__ __forceinline__ void mg_cheb(const MgPlan &P, float *sm, const MgShared &S, float *z, float (&p)[kMgTrips],
+                                        bool up, unsigned tag, int *status)
+{
+    const MgLevel &lv = P.lv[0];
+    int n0, cnt;
+    mg_own_range(lv, blockIdx.x, n0, cnt);
+    if (cnt <= 0) return;
+    const int H = lv.Nx + 1;
+    float *ze = sm + P.sm_vec;
+#pragma unroll
+    for (int k = 1; k < kMgDegree; k++) {
+        for (int c = threadIdx.x; c < cnt; c += kMgThreads) ze[H + c] = z[c];
+        mg_stage(mg_step_words(P, k - 1, up), lv.nn, n0 - H, n0, ze, n0 + cnt, n0 + cnt + H, ze + H + cnt, tag, status);
+        unsigned long long *out = mg_step_words(P, k, up);
+#pragma unroll
+        for (int t = 0; t < kMgTrips; t++) {
+            const int c = threadIdx.x + t * kMgThreads;
+            if (c >= cnt) continue;
+            const float *v = ze + H + c;
+            float acc = 0.0f;
+#pragma unroll
+            for (int q = 0; q < 9; q++) acc = fmaf(sm[q * lv.C + c], v[(q / 3 - 1) * lv.Nx + (q % 3 - 1)], acc);
+            p[t] = fmaf(cheb_a(k), p[t], cheb_b(k) * sm[9 * lv.C + c] * (S.b[c] - acc));
+            const float zn = z[c] + p[t];
+            z[c] = zn;
+            mg_st(out + n0 + c, zn, tag);
+        }
+        __syncthreads();
+    }
 }
 
 // Restriction to the spread level c from the spread level c - 1: the fine
@@ -1455,10 +1512,13 @@ __device__ __forceinline__ void mg_restrict_to_held(const MgPlan &P, float *sm, 
 //   z = z2 + omega D_l1^-1 (res - A P zc)   (published; zero off the unknowns)
 // The coarse rows holding the parents of the nodes n0 - H .. n0 + cnt + H
 // are staged, P zc is formed at those nodes, then the stencil runs.  zown:
-// this block's results also into shared memory (level 0), or null.
+// this block's results also into shared memory, or null; level 0 takes step 0
+// of its Chebyshev recurrence here (correction in p) and the others after.
 __device__ __forceinline__ void mg_prolong(const MgPlan &P, float *sm, int l, const MgShared &S, unsigned tag,
-                                           int *status, float *zown)
+                                           int *status, float *zown, float (&p0)[kMgTrips])
 {
+    const float step = l == 0 ? cheb_b(0) : kMgOmega;
+    unsigned long long *out = l == 0 ? mg_step_words(P, 0, true) : P.zf + P.lv[l].g;
     const MgLevel &lv = P.lv[l], &Cl = P.lv[l + 1];
     int n0, cnt;
     mg_own_range(lv, blockIdx.x, n0, cnt);
@@ -1487,15 +1547,19 @@ __device__ __forceinline__ void mg_prolong(const MgPlan &P, float *sm, int l, co
         pz[u] = v;
     }
     __syncthreads();
-    for (int k = threadIdx.x; k < cnt; k += kMgThreads) {
+#pragma unroll
+    for (int t = 0; t < kMgTrips; t++) {
+        const int k = threadIdx.x + t * kMgThreads;
+        if (k >= cnt) continue;
         const int n = n0 + k;
         const float *p = pz + H + k;
         float acc = 0.0f;
 #pragma unroll
         for (int q = 0; q < 9; q++) acc = fmaf(mg_coef(P, sm, l, q, k, n), p[(q / 3 - 1) * lv.Nx + (q % 3 - 1)], acc);
         const float li = mg_l1inv(P, sm, l, k, n);
-        const float z = (li == 0.0f) ? 0.0f : S.z1[k] + p[0] + kMgOmega * li * (S.res[k] - acc);
-        mg_st(P.zf + lv.g + n, z, tag);
+        p0[t] = step * li * (S.res[k] - acc);
+        const float z = (li == 0.0f) ? 0.0f : S.z1[k] + p[0] + p0[t];
+        mg_st(out + n, z, tag);
         if (zown != nullptr) zown[k] = z;
     }
     __syncthreads();
@@ -1595,6 +1659,85 @@ __device__ __forceinline__ void mgh_prolong(const MgHeld &H, const MgHeld &Cz, c
     __syncthreads();
 }
 
+// Level 0's prolongation and Chebyshev step 0 where it is held: like
+// mgh_prolong, with b kept (P zc goes through zf) and the step's correction
+// in p.
+__device__ __forceinline__ void mgh_prolong0(const MgHeld &H, const MgHeld &Cz, const MgLevel &Cl,
+                                             float (&p)[kMgTrips])
+{
+    for (int n = threadIdx.x; n < H.nn; n += blockDim.x) {
+        const int j = n / H.Nx, i = n - j * H.Nx;
+        int px0, px1, py0, py1;
+        const int npx = mg_parents(i, Cl.cx, px0, px1);
+        const int npy = mg_parents(j, Cl.cy, py0, py1);
+        const float *r0 = Cz.zf + py0 * Cz.Nx, *r1 = Cz.zf + py1 * Cz.Nx;
+        float pz = r0[px0];
+        if (npx == 2) pz += r0[px1];
+        if (npy == 2) pz += r1[px0];
+        if (npx == 2 && npy == 2) pz += r1[px1];
+        H.zf[n] = pz * (((npx == 2) ? 0.5f : 1.0f) * ((npy == 2) ? 0.5f : 1.0f));
+    }
+    __syncthreads();
+    float zn[kMgTrips];
+#pragma unroll
+    for (int t = 0; t < kMgTrips; t++) {
+        const int n = threadIdx.x + t * kMgThreads;
+        zn[t] = 0.0f;
+        if (n >= H.nn) continue;
+        const int j = n / H.Nx, i = n - j * H.Nx;
+        float acc = 0.0f;
+#pragma unroll
+        for (int q = 0; q < 9; q++) {
+            const int di = q % 3 - 1, dj = q / 3 - 1;
+            if (i + di < 0 || i + di >= H.Nx || j + dj < 0 || j + dj >= H.Ny) continue;
+            acc = fmaf(H.coef[q * H.nn + n], H.zf[n + dj * H.Nx + di], acc);
+        }
+        const float li = H.l1inv[n];
+        p[t] = cheb_b(0) * li * (H.res[n] - acc);
+        zn[t] = (li == 0.0f) ? 0.0f : H.z1[n] + H.zf[n] + p[t];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int t = 0; t < kMgTrips; t++) {
+        const int n = threadIdx.x + t * kMgThreads;
+        if (n < H.nn) H.zf[n] = zn[t];
+    }
+    __syncthreads();
+}
+
+// Chebyshev steps 1 .. kMgDegree - 1 on z of a held level 0 (its rows skip
+// nodes outside the grid); p: the correction of each of this thread's nodes.
+__device__ __forceinline__ void mgh_cheb(const MgHeld &H, float *z, float (&p)[kMgTrips])
+{
+#pragma unroll
+    for (int k = 1; k < kMgDegree; k++) {
+        float zn[kMgTrips];
+#pragma unroll
+        for (int t = 0; t < kMgTrips; t++) {
+            const int n = threadIdx.x + t * kMgThreads;
+            zn[t] = 0.0f;
+            if (n >= H.nn) continue;
+            const int j = n / H.Nx, i = n - j * H.Nx;
+            float acc = 0.0f;
+#pragma unroll
+            for (int q = 0; q < 9; q++) {
+                const int di = q % 3 - 1, dj = q / 3 - 1;
+                if (i + di < 0 || i + di >= H.Nx || j + dj < 0 || j + dj >= H.Ny) continue;
+                acc = fmaf(H.coef[q * H.nn + n], z[n + dj * H.Nx + di], acc);
+            }
+            p[t] = fmaf(cheb_a(k), p[t], cheb_b(k) * H.l1inv[n] * (H.b[n] - acc));
+            zn[t] = z[n] + p[t];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int t = 0; t < kMgTrips; t++) {
+            const int n = threadIdx.x + t * kMgThreads;
+            if (n < H.nn) z[n] = zn[t];
+        }
+        __syncthreads();
+    }
+}
+
 // The V-cycle on b0 (already in level 0's b): the result lands in level 0's
 // zf words with this tag.  Levels 0 .. Lg - 1 are spread over the blocks;
 // block 0 runs levels Lg .. L - 1 in its shared memory and publishes level
@@ -1607,8 +1750,15 @@ __device__ void mg_vcycle(const MgPlan &P, float *sm, const double *cinv, unsign
         defer();
         // one block holds every level
         const MgHeld H = mg_held(sm, P.lv[0]);
-        for (int n = threadIdx.x; n < H.nn; n += blockDim.x) H.z1[n] = kMgOmega * H.l1inv[n] * H.b[n];
+        float p[kMgTrips];
+#pragma unroll
+        for (int t = 0; t < kMgTrips; t++) {
+            const int n = threadIdx.x + t * kMgThreads;
+            p[t] = 0.0f;
+            if (n < H.nn) H.z1[n] = p[t] = cheb_b(0) * H.l1inv[n] * H.b[n];
+        }
         __syncthreads();
+        mgh_cheb(H, H.z1, p);
         for (int l = 0; l + 1 < L; l++) {
             const MgHeld Hl = mg_held(sm, P.lv[l]);
             mgh_residual(Hl);
@@ -1621,7 +1771,11 @@ __device__ void mg_vcycle(const MgPlan &P, float *sm, const double *cinv, unsign
             Hc.zf[threadIdx.x] = (float)z;
         }
         __syncthreads();
-        for (int l = L - 2; l >= 0; l--) mgh_prolong(mg_held(sm, P.lv[l]), mg_held(sm, P.lv[l + 1]), P.lv[l + 1]);
+        for (int l = L - 2; l >= 1; l--) mgh_prolong(mg_held(sm, P.lv[l]), mg_held(sm, P.lv[l + 1]), P.lv[l + 1]);
+        // level 0: prolongation (its b is kept for the smoother: P zc goes to
+        // zf), then the Chebyshev steps from z1 + P zc
+        mgh_prolong0(H, mg_held(sm, P.lv[1]), P.lv[1], p);
+        mgh_cheb(H, H.zf, p);
         return;
     }
     {
@@ -1630,14 +1784,23 @@ __device__ void mg_vcycle(const MgPlan &P, float *sm, const double *cinv, unsign
         const MgShared S = mg_shared(sm, lv);
         int n0, cnt;
         mg_own_range(lv, blockIdx.x, n0, cnt);
-        for (int k = threadIdx.x; k < cnt; k += kMgThreads) {
-            const float z = kMgOmega * sm[9 * lv.C + k] * S.b[k];
+        unsigned long long *out = mg_step_words(P, 0, false);
+        float p[kMgTrips];
+#pragma unroll
+        for (int t = 0; t < kMgTrips; t++) {
+            const int k = threadIdx.x + t * kMgThreads;
+            p[t] = 0.0f;
+            if (k >= cnt) continue;
+            const float z = cheb_b(0) * sm[9 * lv.C + k] * S.b[k];
+            p[t] = z;
             S.z1[k] = z;
-            mg_st(P.z1 + n0 + k, z, tag);
+            mg_st(out + n0 + k, z, tag);
         }
+        __syncthreads();
+        mg_cheb(P, sm, S, S.z1, p, false, tag, status);
     }
     for (int l = 0; l < Lg; l++) {
-        mg_residual(P, sm, l, mg_shared(sm, P.lv[l]), tag, status);
+        mg_residual(P, sm, l, mg_shared(sm, P.lv[l]), P.z1 + P.lv[l].g, tag, status);
         if (l + 1 < Lg) mg_restrict(P, sm, l + 1, mg_shared(sm, P.lv[l + 1]), tag, status);
     }
     mg_restrict_to_held(P, sm, Lg, tag, status);
@@ -1675,8 +1838,10 @@ __device__ void mg_vcycle(const MgPlan &P, float *sm, const double *cinv, unsign
         for (int n = threadIdx.x; n < H.nn; n += blockDim.x) mg_st(P.zf + P.lv[Lg].g + n, H.zf[n], tag);
         __syncthreads();      // the staging area of the spread phases aliases the held vectors
     }
+    float p[kMgTrips] = {};
     for (int l = Lg - 1; l >= 0; l--)
-        mg_prolong(P, sm, l, mg_shared(sm, P.lv[l]), tag, status, l == 0 ? sm + P.sm_zf0 : nullptr);
+        mg_prolong(P, sm, l, mg_shared(sm, P.lv[l]), tag, status, l == 0 ? sm + P.sm_zf0 : nullptr, p);
+    mg_cheb(P, sm, mg_shared(sm, P.lv[0]), sm + P.sm_zf0, p, true, tag, status);
 }
 
 // Shared memory of pcg_mg_kernel (the offsets are in the plan): level 0's
@@ -1697,9 +1862,15 @@ __global__ void __launch_bounds__(kMgThreads, 1) pcg_mg_kernel(SolveArgs S, cons
     // the level table, indexed by level below, from global memory into
     // shared memory
     __shared__ MgPlan P;
+    __shared__ double sh_unit[2];          // constants as registers (mat::Unit)
     for (int e = threadIdx.x; e < (int)(sizeof(MgPlan) / sizeof(int)); e += blockDim.x)
         reinterpret_cast<int *>(&P)[e] = __ldg(reinterpret_cast<const int *>(plan) + e);
+    if (threadIdx.x == 0) {
+        sh_unit[0] = 1.0;
+        sh_unit[1] = -0.0;
+    }
     __syncthreads();
+    const mat::Unit u{sh_unit[0], sh_unit[1]};
     float *sm = reinterpret_cast<float *>(smd);
     const int Nx = S.Nx, Ny = S.Ny, nn = Nx * Ny;
     const int nblocks = gridDim.x;
@@ -1771,14 +1942,14 @@ __global__ void __launch_bounds__(kMgThreads, 1) pcg_mg_kernel(SolveArgs S, cons
     // start forms r = b - A x and its sums after the set-up instead).
     if (!warm) {
         double part0[4] = {bbp, 0, 0, 0};
-        mg_sum4(part0, scratch);
+        mg_sum4(u, part0, scratch);
         if (threadIdx.x == 0) S.partials[blockIdx.x] = part0[0];
     }
     if (!tile_grid_barrier(S.barrier, ++episode * (unsigned)nblocks, S.status)) return;
     double bb0 = 0;
     if (!warm) {
         double tot[4];
-        mg_totals4(S.partials, nblocks, tot, scratch, 1);
+        mg_totals4(u, S.partials, nblocks, tot, scratch, 1);
         bb0 = tot[0];
     }
     // every block has read the tag counter: reserve this solve's tags
@@ -1883,7 +2054,7 @@ __global__ void __launch_bounds__(kMgThreads, 1) pcg_mg_kernel(SolveArgs S, cons
             part[0] = fma(b, b, part[0]);
             part[1] = fma(rk, rk, part[1]);
         }
-        mg_sum4(part, scratch);
+        mg_sum4(u, part, scratch);
         if (threadIdx.x == 0) {
             S.partials[0 * nblocks + blockIdx.x] = part[0];
             S.partials[1 * nblocks + blockIdx.x] = part[1];
@@ -1891,7 +2062,7 @@ __global__ void __launch_bounds__(kMgThreads, 1) pcg_mg_kernel(SolveArgs S, cons
             S.partials[3 * nblocks + blockIdx.x] = 0;
         }
         if (!tile_grid_barrier(S.barrier, ++episode * (unsigned)nblocks, S.status)) return;
-        mg_totals4(S.partials, nblocks, part, scratch);
+        mg_totals4(u, S.partials, nblocks, part, scratch);
         bb = part[0];
         rr = part[1];
     }
@@ -1911,8 +2082,8 @@ __global__ void __launch_bounds__(kMgThreads, 1) pcg_mg_kernel(SolveArgs S, cons
     // |r| and its reciprocal, formed once by thread 0 (GB300 runs FP64 at
     // 1/64 of the FP32 rate)
     if (threadIdx.x == 0 && !converged) {
-        sh_scalar[3] = sqrt(rr);
-        sh_scalar[4] = 1.0 / sh_scalar[3];
+        sh_scalar[3] = mat::root(rr);
+        sh_scalar[4] = mat::quot(1.0, sh_scalar[3]);
     }
     __syncthreads();
     double sig_u = 0;       // u = sig_u zf0 (the last V-cycle's result)
@@ -1940,7 +2111,7 @@ __global__ void __launch_bounds__(kMgThreads, 1) pcg_mg_kernel(SolveArgs S, cons
 #pragma unroll
             for (int t = 0; t < kMgTrips; t++) {
                 const int k = threadIdx.x + t * kMgThreads;
-                if (k < cnt) Sh.b[k] = (float)(r[k] * isig);
+                if (k < cnt) Sh.b[k] = (float)u.mul(r[k], isig);
             }
         }
         const unsigned tag = tag0 + (unsigned)v;
@@ -1953,7 +2124,7 @@ __global__ void __launch_bounds__(kMgThreads, 1) pcg_mg_kernel(SolveArgs S, cons
                 const int k = threadIdx.x + t * kMgThreads;
                 if (k >= cnt) continue;
                 const int n = n0 + k;
-                const double pk = fma(beta, S.p[n], sig_prev * (double)zf0[k]);
+                const double pk = fma(beta, S.p[n], u.mul(sig_prev, mg_wide(zf0[k])));
                 S.p[n] = pk;
                 x[t] = fma(alpha, pk, x[t]);
             }
@@ -1984,10 +2155,10 @@ __global__ void __launch_bounds__(kMgThreads, 1) pcg_mg_kernel(SolveArgs S, cons
                     // level 0 reads no node outside the level)
                     const int d = (q / 3 - 1) * Nx + (q % 3 - 1), m = n + d;
                     const float zq = !held0 ? st[H + k + d] : (m < 0 || m >= nn) ? 0.0f : zh[m];
-                    az = fma(S.coef[(size_t)q * nn + n], (double)zq, az);
+                    az = fma(S.coef[(size_t)q * nn + n], mg_wide(zq), az);
                 }
                 const float zo = held0 ? zh[n] : st[H + k];
-                const double uk = sig * (double)zo, wk = sig * az, rk = r[k];
+                const double uk = u.mul(sig, mg_wide(zo)), wk = u.mul(sig, az), rk = r[k];
                 zf0[k] = zo;
                 w[k] = wk;
                 part[0] = fma(rk, uk, part[0]);
@@ -1997,13 +2168,13 @@ __global__ void __launch_bounds__(kMgThreads, 1) pcg_mg_kernel(SolveArgs S, cons
             }
         }
         __syncthreads();      // the scratch aliases the held levels' vectors (a held level 0's zf)
-        mg_sum4(part, scratch);
+        mg_sum4(u, part, scratch);
         if (threadIdx.x == 0) {
 #pragma unroll
             for (int c = 0; c < 4; c++) S.partials[c * nblocks + blockIdx.x] = part[c];
         }
         if (!tile_grid_barrier(S.barrier, ++episode * (unsigned)nblocks, S.status)) return;
-        mg_totals4(S.partials, nblocks, part, scratch);
+        mg_totals4(u, S.partials, nblocks, part, scratch);
         const double gn = part[0], dl = part[1], sg = part[2];
         rr = part[3];
         if (threadIdx.x == 0) {
@@ -2015,19 +2186,21 @@ __global__ void __launch_bounds__(kMgThreads, 1) pcg_mg_kernel(SolveArgs S, cons
             } else if (it >= S.maxit) {
                 next = 1;
             } else {
-                const double bn = (v == 0) ? 0.0 : -alpha * sg / gamma;
+                const double bn = (v == 0) ? 0.0 : mat::quot(-alpha * sg, gamma);
                 const double pn = dl + 2.0 * bn * sg + bn * bn * pi;
                 if (!(pn > 0)) {
                     next = 1;                   // breakdown: report non-convergence
                 } else {
                     sh_scalar[0] = bn;
                     sh_scalar[1] = pn;
-                    sh_scalar[2] = gn / pn;
-                    sh_scalar[3] = sqrt(rr);
-                    sh_scalar[4] = 1.0 / sh_scalar[3];
+                    sh_scalar[2] = mat::quot(gn, pn);
                 }
             }
             sh_next = next;
+        } else if (threadIdx.x == 32 && rr > 0) {
+            // another sub-partition forms |r| and its reciprocal meanwhile
+            sh_scalar[3] = mat::root(rr);
+            sh_scalar[4] = mat::quot(1.0, sh_scalar[3]);
         }
         __syncthreads();
         const int next = sh_next;
@@ -2300,9 +2473,9 @@ int mpmg_nonlocal_init(mpmg_ctx *ctx)
             MPMG_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&mg_per_sm, pcg_mg_kernel, kMgThreads, smem));
             if (mg_per_sm >= 1) {
                 MPMG_CHECK(cudaMalloc(&ctx->mg_rows, 11 * (size_t)total * sizeof(float)));
-                MPMG_CHECK(cudaMalloc(&ctx->mg_words, 3 * (size_t)total * sizeof(unsigned long long)));
-                MPMG_CHECK(cudaMemsetAsync(ctx->mg_words, 0, 3 * (size_t)total * sizeof(unsigned long long),
-                                           ctx->stream));
+                const size_t words = 3 * (size_t)total + 2 * (kMgDegree - 1) * nn;
+                MPMG_CHECK(cudaMalloc(&ctx->mg_words, words * sizeof(unsigned long long)));
+                MPMG_CHECK(cudaMemsetAsync(ctx->mg_words, 0, words * sizeof(unsigned long long), ctx->stream));
                 MPMG_CHECK(cudaMalloc(&ctx->mg_tag, sizeof(unsigned int)));
                 const unsigned int first_tag = 1;   // the pools start with tag 0
                 MPMG_CHECK(cudaMemcpyAsync(ctx->mg_tag, &first_tag, sizeof(first_tag), cudaMemcpyHostToDevice,
@@ -2313,6 +2486,7 @@ int mpmg_nonlocal_init(mpmg_ctx *ctx)
                 P.z1 = ctx->mg_words;
                 P.res = ctx->mg_words + total;
                 P.zf = ctx->mg_words + 2 * (size_t)total;
+                P.zs = ctx->mg_words + 3 * (size_t)total;
                 P.tag = ctx->mg_tag;
                 ctx->mg_host = new MgPlan(P);
                 MPMG_CHECK(cudaMalloc(&ctx->mg_dev, sizeof(MgPlan)));
