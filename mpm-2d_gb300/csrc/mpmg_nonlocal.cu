@@ -32,6 +32,7 @@ struct MgLevel {
     int b0;                // first block that owns nodes of the level (blocks b0, b0 + 1, ...
                            // own C nodes each)
     int cx, cy;            // coarsened from the finer level along x, y (level 0: 0)
+    MpmgDiv div;           // by Nx
     int local;             // 1: block 0 holds the whole level (C = nn) in shared memory
     int g;                 // first node of the level in the global pools
     int sm;                // shared memory (floats): spread level: its b, z1, res; held
@@ -53,6 +54,7 @@ struct MgPlan {
     unsigned long long *z1, *res, *zf;   // [total] tagged words each
     unsigned long long *zs;              // [2 (kMgDegree - 1)][level 0's nodes] tagged words: the
                                          // smoothing steps before the last, down then up
+    unsigned long long *gather;          // [2][4][nblocks][2] tagged words (mg_gather4)
     unsigned int *tag;     // tag counter
 };
 
@@ -278,27 +280,55 @@ __device__ __forceinline__ void grid_total3(const double *partials, int a, int b
 // elements around the node (south-west, south-east, north-west, north-east),
 // each element's corners in order.  The node is corner a = TR, TL, BR, BL of
 // them; corner b of an element lies at offset (bx, by) from its BL node, so
-// every stencil index is a compile-time constant.
-__device__ __forceinline__ void build_row(const SolveArgs &S, int i, int j, double cf[9], double *rhs)
+// every stencil index is a compile-time constant.  A sum starts from its first
+// term (an entry has one, two or four), and the additions go through the unit:
+// the rows of a solve are bound by the FP64 pipe.
+__device__ __forceinline__ void build_row(const SolveArgs &S, const mat::Unit &u, int i, int j, double cf[9],
+                                          double *rhs)
 {
     constexpr int qx[4] = {-1, 0, -1, 0}, qy[4] = {-1, -1, 0, 0};   // element offset of each quadrant
     constexpr int qa[4] = {2, 3, 1, 0};                             // the node's corner in it
     constexpr int bx[4] = {0, 1, 1, 0}, by[4] = {0, 0, 1, 1};       // corner offsets BL BR TR TL
-    double f = 0;
+    bool have[4];
+    double k[4][4], f[4];
 #pragma unroll
     for (int q = 0; q < 4; q++) {
         const int ci = i + qx[q], cj = j + qy[q];
-        if (ci < 0 || cj < 0 || ci >= S.Ex || cj >= S.Ey) continue;
-        const int e = cj * S.Ex + ci;
-        if (S.counts != nullptr ? S.counts[e] == 0 : S.cell_start[e] == S.cell_start[e + 1]) continue;
+        have[q] = ci >= 0 && cj >= 0 && ci < S.Ex && cj < S.Ey;
+        const int e = have[q] ? cj * S.Ex + ci : 0;
+        if (have[q]) have[q] = S.counts != nullptr ? S.counts[e] != 0 : S.cell_start[e] != S.cell_start[e + 1];
 #pragma unroll
-        for (int b = 0; b < 4; b++) {
-            const int di = qx[q] + bx[b], dj = qy[q] + by[b];
-            cf[3 * (dj + 1) + (di + 1)] += S.elem_k[(size_t)sym_index(qa[q], b) * S.ne + e];
-        }
-        f += S.elem_f[(size_t)qa[q] * S.ne + e];
+        for (int b = 0; b < 4; b++) k[q][b] = have[q] ? S.elem_k[(size_t)sym_index(qa[q], b) * S.ne + e] : 0.0;
+        f[q] = have[q] ? S.elem_f[(size_t)qa[q] * S.ne + e] : 0.0;
     }
-    *rhs = f;
+    bool seen[9];
+#pragma unroll
+    for (int d = 0; d < 9; d++) seen[d] = false;
+    if (have[0] && have[1] && have[2] && have[3]) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+#pragma unroll
+            for (int b = 0; b < 4; b++) {
+                const int d = 3 * (qy[q] + by[b] + 1) + (qx[q] + bx[b] + 1);
+                cf[d] = seen[d] ? u.add(cf[d], k[q][b]) : k[q][b];
+                seen[d] = true;
+            }
+        }
+        *rhs = u.add(u.add(u.add(f[0], f[1]), f[2]), f[3]);
+    } else {
+        double r = 0;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            if (!have[q]) continue;
+#pragma unroll
+            for (int b = 0; b < 4; b++) {
+                const int d = 3 * (qy[q] + by[b] + 1) + (qx[q] + bx[b] + 1);
+                cf[d] = u.add(cf[d], k[q][b]);
+            }
+            r = u.add(r, f[q]);
+        }
+        *rhs = r;
+    }
 }
 
 // dinv == +0 (not an unknown) tested on the integer pipe: dinv is either a
@@ -338,6 +368,7 @@ __device__ __forceinline__ double apply_stencil(const SolveArgs &S, int n, int i
 //   beta = gamma' / gamma;  alpha = gamma' / (delta - beta gamma' / alpha)
 __global__ void __launch_bounds__(kSolveThreads, 2) pcg_kernel(SolveArgs S)
 {
+    const mat::Unit u{1.0, -0.0};
     const int nn = S.Nx * S.Ny;
     const int nblocks = gridDim.x;
     const int stride = gridDim.x * blockDim.x;
@@ -352,7 +383,7 @@ __global__ void __launch_bounds__(kSolveThreads, 2) pcg_kernel(SolveArgs S)
         const bool dof = S.node_m[n] > S.dof_tol;
         bool coupled = false;
         if (dof) {
-            build_row(S, i, j, cf, &f);
+            build_row(S, u, i, j, cf, &f);
 #pragma unroll
             for (int q = 0; q < 9; q++) coupled |= (__double_as_longlong(cf[q]) << 1) != 0;
             cf[4] += S.shift;
@@ -722,6 +753,7 @@ __device__ __forceinline__ void tile_halo(const double *g, int n0, int n1, int n
 
 __global__ void __launch_bounds__(kTileThreads, 1) pcg_tile_kernel(SolveArgs S, int C, int warm, unsigned int *flags)
 {
+    const mat::Unit u{1.0, -0.0};
     extern __shared__ double sm[];
     const int Nx = S.Nx, Ny = S.Ny, nn = Nx * Ny, H = Nx + 1;
     const int nblocks = gridDim.x;
@@ -748,7 +780,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) pcg_tile_kernel(SolveArgs S, 
         const bool dof = S.node_m[n] > S.dof_tol;
         bool coupled = false;
         if (dof) {
-            build_row(S, i, j, cf, &f);
+            build_row(S, u, i, j, cf, &f);
 #pragma unroll
             for (int q = 0; q < 9; q++) coupled |= (__double_as_longlong(cf[q]) << 1) != 0;
             cf[4] += S.shift;
@@ -1359,13 +1391,74 @@ __device__ __forceinline__ void mg_totals4(const mat::Unit &u, const double *par
     __syncthreads();
 }
 
-// An FP32 value (subnormals as zero) as a double, in integer arithmetic: the
-// conversion instruction runs on the FP64 pipe.
-__device__ __forceinline__ double mg_wide(float f)
+// 2^e times an FP32 value (subnormals as zero) as a double, and 2^e times a
+// double rounded to FP32 (below FP32's normal range: zero), in integer
+// arithmetic: the conversion instructions run on the FP64 pipe.  Both are for
+// vectors of order one and |e| < 800.
+__device__ __forceinline__ double mg_wide(float f, int e)
 {
     const unsigned b = __float_as_uint(f), m = b & 0x7fffffffu;
     if (m < 0x00800000u) return 0.0;
-    return __hiloint2double((int)((b & 0x80000000u) | ((m >> 3) + (896u << 20))), (int)(b << 29));
+    return __hiloint2double((int)((b & 0x80000000u) | ((m >> 3) + ((unsigned)(896 + e) << 20))), (int)(b << 29));
+}
+
+__device__ __forceinline__ float mg_narrow(double x, int e)
+{
+    const long long b = __double_as_longlong(x);
+    const unsigned long long m = (unsigned long long)b & 0x7fffffffffffffffULL;
+    const int f = (int)(m >> 52) + e;       // exponent field, double's bias
+    if (f < 897 || f > 1150) return f > 1150 ? (float)x : 0.0f;
+    const unsigned long long r = (m + 0x0fffffffULL + ((m >> 29) & 1)) >> 29;   // to nearest even
+    return __uint_as_float((unsigned)((unsigned long long)b >> 32 & 0x80000000u) |
+                           ((unsigned)r + ((unsigned)(e - 896) << 23)));
+}
+
+// All-gather of the four per-block inner products of V-cycle `tag`: each block
+// publishes its values as tagged words (a double as two), and warp c waits for
+// value c of every block and adds them in block order (lane l the blocks l,
+// l + 32, ..., then a shuffle tree).  A block goes on only when every block has
+// published, and every block publishes after its last read of the V-cycle's
+// words: this is the grid barrier between V-cycles too, in one round trip
+// instead of an arrival, a release and a read.  Two buffers, by the V-cycle's
+// parity: a block that runs ahead writes the next but one only after every
+// block has published, hence read, the one between.
+__device__ __forceinline__ void mg_gather4(const mat::Unit &u, unsigned long long *words, double v[4], int nblocks,
+                                           double *scratch, unsigned tag, int *status)
+{
+    const int nt = blockDim.x;
+    if (threadIdx.x < 4) {
+        const unsigned long long b = (unsigned long long)__double_as_longlong(
+            threadIdx.x == 0 ? v[0] : threadIdx.x == 1 ? v[1] : threadIdx.x == 2 ? v[2] : v[3]);
+        unsigned long long *w = words + 2 * ((size_t)threadIdx.x * nblocks + blockIdx.x);
+        const unsigned long long t = (unsigned long long)tag << 32;
+        asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(w), "l"(t | (b & 0xffffffffu)));
+        asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(w + 1), "l"(t | (b >> 32)));
+    }
+    if (threadIdx.x < 128) {
+        const int lane = threadIdx.x & 31, c = threadIdx.x >> 5;
+        constexpr int kMax = 8;     // blocks <= 32 * kMax
+        unsigned long long p[kMax][2];
+        const unsigned long long *base = words + 2 * (size_t)c * nblocks;
+#pragma unroll
+        for (int q = 0; q < kMax; q++) {
+            const int t = lane + 32 * q;
+#pragma unroll
+            for (int h = 0; h < 2; h++) p[q][h] = t < nblocks ? mg_ld(base + 2 * t + h) : mg_zero(tag);
+        }
+        mg_resolve(p, tag, status, [&](int q, int h) { return base + 2 * (lane + 32 * q) + h; });
+        double x = 0;
+#pragma unroll
+        for (int q = 0; q < kMax; q++)
+            if (32 * q < nblocks)
+                x = u.add(x, __longlong_as_double((long long)((p[q][1] << 32) | (p[q][0] & 0xffffffffu))));
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) x = u.add(x, __shfl_down_sync(0xffffffffu, x, off));
+        if (lane == 0) scratch[4 * nt + c] = x;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < 4; c++) v[c] = scratch[4 * nt + c];
+    __syncthreads();
 }
 
 // The phases of a level spread over the blocks.  Block b owns the nodes
@@ -1460,7 +1553,7 @@ __device__ __forceinline__ void mg_restrict(const MgPlan &P, float *sm, int c, c
     float *rf = sm + P.sm_vec;          // fine residual rows fa .. fb
     mg_stage(P.res + F.g, F.nn, fa * F.Nx, (fb + 1) * F.Nx, rf, 0, 0, rf, tag, status);
     for (int k = threadIdx.x; k < cnt; k += kMgThreads) {
-        const int I = c0 + k, cj = I / lv.Nx, ci = I - cj * lv.Nx;
+        const int I = c0 + k, cj = (int)mpmg_div((uint32_t)I, lv.div), ci = I - cj * lv.Nx;
         float b = 0.0f;
 #pragma unroll
         for (int q = 0; q < 9; q++) {
@@ -1493,7 +1586,7 @@ __device__ __forceinline__ void mg_restrict_to_held(const MgPlan &P, float *sm, 
     float *rf = sm + P.sm_vec;          // fine residual rows fa .. fb
     mg_stage(P.res + F.g, F.nn, fa * F.Nx, (fb + 1) * F.Nx, rf, 0, 0, rf, tag, status);
     for (int k = threadIdx.x; k < cnt; k += kMgThreads) {
-        const int I = c0 + k, cj = I / lv.Nx, ci = I - cj * lv.Nx;
+        const int I = c0 + k, cj = (int)mpmg_div((uint32_t)I, lv.div), ci = I - cj * lv.Nx;
         float b = 0.0f;
 #pragma unroll
         for (int q = 0; q < 9; q++) {
@@ -1533,7 +1626,7 @@ __device__ __forceinline__ void mg_prolong(const MgPlan &P, float *sm, int l, co
         const int m = n0 - H + u;
         float v = 0.0f;
         if (m >= 0 && m < lv.nn) {
-            const int j = m / lv.Nx, i = m - j * lv.Nx;
+            const int j = (int)mpmg_div((uint32_t)m, lv.div), i = m - j * lv.Nx;
             int px0, px1, py0, py1;
             const int npx = mg_parents(i, Cl.cx, px0, px1);
             const int npy = mg_parents(j, Cl.cy, py0, py1);
@@ -1571,6 +1664,7 @@ struct MgHeld {
     const float *coef, *l1inv;
     float *b, *z1, *res, *zf;
     int Nx, Ny, nn;
+    MpmgDiv div;
 };
 
 __device__ __forceinline__ MgHeld mg_held(float *sm, const MgLevel &lv)
@@ -1585,21 +1679,29 @@ __device__ __forceinline__ MgHeld mg_held(float *sm, const MgLevel &lv)
     h.Nx = lv.Nx;
     h.Ny = lv.Ny;
     h.nn = lv.nn;
+    h.div = lv.div;
     return h;
+}
+
+// (A z)(n) on a held level.  Entries towards nodes outside the grid are zero,
+// so a neighbour that wraps around a row end multiplies a finite value by
+// zero; only the level's ends are tested.
+__device__ __forceinline__ float mgh_stencil(const MgHeld &H, int n, const float *z)
+{
+    float acc = 0.0f;
+#pragma unroll
+    for (int q = 0; q < 9; q++) {
+        const int m = n + (q / 3 - 1) * H.Nx + (q % 3 - 1);
+        if ((unsigned)m < (unsigned)H.nn) acc = fmaf(H.coef[q * H.nn + n], z[m], acc);
+    }
+    return acc;
 }
 
 // res = b - A z1 on a held level.
 __device__ __forceinline__ void mgh_residual(const MgHeld &H)
 {
     for (int n = threadIdx.x; n < H.nn; n += blockDim.x) {
-        const int j = n / H.Nx, i = n - j * H.Nx;
-        float acc = 0.0f;
-#pragma unroll
-        for (int q = 0; q < 9; q++) {
-            const int di = q % 3 - 1, dj = q / 3 - 1;
-            if (i + di < 0 || i + di >= H.Nx || j + dj < 0 || j + dj >= H.Ny) continue;
-            acc = fmaf(H.coef[q * H.nn + n], H.z1[n + dj * H.Nx + di], acc);
-        }
+        const float acc = mgh_stencil(H, n, H.z1);
         H.res[n] = H.b[n] - acc;
     }
     __syncthreads();
@@ -1610,7 +1712,7 @@ __device__ __forceinline__ void mgh_residual(const MgHeld &H)
 __device__ __forceinline__ void mgh_restrict(const MgHeld &F, const MgHeld &H, const MgLevel &lv, bool coarsest)
 {
     for (int I = threadIdx.x; I < H.nn; I += blockDim.x) {
-        const int cj = I / H.Nx, ci = I - cj * H.Nx;
+        const int cj = (int)mpmg_div((uint32_t)I, H.div), ci = I - cj * H.Nx;
         float b = 0.0f;
 #pragma unroll
         for (int q = 0; q < 9; q++) {
@@ -1632,7 +1734,7 @@ __device__ __forceinline__ void mgh_restrict(const MgHeld &F, const MgHeld &H, c
 __device__ __forceinline__ void mgh_prolong(const MgHeld &H, const MgHeld &Cz, const MgLevel &Cl)
 {
     for (int n = threadIdx.x; n < H.nn; n += blockDim.x) {
-        const int j = n / H.Nx, i = n - j * H.Nx;
+        const int j = (int)mpmg_div((uint32_t)n, H.div), i = n - j * H.Nx;
         int px0, px1, py0, py1;
         const int npx = mg_parents(i, Cl.cx, px0, px1);
         const int npy = mg_parents(j, Cl.cy, py0, py1);
@@ -1645,14 +1747,7 @@ __device__ __forceinline__ void mgh_prolong(const MgHeld &H, const MgHeld &Cz, c
     }
     __syncthreads();
     for (int n = threadIdx.x; n < H.nn; n += blockDim.x) {
-        const int j = n / H.Nx, i = n - j * H.Nx;
-        float acc = 0.0f;
-#pragma unroll
-        for (int q = 0; q < 9; q++) {
-            const int di = q % 3 - 1, dj = q / 3 - 1;
-            if (i + di < 0 || i + di >= H.Nx || j + dj < 0 || j + dj >= H.Ny) continue;
-            acc = fmaf(H.coef[q * H.nn + n], H.b[n + dj * H.Nx + di], acc);
-        }
+        const float acc = mgh_stencil(H, n, H.b);
         const float li = H.l1inv[n];
         H.zf[n] = (li == 0.0f) ? 0.0f : H.z1[n] + H.b[n] + kMgOmega * li * (H.res[n] - acc);
     }
@@ -1666,7 +1761,7 @@ __device__ __forceinline__ void mgh_prolong0(const MgHeld &H, const MgHeld &Cz, 
                                              float (&p)[kMgTrips])
 {
     for (int n = threadIdx.x; n < H.nn; n += blockDim.x) {
-        const int j = n / H.Nx, i = n - j * H.Nx;
+        const int j = (int)mpmg_div((uint32_t)n, H.div), i = n - j * H.Nx;
         int px0, px1, py0, py1;
         const int npx = mg_parents(i, Cl.cx, px0, px1);
         const int npy = mg_parents(j, Cl.cy, py0, py1);
@@ -1684,14 +1779,7 @@ __device__ __forceinline__ void mgh_prolong0(const MgHeld &H, const MgHeld &Cz, 
         const int n = threadIdx.x + t * kMgThreads;
         zn[t] = 0.0f;
         if (n >= H.nn) continue;
-        const int j = n / H.Nx, i = n - j * H.Nx;
-        float acc = 0.0f;
-#pragma unroll
-        for (int q = 0; q < 9; q++) {
-            const int di = q % 3 - 1, dj = q / 3 - 1;
-            if (i + di < 0 || i + di >= H.Nx || j + dj < 0 || j + dj >= H.Ny) continue;
-            acc = fmaf(H.coef[q * H.nn + n], H.zf[n + dj * H.Nx + di], acc);
-        }
+        const float acc = mgh_stencil(H, n, H.zf);
         const float li = H.l1inv[n];
         p[t] = cheb_b(0) * li * (H.res[n] - acc);
         zn[t] = (li == 0.0f) ? 0.0f : H.z1[n] + H.zf[n] + p[t];
@@ -1717,14 +1805,7 @@ __device__ __forceinline__ void mgh_cheb(const MgHeld &H, float *z, float (&p)[k
             const int n = threadIdx.x + t * kMgThreads;
             zn[t] = 0.0f;
             if (n >= H.nn) continue;
-            const int j = n / H.Nx, i = n - j * H.Nx;
-            float acc = 0.0f;
-#pragma unroll
-            for (int q = 0; q < 9; q++) {
-                const int di = q % 3 - 1, dj = q / 3 - 1;
-                if (i + di < 0 || i + di >= H.Nx || j + dj < 0 || j + dj >= H.Ny) continue;
-                acc = fmaf(H.coef[q * H.nn + n], z[n + dj * H.Nx + di], acc);
-            }
+            const float acc = mgh_stencil(H, n, z);
             p[t] = fmaf(cheb_a(k), p[t], cheb_b(k) * H.l1inv[n] * (H.b[n] - acc));
             zn[t] = z[n] + p[t];
         }
@@ -1855,6 +1936,20 @@ inline size_t pcg_mg_smem(const MgPlan &P)
     return (size_t)P.sm_fp64 * sizeof(float) + doubles * sizeof(double);
 }
 
+// The exponent k of the power of two with 2^k <= sqrt(rr) < 2^(k + 1) (or
+// nearly: rr is positive and finite).
+__device__ __forceinline__ int mg_scale(double rr)
+{
+    return (((__double2hiint(rr) >> 20) & 0x7ff) - 1023) >> 1;
+}
+
+// a > b for a, b not -0 (nodal masses and their threshold), on the bit
+// patterns.
+__device__ __forceinline__ bool above(double a, double b)
+{
+    return __double_as_longlong(a) > __double_as_longlong(b) && !mat::is_nan(a);
+}
+
 __global__ void __launch_bounds__(kMgThreads, 1) pcg_mg_kernel(SolveArgs S, const MgPlan *__restrict__ plan,
                                                                 int warm)
 {
@@ -1904,15 +1999,15 @@ __global__ void __launch_bounds__(kMgThreads, 1) pcg_mg_kernel(SolveArgs S, cons
         const int n = n0 + k, j = n / Nx, i = n - j * Nx;
         double cf[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
         double f = 0;
-        const bool dof = S.node_m[n] > S.dof_tol;
+        const bool dof = above(S.node_m[n], S.dof_tol);
         bool coupled = false;
         if (dof) {
-            build_row(S, i, j, cf, &f);
+            build_row(S, u, i, j, cf, &f);
 #pragma unroll
             for (int q = 0; q < 9; q++) coupled |= (__double_as_longlong(cf[q]) << 1) != 0;
-            cf[4] += S.shift;
+            cf[4] = u.add(cf[4], S.shift);
         }
-        const bool unknown = dof && cf[4] > 0;
+        const bool unknown = dof && mat::is_pos(cf[4]);
         if (unknown) {
             r[k] = f;
             x[t] = (warm && coupled) ? S.x[n] : 0.0;
@@ -1931,11 +2026,12 @@ __global__ void __launch_bounds__(kMgThreads, 1) pcg_mg_kernel(SolveArgs S, cons
         for (int q = 0; q < 9; q++) {
             const int di = q % 3 - 1, dj = q / 3 - 1;
             const bool in = i + di >= 0 && i + di < Nx && j + dj >= 0 && j + dj < Ny;
-            const bool nbu = unknown && (q == 4 || (in && S.node_m[n + dj * Nx + di] > S.dof_tol));
-            a[q] = nbu ? (float)cf[q] : 0.0f;
-            if (nbu) rsum += cf[q];
+            const bool nbu = unknown && (q == 4 || (in && above(S.node_m[n + dj * Nx + di], S.dof_tol)));
+            const double c = nbu ? cf[q] : 0.0;
+            a[q] = mg_narrow(c, 0);
+            rsum = q == 0 ? c : u.add(rsum, c);
         }
-        mg_put_row(P, n, a, (float)rsum, sm, k, L0.C);
+        mg_put_row(P, n, a, mg_narrow(rsum, 0), sm, k, L0.C);
         if (unknown) bbp = fma(f, f, bbp);
     }
     // From a zero start r = b: <b, b> rides on the first grid barrier (a warm
@@ -2079,16 +2175,11 @@ __global__ void __launch_bounds__(kMgThreads, 1) pcg_mg_kernel(SolveArgs S, cons
     } else if (rr <= target) {
         converged = true;                                 // the start already meets the tolerance
     }
-    // |r| and its reciprocal, formed once by thread 0 (GB300 runs FP64 at
-    // 1/64 of the FP32 rate)
-    if (threadIdx.x == 0 && !converged) {
-        sh_scalar[3] = mat::root(rr);
-        sh_scalar[4] = mat::quot(1.0, sh_scalar[3]);
-    }
-    __syncthreads();
-    double sig_u = 0;       // u = sig_u zf0 (the last V-cycle's result)
+    // The V-cycle works on r scaled to order one by a power of two near 1 / |r|
+    // (an exponent shift, no multiplication): u = 2^sc zf0 is its result.
+    int sc = mg_scale(rr);
     for (int v = 0; !converged && !failed; v++) {
-        const double sig_prev = sig_u;
+        const int sc_prev = sc;
         if (v > 0) {
             // s = w + beta s, r -= alpha s (the V-cycle's input); p and x
             // follow inside the V-cycle (defer below)
@@ -2102,20 +2193,18 @@ __global__ void __launch_bounds__(kMgThreads, 1) pcg_mg_kernel(SolveArgs S, cons
             }
             it++;
         }
-        // u = |r| V(r / |r|) (|r| of the last reduction), w = A u, and the
-        // inner products
-        const double sig = sh_scalar[3], isig = sh_scalar[4];
-        sig_u = sig;
+        // u = 2^sc V(2^-sc r), w = A u, and the inner products
+        sc = mg_scale(rr);
         {
             const MgShared Sh = mg_shared(sm, L0);
 #pragma unroll
             for (int t = 0; t < kMgTrips; t++) {
                 const int k = threadIdx.x + t * kMgThreads;
-                if (k < cnt) Sh.b[k] = (float)u.mul(r[k], isig);
+                if (k < cnt) Sh.b[k] = mg_narrow(r[k], -sc);
             }
         }
         const unsigned tag = tag0 + (unsigned)v;
-        // p = u + beta p, x += alpha p, with u = sig_prev zf0 (the last
+        // p = u + beta p, x += alpha p, with u = 2^sc_prev zf0 (the last
         // V-cycle's result, in zf0 until level 0's prolongation)
         auto defer = [&]() {
             if (v == 0) return;
@@ -2124,7 +2213,7 @@ __global__ void __launch_bounds__(kMgThreads, 1) pcg_mg_kernel(SolveArgs S, cons
                 const int k = threadIdx.x + t * kMgThreads;
                 if (k >= cnt) continue;
                 const int n = n0 + k;
-                const double pk = fma(beta, S.p[n], u.mul(sig_prev, mg_wide(zf0[k])));
+                const double pk = fma(beta, S.p[n], mg_wide(zf0[k], sc_prev));
                 S.p[n] = pk;
                 x[t] = fma(alpha, pk, x[t]);
             }
@@ -2155,10 +2244,10 @@ __global__ void __launch_bounds__(kMgThreads, 1) pcg_mg_kernel(SolveArgs S, cons
                     // level 0 reads no node outside the level)
                     const int d = (q / 3 - 1) * Nx + (q % 3 - 1), m = n + d;
                     const float zq = !held0 ? st[H + k + d] : (m < 0 || m >= nn) ? 0.0f : zh[m];
-                    az = fma(S.coef[(size_t)q * nn + n], mg_wide(zq), az);
+                    az = fma(S.coef[(size_t)q * nn + n], mg_wide(zq, sc), az);
                 }
                 const float zo = held0 ? zh[n] : st[H + k];
-                const double uk = u.mul(sig, mg_wide(zo)), wk = u.mul(sig, az), rk = r[k];
+                const double uk = mg_wide(zo, sc), wk = az, rk = r[k];
                 zf0[k] = zo;
                 w[k] = wk;
                 part[0] = fma(rk, uk, part[0]);
@@ -2169,12 +2258,7 @@ __global__ void __launch_bounds__(kMgThreads, 1) pcg_mg_kernel(SolveArgs S, cons
         }
         __syncthreads();      // the scratch aliases the held levels' vectors (a held level 0's zf)
         mg_sum4(u, part, scratch);
-        if (threadIdx.x == 0) {
-#pragma unroll
-            for (int c = 0; c < 4; c++) S.partials[c * nblocks + blockIdx.x] = part[c];
-        }
-        if (!tile_grid_barrier(S.barrier, ++episode * (unsigned)nblocks, S.status)) return;
-        mg_totals4(u, S.partials, nblocks, part, scratch);
+        mg_gather4(u, P.gather + (size_t)(v & 1) * 8 * nblocks, part, nblocks, scratch, tag, S.status);
         const double gn = part[0], dl = part[1], sg = part[2];
         rr = part[3];
         if (threadIdx.x == 0) {
@@ -2186,8 +2270,8 @@ __global__ void __launch_bounds__(kMgThreads, 1) pcg_mg_kernel(SolveArgs S, cons
             } else if (it >= S.maxit) {
                 next = 1;
             } else {
-                const double bn = (v == 0) ? 0.0 : mat::quot(-alpha * sg, gamma);
-                const double pn = dl + 2.0 * bn * sg + bn * bn * pi;
+                const double bn = (v == 0) ? 0.0 : mat::quot(u.mul(-alpha, sg), gamma);
+                const double pn = fma(bn, fma(bn, pi, u.add(sg, sg)), dl);
                 if (!(pn > 0)) {
                     next = 1;                   // breakdown: report non-convergence
                 } else {
@@ -2197,10 +2281,6 @@ __global__ void __launch_bounds__(kMgThreads, 1) pcg_mg_kernel(SolveArgs S, cons
                 }
             }
             sh_next = next;
-        } else if (threadIdx.x == 32 && rr > 0) {
-            // another sub-partition forms |r| and its reciprocal meanwhile
-            sh_scalar[3] = mat::root(rr);
-            sh_scalar[4] = mat::quot(1.0, sh_scalar[3]);
         }
         __syncthreads();
         const int next = sh_next;
@@ -2375,6 +2455,7 @@ int mpmg_nonlocal_init(mpmg_ctx *ctx)
             lv.Nx = Nx;
             lv.Ny = Ny;
             lv.nn = Nx * Ny;
+            lv.div = mpmg_div_init((uint32_t)Nx);
             // on one block every level is held; otherwise level 0 is spread
             // and the coarser levels of at most kMgLocal nodes are held
             lv.local = (nb == 1 || (L > 0 && lv.nn <= kMgLocal)) ? 1 : 0;
@@ -2473,7 +2554,7 @@ int mpmg_nonlocal_init(mpmg_ctx *ctx)
             MPMG_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&mg_per_sm, pcg_mg_kernel, kMgThreads, smem));
             if (mg_per_sm >= 1) {
                 MPMG_CHECK(cudaMalloc(&ctx->mg_rows, 11 * (size_t)total * sizeof(float)));
-                const size_t words = 3 * (size_t)total + 2 * (kMgDegree - 1) * nn;
+                const size_t words = 3 * (size_t)total + 2 * (kMgDegree - 1) * nn + 16 * (size_t)nb;
                 MPMG_CHECK(cudaMalloc(&ctx->mg_words, words * sizeof(unsigned long long)));
                 MPMG_CHECK(cudaMemsetAsync(ctx->mg_words, 0, words * sizeof(unsigned long long), ctx->stream));
                 MPMG_CHECK(cudaMalloc(&ctx->mg_tag, sizeof(unsigned int)));
@@ -2487,6 +2568,7 @@ int mpmg_nonlocal_init(mpmg_ctx *ctx)
                 P.res = ctx->mg_words + total;
                 P.zf = ctx->mg_words + 2 * (size_t)total;
                 P.zs = ctx->mg_words + 3 * (size_t)total;
+                P.gather = P.zs + 2 * (kMgDegree - 1) * nn;
                 P.tag = ctx->mg_tag;
                 ctx->mg_host = new MgPlan(P);
                 MPMG_CHECK(cudaMalloc(&ctx->mg_dev, sizeof(MgPlan)));
