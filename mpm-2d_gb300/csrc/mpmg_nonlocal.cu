@@ -43,10 +43,12 @@ struct MgLevel {
 struct MgPlan {
     int L, nblocks, total; // levels, blocks, nodes over all levels
     int Lg;                // first level held by block 0 (levels Lg .. L - 1)
-    int sm_zf0, sm_vec, sm_fp64;   // shared memory (floats): level 0's own V-cycle
+    int sm_zf0, sm_vec, sm_alt, sm_fp64;   // shared memory (floats): level 0's own V-cycle
                                    // results; the held levels' vectors (also the
                                    // reduction scratch and the staging area of the
-                                   // spread phases); the FP64 region
+                                   // spread phases); a second extended vector of level 0
+                                   // (in the held levels' rows, which only block 0 uses);
+                                   // the FP64 region
     MgLevel lv[kMgMaxLevels];
     float *coef;           // [9][total]: 9-point rows, q = 3 (dj + 1) + (di + 1)
     float *rsum;           // [total]: row sums
@@ -1018,17 +1020,17 @@ inline size_t pcg_tile_smem(int C, int Nx)
 // Synchronisation between blocks.  Each phase writes its level vector to
 // global memory as 64-bit words: an FP32 value plus a 32-bit tag that names
 // the V-cycle.  A phase stages the words it needs from other blocks (a halo
-// or a band of rows) into shared memory once; if some carry an older tag, a
-// lane polls one of them with a pause after each stale answer and, once that
-// one is current, the warp loads its stale words again together.  A word is stored with one
-// single-copy-atomic 64-bit store, so its value and tag arrive together,
-// with no fences or flags.
-//   * Each phase vector is written once per V-cycle, and the outer grid
-//     barrier separates V-cycles, so no value is overwritten while a reader
-//     may still need it.
+// or a band of rows) into shared memory once, loading those with an older tag
+// again until they are current.  A word is stored with one single-copy-atomic
+// 64-bit store, so its value and tag arrive together, with no fences or flags.
+//   * Each phase vector is written once per V-cycle, and the gather of the
+//     outer inner products (mg_gather4) separates V-cycles, so no value is
+//     overwritten while a reader may still need it.
 //   * Each solve reserves its tags (maxit + 2, from a counter in device
 //     memory), so it never accepts a word written by an earlier solve.
 //   * Polls are bounded, like the barriers.
+// Where only neighbours read a vector (level 0's smoothing steps and result),
+// only the Nx + 1 nodes at either end of a block's range are published.
 
 constexpr int kMgThreads = 512;
 constexpr int kMgTrips = 4;            // nodes of a level a thread owns at most
@@ -1049,8 +1051,8 @@ constexpr float cheb_b(int k) { return k == 0 ? 1.0f / kChebTheta : 2.0f * cheb_
 // polls of one wait before it gives up (a poll is one L2 round trip, about
 // a microsecond: a few seconds in all)
 constexpr long long kMgPollLimit = 1ll << 22;
-// sleep of a waiting warp after a stale answer (ns)
-constexpr unsigned kMgNap = 128;
+// sleep of a waiting warp between its rounds of loads (ns)
+constexpr unsigned kMgNap = 40;
 
 __device__ __forceinline__ unsigned long long mg_ld(const unsigned long long *p)
 {
@@ -1087,32 +1089,25 @@ __device__ __forceinline__ bool mg_give_up(long long polls, int *status)
 }
 
 // Waits until every word of v carries `tag` (addr(t, q) is the address of
-// word q of trip t, for T trips of Q words).  Called by whole warps.  While some lane holds stale
-// words, one lane polls one of them and the warp sleeps kMgNap ns after a
-// stale answer; once that word is current, every lane loads its stale words
-// again together.  A phase so waits a round trip or two after its last
-// input is written, while a waiting warp neither floods L2 with polls (which
-// slows the stores it waits for) nor takes many issue slots from the warps
-// that compute.  Bounded (kMgPollLimit polls, or another block's timeout):
-// then the spin error is set and the words read 0.
+// word q of trip t, for T trips of Q words).  Called by whole warps.  While some
+// lane holds stale words, every lane loads its stale words again, kMgNap ns
+// after the last round: the staged phases wait for a thousand words a block at
+// most, so this floods nothing, and a word is in a register one round trip
+// after it is visible (one lane polling one word and the rest reloaded after
+// it cost a second round trip: 0.456 against 0.441 ms a step on the 130^2
+// silo).  Bounded (kMgPollLimit polls, or another block's timeout): then the
+// spin error is set and the words read 0.
 template <int T, int Q, class Addr>
 __device__ __forceinline__ void mg_resolve(unsigned long long (&v)[T][Q], unsigned tag, int *status, Addr addr)
 {
-    const unsigned lane = threadIdx.x & 31u;
     for (long long polls = 1;; polls++) {
-        int ft = -1, fq = 0;
+        bool stale = false;
 #pragma unroll
-        for (int t = T - 1; t >= 0; t--) {
+        for (int t = 0; t < T; t++) {
 #pragma unroll
-            for (int q = Q - 1; q >= 0; q--) {
-                if ((unsigned)(v[t][q] >> 32) != tag) {
-                    ft = t;
-                    fq = q;
-                }
-            }
+            for (int q = 0; q < Q; q++) stale |= (unsigned)(v[t][q] >> 32) != tag;
         }
-        const unsigned stale = __ballot_sync(0xffffffffu, ft >= 0);
-        if (stale == 0) return;
+        if (!__any_sync(0xffffffffu, stale)) return;
         if (mg_give_up(polls, status)) {
 #pragma unroll
             for (int t = 0; t < T; t++) {
@@ -1121,13 +1116,7 @@ __device__ __forceinline__ void mg_resolve(unsigned long long (&v)[T][Q], unsign
             }
             return;
         }
-        const unsigned leader = __ffs(stale) - 1;
-        int fresh = 0;
-        if (lane == leader) fresh = (unsigned)(mg_ld(addr(ft, fq)) >> 32) == tag;
-        if (!__shfl_sync(0xffffffffu, fresh, leader)) {
-            __nanosleep(kMgNap);
-            continue;
-        }
+        __nanosleep(kMgNap);
 #pragma unroll
         for (int t = 0; t < T; t++) {
 #pragma unroll
@@ -1277,12 +1266,31 @@ __device__ __forceinline__ constexpr bool mg_par2(int o)
     return CO ? (o & 1) != 0 : false;
 }
 
+// Rows of a fine level for the Galerkin products: entry q and row sum of node
+// n, from the global pools (a level spread over the blocks) or from block 0's
+// shared memory (a held level, whose row sums sit in its zf slots during the
+// set-up): a held level's products there wait 30 cycles a load, not an L2 round
+// trip.
+struct MgRowsGlobal {
+    const float *coef, *rs;
+    int total;
+    __device__ __forceinline__ float at(int q, int n) const { return __ldcg(coef + (size_t)q * total + n); }
+    __device__ __forceinline__ float sum(int n) const { return __ldcg(rs + n); }
+};
+struct MgRowsHeld {
+    const float *coef, *rs;
+    int nn;
+    __device__ __forceinline__ float at(int q, int n) const { return coef[q * nn + n]; }
+    __device__ __forceinline__ float sum(int n) const { return rs[n]; }
+};
+
 // Galerkin row of coarse node (ci, cj) of level c from the rows of level
 // c - 1: the nine entries of P^T A P, the row sum P^T s, and the diagonal
 // set to the row sum minus the off-diagonal entries.  CX, CY: the level is
 // coarsened along x, y (every index into the row is then a constant).
-template <int CX, int CY>
-__device__ void mg_galerkin_row_t(const MgPlan &P, int c, int I, int ci, int cj, float *held)
+template <int CX, int CY, class Rows>
+__device__ __forceinline__ void mg_galerkin_row_t(const MgPlan &P, const Rows &R, int c, int I, int ci, int cj,
+                                                  float *held, float *held_sum)
 {
     const MgLevel &F = P.lv[c - 1], &Cl = P.lv[c];
     float acc[9];
@@ -1302,8 +1310,8 @@ __device__ void mg_galerkin_row_t(const MgPlan &P, int c, int I, int ci, int cj,
             in[sx] = (CX || sx == 1) && fx >= 0 && fx < F.Nx && fy >= 0 && fy < F.Ny;
             const int fi = in[sx] ? fy * F.Nx + fx : 0;
 #pragma unroll
-            for (int q = 0; q < 9; q++) a[sx][q] = in[sx] ? __ldcg(P.coef + (size_t)q * P.total + F.g + fi) : 0.0f;
-            sf[sx] = in[sx] ? __ldcg(P.rsum + F.g + fi) : 0.0f;
+            for (int q = 0; q < 9; q++) a[sx][q] = in[sx] ? R.at(q, fi) : 0.0f;
+            sf[sx] = in[sx] ? R.sum(fi) : 0.0f;
         }
 #pragma unroll
         for (int sx = 0; sx < 3; sx++) {
@@ -1327,15 +1335,18 @@ __device__ void mg_galerkin_row_t(const MgPlan &P, int c, int I, int ci, int cj,
     }
     acc[4] = srow - (((acc[0] + acc[1]) + (acc[2] + acc[3])) + ((acc[5] + acc[6]) + (acc[7] + acc[8])));
     mg_put_row(P, Cl.g + I, acc, srow, held, I, Cl.nn);
+    if (held_sum != nullptr) held_sum[I] = srow;
 }
 
-__device__ __noinline__ void mg_galerkin_row(const MgPlan &P, int c, int I, int ci, int cj, float *held)
+template <class Rows>
+__device__ __noinline__ void mg_galerkin_row(const MgPlan &P, const Rows R, int c, int I, float *held, float *held_sum)
 {
     const MgLevel &Cl = P.lv[c];
-    if (Cl.cx && Cl.cy) mg_galerkin_row_t<1, 1>(P, c, I, ci, cj, held);
-    else if (Cl.cx) mg_galerkin_row_t<1, 0>(P, c, I, ci, cj, held);
-    else if (Cl.cy) mg_galerkin_row_t<0, 1>(P, c, I, ci, cj, held);
-    else mg_galerkin_row_t<0, 0>(P, c, I, ci, cj, held);
+    const int cj = (int)mpmg_div((uint32_t)I, Cl.div), ci = I - cj * Cl.Nx;
+    if (Cl.cx && Cl.cy) mg_galerkin_row_t<1, 1>(P, R, c, I, ci, cj, held, held_sum);
+    else if (Cl.cx) mg_galerkin_row_t<1, 0>(P, R, c, I, ci, cj, held, held_sum);
+    else if (Cl.cy) mg_galerkin_row_t<0, 1>(P, R, c, I, ci, cj, held, held_sum);
+    else mg_galerkin_row_t<0, 0>(P, R, c, I, ci, cj, held, held_sum);
 }
 
 // Sum of four values over the block in a fixed order, returned to every
@@ -1504,9 +1515,25 @@ __device__ __forceinline__ unsigned long long *mg_step_words(const MgPlan &P, in
     return P.zs + (size_t)(k + (up ? kMgDegree - 1 : 0)) * P.lv[0].nn;
 }
 
-// Level 0's Chebyshev steps 1 .. kMgDegree - 1 on z (S.z1 down, zown up),
-// whose step 0 is published and whose last correction is p: each stages the
-// halo of the step before, forms r = b - A z and steps.
+// Node of a block's range that trip slot idx handles at level 0: the Nx + 1
+// nodes at either end first (the neighbours wait for those), then the rest.
+__device__ __forceinline__ int mg_slot(int idx, int cnt, int H)
+{
+    if (cnt <= 2 * H || idx < H) return idx;
+    return idx < 2 * H ? cnt - 2 * H + idx : idx - H;
+}
+
+__device__ __forceinline__ bool mg_edge(int k, int cnt, int H)
+{
+    return k < H || k >= cnt - H;
+}
+
+// Level 0's Chebyshev steps 1 .. kMgDegree - 1.  Step 0 is published, its values
+// are at ze + H (ze: P.sm_vec) and its corrections in p, slot t of a thread at
+// mg_slot(threadIdx.x + t kMgThreads).  Each step stages the halo of the step
+// before, forms r = b - A z and steps into the other of two extended vectors;
+// the range's ends come first, so that they travel while the rest is formed.
+// The last step goes to z (own nodes).
 __device__ __forceinline__ void mg_cheb(const MgPlan &P, float *sm, const MgShared &S, float *z, float (&p)[kMgTrips],
                                         bool up, unsigned tag, int *status)
 {
@@ -1515,27 +1542,31 @@ __device__ __forceinline__ void mg_cheb(const MgPlan &P, float *sm, const MgShar
     mg_own_range(lv, blockIdx.x, n0, cnt);
     if (cnt <= 0) return;
     const int H = lv.Nx + 1;
-    float *ze = sm + P.sm_vec;
+    float *cur = sm + P.sm_vec, *other = sm + P.sm_alt;
 #pragma unroll
     for (int k = 1; k < kMgDegree; k++) {
-        for (int c = threadIdx.x; c < cnt; c += kMgThreads) ze[H + c] = z[c];
-        mg_stage(mg_step_words(P, k - 1, up), lv.nn, n0 - H, n0, ze, n0 + cnt, n0 + cnt + H, ze + H + cnt, tag, status);
+        mg_stage(mg_step_words(P, k - 1, up), lv.nn, n0 - H, n0, cur, n0 + cnt, n0 + cnt + H, cur + H + cnt, tag, status);
         unsigned long long *out = mg_step_words(P, k, up);
 #pragma unroll
         for (int t = 0; t < kMgTrips; t++) {
-            const int c = threadIdx.x + t * kMgThreads;
-            if (c >= cnt) continue;
-            const float *v = ze + H + c;
+            const int idx = threadIdx.x + t * kMgThreads;
+            if (idx >= cnt) continue;
+            const int c = mg_slot(idx, cnt, H);
+            const float *v = cur + H + c;
             float acc = 0.0f;
 #pragma unroll
             for (int q = 0; q < 9; q++) acc = fmaf(sm[q * lv.C + c], v[(q / 3 - 1) * lv.Nx + (q % 3 - 1)], acc);
             p[t] = fmaf(cheb_a(k), p[t], cheb_b(k) * sm[9 * lv.C + c] * (S.b[c] - acc));
-            const float zn = z[c] + p[t];
-            z[c] = zn;
-            mg_st(out + n0 + c, zn, tag);
+            const float zn = v[0] + p[t];
+            if (mg_edge(c, cnt, H)) mg_st(out + n0 + c, zn, tag);
+            if (k == kMgDegree - 1) z[c] = zn;
+            else other[H + c] = zn;
         }
-        __syncthreads();
+        float *swap = cur;
+        cur = other;
+        other = swap;
     }
+    __syncthreads();
 }
 
 // Restriction to the spread level c from the spread level c - 1: the fine
@@ -1604,11 +1635,11 @@ __device__ __forceinline__ void mg_restrict_to_held(const MgPlan &P, float *sm, 
 // solution of level l + 1: with z2 = z1 + P zc and res = b - A z1,
 //   z = z2 + omega D_l1^-1 (res - A P zc)   (published; zero off the unknowns)
 // The coarse rows holding the parents of the nodes n0 - H .. n0 + cnt + H
-// are staged, P zc is formed at those nodes, then the stencil runs.  zown:
-// this block's results also into shared memory, or null; level 0 takes step 0
-// of its Chebyshev recurrence here (correction in p) and the others after.
+// are staged, P zc is formed at those nodes, then the stencil runs;
+// level 0 takes step 0 of its Chebyshev recurrence here (correction in p0) and
+// the others after (mg_cheb, whose staging ends with a block barrier).
 __device__ __forceinline__ void mg_prolong(const MgPlan &P, float *sm, int l, const MgShared &S, unsigned tag,
-                                           int *status, float *zown, float (&p0)[kMgTrips])
+                                           int *status, float (&p0)[kMgTrips])
 {
     const float step = l == 0 ? cheb_b(0) : kMgOmega;
     unsigned long long *out = l == 0 ? mg_step_words(P, 0, true) : P.zf + P.lv[l].g;
@@ -1640,10 +1671,12 @@ __device__ __forceinline__ void mg_prolong(const MgPlan &P, float *sm, int l, co
         pz[u] = v;
     }
     __syncthreads();
+    float zn[kMgTrips];
 #pragma unroll
     for (int t = 0; t < kMgTrips; t++) {
-        const int k = threadIdx.x + t * kMgThreads;
-        if (k >= cnt) continue;
+        const int idx = threadIdx.x + t * kMgThreads;
+        if (idx >= cnt) continue;
+        const int k = l == 0 ? mg_slot(idx, cnt, H) : idx;
         const int n = n0 + k;
         const float *p = pz + H + k;
         float acc = 0.0f;
@@ -1651,11 +1684,17 @@ __device__ __forceinline__ void mg_prolong(const MgPlan &P, float *sm, int l, co
         for (int q = 0; q < 9; q++) acc = fmaf(mg_coef(P, sm, l, q, k, n), p[(q / 3 - 1) * lv.Nx + (q % 3 - 1)], acc);
         const float li = mg_l1inv(P, sm, l, k, n);
         p0[t] = step * li * (S.res[k] - acc);
-        const float z = (li == 0.0f) ? 0.0f : S.z1[k] + p[0] + p0[t];
-        mg_st(out + n, z, tag);
-        if (zown != nullptr) zown[k] = z;
+        zn[t] = (li == 0.0f) ? 0.0f : S.z1[k] + p[0] + p0[t];
+        if (l > 0 || mg_edge(k, cnt, H)) mg_st(out + n, zn[t], tag);
     }
     __syncthreads();
+    if (l > 0) return;
+    // level 0's step 0 where mg_cheb reads it (in the place of P zc)
+#pragma unroll
+    for (int t = 0; t < kMgTrips; t++) {
+        const int idx = threadIdx.x + t * kMgThreads;
+        if (idx < cnt) pz[H + mg_slot(idx, cnt, H)] = zn[t];
+    }
 }
 
 // Phases of the levels held by block 0: shared memory only, a block barrier
@@ -1860,7 +1899,8 @@ __device__ void mg_vcycle(const MgPlan &P, float *sm, const double *cinv, unsign
         return;
     }
     {
-        // pre-smoothing at level 0
+        // pre-smoothing at level 0 (b is this block's from before: a barrier)
+        __syncthreads();
         const MgLevel &lv = P.lv[0];
         const MgShared S = mg_shared(sm, lv);
         int n0, cnt;
@@ -1869,15 +1909,15 @@ __device__ void mg_vcycle(const MgPlan &P, float *sm, const double *cinv, unsign
         float p[kMgTrips];
 #pragma unroll
         for (int t = 0; t < kMgTrips; t++) {
-            const int k = threadIdx.x + t * kMgThreads;
+            const int idx = threadIdx.x + t * kMgThreads;
             p[t] = 0.0f;
-            if (k >= cnt) continue;
+            if (idx >= cnt) continue;
+            const int H = lv.Nx + 1, k = mg_slot(idx, cnt, H);
             const float z = cheb_b(0) * sm[9 * lv.C + k] * S.b[k];
             p[t] = z;
-            S.z1[k] = z;
-            mg_st(out + n0 + k, z, tag);
+            sm[P.sm_vec + H + k] = z;
+            if (mg_edge(k, cnt, H)) mg_st(out + n0 + k, z, tag);
         }
-        __syncthreads();
         mg_cheb(P, sm, S, S.z1, p, false, tag, status);
     }
     for (int l = 0; l < Lg; l++) {
@@ -1921,7 +1961,7 @@ __device__ void mg_vcycle(const MgPlan &P, float *sm, const double *cinv, unsign
     }
     float p[kMgTrips] = {};
     for (int l = Lg - 1; l >= 0; l--)
-        mg_prolong(P, sm, l, mg_shared(sm, P.lv[l]), tag, status, l == 0 ? sm + P.sm_zf0 : nullptr, p);
+        mg_prolong(P, sm, l, mg_shared(sm, P.lv[l]), tag, status, p);
     mg_cheb(P, sm, mg_shared(sm, P.lv[0]), sm + P.sm_zf0, p, true, tag, status);
 }
 
@@ -2058,9 +2098,14 @@ __global__ void __launch_bounds__(kMgThreads, 1) pcg_mg_kernel(SolveArgs S, cons
         const MgLevel &lv = P.lv[c];
         int c0, ccnt;
         mg_own_range(lv, blockIdx.x, c0, ccnt);
+        const MgLevel &F = P.lv[c - 1];
+        float *held = lv.local ? sm + lv.sm : nullptr, *held_sum = lv.local ? sm + lv.smv + 3 * lv.nn : nullptr;
+        const MgRowsGlobal Rg{P.coef + F.g, P.rsum + F.g, P.total};
+        const MgRowsHeld Rh{sm + F.sm, sm + F.smv + 3 * F.nn, F.nn};
         for (int k = threadIdx.x; k < ccnt; k += kMgThreads) {
-            const int I = c0 + k, cj = I / lv.Nx, ci = I - cj * lv.Nx;
-            mg_galerkin_row(P, c, I, ci, cj, lv.local ? sm + lv.sm : nullptr);
+            // (a held level 0 keeps its row sums in global memory only)
+            if (F.local && c > 1) mg_galerkin_row(P, Rh, c, c0 + k, held, held_sum);
+            else mg_galerkin_row(P, Rg, c, c0 + k, held, held_sum);
         }
         if (!lv.local) {
             if (!tile_grid_barrier(S.barrier, ++episode * (unsigned)nblocks, S.status)) return;
@@ -2096,7 +2141,7 @@ __global__ void __launch_bounds__(kMgThreads, 1) pcg_mg_kernel(SolveArgs S, cons
         for (int piv = 0; piv < nc; piv++) {
             if (threadIdx.x == 0) {
                 const double d = gj[piv * w2 + piv];
-                sh_scalar[0] = d > 0 ? 1.0 / d : 0.0;     // one reciprocal a pivot
+                sh_scalar[0] = d > 0 ? mat::quot(1.0, d) : 0.0;     // one reciprocal a pivot
             }
             __syncthreads();
             const double id = sh_scalar[0];
@@ -2492,11 +2537,14 @@ int mpmg_nonlocal_init(mpmg_ctx *ctx)
                 P.lv[l].sm = off;                        // spread levels: b, z1, res
                 off += 3 * P.lv[l].C;
             }
+            P.sm_alt = off;
             for (int l = P.Lg; l < L; l++) {
                 if (l == 0) continue;                    // a held level 0 keeps its rows at 0
                 P.lv[l].sm = off;                        // held levels' rows
                 off += 10 * P.lv[l].nn;
             }
+            const int alt = P.Lg > 0 ? P.lv[0].C + 2 * (P.lv[0].Nx + 1) : 0;
+            if (off < P.sm_alt + alt) off = P.sm_alt + alt;
             P.sm_zf0 = off;
             off += P.lv[0].C;
             off = (off + 1) & ~1;
