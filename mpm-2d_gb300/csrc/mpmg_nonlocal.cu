@@ -1130,7 +1130,7 @@ __device__ __forceinline__ void mg_resolve(unsigned long long (&v)[T][Q], unsign
 // Copies the words of two node ranges of a level vector (nn nodes), [a0, a1)
 // to d0 and [b0, b1) to d1, as floats once they carry `tag`; nodes outside
 // the level read 0.  Called by the whole block; ends with a block barrier.
-__device__ __forceinline__ void mg_stage(const unsigned long long *w, int nn, int a0, int a1, float *d0, int b0,
+__device__ __noinline__ void mg_stage(const unsigned long long *w, int nn, int a0, int a1, float *d0, int b0,
                                          int b1, float *d1, unsigned tag, int *status)
 {
     constexpr int T = 4;
@@ -1494,6 +1494,7 @@ __device__ __forceinline__ void mg_residual(const MgPlan &P, float *sm, int l, c
     float *ze = sm + P.sm_vec;          // z1 at nodes n0 - H .. n0 + cnt + H
     for (int k = threadIdx.x; k < cnt; k += kMgThreads) ze[H + k] = S.z1[k];
     mg_stage(words, lv.nn, n0 - H, n0, ze, n0 + cnt, n0 + cnt + H, ze + H + cnt, tag, status);
+#pragma unroll 1
     for (int k = threadIdx.x; k < cnt; k += kMgThreads) {
         const int n = n0 + k;
         const float *z = ze + H + k;
@@ -1529,38 +1530,41 @@ __device__ __forceinline__ bool mg_edge(int k, int cnt, int H)
 }
 
 // Level 0's Chebyshev steps 1 .. kMgDegree - 1.  Step 0 is published, its values
-// are at ze + H (ze: P.sm_vec) and its corrections in p, slot t of a thread at
-// mg_slot(threadIdx.x + t kMgThreads).  Each step stages the halo of the step
-// before, forms r = b - A z and steps into the other of two extended vectors;
-// the range's ends come first, so that they travel while the rest is formed.
-// The last step goes to z (own nodes).
-__device__ __forceinline__ void mg_cheb(const MgPlan &P, float *sm, const MgShared &S, float *z, float (&p)[kMgTrips],
-                                        bool up, unsigned tag, int *status)
+// are at cur + H and its corrections in S.res.  Each step stages the halo of the
+// step before, forms r = b - A z and steps into the other of two extended
+// vectors; the range's ends come first, so that they travel while the rest is
+// formed.  The last step goes to z (own nodes).  One rolled loop, called for
+// both ways: the V-cycle's phases run once each an iteration, and their code
+// misses the instruction cache where it is unrolled (a step of 512 nodes took
+// 1.5 to 2.3 us of straight-line code).
+__device__ __noinline__ void mg_cheb(const MgPlan &P, float *sm, const MgShared S, float *z, float *cur, float *other,
+                                     bool up, unsigned tag, int *status)
 {
     const MgLevel &lv = P.lv[0];
     int n0, cnt;
     mg_own_range(lv, blockIdx.x, n0, cnt);
     if (cnt <= 0) return;
-    const int H = lv.Nx + 1;
-    float *cur = sm + P.sm_vec, *other = sm + P.sm_alt;
-#pragma unroll
+    const int Nx = lv.Nx, H = Nx + 1, C = lv.C;
+    const float *li = sm + 9 * C;
+#pragma unroll 1
     for (int k = 1; k < kMgDegree; k++) {
         mg_stage(mg_step_words(P, k - 1, up), lv.nn, n0 - H, n0, cur, n0 + cnt, n0 + cnt + H, cur + H + cnt, tag, status);
-        unsigned long long *out = mg_step_words(P, k, up);
-#pragma unroll
-        for (int t = 0; t < kMgTrips; t++) {
-            const int idx = threadIdx.x + t * kMgThreads;
-            if (idx >= cnt) continue;
+        unsigned long long *out = mg_step_words(P, k, up) + n0;
+        const float ca = k == 1 ? cheb_a(1) : cheb_a(2), cb = k == 1 ? cheb_b(1) : cheb_b(2);
+        static_assert(kMgDegree <= 3, "the coefficients above");
+        float *dst = k == kMgDegree - 1 ? z : other + H;
+#pragma unroll 1
+        for (int idx = threadIdx.x; idx < cnt; idx += kMgThreads) {
             const int c = mg_slot(idx, cnt, H);
-            const float *v = cur + H + c;
+            const float *v = cur + H + c, *a = sm + c;
             float acc = 0.0f;
 #pragma unroll
-            for (int q = 0; q < 9; q++) acc = fmaf(sm[q * lv.C + c], v[(q / 3 - 1) * lv.Nx + (q % 3 - 1)], acc);
-            p[t] = fmaf(cheb_a(k), p[t], cheb_b(k) * sm[9 * lv.C + c] * (S.b[c] - acc));
-            const float zn = v[0] + p[t];
-            if (mg_edge(c, cnt, H)) mg_st(out + n0 + c, zn, tag);
-            if (k == kMgDegree - 1) z[c] = zn;
-            else other[H + c] = zn;
+            for (int q = 0; q < 9; q++) acc = fmaf(a[q * C], v[(q / 3 - 1) * Nx + (q % 3 - 1)], acc);
+            const float p = fmaf(ca, S.res[c], cb * li[c] * (S.b[c] - acc));
+            S.res[c] = p;
+            const float zn = v[0] + p;
+            if (mg_edge(c, cnt, H)) mg_st(out + c, zn, tag);
+            dst[c] = zn;
         }
         float *swap = cur;
         cur = other;
@@ -1583,6 +1587,7 @@ __device__ __forceinline__ void mg_restrict(const MgPlan &P, float *sm, int c, c
     mg_fine_rows(lv, F, c0, cnt, fa, fb);
     float *rf = sm + P.sm_vec;          // fine residual rows fa .. fb
     mg_stage(P.res + F.g, F.nn, fa * F.Nx, (fb + 1) * F.Nx, rf, 0, 0, rf, tag, status);
+#pragma unroll 1
     for (int k = threadIdx.x; k < cnt; k += kMgThreads) {
         const int I = c0 + k, cj = (int)mpmg_div((uint32_t)I, lv.div), ci = I - cj * lv.Nx;
         float b = 0.0f;
@@ -1616,6 +1621,7 @@ __device__ __forceinline__ void mg_restrict_to_held(const MgPlan &P, float *sm, 
     mg_fine_rows(lv, F, c0, cnt, fa, fb);
     float *rf = sm + P.sm_vec;          // fine residual rows fa .. fb
     mg_stage(P.res + F.g, F.nn, fa * F.Nx, (fb + 1) * F.Nx, rf, 0, 0, rf, tag, status);
+#pragma unroll 1
     for (int k = threadIdx.x; k < cnt; k += kMgThreads) {
         const int I = c0 + k, cj = (int)mpmg_div((uint32_t)I, lv.div), ci = I - cj * lv.Nx;
         float b = 0.0f;
@@ -1636,10 +1642,10 @@ __device__ __forceinline__ void mg_restrict_to_held(const MgPlan &P, float *sm, 
 //   z = z2 + omega D_l1^-1 (res - A P zc)   (published; zero off the unknowns)
 // The coarse rows holding the parents of the nodes n0 - H .. n0 + cnt + H
 // are staged, P zc is formed at those nodes, then the stencil runs;
-// level 0 takes step 0 of its Chebyshev recurrence here (correction in p0) and
-// the others after (mg_cheb, whose staging ends with a block barrier).
+// level 0 takes step 0 of its Chebyshev recurrence here (correction in S.res)
+// and the others after (mg_cheb).
 __device__ __forceinline__ void mg_prolong(const MgPlan &P, float *sm, int l, const MgShared &S, unsigned tag,
-                                           int *status, float (&p0)[kMgTrips])
+                                           int *status)
 {
     const float step = l == 0 ? cheb_b(0) : kMgOmega;
     unsigned long long *out = l == 0 ? mg_step_words(P, 0, true) : P.zf + P.lv[l].g;
@@ -1653,6 +1659,7 @@ __device__ __forceinline__ void mg_prolong(const MgPlan &P, float *sm, int l, co
     float *pz = sm + P.sm_vec;          // P zc at nodes n0 - H .. n0 + cnt + H
     float *cz = pz + E;                 // coarse rows ya .. yb
     mg_stage(P.zf + Cl.g, Cl.nn, ya * Cl.Nx, (yb + 1) * Cl.Nx, cz, 0, 0, cz, tag, status);
+#pragma unroll 1
     for (int u = threadIdx.x; u < E; u += kMgThreads) {
         const int m = n0 - H + u;
         float v = 0.0f;
@@ -1671,11 +1678,9 @@ __device__ __forceinline__ void mg_prolong(const MgPlan &P, float *sm, int l, co
         pz[u] = v;
     }
     __syncthreads();
-    float zn[kMgTrips];
-#pragma unroll
-    for (int t = 0; t < kMgTrips; t++) {
-        const int idx = threadIdx.x + t * kMgThreads;
-        if (idx >= cnt) continue;
+    float *z0 = sm + P.sm_alt + H;      // level 0's step 0, where mg_cheb reads it
+#pragma unroll 1
+    for (int idx = threadIdx.x; idx < cnt; idx += kMgThreads) {
         const int k = l == 0 ? mg_slot(idx, cnt, H) : idx;
         const int n = n0 + k;
         const float *p = pz + H + k;
@@ -1683,18 +1688,15 @@ __device__ __forceinline__ void mg_prolong(const MgPlan &P, float *sm, int l, co
 #pragma unroll
         for (int q = 0; q < 9; q++) acc = fmaf(mg_coef(P, sm, l, q, k, n), p[(q / 3 - 1) * lv.Nx + (q % 3 - 1)], acc);
         const float li = mg_l1inv(P, sm, l, k, n);
-        p0[t] = step * li * (S.res[k] - acc);
-        zn[t] = (li == 0.0f) ? 0.0f : S.z1[k] + p[0] + p0[t];
-        if (l > 0 || mg_edge(k, cnt, H)) mg_st(out + n, zn[t], tag);
+        const float d = step * li * (S.res[k] - acc);
+        const float z = (li == 0.0f) ? 0.0f : S.z1[k] + p[0] + d;
+        if (l > 0 || mg_edge(k, cnt, H)) mg_st(out + n, z, tag);
+        if (l == 0) {
+            S.res[k] = d;
+            z0[k] = z;
+        }
     }
     __syncthreads();
-    if (l > 0) return;
-    // level 0's step 0 where mg_cheb reads it (in the place of P zc)
-#pragma unroll
-    for (int t = 0; t < kMgTrips; t++) {
-        const int idx = threadIdx.x + t * kMgThreads;
-        if (idx < cnt) pz[H + mg_slot(idx, cnt, H)] = zn[t];
-    }
 }
 
 // Phases of the levels held by block 0: shared memory only, a block barrier
@@ -1906,19 +1908,16 @@ __device__ void mg_vcycle(const MgPlan &P, float *sm, const double *cinv, unsign
         int n0, cnt;
         mg_own_range(lv, blockIdx.x, n0, cnt);
         unsigned long long *out = mg_step_words(P, 0, false);
-        float p[kMgTrips];
-#pragma unroll
-        for (int t = 0; t < kMgTrips; t++) {
-            const int idx = threadIdx.x + t * kMgThreads;
-            p[t] = 0.0f;
-            if (idx >= cnt) continue;
-            const int H = lv.Nx + 1, k = mg_slot(idx, cnt, H);
+        const int H = lv.Nx + 1;
+#pragma unroll 1
+        for (int idx = threadIdx.x; idx < cnt; idx += kMgThreads) {
+            const int k = mg_slot(idx, cnt, H);
             const float z = cheb_b(0) * sm[9 * lv.C + k] * S.b[k];
-            p[t] = z;
+            S.res[k] = z;
             sm[P.sm_vec + H + k] = z;
             if (mg_edge(k, cnt, H)) mg_st(out + n0 + k, z, tag);
         }
-        mg_cheb(P, sm, S, S.z1, p, false, tag, status);
+        mg_cheb(P, sm, S, S.z1, sm + P.sm_vec, sm + P.sm_alt, false, tag, status);
     }
     for (int l = 0; l < Lg; l++) {
         mg_residual(P, sm, l, mg_shared(sm, P.lv[l]), P.z1 + P.lv[l].g, tag, status);
@@ -1959,10 +1958,8 @@ __device__ void mg_vcycle(const MgPlan &P, float *sm, const double *cinv, unsign
         for (int n = threadIdx.x; n < H.nn; n += blockDim.x) mg_st(P.zf + P.lv[Lg].g + n, H.zf[n], tag);
         __syncthreads();      // the staging area of the spread phases aliases the held vectors
     }
-    float p[kMgTrips] = {};
-    for (int l = Lg - 1; l >= 0; l--)
-        mg_prolong(P, sm, l, mg_shared(sm, P.lv[l]), tag, status, p);
-    mg_cheb(P, sm, mg_shared(sm, P.lv[0]), sm + P.sm_zf0, p, true, tag, status);
+    for (int l = Lg - 1; l >= 0; l--) mg_prolong(P, sm, l, mg_shared(sm, P.lv[l]), tag, status);
+    mg_cheb(P, sm, mg_shared(sm, P.lv[0]), sm + P.sm_zf0, sm + P.sm_alt, sm + P.sm_vec, true, tag, status);
 }
 
 // Shared memory of pcg_mg_kernel (the offsets are in the plan): level 0's
