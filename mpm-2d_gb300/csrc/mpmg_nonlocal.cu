@@ -37,6 +37,7 @@ struct MgLevel {
     int g;                 // first node of the level in the global pools
     int sm;                // shared memory (floats): spread level: its b, z1, res; held
                            // level: its rows (coef[9][nn], l1inv[nn])
+    int smr;               // spread level: its rows (coef[9][C], l1inv[C])
     int smv;               // held level: its b, z1, res, zf (shared memory, floats)
 };
 
@@ -47,8 +48,8 @@ struct MgPlan {
                                    // results; the held levels' vectors (also the
                                    // reduction scratch and the staging area of the
                                    // spread phases); a second extended vector of level 0
-                                   // (in the held levels' rows, which only block 0 uses);
-                                   // the FP64 region
+                                   // (in the held levels' rows, which only block 0 uses,
+                                   // as are the spread levels' rows); the FP64 region
     MgLevel lv[kMgMaxLevels];
     float *coef;           // [9][total]: 9-point rows, q = 3 (dj + 1) + (di + 1)
     float *rsum;           // [total]: row sums
@@ -1033,6 +1034,7 @@ inline size_t pcg_tile_smem(int C, int Nx)
 // only the Nx + 1 nodes at either end of a block's range are published.
 
 constexpr int kMgThreads = 512;
+constexpr int kMgBlocks = 160;         // blocks of the solve at most (mg_gather4: five a lane)
 constexpr int kMgTrips = 4;            // nodes of a level a thread owns at most
 constexpr int kMgLocal = kMgTrips * kMgThreads;   // levels this small are held by block 0
 constexpr int kMgCoarse = 9;           // nodes of the coarsest level at most (3 x 3)
@@ -1158,8 +1160,8 @@ __device__ __noinline__ void mg_stage(const unsigned long long *w, int nn, int a
 }
 
 // Per-level arrays in shared memory (floats).  A level spread over the
-// blocks keeps its b, z1, res (C each) at lv.sm; level 0 also keeps its rows
-// at float 0 (coef0[9][C0], l1inv0[C0]).  A level held by block 0 keeps its
+// blocks keeps its b, z1, res (C each) at lv.sm and its rows (coef[9][C],
+// l1inv[C]) at lv.smr (level 0: float 0).  A level held by block 0 keeps its
 // rows at lv.sm and b, z1, res, zf (nn each) at lv.smv.
 struct MgShared {
     float *b, *z1, *res;
@@ -1172,21 +1174,6 @@ __device__ __forceinline__ MgShared mg_shared(float *sm, const MgLevel &lv)
     s.z1 = s.b + lv.C;
     s.res = s.z1 + lv.C;
     return s;
-}
-
-// Row entry q of own node k (global node n) of level l, and D_l1^-1.
-__device__ __forceinline__ float mg_coef(const MgPlan &P, const float *sm, int l, int q, int k, int n)
-{
-    if (l == 0) return sm[q * P.lv[0].C + k];
-    if (P.lv[l].local) return sm[P.lv[l].sm + q * P.lv[l].nn + n];
-    return __ldcg(P.coef + (size_t)q * P.total + P.lv[l].g + n);
-}
-
-__device__ __forceinline__ float mg_l1inv(const MgPlan &P, const float *sm, int l, int k, int n)
-{
-    if (l == 0) return sm[9 * P.lv[0].C + k];
-    if (P.lv[l].local) return sm[P.lv[l].sm + 9 * P.lv[l].nn + n];
-    return __ldcg(P.l1inv + P.lv[l].g + n);
 }
 
 // Coarse parents of fine coordinate g along a direction: g even (or the
@@ -1290,7 +1277,7 @@ struct MgRowsHeld {
 // coarsened along x, y (every index into the row is then a constant).
 template <int CX, int CY, class Rows>
 __device__ __forceinline__ void mg_galerkin_row_t(const MgPlan &P, const Rows &R, int c, int I, int ci, int cj,
-                                                  float *held, float *held_sum)
+                                                  float *held, float *held_sum, int k, int nn)
 {
     const MgLevel &F = P.lv[c - 1], &Cl = P.lv[c];
     float acc[9];
@@ -1334,19 +1321,20 @@ __device__ __forceinline__ void mg_galerkin_row_t(const MgPlan &P, const Rows &R
         }
     }
     acc[4] = srow - (((acc[0] + acc[1]) + (acc[2] + acc[3])) + ((acc[5] + acc[6]) + (acc[7] + acc[8])));
-    mg_put_row(P, Cl.g + I, acc, srow, held, I, Cl.nn);
-    if (held_sum != nullptr) held_sum[I] = srow;
+    mg_put_row(P, Cl.g + I, acc, srow, held, k, nn);
+    if (held_sum != nullptr) held_sum[k] = srow;
 }
 
 template <class Rows>
-__device__ __noinline__ void mg_galerkin_row(const MgPlan &P, const Rows R, int c, int I, float *held, float *held_sum)
+__device__ __noinline__ void mg_galerkin_row(const MgPlan &P, const Rows R, int c, int I, float *held, float *held_sum,
+                                             int k)
 {
     const MgLevel &Cl = P.lv[c];
     const int cj = (int)mpmg_div((uint32_t)I, Cl.div), ci = I - cj * Cl.Nx;
-    if (Cl.cx && Cl.cy) mg_galerkin_row_t<1, 1>(P, R, c, I, ci, cj, held, held_sum);
-    else if (Cl.cx) mg_galerkin_row_t<1, 0>(P, R, c, I, ci, cj, held, held_sum);
-    else if (Cl.cy) mg_galerkin_row_t<0, 1>(P, R, c, I, ci, cj, held, held_sum);
-    else mg_galerkin_row_t<0, 0>(P, R, c, I, ci, cj, held, held_sum);
+    if (Cl.cx && Cl.cy) mg_galerkin_row_t<1, 1>(P, R, c, I, ci, cj, held, held_sum, k, Cl.C);
+    else if (Cl.cx) mg_galerkin_row_t<1, 0>(P, R, c, I, ci, cj, held, held_sum, k, Cl.C);
+    else if (Cl.cy) mg_galerkin_row_t<0, 1>(P, R, c, I, ci, cj, held, held_sum, k, Cl.C);
+    else mg_galerkin_row_t<0, 0>(P, R, c, I, ci, cj, held, held_sum, k, Cl.C);
 }
 
 // Sum of four values over the block in a fixed order, returned to every
@@ -1447,7 +1435,7 @@ __device__ __forceinline__ void mg_gather4(const mat::Unit &u, unsigned long lon
     }
     if (threadIdx.x < 128) {
         const int lane = threadIdx.x & 31, c = threadIdx.x >> 5;
-        constexpr int kMax = 8;     // blocks <= 32 * kMax
+        constexpr int kMax = kMgBlocks / 32;
         unsigned long long p[kMax][2];
         const unsigned long long *base = words + 2 * (size_t)c * nblocks;
 #pragma unroll
@@ -1490,6 +1478,8 @@ __device__ __forceinline__ void mg_residual(const MgPlan &P, float *sm, int l, c
     int n0, cnt;
     mg_own_range(lv, blockIdx.x, n0, cnt);
     if (cnt <= 0) return;
+    const int C = lv.C;
+    const float *rows = sm + lv.smr;
     const int H = lv.Nx + 1;
     float *ze = sm + P.sm_vec;          // z1 at nodes n0 - H .. n0 + cnt + H
     for (int k = threadIdx.x; k < cnt; k += kMgThreads) ze[H + k] = S.z1[k];
@@ -1498,9 +1488,10 @@ __device__ __forceinline__ void mg_residual(const MgPlan &P, float *sm, int l, c
     for (int k = threadIdx.x; k < cnt; k += kMgThreads) {
         const int n = n0 + k;
         const float *z = ze + H + k;
+        const float *a = rows + k;
         float acc = 0.0f;
 #pragma unroll
-        for (int q = 0; q < 9; q++) acc = fmaf(mg_coef(P, sm, l, q, k, n), z[(q / 3 - 1) * lv.Nx + (q % 3 - 1)], acc);
+        for (int q = 0; q < 9; q++) acc = fmaf(a[q * C], z[(q / 3 - 1) * lv.Nx + (q % 3 - 1)], acc);
         const float r = S.b[k] - acc;
         S.res[k] = r;
         mg_st(P.res + lv.g + n, r, tag);
@@ -1599,7 +1590,7 @@ __device__ __forceinline__ void mg_restrict(const MgPlan &P, float *sm, int c, c
             b = fmaf(w, rf[(fy - fa) * F.Nx + fx], b);
         }
         S.b[k] = b;
-        const float z = kMgOmega * mg_l1inv(P, sm, c, k, I) * b;
+        const float z = kMgOmega * sm[lv.smr + 9 * lv.C + k] * b;
         S.z1[k] = z;
         mg_st(P.z1 + lv.g + I, z, tag);
     }
@@ -1653,6 +1644,8 @@ __device__ __forceinline__ void mg_prolong(const MgPlan &P, float *sm, int l, co
     int n0, cnt;
     mg_own_range(lv, blockIdx.x, n0, cnt);
     if (cnt <= 0) return;
+    const int C = lv.C;
+    const float *rows = sm + lv.smr;
     const int H = lv.Nx + 1, E = cnt + 2 * H;
     int ya, yb;
     mg_parent_rows(lv, Cl, n0, cnt, ya, yb);
@@ -1684,10 +1677,11 @@ __device__ __forceinline__ void mg_prolong(const MgPlan &P, float *sm, int l, co
         const int k = l == 0 ? mg_slot(idx, cnt, H) : idx;
         const int n = n0 + k;
         const float *p = pz + H + k;
+        const float *a = rows + k;
         float acc = 0.0f;
 #pragma unroll
-        for (int q = 0; q < 9; q++) acc = fmaf(mg_coef(P, sm, l, q, k, n), p[(q / 3 - 1) * lv.Nx + (q % 3 - 1)], acc);
-        const float li = mg_l1inv(P, sm, l, k, n);
+        for (int q = 0; q < 9; q++) acc = fmaf(a[q * C], p[(q / 3 - 1) * lv.Nx + (q % 3 - 1)], acc);
+        const float li = rows[9 * C + k];
         const float d = step * li * (S.res[k] - acc);
         const float z = (li == 0.0f) ? 0.0f : S.z1[k] + p[0] + d;
         if (l > 0 || mg_edge(k, cnt, H)) mg_st(out + n, z, tag);
@@ -2027,12 +2021,8 @@ __global__ void __launch_bounds__(kMgThreads, 1) pcg_mg_kernel(SolveArgs S, cons
     // start; FP32 rows (global for the Galerkin products, and this block's in
     // shared memory).  Entries towards nodes that are not unknowns are left
     // out of the FP32 rows, whose own rows are zero.
-#pragma unroll
-    for (int t = 0; t < kMgTrips; t++) {
-        const int k = threadIdx.x + t * kMgThreads;
-        x[t] = 0;
-        sv[t] = 0;
-        if (k >= cnt) continue;
+#pragma unroll 1
+    for (int k = threadIdx.x; k < cnt; k += kMgThreads) {
         const int n = n0 + k, j = n / Nx, i = n - j * Nx;
         double cf[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
         double f = 0;
@@ -2047,8 +2037,9 @@ __global__ void __launch_bounds__(kMgThreads, 1) pcg_mg_kernel(SolveArgs S, cons
         const bool unknown = dof && mat::is_pos(cf[4]);
         if (unknown) {
             r[k] = f;
-            x[t] = (warm && coupled) ? S.x[n] : 0.0;
+            if (!warm || !coupled) S.x[n] = 0;
         } else {
+            S.x[n] = 0;
             r[k] = 0;
 #pragma unroll
             for (int q = 0; q < 9; q++) cf[q] = 0;
@@ -2056,7 +2047,6 @@ __global__ void __launch_bounds__(kMgThreads, 1) pcg_mg_kernel(SolveArgs S, cons
         S.p[n] = 0;
 #pragma unroll
         for (int q = 0; q < 9; q++) S.coef[(size_t)q * nn + n] = cf[q];
-        S.x[n] = x[t];
         double rsum = 0;
         float a[9];
 #pragma unroll
@@ -2070,6 +2060,12 @@ __global__ void __launch_bounds__(kMgThreads, 1) pcg_mg_kernel(SolveArgs S, cons
         }
         mg_put_row(P, n, a, mg_narrow(rsum, 0), sm, k, L0.C);
         if (unknown) bbp = fma(f, f, bbp);
+    }
+#pragma unroll
+    for (int t = 0; t < kMgTrips; t++) {
+        const int k = threadIdx.x + t * kMgThreads;
+        x[t] = warm && k < cnt ? S.x[n0 + k] : 0.0;
+        sv[t] = 0;
     }
     // From a zero start r = b: <b, b> rides on the first grid barrier (a warm
     // start forms r = b - A x and its sums after the set-up instead).
@@ -2096,13 +2092,15 @@ __global__ void __launch_bounds__(kMgThreads, 1) pcg_mg_kernel(SolveArgs S, cons
         int c0, ccnt;
         mg_own_range(lv, blockIdx.x, c0, ccnt);
         const MgLevel &F = P.lv[c - 1];
-        float *held = lv.local ? sm + lv.sm : nullptr, *held_sum = lv.local ? sm + lv.smv + 3 * lv.nn : nullptr;
+        // a level's rows also go to the shared memory of the block that works
+        // on them: block 0's held levels, the other blocks' share of a spread one
+        float *held = lv.local ? sm + lv.sm : sm + lv.smr, *held_sum = lv.local ? sm + lv.smv + 3 * lv.nn : nullptr;
         const MgRowsGlobal Rg{P.coef + F.g, P.rsum + F.g, P.total};
         const MgRowsHeld Rh{sm + F.sm, sm + F.smv + 3 * F.nn, F.nn};
         for (int k = threadIdx.x; k < ccnt; k += kMgThreads) {
             // (a held level 0 keeps its row sums in global memory only)
-            if (F.local && c > 1) mg_galerkin_row(P, Rh, c, c0 + k, held, held_sum);
-            else mg_galerkin_row(P, Rg, c, c0 + k, held, held_sum);
+            if (F.local && c > 1) mg_galerkin_row(P, Rh, c, c0 + k, held, held_sum, k);
+            else mg_galerkin_row(P, Rg, c, c0 + k, held, held_sum, k);
         }
         if (!lv.local) {
             if (!tile_grid_barrier(S.barrier, ++episode * (unsigned)nblocks, S.status)) return;
@@ -2248,12 +2246,15 @@ __global__ void __launch_bounds__(kMgThreads, 1) pcg_mg_kernel(SolveArgs S, cons
         const unsigned tag = tag0 + (unsigned)v;
         // p = u + beta p, x += alpha p, with u = 2^sc_prev zf0 (the last
         // V-cycle's result, in zf0 until level 0's prolongation)
+        // and <r, r>
+        double rr_part = 0;
         auto defer = [&]() {
-            if (v == 0) return;
 #pragma unroll
             for (int t = 0; t < kMgTrips; t++) {
                 const int k = threadIdx.x + t * kMgThreads;
                 if (k >= cnt) continue;
+                rr_part = fma(r[k], r[k], rr_part);
+                if (v == 0) continue;
                 const int n = n0 + k;
                 const double pk = fma(beta, S.p[n], mg_wide(zf0[k], sc_prev));
                 S.p[n] = pk;
@@ -2273,7 +2274,8 @@ __global__ void __launch_bounds__(kMgThreads, 1) pcg_mg_kernel(SolveArgs S, cons
                 for (int k = threadIdx.x; k < cnt; k += kMgThreads) st[H + k] = zf0[k];
                 mg_stage(P.zf, nn, n0 - H, n0, st, n0 + cnt, n0 + cnt + H, st + H + cnt, tag, S.status);
             }
-            part[0] = part[1] = part[2] = part[3] = 0;
+            part[0] = part[1] = part[2] = 0;
+            part[3] = rr_part;
 #pragma unroll
             for (int t = 0; t < kMgTrips; t++) {
                 const int k = threadIdx.x + t * kMgThreads;
@@ -2295,7 +2297,6 @@ __global__ void __launch_bounds__(kMgThreads, 1) pcg_mg_kernel(SolveArgs S, cons
                 part[0] = fma(rk, uk, part[0]);
                 part[1] = fma(wk, uk, part[1]);
                 part[2] = fma(sv[t], uk, part[2]);
-                part[3] = fma(rk, rk, part[3]);
             }
         }
         __syncthreads();      // the scratch aliases the held levels' vectors (a held level 0's zf)
@@ -2489,6 +2490,7 @@ int mpmg_nonlocal_init(mpmg_ctx *ctx)
         // a grid whose level 0 fits one block runs on one block
         int nb = nn <= (size_t)kMgLocal ? 1 : (int)((nn + kMgThreads - 1) / kMgThreads);
         if (nb > sms) nb = sms;
+        if (nb > kMgBlocks) nb = kMgBlocks;
         if (nb < 1) nb = 1;
         int Nx = ctx->cfg.Nx, Ny = ctx->cfg.Ny, L = 0, total = 0, cxs = 0, cys = 0;
         bool ok = Nx >= 1 && Ny >= 1;
@@ -2501,11 +2503,12 @@ int mpmg_nonlocal_init(mpmg_ctx *ctx)
             // on one block every level is held; otherwise level 0 is spread
             // and the coarser levels of at most kMgLocal nodes are held
             lv.local = (nb == 1 || (L > 0 && lv.nn <= kMgLocal)) ? 1 : 0;
-            // a spread level 0 is shared by blocks 1 .. nb - 1: block 0, which
-            // runs the held levels, then has no level-0 work (the outer
+            // the spread levels are shared by blocks 1 .. nb - 1: block 0, which
+            // runs the held levels, then has no other work (the outer
             // iteration's p and x updates of the other blocks run while it
-            // holds the V-cycle)
-            lv.b0 = (L == 0 && !lv.local) ? 1 : 0;
+            // holds the V-cycle), and the others' rows of the spread levels
+            // fit where block 0 keeps the held ones
+            lv.b0 = lv.local ? 0 : 1;
             lv.C = lv.local ? lv.nn : (lv.nn + (nb - lv.b0) - 1) / (nb - lv.b0);
             lv.cx = cxs;
             lv.cy = cys;
@@ -2540,8 +2543,13 @@ int mpmg_nonlocal_init(mpmg_ctx *ctx)
                 P.lv[l].sm = off;                        // held levels' rows
                 off += 10 * P.lv[l].nn;
             }
-            const int alt = P.Lg > 0 ? P.lv[0].C + 2 * (P.lv[0].Nx + 1) : 0;
-            if (off < P.sm_alt + alt) off = P.sm_alt + alt;
+            int alt = P.sm_alt + (P.Lg > 0 ? P.lv[0].C + 2 * (P.lv[0].Nx + 1) : 0);
+            P.lv[0].smr = 0;
+            for (int l = 1; l < P.Lg; l++) {
+                P.lv[l].smr = alt;                       // spread levels' rows (blocks 1 .. nb - 1)
+                alt += 10 * P.lv[l].C;
+            }
+            if (off < alt) off = alt;
             P.sm_zf0 = off;
             off += P.lv[0].C;
             off = (off + 1) & ~1;
