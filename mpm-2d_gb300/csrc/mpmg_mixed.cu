@@ -1112,8 +1112,12 @@ __global__ void __launch_bounds__(kG2PTile, 768 / kG2PTile) mx_g2p_kernel(
 // g_nonlocal_mu2 element blocks and right-hand sides (g_nonlocal_mu2.c:418-507)
 // from the stored particles of this step's binned order: start-of-step shape
 // functions (the local coordinates still in S.A), updated volume, dense flag,
-// local fluidity and cooperativity from the G2P.  FP32 sums of an element's
-// few particles, stored in FP64 for the solver.
+// local fluidity and cooperativity from the G2P.  The sums are FP64: an element
+// with few particles has a block of deficient rank, and FP32 sums make its null
+// vectors' eigenvalues as often negative as positive at 1e-8 of the diagonal,
+// far above the matrix's shift, so that the conjugate gradients broke down on
+// about one step in 600 of a draining silo.  The gradient part comes from five
+// moments of v, as in the FP64 step's assembly.
 __device__ __forceinline__ int sym_index_m(int a, int b)
 {
     if (a > b) {
@@ -1134,32 +1138,43 @@ __global__ void __launch_bounds__(128) mx_assemble_kernel(int ne, float inv_h, c
     if (e >= ne) return;
     const int k0 = cell_start[e], k1 = cell_start[e + 1];
     if (k0 == k1) return;
-    float K[10], F[4];
+    double K[10], F[4];
 #pragma unroll
-    for (int k = 0; k < 10; k++) K[k] = 0.0f;
+    for (int k = 0; k < 10; k++) K[k] = 0;
 #pragma unroll
-    for (int k = 0; k < 4; k++) F[k] = 0.0f;
+    for (int k = 0; k < 4; k++) F[k] = 0;
+    double m0 = 0, ma = 0, maa = 0, mb = 0, mbb = 0;
     for (int k = k0; k < k1; k++) {
         const uint32_t i = perm[k];
         const float4 f4 = nl.F[i];
         if (f4.w == 0.0f) continue;      // not dense
         const float4 a4 = SA[i];
-        const float a = a4.x, b = a4.y, ox = 1.0f - a, oy = 1.0f - b;
-        const float sf[4] = {ox * oy, a * oy, a * b, ox * b};
-        const float gx[4] = {-oy * inv_h, oy * inv_h, b * inv_h, -b * inv_h};
-        const float gy[4] = {-ox * inv_h, -a * inv_h, a * inv_h, ox * inv_h};
-        const float vol = f4.w, xi = f4.z, fv = vol * f4.y * xi;
+        const double a = a4.x, b = a4.y, ox = 1 - a, oy = 1 - b;
+        const double s[4] = {ox * oy, a * oy, a * b, ox * b};
+        const double vol = f4.w, w = vol * f4.z, fv = w * f4.y;
 #pragma unroll
         for (int r = 0; r < 4; r++) {
-            F[r] += fv * sf[r];
+            const double ws = w * s[r];
+            F[r] = fma(fv, s[r], F[r]);
 #pragma unroll
-            for (int c = r; c < 4; c++) K[sym_index_m(r, c)] += vol * (xi * sf[r] * sf[c] + (gx[r] * gx[c] + gy[r] * gy[c]));
+            for (int c = r; c < 4; c++) K[sym_index_m(r, c)] = fma(ws, s[c], K[sym_index_m(r, c)]);
         }
+        const double va = vol * a, vb = vol * b;
+        m0 += vol;
+        ma += va;
+        mb += vb;
+        maa = fma(va, a, maa);
+        mbb = fma(vb, b, mbb);
     }
+    // sum v grad s_r . grad s_c h^2, h grad s = ((-oy, -ox), (oy, -a), (b, a), (-b, ox))
+    const double sxx = m0 - 2 * ma + maa, syy = m0 - 2 * mb + mbb, g02 = (maa - ma) + (mbb - mb);   // sxx: ox^2
+    const double gg[10] = {syy + sxx, (ma - maa) - syy, g02, (mb - mbb) - sxx, syy + maa,
+                           (mb - mbb) - maa, g02, mbb + maa, (ma - maa) - mbb, mbb + sxx};
+    const double ih2 = (double)inv_h * inv_h;
 #pragma unroll
-    for (int k = 0; k < 10; k++) elem_k[(size_t)k * ne + e] = (double)K[k];
+    for (int k = 0; k < 10; k++) elem_k[(size_t)k * ne + e] = fma(gg[k], ih2, K[k]);
 #pragma unroll
-    for (int k = 0; k < 4; k++) elem_f[(size_t)k * ne + e] = (double)F[k];
+    for (int k = 0; k < 4; k++) elem_f[(size_t)k * ne + e] = F[k];
 }
 
 // After the solve: the nodal fluidity at each particle's start-of-step
