@@ -30,66 +30,98 @@ __device__ __forceinline__ double dvd_known(double a, double b, double y)
     return __fma_rn(r, y, q);
 }
 
-// A divisor b fixed for the run, with its reciprocal as an unevaluated sum
-// zh + zl (zh = RN(1/b), zl = RN(1/b - zh)), formed on the host.
+// A divisor b fixed for the run: 1 / |b| = Z 2^(ez - 64) with Z the top 64
+// bits (truncated) of the reciprocal, formed on the host.
 struct Known {
-    double b, zh, zl;
-    double nz;   // -0 (see Unit)
-    int two;   // RN(a zh + RN(a zl)) is RN(a / b) for every normal a
+    double b;
+    uint64_t Z;
+    int ez;                 // exponent of 1 / |b| (out of every range where b is not moderate)
 };
 
-// The two-operation quotient of Brisebarre, Muller and Raina ("Accelerating
-// correctly rounded floating-point division when the divisor is known in
-// advance", IEEE Trans. Computers 53(8), 2004).  Scaled to [1, 2) each, with
-// B = 2^52 b and A = 2^52 a: a zh + RN(a zl) is within 2^-106 of a / b (half
-// an ulp of zl times a, plus half an ulp of a zl), and a quotient's distance
-// from a midpoint of two doubles is |D| / (B 2^53) for a >= b and
-// |D| / (B 2^54) for a < b, D = A 2^53 - (2 M + 1) B (or with 2^54) a nonzero
-// integer.  So a >= b always rounds correctly, and a < b unless |D| = 1, which
-// needs an odd B and then fixes 2 M + 1 = -D / B modulo 2^54: `two` records
-// that these two numerators come out right.
 inline Known make_known(double b)
 {
     Known k;
     k.b = b;
-    k.zh = 1.0 / b;
-    k.zl = 0.0;
-    k.nz = -0.0;
-    k.two = 0;
+    k.Z = 0;
+    k.ez = 1 << 20;
     const double m = fabs(b);
     if (!(m > 0x1p-400 && m < 0x1p400)) return k;
-    k.zl = fma(-b, k.zh, 1.0) / b;
-    k.two = 1;
     int e;
-    const uint64_t B = (uint64_t)ldexp(frexp(m, &e), 53);
-    if ((B & 1) == 0) return k;
-    const double bm = (double)B, zh = 1.0 / bm, zl = fma(-bm, zh, 1.0) / bm;
-    uint64_t inv = B;                                   // B^-1 mod 2^64 by Newton's iteration
-    for (int i = 0; i < 5; i++) inv *= 2 - B * inv;
-    const uint64_t mask = (1ull << 54) - 1;
-    for (int sign = 0; sign < 2; sign++) {
-        const uint64_t odd = (sign ? inv : 0 - inv) & mask;
-        const unsigned __int128 prod = (unsigned __int128)odd * B + (sign ? (unsigned __int128)0 : 1) -
-                                       (sign ? (unsigned __int128)1 : 0);
-        const uint64_t A = (uint64_t)(prod >> 54);
-        if (A < (1ull << 52) || A >= B) continue;
-        const double a = (double)A;
-        if (fma(a, zh, a * zl) != a / bm) k.two = 0;
-    }
+    const uint64_t B = (uint64_t)ldexp(frexp(m, &e), 53);      // m = B 2^(e - 53), 2^52 <= B < 2^53
+    // 2^116 / B in [2^63, 2^64]
+    const unsigned __int128 z = ((unsigned __int128)1 << 116) / B;
+    k.Z = (z >> 64) != 0 ? ~0ull : (uint64_t)z;                // B = 2^52: 2^64 - 1 stands for 2^64
+    k.ez = 1 - e;
     return k;
 }
 
-static __device__ __noinline__ double dvd_slow(double a, double b, double y)
+// The compiler's operations, out of line: the rare operands the shortcuts
+// below leave to them.  (Under a predicate instead of a branch they would cost
+// the FP64 pipe what they cost when they run.)
+static __device__ __noinline__ double div_ieee(double a, double b)
 {
-    return dvd_known(a, b, y);
+    return __ddiv_rn(a, b);
+}
+static __device__ __noinline__ double mul_ieee(double a, double b)
+{
+    return __dmul_rn(a, b);
+}
+static __device__ __noinline__ double sqrt_ieee(double a)
+{
+    return __dsqrt_rn(a);
 }
 
-// a / b correctly rounded, for normal operands and quotients (and a = 0, which
-// gives a zero), in two FP64 operations for all but rare divisors.
+// a / b correctly rounded without an FP64 operation.  With a's 53-bit
+// significand at the top of A and Z truncated, the exact quotient's 64-bit
+// significand lies in [P, P + 2), P the high word of A Z, and in [P, P + 4)
+// after the normalising shift.  Its 11 bits below the double's decide the
+// rounding (a quotient is never a midpoint) unless they are within 4 of half:
+// those four patterns of 2048, and operands or results outside the normal
+// range, take the compiler's division.  A zero is returned as one.
 __device__ __forceinline__ double dvd_const(double a, const Known &k)
 {
-    if (!k.two) return dvd_slow(a, k.b, k.zh);
-    return __fma_rn(a, k.zh, __fma_rn(a, k.zl, k.nz));
+    const int hi = __double2hiint(a), lo = __double2loint(a);
+    const int e = (hi >> 20) & 0x7ff;
+    const uint64_t A = ((uint64_t)(uint32_t)((hi & 0xfffff) | 0x100000) << 32 | (uint32_t)lo) << 11;
+    uint64_t P = __umul64hi(A, k.Z);
+    const int s = (int)(P >> 63) ^ 1;
+    P <<= s;
+    const int low = (int)P & 0x7ff, er = e + k.ez - s;
+    const int sign = (hi ^ __double2hiint(k.b)) & (int)0x80000000;
+    if ((unsigned)(e - 1) >= 2046u || (unsigned)(er - 1) >= 2046u || (unsigned)(low - 0x3fc) < 4u) {
+        if (((hi << 1) | lo) == 0 && k.Z != 0) return __hiloint2double(sign, 0);
+        return div_ieee(a, k.b);
+    }
+    const uint64_t m = (P >> 11) + (uint64_t)(low >> 10) + ((uint64_t)(uint32_t)(er - 1) << 52);
+    return __hiloint2double((int)(m >> 32) | sign, (int)m);
+}
+
+// RN(a b) in integer arithmetic: the FP64 pipe issues one instruction a warp in
+// 64 cycles and bounds the kernels that use this, while their integer pipe
+// idles, and a product takes about 40 integer instructions.  With both
+// significands at the top of 64 bits the exact product's upper 64 bits lie in
+// [P, P + 3), P the high parts of three of the four 32-bit products, and in
+// [P, P + 6) after the normalising shift; the 11 bits below the double's
+// decide the rounding unless they lie next to half (six patterns of 2048, a
+// tie among them).  Those, and operands outside 2^-255 .. 2^256 (zeros, for
+// one), take the FP64 instruction.
+__device__ __forceinline__ double imul(double a, double b)
+{
+    const int ha = __double2hiint(a), hb = __double2hiint(b);
+    const unsigned la = (unsigned)__double2loint(a), lb = (unsigned)__double2loint(b);
+    const unsigned Ah = __funnelshift_l(la, (unsigned)ha, 11) | 0x80000000u, Al = la << 11;
+    const unsigned Bh = __funnelshift_l(lb, (unsigned)hb, 11) | 0x80000000u, Bl = lb << 11;
+    const unsigned ea = (unsigned)(ha & 0x7ff00000) - (768u << 20), eb = (unsigned)(hb & 0x7ff00000) - (768u << 20);
+    unsigned long long P = (unsigned long long)Ah * Bh + __umulhi(Ah, Bl) + __umulhi(Al, Bh);
+    const unsigned up = (unsigned)(P >> 63);
+    P <<= up ^ 1u;
+    const unsigned low = (unsigned)P & 0x7ffu;
+    if ((ea | eb) >= (512u << 20) || low - 0x3fbu < 6u) return mul_ieee(a, b);
+    const unsigned long long m = (P >> 11) + (low >> 10);
+    // biased exponents 768 + x and 768 + y give 513 + x + y (the significand's
+    // leading one adds the rest)
+    const unsigned e = ea + eb + (512u << 20) + (up << 20);
+    return __hiloint2double((int)((unsigned)(m >> 32) + e + ((unsigned)(ha ^ hb) & 0x80000000u)), (int)(unsigned)m);
 }
 
 // Sign and order tests on the bit patterns (the FP64 pipe issues a compare at
@@ -117,24 +149,26 @@ __device__ __forceinline__ bool is_finite(double a)
 {
     return (__double2hiint(a) & 0x7ff00000) != 0x7ff00000;
 }
-// IEEE square root and quotient in three FP64 operations.  GB300's FP64 pipe
-// runs at 1/64 of its FP32 rate and bounds the kernels that use these, while
-// the integer and FP32 pipes idle: so the seed is refined there.  The operand's
-// 52-bit significand is split into an FP32 head and tail, the approximate FP32
-// reciprocal (root) gives the result's head, and the head's residual, exact in
-// an FP32 FMA, its tail: head + tail is good to about 2^-44 and is assembled
-// into a double by integer addition (the head held in [1, 2], where the
-// double's spacing is one).  One FP64 correction with the exact
-// residual then lands within 2^-64 relative of the value before its rounding,
-// so the rounded result is at most one ulp from the correctly rounded one, and
-// the residual of that result (exact: it has at most 53 bits) decides: it is
-// kept where its magnitude is at most that of half an ulp, else moved by one.
-// A square root or quotient of doubles is never a midpoint, so this decision
-// is exact.  The compiler's operations issue eight FP64 instructions each; with
-// these, the two-operation constant quotients and the integer compares above,
-// the G2P with g_local_mu2 went from 211 to 164 FP64 instructions a particle
-// and from 417 to 327 us at 1 048 576 particles.  Zeros, negatives, non-finite values and exponents near the ends
-// of the range take the compiler's operation.
+
+// IEEE square root and quotient in one FP64 operation.  GB300's FP64 pipe runs
+// at 1/64 of its FP32 rate and bounds the kernels that use these, while the
+// integer and FP32 pipes idle: so all but the residual is formed there.  The
+// operand's 52-bit significand is split into an FP32 head and tail, the
+// approximate FP32 reciprocal (root) gives the result's head, and the head's
+// residual, exact in an FP32 FMA, its tail: head + tail is good to about 2^-44
+// and is assembled into a double by integer addition (the head held in [1, 2],
+// where the double's spacing is one).  The exact residual of that double (the
+// one FP64 FMA) times the FP32 reciprocal is the rest of the result in units
+// of its last place, at most 512 of them and known to 2^-12: its nearest
+// integer is added to the bit pattern.  The result is then the correctly
+// rounded one (a square root or quotient of doubles is never a midpoint)
+// unless the rest lies within 2^-11 of half a unit (one operand in 1024): those,
+// results at the ends of a binade, zeros, negatives, non-finite values and
+// exponents near the ends of the range take the compiler's operation.  That
+// one issues eight FP64 instructions; with these, the integer quotients by
+// constants and products above and the integer compares, the G2P with
+// g_local_mu2 issues 72 FP64 instructions a warp of particles (211 with the
+// compiler's operations): 156 us at 1 048 576 particles, 417 with those.
 
 // The FP32 head (in [1, 2)) and tail of a double's significand.
 __device__ __forceinline__ float sig_head(int hi, int lo, int exponent)
@@ -161,71 +195,75 @@ __device__ __forceinline__ double small_int(int c)
     return __hiloint2double(c == 0 ? 0 : (int)(((1022u + 31 - z) << 20) + (m >> 11)), c == 0 ? 0 : (int)(m << 21));
 }
 
+// A residual r times 2^e as FP32 (truncated; zero stays zero), for results of
+// moderate exponent.
+__device__ __forceinline__ float residual(double r, int e)
+{
+    const int hi = __double2hiint(r), lo = __double2loint(r);
+    const int f = ((hi >> 20) & 0x7ff) + e;
+    const int b = (hi & (int)0x80000000) | ((f - 896) << 23) | ((hi & 0xfffff) << 3) | (int)((unsigned)lo >> 29);
+    return (unsigned)(f - 897) < 254u ? __int_as_float(b) : 0.0f;
+}
+
+// The bit pattern s0 moved by d units, or false where that does not decide the
+// rounding or leaves the binade of exponent field f.
+__device__ __forceinline__ bool settle(long long &s0, float d, int f)
+{
+    const float t = rintf(d);
+    const long long s = s0 + (long long)(int)t;
+    const bool ok = fabsf(d - t) <= 0.5f - 0x1p-11f && fabsf(d) < 512.0f && (int)(s0 >> 52) == f && (int)(s >> 52) == f;
+    s0 = s;
+    return ok;
+}
+
 // sqrt(2^E x).
 template <int E = 0>
 __device__ __forceinline__ double root(double x)
 {
-    if ((unsigned)__double2hiint(x) - (223u << 20) >= (1600u << 20))   // outside 2^-800 .. 2^800
-        return __dsqrt_rn(E == 0 ? x : __dmul_rn(x, E == -1 ? 0.5 : 2.0));
+    static_assert(E == 0 || E == -1, "the fallback's factor");
     const int hi = __double2hiint(x) + (E << 20), lo = __double2loint(x);
-    if (E != 0) x = __hiloint2double(hi, lo);
+    const double xs = __hiloint2double(hi, lo);
     const int e = (hi >> 20) - 1023, odd = e & 1, k = e >> 1;
     // x = m 4^k, m = head + tail in [1, 4)
     const float mh = sig_head(hi, lo, odd), ml = sig_tail(lo, odd ? 0x1p-22f : 0x1p-23f);
     const float y = rsqrtf(mh);
     const float sh = fminf(fmaxf(mh * y, 1.0f), 2.0f);
     const float sl = 0.5f * y * (__fmaf_rn(-sh, sh, mh) + ml);
-    const long long sb = widen(sh, k) + ((long long)__float2int_rn(sl * 0x1p50f) << 2);
-    const double s0 = __longlong_as_double(sb);
-    const double h = __longlong_as_double(widen(y, -k - 1));
-    const double s = __fma_rn(__fma_rn(-s0, s0, x), h, s0);
-    const double r = __fma_rn(-s, s, x);
-    // sqrt(x) <= s + u/2 iff r <= s u, and sqrt(x) >= s - u/2 iff r > -s u
-    // (r and s u are multiples of u^2); below a power of two the gap is half
-    long long b = __double_as_longlong(s);
-    const long long su = b + ((long long)((int)(b >> 52) - 1023 - 52) << 52);
-    const long long rb = __double_as_longlong(r), mag = rb & 0x7fffffffffffffffLL;
-    if (rb >= 0) b += mag > su ? 1 : 0;
-    else b -= mag >= su - ((b & 0xfffffffffffffLL) == 0 ? (1LL << 52) : 0) ? 1 : 0;
-    return __longlong_as_double(b);
+    long long s = widen(sh, k) + ((long long)__float2int_rn(sl * 0x1p50f) << 2);
+    const double s0 = __longlong_as_double(s);
+    const double r = __fma_rn(-s0, s0, xs);
+    // sqrt(x) - s0 = r / (2 s0), in units 2^(k - 52)
+    const bool fine = settle(s, residual(r, 51 - 2 * k) * y, 1023 + k);
+    if (!fine || (unsigned)__double2hiint(x) - (223u << 20) >= (1600u << 20))   // outside 2^-800 .. 2^800
+        return sqrt_ieee(E == 0 ? x : __dmul_rn(x, 0.5));
+    return __longlong_as_double(s);
 }
 
 // 2^E a / b.
 template <int E = 0>
 __device__ __forceinline__ double quot(double a, double b)
 {
-    int ah = __double2hiint(a) & 0x7fffffff;
-    const int al = __double2loint(a);
-    const int bh = __double2hiint(b) & 0x7fffffff, bl = __double2loint(b);
-    if ((unsigned)ah - (623u << 20) >= (800u << 20) || (unsigned)bh - (623u << 20) >= (800u << 20))
-        return __ddiv_rn(E == 0 ? a : __dmul_rn(a, 2.0), b);   // outside 2^-400 .. 2^400
     static_assert(E == 0 || E == 1, "the fallback's factor");
-    ah += E << 20;
-    const long long ab = (long long)((unsigned long long)(unsigned)ah << 32 | (unsigned)al);
-    const long long bb = __double_as_longlong(b) & 0x7fffffffffffffffLL;
+    const int ah = (__double2hiint(a) & 0x7fffffff) + (E << 20), al = __double2loint(a);
+    const int bh = __double2hiint(b) & 0x7fffffff, bl = __double2loint(b);
+    const double am = __hiloint2double(ah, al), bm = __hiloint2double(bh, bl);
     const long long frac = 0xfffffffffffffLL;
     // significands scaled so that the quotient's lies in [1, 2)
-    const int up = (ab & frac) < (bb & frac) ? 1 : 0;
+    const int up = (__double_as_longlong(am) & frac) < (__double_as_longlong(bm) & frac) ? 1 : 0;
     const float afh = sig_head(ah, al, up), afl = sig_tail(al, up ? 0x1p-22f : 0x1p-23f);
     const float bfh = sig_head(bh, bl, 0), bfl = sig_tail(bl, 0x1p-23f);
     const float y = __fdividef(1.0f, bfh);
     const float qh = fminf(fmaxf(afh * y, 1.0f), 2.0f);
     const float ql = __fmaf_rn(-qh, bfl, __fmaf_rn(-qh, bfh, afh) + afl) * y;
     const int eb = (bh >> 20) - 1023, eq = (ah >> 20) - 1023 - eb - up;
-    const double am = __longlong_as_double(ab), bm = __longlong_as_double(bb);
-    const double q0 = __longlong_as_double(widen(qh, eq) + ((long long)__float2int_rn(ql * 0x1p50f) << 2));
-    const double yd = __longlong_as_double(widen(y, -eb));
-    const double q = __fma_rn(__fma_rn(-bm, q0, am), yd, q0);
-    const double r = __fma_rn(-bm, q, am);
-    // |a - b q| against b times half the gap to the neighbour (the gap below a
-    // power of two is half the one above)
-    long long qb = __double_as_longlong(q);
-    const long long rb = __double_as_longlong(r), mag = rb & 0x7fffffffffffffffLL;
-    const long long above = bb + ((long long)((int)(qb >> 52) - 1023 - 53) << 52);
-    if (rb >= 0) qb += mag > above ? 1 : 0;
-    else qb -= mag > above - ((qb & frac) == 0 ? (1LL << 52) : 0) ? 1 : 0;
-    const long long sign = (__double_as_longlong(a) ^ __double_as_longlong(b)) & (long long)0x8000000000000000ULL;
-    return __longlong_as_double(qb | sign);
+    long long q = widen(qh, eq) + ((long long)__float2int_rn(ql * 0x1p50f) << 2);
+    const double r = __fma_rn(-bm, __longlong_as_double(q), am);
+    // a / b - q0 = r / b, in units 2^(eq - 52)
+    const bool fine = settle(q, residual(r, 52 - eb - eq) * y, 1023 + eq);
+    if (!fine || (unsigned)((ah >> 20) - 624) >= 799u || (unsigned)((bh >> 20) - 624) >= 799u)   // 2^-399 .. 2^399
+        return div_ieee(E == 0 ? a : __dmul_rn(a, 2.0), b);
+    const int sign = (__double2hiint(a) ^ __double2hiint(b)) & (int)0x80000000;
+    return __hiloint2double((int)(q >> 32) | sign, (int)q);
 }
 
 // Products, sums and constants for the FP64 pipe.  On GB300 a DFMA whose three
@@ -247,8 +285,13 @@ struct Elastic : Unit {
     double G, K, lambda, dt;
     double twoG;            // 2 G, exact
     double Gdt;             // RN(G dt)
-    double half, two, sixth, mfour;   // 1/2, 2, RN(1/6), -4
+    double half, two, mfour;
     Known k3, kG, kdt, kGdt;     // 3, G, dt and RN(G dt) as divisors
+};
+
+// The same with integer products.
+struct SoftElastic : Elastic {
+    __device__ __forceinline__ double mul(double a, double b) const { return imul(a, b); }
 };
 
 inline Elastic make_elastic(double G, double K, double lambda, double dt)
@@ -264,7 +307,6 @@ inline Elastic make_elastic(double G, double K, double lambda, double dt)
     el.Gdt = G * dt;
     el.half = 0.5;
     el.two = 2.0;
-    el.sixth = 1.0 / 6.0;
     el.mfour = -4.0;
     el.k3 = make_known(3.0);
     el.kG = make_known(G);
@@ -274,10 +316,13 @@ inline Elastic make_elastic(double G, double K, double lambda, double dt)
 }
 
 // exp(x) for the volume update v <- v exp(dt tr D), whose argument is tiny at
-// any stable time step: where |x| < 2^-14 the degree-3 Taylor polynomial about
-// 0 in Horner form (truncation below x^4 / 24 < 2^-60), where |x| < 2^-9 the
-// degree-5 one (below x^6 / 720 < 2^-63), either under a tenth of an ulp of the
-// result, so the result lies within about half an ulp of e^x; elsewhere exp().
+// any stable time step.  Where |x| < 2^-14 it is the degree-4 Taylor polynomial
+// (truncation below x^5 / 120 < 2^-76) as a 64-bit integer in units of 2^-62,
+// without an FP64 operation: x is shifted into place, x^2 / 2 is an integer
+// product, and the rest, below 2^-44, comes from FP32 to 2^-66.  Where
+// |x| < 2^-9 it is the degree-5 polynomial in Horner form (truncation below
+// x^6 / 720 < 2^-63).  Either is within a hundredth of an ulp before its last
+// rounding, so the result lies within about half an ulp of e^x; elsewhere exp().
 static __device__ __noinline__ double exp_wide(double x)
 {
     if ((__double2hiint(x) & 0x7fffffff) >= 0x3f600000) return exp(x);
@@ -288,16 +333,27 @@ static __device__ __noinline__ double exp_wide(double x)
     return __fma_rn(p, x, 1.0);
 }
 
-__device__ __forceinline__ double exp_small(double x, double one = 1.0, double half = 0.5, double sixth = 1.0 / 6.0)
+__device__ __forceinline__ double exp_small(double x)
 {
-    if ((__double2hiint(x) & 0x7fffffff) >= 0x3f100000) return exp_wide(x);
-    double p = __fma_rn(x, sixth, half);
-    p = __fma_rn(p, x, one);
-    return __fma_rn(p, x, one);
+    const int hi = __double2hiint(x), lo = __double2loint(x);
+    const int e = (hi >> 20) & 0x7ff;
+    if (e >= 1023 - 14) return exp_wide(x);
+    const unsigned long long sig =
+        ((unsigned long long)(unsigned)((hi & 0xfffff) | 0x100000) << 32 | (unsigned)lo) << 11;
+    // below 2^-62 x does not count
+    const long long X = (long long)(sig >> min(1024 - e, 63));
+    const float xf = __int_as_float((hi & (int)0x80000000) | (max(e, 960) - 896) << 23 | (hi & 0xfffff) << 3);
+    const int w = __float2int_rn(xf * xf * xf * __fmaf_rn(xf, 1.0f / 24.0f, 1.0f / 6.0f) * 0x1p62f);
+    const long long r = (1LL << 62) + (long long)__umul64hi(2 * X, X) + w + (hi < 0 ? -X : X);
+    // rounded to 2^-52 from one upwards, to 2^-53 below
+    const bool up = r >= 1LL << 62;
+    const long long m = up ? (r + 512) >> 10 : (r + 256) >> 9;
+    return __hiloint2double((int)(m >> 32) + ((up ? 1022 : 1021) << 20), (int)m);
 }
 
 // isolin calculate_stress_threaded, materialsrc/isolin.c:75-116.
-__device__ __forceinline__ void isolin(const Elastic &el, double exx, double exy, double eyy,
+template <class E>
+__device__ __forceinline__ void isolin(const E &el, double exx, double exy, double eyy,
                                        double wxy, double &sxx, double &sxy, double &syy)
 {
     const auto mul = [&](double a, double b) { return el.mul(a, b); };
@@ -320,7 +376,8 @@ __device__ __forceinline__ void isolin(const Elastic &el, double exx, double exy
 // negative_root, g_local_mu2.c:90-99 (also g_nonlocal_mu2.c:226-235), with
 // a = 1: the products by 4 and 2 are exact, so they ride in an FMA and in the
 // quotient's exponent.
-__device__ __forceinline__ double negative_root(const Elastic &el, double b, double c)
+template <class E>
+__device__ __forceinline__ double negative_root(const E &el, double b, double c)
 {
     const double disc = root(__fma_rn(el.mfour, c, el.mul(b, b)));
     if (is_pos(b)) return el.mul(el.half, el.sub(-b, disc));
@@ -346,7 +403,8 @@ struct Mu2Params {
 // Only m inside the bracket, and any operand that is not a normal positive
 // number above 2^-959 (or a NaN), takes the division.  Positive normal
 // products and m order as integers; the dense side is tested first.
-__device__ __forceinline__ bool below_density(const Unit &u, double m, double v, const Mu2Params &mp)
+template <class U>
+__device__ __forceinline__ bool below_density(const U &u, double m, double v, const Mu2Params &mp)
 {
     const long long mb = __double_as_longlong(m), vb = __double_as_longlong(v);
     if (vb > 0x0400000000000000LL && vb < 0x7ff0000000000000LL && mb > 0x0400000000000000LL &&
@@ -362,9 +420,10 @@ __device__ __forceinline__ bool below_density(const Unit &u, double m, double v,
 // [0, 0, Tzz]] (the z-shear components stay zero and T stays symmetric
 // because L has no z entries).  The expressions are the tensor.c sums with
 // their zero terms removed, in the same order.
-__device__ __forceinline__ void g_local_mu2(const Elastic &el, const Mu2Params &mp, double m,
-                                            double v, double exx, double exy, double eyy,
-                                            double wxy, double &Txx, double &Txy, double &Tyy,
+template <class E>
+__device__ __forceinline__ void g_local_mu2(const E &el, const Mu2Params &mp, double m,
+                                            double v, double exx, double eyy, double d2,
+                                            double w2, double &Txx, double &Txy, double &Tyy,
                                             double &Tzz, double &gammap, double &gammadotp)
 {
     const auto mul = [&](double a, double b) { return el.mul(a, b); };
@@ -372,15 +431,14 @@ __device__ __forceinline__ void g_local_mu2(const Elastic &el, const Mu2Params &
     const auto sub = [&](double a, double b) { return el.sub(a, b); };
     const double G = el.G, dt = el.dt;
     const double lambda = el.lambda;   // K - 2 G / 3, formed on the host with the same roundings
-    // L (:191-199), W = skw(L), D = sym(L) (tensor.c:330-384)
+    // d2 = Lxy + Lyx = 2 Dxy, w2 = Lxy - Lyx = 2 Wxy (L :191-199, W = skw(L),
+    // D = sym(L) tensor.c:330-384).
     // Exact shortcuts, bit for bit the reference's values for normal
     // operands below DBL_MAX / 2 (a halving or doubling commutes with a
-    // rounding): 0.5 (x + x) is x; with w2 = Lxy - Lyx = 2 Wxy, W T - T W has
+    // rounding): 0.5 (x + x) is x; W T - T W has
     // xx entry RN(Wxy Txy) + RN(Wxy Txy) = RN(w2 Txy), yy entry its negative,
     // and xy entry half of RN(w2 Tyy) - RN(Txx w2), added with one rounding by
-    // an FMA; with d2 = Lxy + Lyx = 2 Dxy, Dxy 2G is d2 G; 0 * 2G is +0.
-    const double Lxy = add(exy, wxy), Lyx = sub(exy, wxy);
-    const double w2 = sub(Lxy, Lyx), d2 = add(Lxy, Lyx);
+    // an FMA; Dxy 2G is d2 G; 0 * 2G is +0.
     const double trD = add(exx, eyy);
     // Jaumann term JS = W T - T W (:209-212)
     const double JSxx = mul(w2, Txy);
@@ -451,8 +509,8 @@ struct ReturnParams {
     double mu_s, mu_2, I0, grains_rho, grains_d, rho_critical;
 };
 
-template <bool TRIAL3D, bool MU_I, bool BETA>
-__device__ __forceinline__ void plane_return(const Elastic &el, const ReturnParams &rp, double m, double v,
+template <bool TRIAL3D, bool MU_I, bool BETA, class E>
+__device__ __forceinline__ void plane_return(const E &el, const ReturnParams &rp, double m, double v,
                                              double exx, double exy, double eyy, double wxy, double &sxx,
                                              double &sxy, double &syy, double &szz, double &beta,
                                              double &gammap, double &gammadotp)
@@ -530,7 +588,8 @@ __device__ __forceinline__ void plane_return(const Elastic &el, const ReturnPara
 // a rate-dependent return to mu(I) (p + c), c = 0, with mu from the previous
 // step's gammadotp and the start-of-step pressure, and Jaumann terms of the
 // opposite sign to isolin's.  beta in state[5].
-__device__ __forceinline__ void g_local_mu2_reverse(const Elastic &el, const Mu2Params &mp, double m, double v,
+template <class E>
+__device__ __forceinline__ void g_local_mu2_reverse(const E &el, const Mu2Params &mp, double m, double v,
                                                     double exx, double exy, double eyy, double wxy, double &sxx,
                                                     double &sxy, double &syy, double &beta, double &gammap,
                                                     double &gammadotp)
@@ -686,7 +745,8 @@ __device__ __forceinline__ void ext_stress(const Elastic &el, const Mu2Params &m
 
 // Trial Jaumann stress of g_nonlocal_mu2.c:166-186 (and :271-290), with
 // lambda = K - 2G/3 (the reference leaves it uninitialised at :154).
-__device__ __forceinline__ void nonlocal_mu2_trial(const Elastic &el, double exx, double exy,
+template <class E>
+__device__ __forceinline__ void nonlocal_mu2_trial(const E &el, double exx, double exy,
                                                    double eyy, double wxy, double sxx, double sxy,
                                                    double syy, double &p_tr, double &t0xx,
                                                    double &t0xy, double &t0yy, double &tau_tr)
@@ -726,7 +786,8 @@ __device__ __forceinline__ void nonlocal_mu2_trial(const Elastic &el, double exx
 //              as 2 H / (B + sqrt(B^2 - 4 H)) (negative_root's b < 0 branch)
 //   gf_local = (p / (G dt)) (tau / tau_tau - 1) = p (tau - tau_tau) / (G dt tau_tau)
 // and below yield (scale factor 1) gf_local is +0.
-__device__ __forceinline__ void nonlocal_mu2_bulk(const Elastic &el, const Mu2Params &mp, double m,
+template <class E>
+__device__ __forceinline__ void nonlocal_mu2_bulk(const E &el, const Mu2Params &mp, double m,
                                                   double v, double p_tr, double tau_tr, double &dense,
                                                   double &gf_local, double &xisq_inv)
 {
@@ -766,7 +827,8 @@ __device__ __forceinline__ void nonlocal_mu2_bulk(const Elastic &el, const Mu2Pa
 // particle is dense, 0 where it is not), so `dense == 0 || p_tr <= 0` reads
 // `p_d <= 0`. sxx, sxy, syy hold the start-of-step stress, which a NaN trial
 // pressure keeps (neither branch of the reference is taken).
-__device__ __forceinline__ void nonlocal_mu2_stress(const Elastic &el, double gf, double p_d,
+template <class E>
+__device__ __forceinline__ void nonlocal_mu2_stress(const E &el, double gf, double p_d,
                                                     double t0xx, double t0xy, double t0yy,
                                                     double tau_tr, double &sxx, double &sxy,
                                                     double &syy, double &gammap, double &gammadotp)

@@ -298,6 +298,8 @@ __global__ void __launch_bounds__(EB * SPLIT) p2g_cells_kernel(
     const bool do_a = SPLIT == 1 || half == 0, do_b = SPLIT == 1 || half == 1;
     const mat::Unit u{sh_const[0], sh_const[1]};
     const double inv_h = sh_const[2];
+    // integer products where the FP64 pipe is the bound, not a thread's chain
+    auto prod = [&](double a, double b) { return SPLIT == 1 ? mat::imul(a, b) : u.mul(a, b); };
     // the next particle's loads are in flight during this one's arithmetic
     double nx = 0, ny = 0, nm = 0, nvx = 0, nvy = 0, nv = 0, n0 = 0, n1 = 0, n2 = 0;
     auto fetch = [&](int k) {
@@ -320,9 +322,9 @@ __global__ void __launch_bounds__(EB * SPLIT) p2g_cells_kernel(
         if (k + 1 < cnt) fetch(k + 1);
         const double xl = mpmg_local_coord_fma(px, cx, inv_h);
         const double yl = mpmg_local_coord_fma(py, cy, inv_h);
-        const double xy = u.mul(xl, yl);
+        const double xy = prod(xl, yl);
         if (do_a) {
-            const double pmx = u.mul(pvx, pm);
+            const double pmx = prod(pvx, pm);
             mm[0] = u.add(pm, mm[0]);
             mm[1] = fma(xl, pm, mm[1]);
             mm[2] = fma(yl, pm, mm[2]);
@@ -333,8 +335,8 @@ __global__ void __launch_bounds__(EB * SPLIT) p2g_cells_kernel(
             mx[3] = fma(xy, pmx, mx[3]);
         }
         if (do_b) {
-            const double pmy = u.mul(pvy, pm);
-            const double vlx = u.mul(vol, xl), vly = u.mul(vol, yl);
+            const double pmy = prod(pvy, pm);
+            const double vlx = prod(vol, xl), vly = prod(vol, yl);
             my[0] = u.add(pmy, my[0]);
             my[1] = fma(xl, pmy, my[1]);
             my[2] = fma(yl, pmy, my[2]);
@@ -567,7 +569,7 @@ cudaError_t launch_grid(mpmg_ctx *ctx, const GridGeom &g)
 
 // The arithmetic's constants, copied to shared memory (mat::Unit).
 struct G2PConst {
-    mat::Elastic el;
+    mat::SoftElastic el;
     mat::Mu2Params mu2;
     double inv_h, half_inv_h;
 };
@@ -647,7 +649,7 @@ __device__ __forceinline__ Particle load_particle(const G2PArgs &A, int i)
 // The in-plane local returns on particle i (mat::plane_return): szz in
 // state[1] (dp_ri_mt.c:27, g_local_mu2_plane_strain.c:43), beta in state[5],
 // gammap in state[9], gammadotp in state[10].
-template <int MATERIAL>
+template <class E, int MATERIAL>
 __device__ __forceinline__ void plane_return_particle(const G2PArgs &A, const G2PConst &C, int i, const Particle &p,
                                                       double vol, double exx, double exy, double eyy, double wxy)
 {
@@ -657,7 +659,7 @@ __device__ __forceinline__ void plane_return_particle(const G2PArgs &A, const G2
     const mat::ReturnParams rp = {C.mu2.mu_s, C.mu2.mu_2, C.mu2.I0, C.mu2.grains_rho, C.mu2.grains_d,
                                   C.mu2.rho_critical};
     double sxx = p.sxx, sxy = p.sxy, syy = p.syy, szz = p.st1, b = p.st5, gp = p.st9, gdp;
-    mat::plane_return<trial3d, mu_i, beta>(C.el, rp, p.m, vol, exx, exy, eyy, wxy, sxx, sxy, syy, szz, b, gp, gdp);
+    mat::plane_return<trial3d, mu_i, beta>(static_cast<const E &>(C.el), rp, p.m, vol, exx, exy, eyy, wxy, sxx, sxy, syy, szz, b, gp, gdp);
     A.sxx[i] = sxx;
     A.sxy[i] = sxy;
     A.syy[i] = syy;
@@ -669,11 +671,12 @@ __device__ __forceinline__ void plane_return_particle(const G2PArgs &A, const G2
 
 // g_local_mu2_reverse on particle i: beta in state[5], gammap in state[9],
 // gammadotp in state[10] (g_local_mu2_reverse.c:57-64).
+template <class E>
 __device__ __forceinline__ void reverse_particle(const G2PArgs &A, const G2PConst &C, int i, const Particle &p,
                                                  double vol, double exx, double exy, double eyy, double wxy)
 {
     double sxx = p.sxx, sxy = p.sxy, syy = p.syy, b = p.st5, gp = p.st9, gdp = p.st10;
-    mat::g_local_mu2_reverse(C.el, C.mu2, p.m, vol, exx, exy, eyy, wxy, sxx, sxy, syy, b, gp, gdp);
+    mat::g_local_mu2_reverse(static_cast<const E &>(C.el), C.mu2, p.m, vol, exx, exy, eyy, wxy, sxx, sxy, syy, b, gp, gdp);
     A.sxx[i] = sxx;
     A.sxy[i] = sxy;
     A.syy[i] = syy;
@@ -682,21 +685,23 @@ __device__ __forceinline__ void reverse_particle(const G2PArgs &A, const G2PCons
     A.st10[i] = gdp;
 }
 
+template <class E>
 __device__ __forceinline__ void isolin_particle(const G2PArgs &A, const G2PConst &C, int i, const Particle &p,
                                                 double exx, double exy, double eyy, double wxy)
 {
     double sxx = p.sxx, sxy = p.sxy, syy = p.syy;
-    mat::isolin(C.el, exx, exy, eyy, wxy, sxx, sxy, syy);
+    mat::isolin(static_cast<const E &>(C.el), exx, exy, eyy, wxy, sxx, sxy, syy);
     A.sxx[i] = sxx;
     A.sxy[i] = sxy;
     A.syy[i] = syy;
 }
 
+template <class E>
 __device__ __forceinline__ void mu2_particle(const G2PArgs &A, const G2PConst &C, int i, const Particle &p, double vol,
-                                             double exx, double exy, double eyy, double wxy)
+                                             double exx, double eyy, double d2, double w2)
 {
     double Txx = p.sxx, Txy = p.sxy, Tyy = p.syy, Tzz = p.Tzz, gp = p.st9, gdp;
-    mat::g_local_mu2(C.el, C.mu2, p.m, vol, exx, exy, eyy, wxy, Txx, Txy, Tyy, Tzz, gp, gdp);
+    mat::g_local_mu2(static_cast<const E &>(C.el), C.mu2, p.m, vol, exx, eyy, d2, w2, Txx, Txy, Tyy, Tzz, gp, gdp);
     A.sxx[i] = Txx;
     A.sxy[i] = Txy;
     A.syy[i] = Tyy;
@@ -721,11 +726,11 @@ __device__ __forceinline__ Field field_at(double2 c01, double2 c23, double x, do
 
 // One particle inside the grid, element e at the step's start; p.x, p.y leave
 // as the moved position.
-template <int MATERIAL, int PHASE>
+template <class E, int MATERIAL, int PHASE>
 __device__ __forceinline__ void g2p_particle(const G2PArgs &A, const G2PConst &C, int i, int e, Particle &p)
 {
     const GridGeom &g = A.g;
-    const mat::Unit &u = C.el;
+    const E &u = C.el;
     const int cj = e / g.Ex, ci = e - cj * g.Ex;
     const double dt = C.el.dt, inv_h = C.inv_h;
     Field vx, vy;
@@ -775,10 +780,14 @@ __device__ __forceinline__ void g2p_particle(const G2PArgs &A, const G2PConst &C
     // calculate_strainrate_split (process_usl.c:796-803): the sums of
     // grad N_a v_a, scaled by 1 / h once
     const double exx = u.mul(vx.gx, inv_h), eyy = u.mul(vy.gy, inv_h);
-    const double exy = u.mul(C.half_inv_h, u.add(vx.gy, vy.gx));
-    const double wxy = u.mul(C.half_inv_h, u.sub(vx.gy, vy.gx));
+    const double gsum = u.add(vx.gy, vy.gx), gdiff = u.sub(vx.gy, vy.gx);
+    double exy = 0, wxy = 0;
+    if (MATERIAL != MPMG_G_LOCAL_MU2 || A.exx != nullptr) {
+        exy = u.mul(C.half_inv_h, gsum);
+        wxy = u.mul(C.half_inv_h, gdiff);
+    }
     // update_particle_densities_split (process_usl.c:961-970)
-    const double vol = u.mul(p.v, mat::exp_small(u.mul(dt, u.add(exx, eyy)), u.one, C.el.half, C.el.sixth));
+    const double vol = u.mul(p.v, mat::exp_small(u.mul(dt, u.add(exx, eyy))));
     A.v[i] = vol;
     if (A.exx != nullptr) {
         A.exx[i] = exx;
@@ -788,14 +797,14 @@ __device__ __forceinline__ void g2p_particle(const G2PArgs &A, const G2PConst &C
     }
 
     if (MATERIAL == MPMG_ISOLIN) {
-        isolin_particle(A, C, i, p, exx, exy, eyy, wxy);
+        isolin_particle<E>(A, C, i, p, exx, exy, eyy, wxy);
     } else if (MATERIAL == MPMG_G_LOCAL_MU2) {
-        mu2_particle(A, C, i, p, vol, exx, exy, eyy, wxy);
+        mu2_particle<E>(A, C, i, p, vol, exx, eyy, u.mul(inv_h, gsum), u.mul(inv_h, gdiff));
     } else if (MATERIAL == MPMG_DP_RI_MT || MATERIAL == MPMG_G_LOCAL_MU2_PLANE_STRAIN ||
                MATERIAL == MPMG_G_LOCAL_MU2_TRUE_2D) {
-        plane_return_particle<MATERIAL>(A, C, i, p, vol, exx, exy, eyy, wxy);
+        plane_return_particle<E, MATERIAL>(A, C, i, p, vol, exx, exy, eyy, wxy);
     } else if (MATERIAL == MPMG_G_LOCAL_MU2_REVERSE) {
-        reverse_particle(A, C, i, p, vol, exx, exy, eyy, wxy);
+        reverse_particle<E>(A, C, i, p, vol, exx, exy, eyy, wxy);
     } else if (MATERIAL == MPMG_G_LOCAL_MU2_EXT) {
         // first phase only; the stress waits for the nodal Laplacian
         double mu_t = p.st0, gfl;
@@ -804,8 +813,8 @@ __device__ __forceinline__ void g2p_particle(const G2PArgs &A, const G2PConst &C
         A.st4[i] = gfl;
     } else if (MATERIAL == MPMG_G_NONLOCAL_MU2) {
         double p_tr, t0xx, t0xy, t0yy, tau_tr, dense, gfl, xisq;
-        mat::nonlocal_mu2_trial(C.el, exx, exy, eyy, wxy, p.sxx, p.sxy, p.syy, p_tr, t0xx, t0xy, t0yy, tau_tr);
-        mat::nonlocal_mu2_bulk(C.el, C.mu2, p.m, vol, p_tr, tau_tr, dense, gfl, xisq);
+        mat::nonlocal_mu2_trial(u, exx, exy, eyy, wxy, p.sxx, p.sxy, p.syy, p_tr, t0xx, t0xy, t0yy, tau_tr);
+        mat::nonlocal_mu2_bulk(u, C.mu2, p.m, vol, p_tr, tau_tr, dense, gfl, xisq);
         A.st0[i] = dense;
         A.st5[i] = gfl;
         A.st6[i] = xisq;
@@ -829,9 +838,9 @@ __device__ __forceinline__ void stage_const(G2PConst &C, const G2PConst &param)
     for (int k = threadIdx.x; k < (int)(sizeof(G2PConst) / 8); k += blockDim.x) dst[k] = src[k];
 }
 
-// The block's size is the launch's (g2p_threads).  Every thread stays to the
+// The block's size and E are the launch's (g2p_pipe_bound).  Every thread stays to the
 // end: the binning is a warp's work.
-template <int MATERIAL, int PHASE>
+template <class E, int MATERIAL, int PHASE>
 __global__ void __launch_bounds__(128) g2p_kernel(const __grid_constant__ G2PArgs A)
 {
     __shared__ G2PConst C;
@@ -847,7 +856,7 @@ __global__ void __launch_bounds__(128) g2p_kernel(const __grid_constant__ G2PArg
     uint32_t next = A.sentinel;
     if (key != A.sentinel) {
         if (PHASE != G2P_STRAIN) A.in_element[i] = (int)key;
-        g2p_particle<MATERIAL, PHASE>(A, C, i, (int)key, p);
+        g2p_particle<E, MATERIAL, PHASE>(A, C, i, (int)key, p);
         if (PHASE != G2P_MOVE) {
             const int e = mpmg_which_element_fast(p.x, p.y, g.h, g.inv_h, A.inv_hf, g.xmax, g.ymax,
                                                   __double_as_longlong(g.xmax), __double_as_longlong(g.ymax), g.Ex,
@@ -1036,20 +1045,23 @@ __global__ void material_only_kernel(const __grid_constant__ G2PArgs A, int mate
     const G2PConst &C = A.k;
     const double exx = A.exx[i], exy = A.exy[i], eyy = A.eyy[i], wxy = A.wxy[i], vol = A.v[i];
     if (material == MPMG_ISOLIN) {
-        isolin_particle(A, C, i, load_particle<MPMG_ISOLIN, G2P_FULL>(A, i), exx, exy, eyy, wxy);
+        isolin_particle<mat::Elastic>(A, C, i, load_particle<MPMG_ISOLIN, G2P_FULL>(A, i), exx, exy, eyy, wxy);
     } else if (material == MPMG_DP_RI_MT) {
-        plane_return_particle<MPMG_DP_RI_MT>(A, C, i, load_particle<MPMG_DP_RI_MT, G2P_FULL>(A, i), vol, exx, exy,
+        plane_return_particle<mat::Elastic, MPMG_DP_RI_MT>(A, C, i, load_particle<MPMG_DP_RI_MT, G2P_FULL>(A, i), vol, exx, exy,
                                              eyy, wxy);
     } else if (material == MPMG_G_LOCAL_MU2_PLANE_STRAIN) {
-        plane_return_particle<MPMG_G_LOCAL_MU2_PLANE_STRAIN>(
+        plane_return_particle<mat::Elastic, MPMG_G_LOCAL_MU2_PLANE_STRAIN>(
             A, C, i, load_particle<MPMG_G_LOCAL_MU2_PLANE_STRAIN, G2P_FULL>(A, i), vol, exx, exy, eyy, wxy);
     } else if (material == MPMG_G_LOCAL_MU2_TRUE_2D) {
-        plane_return_particle<MPMG_G_LOCAL_MU2_TRUE_2D>(
+        plane_return_particle<mat::Elastic, MPMG_G_LOCAL_MU2_TRUE_2D>(
             A, C, i, load_particle<MPMG_G_LOCAL_MU2_TRUE_2D, G2P_FULL>(A, i), vol, exx, exy, eyy, wxy);
     } else if (material == MPMG_G_LOCAL_MU2_REVERSE) {
-        reverse_particle(A, C, i, load_particle<MPMG_G_LOCAL_MU2_REVERSE, G2P_FULL>(A, i), vol, exx, exy, eyy, wxy);
+        reverse_particle<mat::Elastic>(A, C, i, load_particle<MPMG_G_LOCAL_MU2_REVERSE, G2P_FULL>(A, i), vol, exx, exy, eyy, wxy);
     } else {
-        mu2_particle(A, C, i, load_particle<MPMG_G_LOCAL_MU2, G2P_FULL>(A, i), vol, exx, exy, eyy, wxy);
+        // L's off-diagonal entries, g_local_mu2.c:191-199
+        const double Lxy = mat::add(exy, wxy), Lyx = mat::sub(exy, wxy);
+        mu2_particle<mat::Elastic>(A, C, i, load_particle<MPMG_G_LOCAL_MU2, G2P_FULL>(A, i), vol, exx, eyy, mat::add(Lxy, Lyx),
+                     mat::sub(Lxy, Lyx));
     }
 }
 
@@ -1088,7 +1100,7 @@ G2PArgs make_g2p_args(mpmg_ctx *ctx)
     A.g = make_geom(ctx);
     A.n = (int)ctx->np;
     A.early = early_launch(ctx);
-    A.k.el = mat::make_elastic(ctx->G, ctx->K, ctx->lambda, c.dt);
+    static_cast<mat::Elastic &>(A.k.el) = mat::make_elastic(ctx->G, ctx->K, ctx->lambda, c.dt);
     A.k.inv_h = ctx->inv_h;
     A.k.half_inv_h = 0.5 * ctx->inv_h;
     A.k.mu2.mu_s = c.mp[MPMG_MP_MU_S];
@@ -1143,20 +1155,39 @@ inline int blocks_for(size_t n, int threads)
 
 }  // namespace
 
-// Threads of a G2P block: one warp where every warp can have a sub-partition
-// to itself or nearly so (a 256-thread block would leave most SMs idle), 128
-// beyond that.
-static int g2p_threads(const mpmg_ctx *ctx)
+// More than two warps of particles a sub-partition: the G2P is then bound by
+// the FP64 pipe and takes blocks of four warps and integer products
+// (mat::SoftElastic; g_local_mu2, 1 048 576 particles: 287 -> 254 us a step,
+// 125k: 67 -> 62; isolin, 65k: 40.5 -> 38.8).  Up to there a sub-partition's
+// one or two warps run a serial chain, through an instruction cache that the
+// integer products' longer code overflows: one-warp blocks (a larger one would
+// leave most SMs idle) and FP64 products (31k: 30.7 us, 31.5 with integer ones;
+// 4k: 15.5 and 16.3).
+static bool g2p_pipe_bound(const mpmg_ctx *ctx)
 {
-    return ctx->np <= (size_t)ctx->sms * 4 * 32 * 2 ? 32 : 128;
+    return ctx->np > (size_t)ctx->sms * 4 * 32 * 2;
 }
+
+// The arithmetic of a pipe-bound phase; the move phase has no products.
+template <int PHASE>
+struct BoundArith {
+    using E = mat::SoftElastic;
+};
+template <>
+struct BoundArith<G2P_MOVE> {
+    using E = mat::Elastic;
+};
 
 template <int MATERIAL, int PHASE>
 static cudaError_t launch_g2p(mpmg_ctx *ctx, const G2PArgs &A)
 {
-    const int t = g2p_threads(ctx);
+    const bool bound = g2p_pipe_bound(ctx);
+    const int t = bound ? 128 : 32;
     ctx->launches += 1;
-    return mpmg_launch_pdl(true, g2p_kernel<MATERIAL, PHASE>, dim3(blocks_for(ctx->np, t)), dim3(t), 0, ctx->stream, A);
+    return mpmg_launch_pdl(true,
+                           bound ? g2p_kernel<typename BoundArith<PHASE>::E, MATERIAL, PHASE>
+                                 : g2p_kernel<mat::Elastic, MATERIAL, PHASE>,
+                           dim3(blocks_for(ctx->np, t)), dim3(t), 0, ctx->stream, A);
 }
 
 template <int EB, int SPLIT>
@@ -1230,7 +1261,7 @@ int mpmg_launch_step(mpmg_ctx *ctx)
     // two threads an element in single-warp sets, where that leaves every
     // sub-partition at most one warp
     MPMG_CHECK((ctx->row.filled0 <= (size_t)ctx->sms * 4 * 16 ? launch_p2g<32, 2>(ctx, g, keep_order)
-                                                              : launch_p2g<128, 1>(ctx, g, keep_order)));
+                                                              : launch_p2g<64, 1>(ctx, g, keep_order)));
     mpmg_phase_end(ctx, PH_P2G);
 
     mpmg_phase_begin(ctx, PH_GRID);

@@ -1,5 +1,5 @@
-// Test-only kernels: the library's FP64 square root and quotients
-// (mat::root, mat::quot, mat::dvd_const) against the IEEE
+// Test-only kernels: the library's FP64 square root, quotients
+// (mat::root, mat::quot, mat::dvd_const) and product (mat::imul) against the IEEE
 // operations, on random operands, on operands whose result lies next to a
 // midpoint of two doubles or to a power of two, and on the ends of the range.
 // Built by tests/test_gpu_root.py with nvcc into a temporary shared library.
@@ -34,7 +34,7 @@ __device__ double operand(uint64_t r, int kind, int span)
     return bits(e | (r & frac));
 }
 
-enum { ROOT = 0, QUOT = 1, CONST = 2 };
+enum { ROOT = 0, QUOT = 1, CONST = 2, MUL = 3 };
 
 __global__ void check_kernel(int op, int kind, int span, mat::Known k, long long n, uint64_t seed,
                              unsigned long long *bad, double *example)
@@ -65,6 +65,10 @@ __global__ void check_kernel(int op, int kind, int span, mat::Known k, long long
             if (r1 & 1) b = -b;
             got = r1 & 2 ? mat::quot(a, b) : mat::quot<1>(a, b);
             want = __ddiv_rn(r1 & 2 ? a : 2.0 * a, b);
+        } else if (op == MUL) {
+            if (r1 & 1) b = -b;
+            got = mat::imul(a, b);
+            want = __dmul_rn(a, b);
         } else {
             if (kind & 16) {
                 const double c = operand(mix(r1 ^ half), 0, span);
@@ -88,10 +92,9 @@ __global__ void check_kernel(int op, int kind, int span, mat::Known k, long long
 }  // namespace
 
 // Mismatches among n operands; kind: operand kind of a (bits 0-1) and b (bits
-// 2-3), 16: results next to a midpoint.  b is the divisor of op 2; *two tells
-// which of its two forms ran.
+// 2-3), 16: results next to a midpoint.  b is the divisor of op 2.
 extern "C" int check_op(int op, int kind, int span, double b, long long n, unsigned long long seed,
-                        unsigned long long *mismatches, double *example, int *two)
+                        unsigned long long *mismatches, double *example)
 {
     unsigned long long *d_bad = nullptr;
     double *d_ex = nullptr;
@@ -100,7 +103,6 @@ extern "C" int check_op(int op, int kind, int span, double b, long long n, unsig
     cudaMemset(d_bad, 0, sizeof(*d_bad));
     cudaMemset(d_ex, 0, 4 * sizeof(double));
     const mat::Known k = mat::make_known(b);
-    *two = k.two;
     check_kernel<<<1216, 256>>>(op, kind, span, k, n, seed, d_bad, d_ex);
     cudaError_t e = cudaMemcpy(mismatches, d_bad, sizeof(*d_bad), cudaMemcpyDeviceToHost);
     if (e == cudaSuccess) e = cudaMemcpy(example, d_ex, 4 * sizeof(double), cudaMemcpyDeviceToHost);
