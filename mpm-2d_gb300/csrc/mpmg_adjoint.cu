@@ -8,23 +8,32 @@
 // segment by segment from the last, the forward steps of the segment are run
 // again from its checkpoint with each step's inputs recorded on the device
 // (particle state at the step start, elements and activity after the keys
-// phase, the binned order, the nodal mass, acceleration and velocity, the
-// step's time and gravity), then the segment's steps are reversed one by one:
+// phase, each element's ordered particle list from the step's rows, the nodal
+// mass, acceleration and velocity, the step's time and gravity), then the
+// segment's steps are reversed one by one:
 //
-//   adj_g2p    per particle: the material update (isolin or g_local_mu2),
-//              volume, strain rate, velocity and position gathers, and the
-//              start-of-step shape functions, reversed; writes the particle's
-//              share of the adjoint nodal velocity and acceleration, and the
-//              parameter adjoint (block partial sums)
-//   adj_cells  per element: those shares summed over the element's particles
-//              in the binned order (fixed order, no atomics)
-//   adj_grid   per node: the four elements' sums in colour order, the
-//              boundary masks and the nodal update (v = p/m, a = f/m,
-//              p += dt f) reversed -> adjoint nodal momentum, force and mass
+//   adj_g2p    per particle: the material update (isolin, g_local_mu2 or
+//              g_nonlocal_mu2), volume, strain rate, velocity and position
+//              gathers, and the start-of-step shape functions, reversed;
+//              writes the particle's share of the adjoint nodal velocity and
+//              acceleration, and the parameter adjoint (block partial sums)
+//   adj_node   per node: those shares summed over the particles of its four
+//              elements, in colour order and list order (fixed order, no
+//              atomics), then the boundary masks and the nodal update
+//              (v = p/m, a = f/m, p += dt f) reversed -> adjoint nodal
+//              momentum, force and mass
 //   adj_p2g    per particle: the P2G of mass, momentum and internal force
-//              reversed (a gather from the four nodes)
-//   theta      the step's block partials added, in block order, to the
-//              parameter adjoint
+//              reversed (a gather from the four nodes); one more block adds
+//              the step's block partials to the parameter adjoint
+//
+// The particle kernels are bound by the FP64 pipe (64 cycles a warp
+// instruction), so they work on each nodal field's bilinear coefficients on
+// the element (value, gradient and mixed derivative from the four nodes)
+// instead of on sums over shape functions, and on mat::root, mat::quot and
+// register-operand FMAs.  65 536 particles with g_local_mu2: adj_g2p 76 -> 40 us
+// (672 -> 150 FP64 instructions a warp), adj_p2g 28 -> 16 (248 -> 66), the
+// element and node sums 32 -> 21, the parameter sum 23 -> none of its own, the
+// recorded order 26 -> 2.
 //
 // The element of each particle is held fixed within a step (the map from
 // positions to elements is piecewise constant), and the branches of the
@@ -45,7 +54,7 @@ using fp64::BcParams;
 using fp64::GridGeom;
 using fp64::ShapeFns;
 
-constexpr int kAdjThreads = 256;
+constexpr int kAdjThreads = 128;
 constexpr int kStateFields = 9;     // x y vx vy v sxx sxy syy Tzz
 constexpr int kNodeFields = 5;      // m ax ay vx vy
 
@@ -88,31 +97,64 @@ __device__ void isolin_adj(const MatParams &p, double exx, double exy, double ey
     Tb[3] = 0.0;
 }
 
-// g_local_mu2.c:165-310 (plane strain, T = [[Txx, Txy, 0], [Txy, Tyy, 0],
-// [0, 0, Tzz]]): trial Jaumann stress, deviatoric split, mu(I) return map.
-__device__ void g_local_mu2_adj(const MatParams &p, double m, double v, double exx, double exy, double eyy,
-                                double wxy, double Txx, double Txy, double Tyy, double Tzz, double Tb[4],
-                                MatAdj &a)
+// The constants of the particle kernels, staged in shared memory (mat::Unit).
+struct AdjConst {
+    mat::Elastic el;
+    MatParams mp;
+    mat::Known krho;                // grains_rho as a divisor
+    double ca, caG, caI0;           // G I0 dt / d and its derivatives by G and I0
+    double twodt, twoGdt, ldt;      // 2 dt, 2 G dt, lambda dt
+    double inv_h, half_inv_h;
+};
+
+AdjConst make_adj_const(const MatParams &p, double inv_h)
 {
-    const double G = p.G, dt = p.dt, lambda = p.lambda;
-    const double trD = exx + eyy;
-    const double lt = lambda * trD;
-    const double Ttr_xx = (2.0 * G * exx + lt + 2.0 * wxy * Txy) * dt + Txx;
-    const double Ttr_xy = (2.0 * G * exy + wxy * (Tyy - Txx)) * dt + Txy;
-    const double Ttr_yy = (2.0 * G * eyy + lt - 2.0 * wxy * Txy) * dt + Tyy;
-    const double Ttr_zz = lt * dt + Tzz;
-    const double pm = (Ttr_xx + Ttr_yy + Ttr_zz) / 3.0;
-    const double T0xx = Ttr_xx - pm, T0yy = Ttr_yy - pm, T0zz = Ttr_zz - pm, T0xy = Ttr_xy;
-    const double tt = T0xx * T0xx + 2.0 * T0xy * T0xy + T0yy * T0yy + T0zz * T0zz;
-    const double tau = sqrt(0.5 * tt);
+    AdjConst c;
+    c.el = mat::make_elastic(p.G, p.K, p.lambda, p.dt);
+    c.mp = p;
+    c.krho = mat::make_known(p.grains_rho);
+    c.caG = p.I0 * p.dt / p.grains_d;
+    c.caI0 = p.G * p.dt / p.grains_d;
+    c.ca = p.G * c.caG;
+    c.twodt = 2.0 * p.dt;
+    c.twoGdt = 2.0 * p.G * p.dt;
+    c.ldt = p.lambda * p.dt;
+    c.inv_h = inv_h;
+    c.half_inv_h = 0.5 * inv_h;
+    return c;
+}
+
+// g_local_mu2.c:165-310 (plane strain, T = [[Txx, Txy, 0], [Txy, Tyy, 0],
+// [0, 0, Tzz]]): trial Jaumann stress, deviatoric split, mu(I) return map, with
+// d2 = 2 Dxy and w2 = 2 Wxy.  The return's tau' is a root of
+// t^2 + B t + H = 0 with 2 tau' + B = -disc, so d tau' / dB = tau' / disc and
+// d tau' / dH = 1 / disc.  Adds to a.exx, a.eyy, a.exy, a.wxy as the other laws
+// do (exy and wxy the halves of d2 and w2).
+__device__ __forceinline__ void g_local_mu2_adj(const AdjConst &C, double m, double v, double exx, double eyy,
+                                                double d2, double w2, double Txx, double Txy, double Tyy,
+                                                double Tzz, double Tb[4], MatAdj &a)
+{
+    const mat::Elastic &u = C.el;
+    const MatParams &p = C.mp;
+    const double dt = u.dt;
+    const double trD = u.add(exx, eyy), wxy = u.mul(u.half, w2);
+    const double lt = u.mul(u.lambda, trD), dT = u.sub(Tyy, Txx);
+    const double Ttr_xx = fma(dt, fma(w2, Txy, fma(u.twoG, exx, lt)), Txx);
+    const double Ttr_xy = fma(dt, fma(u.G, d2, u.mul(wxy, dT)), Txy);
+    const double Ttr_yy = fma(dt, fma(-w2, Txy, fma(u.twoG, eyy, lt)), Tyy);
+    const double Ttr_zz = fma(dt, lt, Tzz);
+    const double pm = mat::dvd_const(u.add(u.add(Ttr_xx, Ttr_yy), Ttr_zz), u.k3);
+    const double T0xx = u.sub(Ttr_xx, pm), T0yy = u.sub(Ttr_yy, pm), T0zz = u.sub(Ttr_zz, pm), T0xy = Ttr_xy;
+    const double dev = fma(T0xx, T0xx, fma(T0yy, T0yy, u.mul(T0zz, T0zz)));
+    const double tau = mat::root(fma(u.half, dev, u.mul(T0xy, T0xy)));
     const double pr = -pm;
 
     // adjoint of the trial stress
     double bxx = 0, bxy = 0, byy = 0, bzz = 0;
-    if (m / v < p.rho_critical || !(pr > 0)) {
+    if (mat::quot(m, v) < p.rho_critical || !(pr > 0)) {
         // stress-free (or undefined) branch: T' = 0 does not depend on anything
     } else {
-        const double S0 = p.mu_s * pr;
+        const double S0 = u.mul(p.mu_s, pr);
         if (tau <= S0) {
             // elastic: T' = T0 - p I = T_trial
             bxx = Tb[0];
@@ -120,73 +162,55 @@ __device__ void g_local_mu2_adj(const MatParams &p, double m, double v, double e
             byy = Tb[2];
             bzz = Tb[3];
         } else {
-            const double S2 = p.mu_2 * pr;
-            const double sq = sqrt(pr / p.grains_rho);
-            const double ca = G * p.I0 * dt / p.grains_d;
-            const double alpha = ca * sq;
-            const double B = -(S2 + tau + alpha);
-            const double H = S2 * tau + S0 * alpha;
-            const double disc = sqrt(B * B - 4.0 * H);
-            double taup, dB, dH;     // tau' and its partial derivatives
-            if (B > 0) {
-                taup = 0.5 * (-B - disc);
-                dB = 0.5 * (-1.0 - B / disc);
-                dH = 1.0 / disc;
-            } else {
-                const double q = -B + disc;
-                taup = 2.0 * H / q;
-                const double dqB = -1.0 + B / disc, dqH = -2.0 / disc;
-                dB = -2.0 * H / (q * q) * dqB;
-                dH = 2.0 / q - 2.0 * H / (q * q) * dqH;
-            }
-            const double s = taup / tau;
+            const double S2 = u.mul(p.mu_2, pr);
+            const double sq = mat::root(mat::dvd_const(pr, C.krho));
+            const double alpha = u.mul(C.ca, sq);
+            const double nB = u.add(u.add(S2, tau), alpha);       // -B
+            const double H = fma(S2, tau, u.mul(S0, alpha));
+            const double disc = mat::root(fma(u.mfour, H, u.mul(nB, nB)));
+            const double taup = nB < 0 ? u.mul(u.half, u.sub(nB, disc)) : mat::quot<1>(H, u.add(nB, disc));
+            const double idisc = mat::quot(u.one, disc), itau = mat::quot(u.one, tau);
+            const double s = u.mul(taup, itau);
             // T'_ii = T0_ii s + pm (ii = xx, yy, zz), T'_xy = T0xy s
-            const double sb = Tb[0] * T0xx + Tb[1] * T0xy + Tb[2] * T0yy + Tb[3] * T0zz;
-            double b0xx = Tb[0] * s, b0xy = Tb[1] * s, b0yy = Tb[2] * s, b0zz = Tb[3] * s;
-            double pmb = Tb[0] + Tb[2] + Tb[3];
-            const double taupb = sb / tau;
-            double taub = -sb * taup / (tau * tau);
-            const double Bb = taupb * dB, Hb = taupb * dH;
+            const double sb = fma(Tb[0], T0xx, fma(Tb[1], T0xy, fma(Tb[2], T0yy, u.mul(Tb[3], T0zz))));
+            double pmb = u.add(u.add(Tb[0], Tb[2]), Tb[3]);
+            const double taupb = u.mul(sb, itau);
+            const double Hb = u.mul(taupb, idisc), Bb = u.mul(Hb, taup);
             // H = S2 tau + S0 alpha; B = -(S2 + tau + alpha)
-            double S2b = Hb * tau - Bb;
-            taub += Hb * S2 - Bb;
-            double S0b = Hb * alpha;
-            const double alphab = Hb * S0 - Bb;
+            const double S2b = fma(Hb, tau, -Bb), S0b = u.mul(Hb, alpha), alphab = fma(Hb, S0, -Bb);
+            const double taub = fma(-taupb, s, fma(Hb, S2, -Bb));
             // alpha = ca sqrt(p / rho_g), ca = G I0 dt / d
-            double prb = alphab * ca * 0.5 / (sq * p.grains_rho);
-            const double cab = alphab * sq;
-            a.G += cab * p.I0 * dt / p.grains_d;
-            a.I0 += cab * G * dt / p.grains_d;
-            a.mu_2 += S2b * pr;
-            prb += S2b * p.mu_2;
-            a.mu_s += S0b * pr;
-            prb += S0b * p.mu_s;
-            pmb -= prb;
+            const double cab = u.mul(alphab, sq);
+            a.G = fma(cab, C.caG, a.G);
+            a.I0 = fma(cab, C.caI0, a.I0);
+            a.mu_2 = fma(S2b, pr, a.mu_2);
+            a.mu_s = fma(S0b, pr, a.mu_s);
+            const double prb = fma(S0b, p.mu_s, fma(S2b, p.mu_2, u.mul(u.half, mat::quot(u.mul(alphab, alpha), pr))));
+            pmb = u.sub(pmb, prb);
             // tau = sqrt(tt / 2), tt = T0xx^2 + 2 T0xy^2 + T0yy^2 + T0zz^2
-            const double ttb = taub / (4.0 * tau);
-            b0xx += 2.0 * T0xx * ttb;
-            b0xy += 4.0 * T0xy * ttb;
-            b0yy += 2.0 * T0yy * ttb;
-            b0zz += 2.0 * T0zz * ttb;
+            const double kxy = u.mul(taub, itau), k = u.mul(u.half, kxy);
+            const double b0xx = fma(T0xx, k, u.mul(Tb[0], s)), b0yy = fma(T0yy, k, u.mul(Tb[2], s));
+            const double b0zz = fma(T0zz, k, u.mul(Tb[3], s));
+            bxy = fma(T0xy, kxy, u.mul(Tb[1], s));
             // T0_ii = Ttr_ii - pm, pm = (Ttr_xx + Ttr_yy + Ttr_zz) / 3
-            pmb -= b0xx + b0yy + b0zz;
-            bxx = b0xx + pmb / 3.0;
-            byy = b0yy + pmb / 3.0;
-            bzz = b0zz + pmb / 3.0;
-            bxy = b0xy;
+            const double pm3 = mat::dvd_const(u.sub(u.sub(u.sub(pmb, b0xx), b0yy), b0zz), u.k3);
+            bxx = u.add(b0xx, pm3);
+            byy = u.add(b0yy, pm3);
+            bzz = u.add(b0zz, pm3);
         }
     }
     // trial stress reversed
-    const double trb = bxx + byy + bzz;
-    a.exx += dt * (2.0 * G * bxx + lambda * trb);
-    a.eyy += dt * (2.0 * G * byy + lambda * trb);
-    a.exy += dt * 2.0 * G * bxy;
-    a.wxy += dt * (2.0 * Txy * bxx + (Tyy - Txx) * bxy - 2.0 * Txy * byy);
-    a.G += dt * 2.0 * (exx * bxx + exy * bxy + eyy * byy);
-    a.lambda += dt * trD * trb;
-    Tb[0] = bxx - dt * wxy * bxy;
-    Tb[1] = bxy + dt * 2.0 * wxy * (bxx - byy);
-    Tb[2] = byy + dt * wxy * bxy;
+    const double trb = u.add(u.add(bxx, byy), bzz), lb = u.mul(C.ldt, trb), db = u.sub(bxx, byy), db2 = u.add(db, db);
+    a.exx = fma(C.twoGdt, bxx, lb);
+    a.eyy = fma(C.twoGdt, byy, lb);
+    a.exy = u.mul(C.twoGdt, bxy);
+    a.wxy = u.mul(dt, fma(Txy, db2, u.mul(dT, bxy)));
+    a.G = fma(C.twodt, fma(exx, bxx, u.mul(eyy, byy)), fma(dt, u.mul(d2, bxy), a.G));
+    a.lambda = u.mul(u.mul(dt, trD), trb);
+    const double wdt = u.mul(dt, wxy);
+    Tb[0] = fma(-wdt, bxy, bxx);
+    Tb[1] = fma(wdt, db2, bxy);
+    Tb[2] = fma(wdt, bxy, byy);
     Tb[3] = bzz;
 }
 
@@ -357,17 +381,19 @@ struct AdjStep {
     const double *mass;         // n (constant)
     const int *elem;            // n
     const int *active;          // n
-    const uint32_t *perm;       // n
-    const int *cell_start;      // ne + 1
+    const uint32_t *perm;       // n: the elements' particle lists
+    const int *start;           // ne: where an element's list begins
+    const uint32_t *count;      // ne: and its length
     const double *nodes;        // kNodeFields x nn
     const StepParams *params;   // after the step (t used by the BCs, the step's gravity)
     // adjoints
     const double *adj_in;       // kStateFields x n, of the state after the step
     double *adj_out;            // kStateFields x n, of the state at the step start
-    double *contrib;            // 16 x n: per particle and corner (Ux, Uy, Ax, Ay) adjoint shares
-    double *cell_adj;           // 16 x ne, value-major
-    double *node_adj;           // 5 x nn: pb_x, pb_y, fb_x, fb_y, mb
-    double *theta_part;         // per adj_g2p block: TH_COUNT + (G, K, lambda) partials
+    double *contrib;            // n x 16: per particle and corner (Ux, Uy, Ax, Ay) adjoint shares
+    double *node_adj;           // nn x 6: pb_x, pb_y, fb_x, fb_y, mb, unused
+    double *theta_part;         // per adj_g2p block: the slots' partials
+    double *theta_acc;          // their sums over the steps
+    AdjConst k;
     // g_nonlocal_mu2
     const double *gf_nodes;     // nn: the step's nodal fluidity (solution of the solve)
     double *gfb;                // n: adjoint of the fluidity interpolated at each particle
@@ -377,11 +403,83 @@ struct AdjStep {
 
 constexpr int kThetaSlots = 7;   // mu_s mu_2 I0 (direct) G K lambda, E folded later; A (nonlocal)
 
-__global__ void __launch_bounds__(kAdjThreads) adj_g2p_kernel(AdjStep S)
+// Copies the constants to shared memory (the caller synchronises).
+__device__ __forceinline__ void stage_const(AdjConst &C, const AdjConst &param)
 {
-    __shared__ double red[kAdjThreads / 32][kThetaSlots];
+    static_assert(sizeof(AdjConst) % 8 == 0, "copied as 64-bit words");
+    const unsigned long long *src = reinterpret_cast<const unsigned long long *>(&param);
+    unsigned long long *dst = reinterpret_cast<unsigned long long *>(&C);
+    for (int k = threadIdx.x; k < (int)(sizeof(AdjConst) / 8); k += blockDim.x) dst[k] = src[k];
+}
+
+// A nodal field's bilinear coefficients on an element, q0 + c1 x + c2 y + c3 xy
+// from the corners BL, BR, TR, TL, and h times its gradient at (x, y).
+struct Coef {
+    double q0, c1, c2, c3, gx, gy;
+};
+__device__ __forceinline__ Coef coef_at(const mat::Unit &u, double q0, double q1, double q2, double q3, double x,
+                                        double y)
+{
+    Coef f;
+    f.q0 = q0;
+    f.c1 = u.sub(q1, q0);
+    f.c2 = u.sub(q3, q0);
+    f.c3 = u.sub(u.sub(q2, q3), f.c1);
+    f.gx = fma(y, f.c3, f.c1);
+    f.gy = fma(x, f.c3, f.c2);
+    return f;
+}
+__device__ __forceinline__ double value_at(const Coef &f, double x, double y)
+{
+    return fma(y, f.gy, fma(x, f.c1, f.q0));
+}
+
+// Adds each of eight values over the warp, the sum of value q to lanes with
+// lane / 4 == q: three exchanges that halve the values, then two of one value,
+// nine additions instead of forty.
+__device__ __forceinline__ double warp_sum8(const mat::Unit &u, const double v[8])
+{
+    const int lane = threadIdx.x & 31;
+    double a[4], b[2];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const double keep = lane & 16 ? v[4 + k] : v[k], send = lane & 16 ? v[k] : v[4 + k];
+        a[k] = u.add(keep, __shfl_xor_sync(0xffffffffu, send, 16));
+    }
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const double keep = lane & 8 ? a[2 + k] : a[k], send = lane & 8 ? a[k] : a[2 + k];
+        b[k] = u.add(keep, __shfl_xor_sync(0xffffffffu, send, 8));
+    }
+    const double keep = lane & 4 ? b[1] : b[0], send = lane & 4 ? b[0] : b[1];
+    double c = u.add(keep, __shfl_xor_sync(0xffffffffu, send, 4));
+    c = u.add(c, __shfl_xor_sync(0xffffffffu, c, 2));
+    return u.add(c, __shfl_xor_sync(0xffffffffu, c, 1));
+}
+
+// One particle's corner shares of a field's adjoint where the field enters
+// through its value (adjoint R) and h times its gradient (P, Q): with
+// t1 = P + R x and t2 = Q + R y the corners TR, BR, TL, BL are t1 y + Q x,
+// t1 - TR, t2 - TR and R - t1 - TL.
+__device__ __forceinline__ void corner_shares(const mat::Unit &u, double R, double t1, double t2, double tr,
+                                              double out[4])
+{
+    out[2] = tr;
+    out[1] = u.sub(t1, tr);
+    out[3] = u.sub(t2, tr);
+    out[0] = u.sub(u.sub(R, t1), out[3]);
+}
+
+template <int MATERIAL>
+__global__ void __launch_bounds__(kAdjThreads) adj_g2p_kernel(const __grid_constant__ AdjStep S)
+{
+    __shared__ AdjConst C;
+    __shared__ double red[kAdjThreads / 32][8];
+    stage_const(C, S.k);
+    __syncthreads();
+    const mat::Elastic &u = C.el;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    double th[kThetaSlots] = {0, 0, 0, 0, 0, 0, 0};
+    double th[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     if (i < S.n) {
         const size_t n = (size_t)S.n;
         double in[kStateFields];
@@ -389,54 +487,46 @@ __global__ void __launch_bounds__(kAdjThreads) adj_g2p_kernel(AdjStep S)
         for (int f = 0; f < kStateFields; f++) in[f] = S.adj_in[f * n + i];
         const int e = S.elem[i];
         if (!S.active[i] || e < 0) {
-            // inactive: the state is carried unchanged
+            // inactive: the state is carried unchanged (and no list holds it)
 #pragma unroll
             for (int f = 0; f < kStateFields; f++) S.adj_out[f * n + i] = in[f];
-#pragma unroll
-            for (int k = 0; k < 16; k++) S.contrib[k * n + i] = 0.0;
         } else {
             const GridGeom &g = S.g;
-            const double x = S.state[0 * n + i], y = S.state[1 * n + i];
+            const double px = S.state[0 * n + i], py = S.state[1 * n + i];
             const double V = S.state[4 * n + i];
             const double Txx = S.state[5 * n + i], Txy = S.state[6 * n + i], Tyy = S.state[7 * n + i],
                          Tzz = S.state[8 * n + i];
-            const int ci = e % g.Ex, cj = e / g.Ex;
+            const int cj = e / g.Ex, ci = e - cj * g.Ex;
             const int n0 = cj * g.Nx + ci;
             const int nd[4] = {n0, n0 + 1, n0 + 1 + g.Nx, n0 + g.Nx};
-            const double xl = (x - ci * g.h) * g.inv_h, yl = (y - cj * g.h) * g.inv_h;
-            const ShapeFns f = fp64::shape(xl, yl, g.inv_h);
+            const double inv_h = C.inv_h, dt = u.dt;
+            const double x = mpmg_local_coord_fma(px, mat::small_int(ci), inv_h);
+            const double y = mpmg_local_coord_fma(py, mat::small_int(cj), inv_h);
             const size_t nn = (size_t)S.nn;
-            double ax[4], ay[4], ux[4], uy[4];
+            Coef q[4];          // ax, ay, ux, uy
 #pragma unroll
-            for (int a = 0; a < 4; a++) {
-                ax[a] = S.nodes[1 * nn + nd[a]];
-                ay[a] = S.nodes[2 * nn + nd[a]];
-                ux[a] = S.nodes[3 * nn + nd[a]];
-                uy[a] = S.nodes[4 * nn + nd[a]];
+            for (int k = 0; k < 4; k++) {
+                const double *v = S.nodes + (size_t)(1 + k) * nn;
+                q[k] = coef_at(u, v[nd[0]], v[nd[1]], v[nd[2]], v[nd[3]], x, y);
             }
-            double exx = 0, eyy = 0, dxdy = 0, dydx = 0;
-#pragma unroll
-            for (int a = 0; a < 4; a++) {
-                exx += f.gx[a] * ux[a];
-                eyy += f.gy[a] * uy[a];
-                dxdy += f.gy[a] * ux[a];
-                dydx += f.gx[a] * uy[a];
-            }
-            const double dt = S.dt;
-            const double exy = 0.5 * (dxdy + dydx), wxy = 0.5 * (dxdy - dydx);
-            const double ex = mat::exp_small(dt * (exx + eyy));
-            const double Vn = V * ex;
+            const Coef &qax = q[0], &qay = q[1], &qux = q[2], &quy = q[3];
+            const double exx = u.mul(qux.gx, inv_h), eyy = u.mul(quy.gy, inv_h);
+            const double gsum = u.add(qux.gy, quy.gx), gdiff = u.sub(qux.gy, quy.gx);
+            const double ex = mat::exp_small(u.mul(dt, u.add(exx, eyy)));
+            const double Vn = u.mul(V, ex);
 
             // material
             double Tb[4] = {in[5], in[6], in[7], in[8]};
             MatAdj ma = {};
-            double vnl = 0, snl[4] = {0, 0, 0, 0}, gxnl[4] = {0, 0, 0, 0}, gynl[4] = {0, 0, 0, 0};
-            if (S.material == MPMG_ISOLIN) {
-                isolin_adj(S.mp, exx, exy, eyy, wxy, Txx, Txy, Tyy, Tb, ma);
+            double vnb = in[4], xb = in[0], yb = in[1];
+            if (MATERIAL == MPMG_ISOLIN) {
+                isolin_adj(C.mp, exx, C.half_inv_h * gsum, eyy, C.half_inv_h * gdiff, Txx, Txy, Tyy, Tb, ma);
                 Tb[3] = in[8];      // isolin leaves Tzz alone
-            } else if (S.material == MPMG_G_NONLOCAL_MU2) {
+            } else if (MATERIAL == MPMG_G_NONLOCAL_MU2) {
                 // the element's nodal fluidity g and its adjoint lam: the block's
                 // adjoint is -(lam g^T) symmetrised, the right-hand side's lam
+                const ShapeFns f = fp64::shape(x, y, inv_h);
+                double vnl = 0, snl[4] = {0, 0, 0, 0}, gxnl[4] = {0, 0, 0, 0}, gynl[4] = {0, 0, 0, 0};
                 double gn[4], ln[4], gf = 0;
 #pragma unroll
                 for (int a = 0; a < 4; a++) {
@@ -452,47 +542,58 @@ __global__ void __launch_bounds__(kAdjThreads) adj_g2p_kernel(AdjStep S)
                     for (int b = a; b < 4; b++)
                         kb[sym10(a, b)] = a == b ? -ln[a] * gn[a] : -(ln[a] * gn[b] + ln[b] * gn[a]);
                 }
-                g_nonlocal_mu2_adj(S.mp, S.mass[i], Vn, exx, exy, eyy, wxy, Txx, Txy, Tyy, f, gf, kb, fb, Tb, ma,
-                                   vnl, snl, gxnl, gynl);
+                g_nonlocal_mu2_adj(C.mp, S.mass[i], Vn, exx, C.half_inv_h * gsum, eyy, C.half_inv_h * gdiff, Txx, Txy,
+                                   Tyy, f, gf, kb, fb, Tb, ma, vnl, snl, gxnl, gynl);
                 // the fluidity gather gf = sum N_a g_a, shape values reversed
                 const double gfb = S.gfb[i];
 #pragma unroll
-                for (int a = 0; a < 4; a++) snl[a] += gfb * gn[a];
+                for (int a = 0; a < 4; a++) {
+                    const double sa = fma(gfb, gn[a], snl[a]), hxy = shape_xy(a, inv_h);
+                    xb += sa * f.gx[a] + gynl[a] * hxy;
+                    yb += sa * f.gy[a] + gxnl[a] * hxy;
+                }
+                vnb += vnl;         // the nonlocal assembly also reads V'
                 Tb[3] = in[8];      // plane stress state: Tzz is carried
             } else {
-                g_local_mu2_adj(S.mp, S.mass[i], Vn, exx, exy, eyy, wxy, Txx, Txy, Tyy, Tzz, Tb, ma);
+                g_local_mu2_adj(C, S.mass[i], Vn, exx, eyy, u.mul(gsum, inv_h), u.mul(gdiff, inv_h), Txx, Txy, Tyy,
+                                Tzz, Tb, ma);
             }
-            // volume V' = V exp(dt trD) (the nonlocal assembly also reads V')
-            const double vnb = in[4] + vnl;
-            const double Vb = vnb * ex;
-            const double trb = vnb * Vn * dt;
-            const double exxb = ma.exx + trb, eyyb = ma.eyy + trb;
-            const double dxdyb = 0.5 * (ma.exy + ma.wxy), dydxb = 0.5 * (ma.exy - ma.wxy);
-            // gathers
-            double sb[4], gxb[4], gyb[4];
+            // volume V' = V exp(dt trD)
+            const double Vb = u.mul(vnb, ex);
+            const double trb = u.mul(u.mul(vnb, Vn), dt);
+            // adjoints of the gathers: h times the gradients of ux (Pu, Qu) and
+            // uy (Pv, Qv), and the values of the four fields (R)
+            const double Pu = u.mul(u.add(ma.exx, trb), inv_h), Qv = u.mul(u.add(ma.eyy, trb), inv_h);
+            const double Qu = u.mul(u.add(ma.exy, ma.wxy), C.half_inv_h), Pv = u.mul(u.sub(ma.exy, ma.wxy), C.half_inv_h);
+            double R[4], sh[4][4];      // ux, uy, ax, ay
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                R[k] = u.mul(dt, in[k]);
+                double t1, t2, tr;
+                if (k < 2) {
+                    const double P = k == 0 ? Pu : Pv, Q = k == 0 ? Qu : Qv;
+                    t1 = fma(R[k], x, P);
+                    t2 = fma(R[k], y, Q);
+                    tr = fma(t1, y, u.mul(Q, x));
+                } else {
+                    t1 = u.mul(R[k], x);
+                    t2 = u.mul(R[k], y);
+                    tr = u.mul(t1, y);
+                }
+                corner_shares(u, R[k], t1, t2, tr, sh[k]);
+            }
+            double2 *out = reinterpret_cast<double2 *>(S.contrib + (size_t)i * 16);
 #pragma unroll
             for (int a = 0; a < 4; a++) {
-                const double uxb = exxb * f.gx[a] + dxdyb * f.gy[a] + dt * f.s[a] * in[0];
-                const double uyb = eyyb * f.gy[a] + dydxb * f.gx[a] + dt * f.s[a] * in[1];
-                const double axb = dt * f.s[a] * in[2];
-                const double ayb = dt * f.s[a] * in[3];
-                S.contrib[(a * 4 + 0) * n + i] = uxb;
-                S.contrib[(a * 4 + 1) * n + i] = uyb;
-                S.contrib[(a * 4 + 2) * n + i] = axb;
-                S.contrib[(a * 4 + 3) * n + i] = ayb;
-                sb[a] = dt * (ux[a] * in[0] + uy[a] * in[1] + ax[a] * in[2] + ay[a] * in[3]) + snl[a];
-                gxb[a] = exxb * ux[a] + dydxb * uy[a] + gxnl[a];
-                gyb[a] = eyyb * uy[a] + dxdyb * ux[a] + gynl[a];
+                out[2 * a] = make_double2(sh[0][a], sh[1][a]);
+                out[2 * a + 1] = make_double2(sh[2][a], sh[3][a]);
             }
-            double xb = in[0], yb = in[1];
-#pragma unroll
-            for (int a = 0; a < 4; a++) {
-                const double hxy = shape_xy(a, g.inv_h);
-                xb += sb[a] * f.gx[a] + gyb[a] * hxy;
-                yb += sb[a] * f.gy[a] + gxb[a] * hxy;
-            }
-            S.adj_out[0 * n + i] = xb;
-            S.adj_out[1 * n + i] = yb;
+            // the start-of-step position: the fields' gradients and mixed derivatives
+            double tx = fma(Qv, quy.c3, u.mul(Qu, qux.c3)), ty = fma(Pv, quy.c3, u.mul(Pu, qux.c3));
+            tx = fma(R[0], qux.gx, fma(R[1], quy.gx, fma(R[2], qax.gx, fma(R[3], qay.gx, tx))));
+            ty = fma(R[0], qux.gy, fma(R[1], quy.gy, fma(R[2], qax.gy, fma(R[3], qay.gy, ty))));
+            S.adj_out[0 * n + i] = fma(inv_h, tx, xb);
+            S.adj_out[1 * n + i] = fma(inv_h, ty, yb);
             S.adj_out[2 * n + i] = in[2];
             S.adj_out[3 * n + i] = in[3];
             S.adj_out[4 * n + i] = Vb;
@@ -511,17 +612,12 @@ __global__ void __launch_bounds__(kAdjThreads) adj_g2p_kernel(AdjStep S)
     }
     // block partials of the parameter adjoint (fixed tree order)
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-    for (int k = 0; k < kThetaSlots; k++) {
-        double v = th[k];
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-        if (lane == 0) red[w][k] = v;
-    }
+    const double sum = warp_sum8(u, th);
+    if ((lane & 3) == 0) red[w][lane >> 2] = sum;
     __syncthreads();
     if (threadIdx.x < kThetaSlots) {
-        double v = 0;
-        for (int q = 0; q < kAdjThreads / 32; q++) v += red[q][threadIdx.x];
+        double v = red[0][threadIdx.x];
+        for (int k = 1; k < kAdjThreads / 32; k++) v = u.add(v, red[k][threadIdx.x]);
         S.theta_part[(size_t)blockIdx.x * kThetaSlots + threadIdx.x] = v;
     }
 }
@@ -587,7 +683,8 @@ __global__ void __launch_bounds__(128) adj_nl_rhs_kernel(AdjStep S)
     const size_t n = (size_t)S.n;
     const int ci = e % g.Ex, cj = e / g.Ex;
     double F[4] = {0, 0, 0, 0};
-    for (int k = S.cell_start[e]; k < S.cell_start[e + 1]; k++) {
+    const int k0 = S.start[e], k1 = k0 + (int)S.count[e];
+    for (int k = k0; k < k1; k++) {
         const int i = (int)S.perm[k];
         const double xl = (S.state[0 * n + i] - ci * g.h) * g.inv_h, yl = (S.state[1 * n + i] - cj * g.h) * g.inv_h;
         const ShapeFns f = fp64::shape(xl, yl, g.inv_h);
@@ -599,148 +696,183 @@ __global__ void __launch_bounds__(128) adj_nl_rhs_kernel(AdjStep S)
     for (int a = 0; a < 4; a++) S.rhs[(size_t)a * S.ne + e] = F[a];
 }
 
-// Per element: the corner shares of its particles, in the binned order.
-__global__ void __launch_bounds__(128) adj_cells_kernel(AdjStep S)
+// Per node: the corner shares of the particles around it summed, then the
+// nodal update reversed (grid_kernel of mpmg_step.cu).  Four lanes a node, one
+// for each of Ux, Uy, Ax, Ay (a particle's share of a node is one 32-byte
+// sector): a warp's chain of additions is the particles around its eight nodes.
+__global__ void __launch_bounds__(256) adj_node_kernel(const __grid_constant__ AdjStep S)
 {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= S.ne) return;
-    const int k0 = S.cell_start[e], k1 = S.cell_start[e + 1];
-    double acc[16];
-#pragma unroll
-    for (int k = 0; k < 16; k++) acc[k] = 0.0;
-    const size_t n = (size_t)S.n;
-    for (int k = k0; k < k1; k++) {
-        const int i = (int)S.perm[k];
-#pragma unroll
-        for (int q = 0; q < 16; q++) acc[q] += S.contrib[q * n + i];
-    }
-#pragma unroll
-    for (int q = 0; q < 16; q++) S.cell_adj[(size_t)q * S.ne + e] = acc[q];
-}
-
-// Per node: the nodal update reversed (grid_kernel of mpmg_step.cu).
-__global__ void __launch_bounds__(256) adj_grid_kernel(AdjStep S)
-{
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= S.nn) return;
+    __shared__ AdjConst C;
+    stage_const(C, S.k);
+    __syncthreads();
+    const mat::Unit &u = C.el;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int n = t >> 2, q = t & 3;
+    const bool inside = n < S.nn;
     const GridGeom &g = S.g;
-    const int i = n % g.Nx, j = n / g.Nx;
-    double ub[4] = {0, 0, 0, 0};     // Ux, Uy, Ax, Ay adjoints
-#pragma unroll
-    for (int c = 0; c < 4; c++) {
-        const int ci = ((i & 1) == (c & 1)) ? i : i - 1;
-        const int cj = ((j & 1) == (c >> 1)) ? j : j - 1;
-        if (ci < 0 || cj < 0 || ci >= g.Ex || cj >= g.Ey) continue;
-        const int e = cj * g.Ex + ci;
-        if (S.cell_start[e] == S.cell_start[e + 1]) continue;
-        const int corner = (ci == i) ? ((cj == j) ? 0 : 3) : ((cj == j) ? 1 : 2);
-#pragma unroll
-        for (int q = 0; q < 4; q++) ub[q] += S.cell_adj[(size_t)(corner * 4 + q) * S.ne + e];
-    }
     const size_t nn = (size_t)S.nn;
-    const double m = S.nodes[n];
-    double pbx = 0, pby = 0, fbx = 0, fby = 0, mb = 0;
-    if (m > MPMG_TOL) {
+    const double m = inside ? S.nodes[n] : 0.0;
+    const int i = n % g.Nx, j = n / g.Nx;
+    const bool live = m > MPMG_TOL;
+    double ub = 0;
+    if (live) {
+        int k0[4], cnt[4], corner[4];
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            const int ci = ((i & 1) == (c & 1)) ? i : i - 1;
+            const int cj = ((j & 1) == (c >> 1)) ? j : j - 1;
+            const bool have = ci >= 0 && cj >= 0 && ci < g.Ex && cj < g.Ey;
+            const int e = have ? cj * g.Ex + ci : 0;
+            cnt[c] = have ? (int)S.count[e] : 0;
+            k0[c] = S.start[e];
+            corner[c] = (ci == i) ? ((cj == j) ? 0 : 3) : ((cj == j) ? 1 : 2);
+        }
+        // the first four particles of every element in flight together
+        double v[4][4];
+        uint32_t at[4][4];
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+#pragma unroll
+            for (int k = 0; k < 4; k++) at[c][k] = k < cnt[c] ? S.perm[k0[c] + k] : 0u;
+        }
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                if (k < cnt[c]) v[c][k] = S.contrib[(size_t)at[c][k] * 16 + corner[c] * 4 + q];
+        }
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                if (k < cnt[c]) ub = u.add(ub, v[c][k]);
+            for (int k = 4; k < cnt[c]; k++)
+                ub = u.add(ub, S.contrib[(size_t)S.perm[k0[c] + k] * 16 + corner[c] * 4 + q]);
+        }
+    }
+    // U = (P + dt F) / m, A = F / m on unmasked components: lanes 0 and 1 (2 and
+    // 3 alike) reverse x and y
+    const double other = __shfl_xor_sync(0xffffffffu, ub, 2);
+    const double uc = q < 2 ? ub : other, ac = q < 2 ? other : ub;
+    double pb = 0, fb = 0, mb = 0;
+    if (live) {
         bool bx, by;
         fp64::bc_mask(S.bc, g, i, j, S.params->t, bx, by);
-        const double ax = S.nodes[1 * nn + n], ay = S.nodes[2 * nn + n];
-        const double ux = S.nodes[3 * nn + n], uy = S.nodes[4 * nn + n];
-        // U = (P + dt F) / m, A = F / m on unmasked components
-        if (!bx) {
-            pbx = ub[0] / m;
-            fbx = (ub[2] + S.dt * ub[0]) / m;
-            mb -= (ub[0] * ux + ub[2] * ax) / m;
-        }
-        if (!by) {
-            pby = ub[1] / m;
-            fby = (ub[3] + S.dt * ub[1]) / m;
-            mb -= (ub[1] * uy + ub[3] * ay) / m;
+        if (!((q & 1) ? by : bx)) {
+            const double a = S.nodes[(size_t)(1 + (q & 1)) * nn + n], v = S.nodes[(size_t)(3 + (q & 1)) * nn + n];
+            const double inv_m = mat::quot(u.one, m);
+            pb = u.mul(uc, inv_m);
+            fb = u.mul(fma(C.el.dt, uc, ac), inv_m);
+            mb = -u.mul(fma(uc, v, u.mul(ac, a)), inv_m);
         }
     }
-    S.node_adj[0 * nn + n] = pbx;
-    S.node_adj[1 * nn + n] = pby;
-    S.node_adj[2 * nn + n] = fbx;
-    S.node_adj[3 * nn + n] = fby;
-    S.node_adj[4 * nn + n] = mb;
+    mb = u.add(mb, __shfl_xor_sync(0xffffffffu, mb, 1));
+    if (inside && q < 2) {
+        double *out = S.node_adj + (size_t)n * 6;
+        out[q] = pb;
+        out[2 + q] = fb;
+        if (q == 0) out[4] = mb;
+    }
 }
 
-// Per particle: P2G (p2g_cells_kernel of mpmg_step.cu) reversed.
-__global__ void __launch_bounds__(kAdjThreads) adj_p2g_kernel(AdjStep S)
+// Per particle: P2G (p2g_cells_kernel of mpmg_step.cu) reversed.  With the
+// nodal adjoints as fields: v' = m pb, V' = -T : grad fb, T' = -V sym grad fb,
+// and the position's from grad (m (mb + v pb + g fb_y)) and fb's mixed
+// derivative (the gradients of the shape functions).  The last block adds the
+// step's block partials to the parameter adjoint, a warp a slot.
+__global__ void __launch_bounds__(kAdjThreads) adj_p2g_kernel(const __grid_constant__ AdjStep S)
 {
+    __shared__ AdjConst C;
+    stage_const(C, S.k);
+    __syncthreads();
+    const mat::Elastic &u = C.el;
+    const int blocks = gridDim.x - 1;
+    if ((int)blockIdx.x == blocks) {
+        const int lane = threadIdx.x & 31;
+        for (int slot = threadIdx.x >> 5; slot < kThetaSlots; slot += kAdjThreads / 32) {
+            double v = 0;
+            for (int b = lane; b < blocks; b += 32) v = u.add(v, S.theta_part[(size_t)b * kThetaSlots + slot]);
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) v = u.add(v, __shfl_down_sync(0xffffffffu, v, off));
+            if (lane == 0) S.theta_acc[slot] = u.add(S.theta_acc[slot], v);
+        }
+        return;
+    }
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= S.n) return;
     const int e = S.elem[i];
     if (!S.active[i] || e < 0) return;
     const GridGeom &g = S.g;
-    const size_t n = (size_t)S.n, nn = (size_t)S.nn;
-    const double x = S.state[0 * n + i], y = S.state[1 * n + i];
+    const size_t n = (size_t)S.n;
+    const double px = S.state[0 * n + i], py = S.state[1 * n + i];
     const double vx = S.state[2 * n + i], vy = S.state[3 * n + i];
     const double V = S.state[4 * n + i];
     const double Txx = S.state[5 * n + i], Txy = S.state[6 * n + i], Tyy = S.state[7 * n + i];
     const double mp = S.mass[i];
     const double grav = S.params->gravity;
-    const int ci = e % g.Ex, cj = e / g.Ex;
+    const int cj = e / g.Ex, ci = e - cj * g.Ex;
     const int n0 = cj * g.Nx + ci;
     const int nd[4] = {n0, n0 + 1, n0 + 1 + g.Nx, n0 + g.Nx};
-    const double xl = (x - ci * g.h) * g.inv_h, yl = (y - cj * g.h) * g.inv_h;
-    const ShapeFns f = fp64::shape(xl, yl, g.inv_h);
-    double vxb = 0, vyb = 0, Vb = 0, Txxb = 0, Txyb = 0, Tyyb = 0, xb = 0, yb = 0;
+    const double inv_h = C.inv_h;
+    const double x = mpmg_local_coord_fma(px, mat::small_int(ci), inv_h);
+    const double y = mpmg_local_coord_fma(py, mat::small_int(cj), inv_h);
+    double2 p[4], f[4];
+    double mb[4];
 #pragma unroll
     for (int a = 0; a < 4; a++) {
-        const double pbx = S.node_adj[0 * nn + nd[a]], pby = S.node_adj[1 * nn + nd[a]];
-        const double fbx = S.node_adj[2 * nn + nd[a]], fby = S.node_adj[3 * nn + nd[a]];
-        const double mb = S.node_adj[4 * nn + nd[a]];
-        // m_a += N m; P_a += N m v; F_a += N m b - V T grad N (b = (0, g))
-        const double sb = mb * mp + mp * (vx * pbx + vy * pby) + mp * grav * fby;
-        vxb += f.s[a] * mp * pbx;
-        vyb += f.s[a] * mp * pby;
-        const double tgx = Txx * f.gx[a] + Txy * f.gy[a], tgy = Txy * f.gx[a] + Tyy * f.gy[a];
-        Vb -= fbx * tgx + fby * tgy;
-        Txxb -= V * fbx * f.gx[a];
-        Txyb -= V * (fbx * f.gy[a] + fby * f.gx[a]);
-        Tyyb -= V * fby * f.gy[a];
-        const double gxb = -V * (fbx * Txx + fby * Txy), gyb = -V * (fbx * Txy + fby * Tyy);
-        const double hxy = shape_xy(a, g.inv_h);
-        xb += sb * f.gx[a] + gyb * hxy;
-        yb += sb * f.gy[a] + gxb * hxy;
+        const double *v = S.node_adj + (size_t)nd[a] * 6;
+        p[a] = *reinterpret_cast<const double2 *>(v);
+        f[a] = *reinterpret_cast<const double2 *>(v + 2);
+        mb[a] = v[4];
     }
-    S.adj_out[0 * n + i] += xb;
-    S.adj_out[1 * n + i] += yb;
-    S.adj_out[2 * n + i] += vxb;
-    S.adj_out[3 * n + i] += vyb;
-    S.adj_out[4 * n + i] += Vb;
-    S.adj_out[5 * n + i] += Txxb;
-    S.adj_out[6 * n + i] += Txyb;
-    S.adj_out[7 * n + i] += Tyyb;
+    const Coef pbx = coef_at(u, p[0].x, p[1].x, p[2].x, p[3].x, x, y);
+    const Coef pby = coef_at(u, p[0].y, p[1].y, p[2].y, p[3].y, x, y);
+    const Coef fbx = coef_at(u, f[0].x, f[1].x, f[2].x, f[3].x, x, y);
+    const Coef fby = coef_at(u, f[0].y, f[1].y, f[2].y, f[3].y, x, y);
+    const Coef mbc = coef_at(u, mb[0], mb[1], mb[2], mb[3], x, y);
+    // m_a += N m; P_a += N m v; F_a += N m b - V T grad N (b = (0, g))
+    const double gxy = u.add(fbx.gy, fby.gx);
+    const double Vh = -u.mul(V, inv_h);
+    const double Vb = u.mul(fma(Txx, fbx.gx, fma(Txy, gxy, u.mul(Tyy, fby.gy))), -inv_h);
+    const double wx = fma(vx, pbx.gx, fma(vy, pby.gx, fma(grav, fby.gx, mbc.gx)));
+    const double wy = fma(vx, pbx.gy, fma(vy, pby.gy, fma(grav, fby.gy, mbc.gy)));
+    const double mh = u.mul(mp, inv_h), Vhh = u.mul(Vh, inv_h);
+    const double hx = fma(Txy, fbx.c3, u.mul(Tyy, fby.c3)), hy = fma(Txx, fbx.c3, u.mul(Txy, fby.c3));
+    double *out = S.adj_out + i;
+    out[0 * n] = fma(mh, wx, fma(Vhh, hx, out[0 * n]));
+    out[1 * n] = fma(mh, wy, fma(Vhh, hy, out[1 * n]));
+    out[2 * n] = fma(mp, value_at(pbx, x, y), out[2 * n]);
+    out[3 * n] = fma(mp, value_at(pby, x, y), out[3 * n]);
+    out[4 * n] = u.add(out[4 * n], Vb);
+    out[5 * n] = fma(Vh, fbx.gx, out[5 * n]);
+    out[6 * n] = fma(Vh, gxy, out[6 * n]);
+    out[7 * n] = fma(Vh, fby.gy, out[7 * n]);
 }
 
-// The step's block partials added in block order (one thread per slot).
-__global__ void adj_theta_kernel(const double *__restrict__ part, int blocks, double *__restrict__ acc)
+// The particle state's arrays.
+struct StatePtrs {
+    const double *x, *y, *vx, *vy, *v, *sxx, *sxy, *syy, *Tzz;
+};
+
+__device__ __forceinline__ void copy_state(const StatePtrs &p, int n, int i, double *__restrict__ out)
 {
-    const int k = threadIdx.x;
-    if (k >= kThetaSlots) return;
-    double v = acc[k];
-    for (int b = 0; b < blocks; b++) v += part[(size_t)b * kThetaSlots + k];
-    acc[k] = v;
+    const size_t N = (size_t)n;
+    out[0 * N + i] = p.x[i];
+    out[1 * N + i] = p.y[i];
+    out[2 * N + i] = p.vx[i];
+    out[3 * N + i] = p.vy[i];
+    out[4 * N + i] = p.v[i];
+    out[5 * N + i] = p.sxx[i];
+    out[6 * N + i] = p.sxy[i];
+    out[7 * N + i] = p.syy[i];
+    out[8 * N + i] = p.Tzz ? p.Tzz[i] : 0.0;
 }
 
 // Copies the step-start particle state into a tape slot (one launch).
-__global__ void save_state_kernel(int n, const double *x, const double *y, const double *vx, const double *vy,
-                                  const double *v, const double *sxx, const double *sxy, const double *syy,
-                                  const double *Tzz, double *__restrict__ out)
+__global__ void save_state_kernel(int n, StatePtrs p, double *__restrict__ out)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const size_t N = (size_t)n;
-    out[0 * N + i] = x[i];
-    out[1 * N + i] = y[i];
-    out[2 * N + i] = vx[i];
-    out[3 * N + i] = vy[i];
-    out[4 * N + i] = v[i];
-    out[5 * N + i] = sxx[i];
-    out[6 * N + i] = sxy[i];
-    out[7 * N + i] = syy[i];
-    out[8 * N + i] = Tzz ? Tzz[i] : 0.0;
+    if (i < n) copy_state(p, n, i, out);
 }
 
 __global__ void load_state_kernel(int n, const double *__restrict__ in, double *x, double *y, double *vx,
@@ -761,23 +893,43 @@ __global__ void load_state_kernel(int n, const double *__restrict__ in, double *
 }
 
 // Records the step's outputs the reverse pass needs: elements and activity
-// after the keys phase, the binned order, the nodal fields, the step record.
-__global__ void save_step_kernel(int n, int ne, int nn, const int *in_element, const int *active,
-                                 const uint32_t *perm, const int *cell_start, const double *node_m,
-                                 const double *node_ax, const double *node_ay, const double *node_vx,
-                                 const double *node_vy, const StepParams *sp, int *__restrict__ elem_out,
-                                 int *__restrict__ active_out, uint32_t *__restrict__ perm_out,
-                                 int *__restrict__ cs_out, double *__restrict__ nodes_out,
-                                 StepParams *__restrict__ sp_out)
+// after the keys phase, the ordered list of each element's particles (from the
+// rows the P2G ordered; lists follow one another in the order in which warps
+// take their space, which nothing depends on), the nodal fields, the step
+// record; and the state after the step where the next step is recorded too.
+__global__ void __launch_bounds__(256) save_step_kernel(
+    int n, int ne, int nn, const int *in_element, const int *active, RowView rv, const double *node_m,
+    const double *node_ax, const double *node_ay, const double *node_vx, const double *node_vy, const StepParams *sp,
+    StatePtrs next, int *__restrict__ elem_out, int *__restrict__ active_out, uint32_t *__restrict__ perm_out,
+    int *__restrict__ start_out, uint32_t *__restrict__ count_out, uint32_t *__restrict__ cursor,
+    double *__restrict__ nodes_out, StepParams *__restrict__ sp_out, double *__restrict__ next_out)
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k == 0) *sp_out = *sp;
     if (k < n) {
         elem_out[k] = active[k] ? in_element[k] : -1;
         active_out[k] = active[k];
-        perm_out[k] = perm[k];
+        if (next_out != nullptr) copy_state(next, n, k, next_out);
     }
-    if (k <= ne) cs_out[k] = cell_start[k];
+    const int lane = threadIdx.x & 31;
+    const int cnt = k < ne ? (int)rv.count[k] : 0;
+    int incl = cnt;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int w = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += w;
+    }
+    uint32_t base = 0;
+    if (lane == 31 && incl > 0) base = atomicAdd(cursor, (uint32_t)incl);
+    base = __shfl_sync(0xffffffffu, base, 31) + (uint32_t)(incl - cnt);
+    if (k < ne) {
+        start_out[k] = (int)base;
+        count_out[k] = (uint32_t)cnt;
+        if (cnt > 0) {
+            const uint32_t *list = rv.list(k, cnt);
+            for (int q = 0; q < cnt; q++) perm_out[base + q] = list[q];
+        }
+    }
     if (k < nn) {
         const size_t N = (size_t)nn;
         nodes_out[0 * N + k] = node_m[k];
@@ -823,7 +975,9 @@ struct AdjTape {
     double *seg_state = nullptr;    // K x kStateFields x n
     int *seg_elem = nullptr, *seg_active = nullptr;   // K x n
     uint32_t *seg_perm = nullptr;   // K x n
-    int *seg_cs = nullptr;          // K x (ne + 1)
+    int *seg_start = nullptr;       // K x ne
+    uint32_t *seg_count = nullptr;  // K x ne
+    uint32_t *seg_cursor = nullptr; // K
     double *seg_nodes = nullptr;    // K x kNodeFields x nn
     StepParams *seg_params = nullptr;   // K
     // g_nonlocal_mu2: each recorded step's nodal fluidity and element blocks
@@ -831,7 +985,7 @@ struct AdjTape {
     double *seg_ek = nullptr;       // K x 10 x ne
     // reverse pass
     double *adj[2] = {nullptr, nullptr};   // kStateFields x n
-    double *contrib = nullptr, *cell_adj = nullptr, *node_adj = nullptr;
+    double *contrib = nullptr, *node_adj = nullptr;
     double *theta_part = nullptr, *theta_acc = nullptr;
     double *gfb = nullptr, *rhs = nullptr, *lam = nullptr;   // g_nonlocal_mu2
     double grad[TH_ALL] = {0, 0, 0, 0, 0};   // the last backward pass's parameter gradient
@@ -844,8 +998,8 @@ void mpmg_adj_free(mpmg_ctx *ctx)
     if (t == nullptr) return;
     void *ptrs[] = {t->ck_state, t->ck_active, t->ck_elem, t->ck_params, t->final_state, t->final_active,
                     t->final_elem, t->final_params, t->seg_state, t->seg_elem, t->seg_active, t->seg_perm,
-                    t->seg_cs, t->seg_nodes, t->seg_params, t->adj[0], t->adj[1], t->contrib, t->cell_adj,
-                    t->node_adj, t->theta_part, t->theta_acc, t->seg_gf, t->seg_ek, t->gfb, t->rhs, t->lam};
+                    t->seg_start, t->seg_count, t->seg_cursor, t->seg_nodes, t->seg_params, t->adj[0], t->adj[1],
+                    t->contrib, t->node_adj, t->theta_part, t->theta_acc, t->seg_gf, t->seg_ek, t->gfb, t->rhs, t->lam};
     for (void *p : ptrs) cudaFree(p);
     delete t;
     ctx->adj = nullptr;
@@ -853,12 +1007,16 @@ void mpmg_adj_free(mpmg_ctx *ctx)
 
 namespace {
 
+StatePtrs state_ptrs(const mpmg_ctx *ctx)
+{
+    return StatePtrs{ctx->x, ctx->y, ctx->vx, ctx->vy, ctx->v, ctx->sxx, ctx->sxy, ctx->syy, ctx->Tzz};
+}
+
 int save_state(mpmg_ctx *ctx, double *out)
 {
     const int n = (int)ctx->np;
     if (n == 0) return MPMG_OK;
-    save_state_kernel<<<blocks_for(n, 256), 256, 0, ctx->stream>>>(n, ctx->x, ctx->y, ctx->vx, ctx->vy, ctx->v,
-                                                                    ctx->sxx, ctx->sxy, ctx->syy, ctx->Tzz, out);
+    save_state_kernel<<<blocks_for(n, 256), 256, 0, ctx->stream>>>(n, state_ptrs(ctx), out);
     ctx->launches += 1;
     MPMG_CHECK(cudaGetLastError());
     return MPMG_OK;
@@ -957,12 +1115,14 @@ int mpmg_adj_forward_tape(mpmg_ctx *ctx, int nsteps, int checkpoint_every)
         (rc = dalloc(&t->seg_elem, (size_t)K * n)) != MPMG_OK ||
         (rc = dalloc(&t->seg_active, (size_t)K * n)) != MPMG_OK ||
         (rc = dalloc(&t->seg_perm, (size_t)K * n)) != MPMG_OK ||
-        (rc = dalloc(&t->seg_cs, (size_t)K * (ne + 1))) != MPMG_OK ||
+        (rc = dalloc(&t->seg_start, (size_t)K * ne)) != MPMG_OK ||
+        (rc = dalloc(&t->seg_count, (size_t)K * ne)) != MPMG_OK ||
+        (rc = dalloc(&t->seg_cursor, (size_t)K)) != MPMG_OK ||
         (rc = dalloc(&t->seg_nodes, (size_t)K * kNodeFields * nn)) != MPMG_OK ||
         (rc = dalloc(&t->seg_params, (size_t)K)) != MPMG_OK ||
         (rc = dalloc(&t->adj[0], kStateFields * n)) != MPMG_OK ||
         (rc = dalloc(&t->adj[1], kStateFields * n)) != MPMG_OK || (rc = dalloc(&t->contrib, 16 * n)) != MPMG_OK ||
-        (rc = dalloc(&t->cell_adj, 16 * ne)) != MPMG_OK || (rc = dalloc(&t->node_adj, 5 * nn)) != MPMG_OK ||
+        (rc = dalloc(&t->node_adj, 6 * nn)) != MPMG_OK ||
         (rc = dalloc(&t->theta_part, (size_t)blocks_for(n, kAdjThreads) * kThetaSlots)) != MPMG_OK ||
         (rc = dalloc(&t->theta_acc, kThetaSlots)) != MPMG_OK) {
         mpmg_adj_free(ctx);
@@ -1020,9 +1180,10 @@ int mpmg_adj_backward(mpmg_ctx *ctx, const double *dl_dx, const double *dl_dy, d
     S.dt = ctx->cfg.dt;
     S.mass = ctx->m;
     S.contrib = t->contrib;
-    S.cell_adj = t->cell_adj;
     S.node_adj = t->node_adj;
     S.theta_part = t->theta_part;
+    S.theta_acc = t->theta_acc;
+    S.k = make_adj_const(S.mp, ctx->inv_h);
     S.gfb = t->gfb;
     S.rhs = t->rhs;
     S.lam = t->lam;
@@ -1035,17 +1196,24 @@ int mpmg_adj_backward(mpmg_ctx *ctx, const double *dl_dx, const double *dl_dy, d
         rc = load_state(ctx, t->ck_state + (size_t)c * kStateFields * n, t->ck_active + (size_t)c * n,
                         t->ck_elem + (size_t)c * n, t->ck_params + c);
         if (rc != MPMG_OK) return rc;
+        MPMG_CHECK(cudaMemsetAsync(t->seg_cursor, 0, (size_t)len * sizeof(uint32_t), s));
+        if ((rc = save_state(ctx, t->seg_state)) != MPMG_OK) return rc;
         for (int k = 0; k < len; k++) {
-            if ((rc = save_state(ctx, t->seg_state + (size_t)k * kStateFields * n)) != MPMG_OK) return rc;
             if ((rc = mpmg_fp64_ready(ctx)) != MPMG_OK) return rc;
-            if ((rc = mpmg_launch_step(ctx)) != MPMG_OK) return rc;
-            if ((rc = mpmg_fp64_sort(ctx)) != MPMG_OK) return rc;
-            const int m = (int)(n > ne + 1 ? (n > nn ? n : nn) : (ne + 1 > nn ? ne + 1 : nn));
+            ctx->row.record = true;
+            rc = mpmg_launch_step(ctx);
+            ctx->row.record = false;
+            if (rc != MPMG_OK) return rc;
+            const size_t m = n > ne ? (n > nn ? n : nn) : (ne > nn ? ne : nn);
+            const RowBins &r = ctx->row;
+            const int b = 1 - r.cur;        // the step's rows
             save_step_kernel<<<blocks_for(m, 256), 256, 0, s>>>(
-                (int)n, (int)ne, (int)nn, ctx->in_element, ctx->active, ctx->perm, ctx->cell_start, ctx->node_m,
-                ctx->node_ax, ctx->node_ay, ctx->node_vx, ctx->node_vy, ctx->d_params, t->seg_elem + (size_t)k * n,
-                t->seg_active + (size_t)k * n, t->seg_perm + (size_t)k * n, t->seg_cs + (size_t)k * (ne + 1),
-                t->seg_nodes + (size_t)k * kNodeFields * nn, t->seg_params + k);
+                (int)n, (int)ne, (int)nn, ctx->in_element, ctx->active, RowView{r.count[b], r.rows[b], r.over_list, r.cap},
+                ctx->node_m, ctx->node_ax, ctx->node_ay, ctx->node_vx, ctx->node_vy, ctx->d_params, state_ptrs(ctx),
+                t->seg_elem + (size_t)k * n, t->seg_active + (size_t)k * n, t->seg_perm + (size_t)k * n,
+                t->seg_start + (size_t)k * ne, t->seg_count + (size_t)k * ne, t->seg_cursor + k,
+                t->seg_nodes + (size_t)k * kNodeFields * nn, t->seg_params + k,
+                k + 1 < len ? t->seg_state + (size_t)(k + 1) * kStateFields * n : nullptr);
             ctx->launches += 1;
             if (nonlocal) {
                 MPMG_CHECK(cudaMemcpyAsync(t->seg_gf + (size_t)k * nn, ctx->node_gf, nn * sizeof(double),
@@ -1060,7 +1228,8 @@ int mpmg_adj_backward(mpmg_ctx *ctx, const double *dl_dx, const double *dl_dy, d
             S.elem = t->seg_elem + (size_t)k * n;
             S.active = t->seg_active + (size_t)k * n;
             S.perm = t->seg_perm + (size_t)k * n;
-            S.cell_start = t->seg_cs + (size_t)k * (ne + 1);
+            S.start = t->seg_start + (size_t)k * ne;
+            S.count = t->seg_count + (size_t)k * ne;
             S.nodes = t->seg_nodes + (size_t)k * kNodeFields * nn;
             S.params = t->seg_params + k;
             S.adj_in = t->adj[t->cur];
@@ -1073,17 +1242,21 @@ int mpmg_adj_backward(mpmg_ctx *ctx, const double *dl_dx, const double *dl_dy, d
                 adj_nl_rhs_kernel<<<blocks_for(ne, 128), 128, 0, s>>>(S);
                 ctx->launches += 2;
                 MPMG_CHECK(cudaGetLastError());
-                rc = mpmg_solve_fluidity_system(ctx, t->seg_ek + (size_t)k * 10 * ne, t->rhs, S.nodes, nullptr, S.cell_start,
+                rc = mpmg_solve_fluidity_system(ctx, t->seg_ek + (size_t)k * 10 * ne, t->rhs, S.nodes, S.count, nullptr,
                                                 t->lam, true);
                 if (rc != MPMG_OK) return rc;
             }
             if (n > 0) {
-                adj_g2p_kernel<<<pblocks, kAdjThreads, 0, s>>>(S);
-                adj_cells_kernel<<<blocks_for(ne, 128), 128, 0, s>>>(S);
-                adj_grid_kernel<<<blocks_for(nn, 256), 256, 0, s>>>(S);
-                adj_p2g_kernel<<<pblocks, kAdjThreads, 0, s>>>(S);
-                adj_theta_kernel<<<1, 32, 0, s>>>(t->theta_part, pblocks, t->theta_acc);
-                ctx->launches += 5;
+                switch (S.material) {
+                case MPMG_ISOLIN: adj_g2p_kernel<MPMG_ISOLIN><<<pblocks, kAdjThreads, 0, s>>>(S); break;
+                case MPMG_G_NONLOCAL_MU2:
+                    adj_g2p_kernel<MPMG_G_NONLOCAL_MU2><<<pblocks, kAdjThreads, 0, s>>>(S);
+                    break;
+                default: adj_g2p_kernel<MPMG_G_LOCAL_MU2><<<pblocks, kAdjThreads, 0, s>>>(S); break;
+                }
+                adj_node_kernel<<<blocks_for(4 * nn, 256), 256, 0, s>>>(S);
+                adj_p2g_kernel<<<pblocks + 1, kAdjThreads, 0, s>>>(S);
+                ctx->launches += 3;
             }
             MPMG_CHECK(cudaGetLastError());
             t->cur = 1 - t->cur;

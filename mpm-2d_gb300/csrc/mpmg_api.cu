@@ -122,6 +122,7 @@ int alloc_rows(mpmg_ctx *ctx, const int *emap, size_t n)
     while (r.cap < 64 && filled > 0 && (size_t)r.cap * filled < 2 * inside) r.cap *= 2;
     r.cur = 0;
     r.ready = false;
+    r.record = false;
     r.filled0 = filled;
     int rc = dalloc(&r.n_over, 5);
     r.n_filled = r.n_over + 2;

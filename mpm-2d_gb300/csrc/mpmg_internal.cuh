@@ -125,6 +125,7 @@ struct RowBins {
     uint32_t *over_list;   // n: the ordered lists of elements with more than cap particles
     int cur;
     bool ready;
+    bool record;           // the step's ordered rows are read after it (adjoint)
 };
 
 // Device view of the rows one step works on.  list(e, cnt) is element e's

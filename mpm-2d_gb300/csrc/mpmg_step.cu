@@ -1257,7 +1257,7 @@ int mpmg_launch_step(mpmg_ctx *ctx)
 
     mpmg_phase_begin(ctx, PH_P2G);
     // later phases of these read the ordered rows
-    const bool keep_order = nonlocal || musl || c.material == MPMG_G_LOCAL_MU2_EXT;
+    const bool keep_order = nonlocal || musl || c.material == MPMG_G_LOCAL_MU2_EXT || ctx->row.record;
     // two threads an element in single-warp sets, where that leaves every
     // sub-partition at most one warp
     MPMG_CHECK((ctx->row.filled0 <= (size_t)ctx->sms * 4 * 16 ? launch_p2g<32, 2>(ctx, g, keep_order)
