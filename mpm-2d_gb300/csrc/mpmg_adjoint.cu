@@ -1086,25 +1086,11 @@ int check_adjoint_ctx(const mpmg_ctx *ctx)
     return MPMG_OK;
 }
 
-}  // namespace
-
-extern "C" {
-
-int mpmg_adj_forward_tape(mpmg_ctx *ctx, int nsteps, int checkpoint_every)
+int alloc_tape(mpmg_ctx *ctx, AdjTape *t)
 {
-    if (ctx == nullptr || nsteps < 1 || checkpoint_every < 1) return MPMG_ERR_INVALID;
-    int rc = check_adjoint_ctx(ctx);
-    if (rc != MPMG_OK) return rc;
-    MPMG_CHECK(cudaSetDevice(ctx->dev));
-    mpmg_adj_free(ctx);
-    AdjTape *t = new (std::nothrow) AdjTape();
-    if (t == nullptr) return MPMG_ERR_NOMEM;
-    ctx->adj = t;
     const size_t n = ctx->np, ne = ctx->ne, nn = ctx->nn;
-    const int K = checkpoint_every < nsteps ? checkpoint_every : nsteps;
-    t->K = K;
-    t->nsteps = nsteps;
-    t->nck = (nsteps + K - 1) / K;
+    const int K = t->K;
+    int rc;
     const size_t nck = (size_t)t->nck;
     if ((rc = dalloc(&t->ck_state, nck * kStateFields * n)) != MPMG_OK ||
         (rc = dalloc(&t->ck_active, nck * n)) != MPMG_OK || (rc = dalloc(&t->ck_elem, nck * n)) != MPMG_OK ||
@@ -1125,16 +1111,47 @@ int mpmg_adj_forward_tape(mpmg_ctx *ctx, int nsteps, int checkpoint_every)
         (rc = dalloc(&t->node_adj, 6 * nn)) != MPMG_OK ||
         (rc = dalloc(&t->theta_part, (size_t)blocks_for(n, kAdjThreads) * kThetaSlots)) != MPMG_OK ||
         (rc = dalloc(&t->theta_acc, kThetaSlots)) != MPMG_OK) {
-        mpmg_adj_free(ctx);
         return rc;
     }
     if (ctx->cfg.material == MPMG_G_NONLOCAL_MU2 &&
         ((rc = dalloc(&t->seg_gf, (size_t)K * nn)) != MPMG_OK ||
          (rc = dalloc(&t->seg_ek, (size_t)K * 10 * ne)) != MPMG_OK || (rc = dalloc(&t->gfb, n)) != MPMG_OK ||
          (rc = dalloc(&t->rhs, 4 * ne)) != MPMG_OK || (rc = dalloc(&t->lam, nn)) != MPMG_OK)) {
-        mpmg_adj_free(ctx);
         return rc;
     }
+    return MPMG_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+int mpmg_adj_forward_tape(mpmg_ctx *ctx, int nsteps, int checkpoint_every)
+{
+    if (ctx == nullptr || nsteps < 1 || checkpoint_every < 1) return MPMG_ERR_INVALID;
+    int rc = check_adjoint_ctx(ctx);
+    if (rc != MPMG_OK) return rc;
+    MPMG_CHECK(cudaSetDevice(ctx->dev));
+    const size_t n = ctx->np;
+    const int K = checkpoint_every < nsteps ? checkpoint_every : nsteps, checkpoints = (nsteps + K - 1) / K;
+    // the last run's tape where its buffers have this one's sizes (27
+    // allocations and as many frees took as long as 20 steps of 65k particles)
+    AdjTape *t = ctx->adj;
+    if (t == nullptr || t->K != K || t->nck != checkpoints) {
+        mpmg_adj_free(ctx);
+        t = new (std::nothrow) AdjTape();
+        if (t == nullptr) return MPMG_ERR_NOMEM;
+        ctx->adj = t;
+        t->K = K;
+        t->nck = checkpoints;
+        if ((rc = alloc_tape(ctx, t)) != MPMG_OK) {
+            mpmg_adj_free(ctx);
+            return rc;
+        }
+    }
+    t->nsteps = nsteps;
+    t->cur = 0;
+    for (double &v : t->grad) v = 0;
     // The forward run: checkpoint, then K ordinary steps (CUDA graphs).
     for (int c = 0; c < t->nck; c++) {
         rc = snapshot(ctx, t->ck_state + (size_t)c * kStateFields * n, t->ck_active + (size_t)c * n,
@@ -1301,11 +1318,8 @@ int mpmg_adj_state(mpmg_ctx *ctx, const char *name, double *host_out)
     for (int f = 0; f < kStateFields; f++) {
         if (strcmp(name, names[f]) == 0) {
             MPMG_CHECK(cudaSetDevice(ctx->dev));
-            MPMG_CHECK(cudaStreamSynchronize(ctx->stream));
-            if (ctx->np)
-                MPMG_CHECK(cudaMemcpy(host_out, ctx->adj->adj[ctx->adj->cur] + (size_t)f * ctx->np,
-                                      ctx->np * sizeof(double), cudaMemcpyDeviceToHost));
-            return MPMG_OK;
+            return mpmg_copy_out(ctx, host_out, ctx->adj->adj[ctx->adj->cur] + (size_t)f * ctx->np,
+                                 ctx->np * sizeof(double));
         }
     }
     return MPMG_ERR_UNKNOWN_FIELD;

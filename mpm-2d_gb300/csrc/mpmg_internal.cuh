@@ -74,6 +74,7 @@ struct MixedState {
     int g2p_tile;          // particles a G2P tile (256 or 128)
     int p2g_variant;       // batched P2G tile (kP2GElems / kP2GStage index)
     double *export_buf;    // one FP64 particle field in caller order, for read-back
+    uint32_t *inverse;     // stored position of each of the caller's particles, for read-back
     float4 *nl_T, *nl_F;   // g_nonlocal_mu2: trial stress and bulk fluidity per stored particle
 };
 
@@ -167,6 +168,8 @@ struct mpmg_ctx {
     RowBins row;
     double *elem_coef;
     uint32_t *sort_keys;   // input of mpmg_fp64_sort
+    unsigned char *out_stage;   // pinned, 2 MB: mpmg_copy_out
+    cudaEvent_t out_event[2];
     int sms;
 
     // Cell sort.
@@ -319,7 +322,10 @@ int mpmg_mixed_step(mpmg_ctx *ctx);
 // MPMG_ERR_UNKNOWN_FIELD for names the mixed state does not hold.
 int mpmg_mixed_get(mpmg_ctx *ctx, const char *name, double *out);
 int mpmg_mixed_set(mpmg_ctx *ctx, const char *name, const double *in);
-int mpmg_mixed_get_many(mpmg_ctx *ctx, int count, const char *const *names, double *const *out, bool *done);
+int mpmg_mixed_get_many(mpmg_ctx *ctx, int count, const char *const *names, double *const *out, double *const *dev,
+                        bool *done);
+double *mpmg_device_view(const void *p, size_t bytes);
+int mpmg_copy_out(mpmg_ctx *ctx, void *dst, const void *src, size_t bytes);
 int mpmg_mixed_get_map(mpmg_ctx *ctx, int *in_element, int *active);
 void mpmg_adj_free(mpmg_ctx *ctx);
 

@@ -1420,6 +1420,7 @@ int mpmg_mixed_init(mpmg_ctx *ctx, const double *m, const double *v, const doubl
     if ((rc = dalloc(&s->node4, ctx->nn)) != MPMG_OK) return rc;
     if ((rc = dalloc(&s->node_mass, ctx->nn)) != MPMG_OK) return rc;
     if ((rc = dalloc(&s->export_buf, n)) != MPMG_OK) return rc;
+    if ((rc = dalloc(&s->inverse, n)) != MPMG_OK) return rc;
     if (mat == MPMG_G_NONLOCAL_MU2) {
         // the fluidity solve: FP64 nodal mass (unknown mask), nodal fluidity,
         // element blocks and Krylov vectors, and the per-particle G2P values
@@ -1588,6 +1589,7 @@ void mpmg_mixed_free(mpmg_ctx *ctx)
     cudaFree(s->node4);
     cudaFree(s->node_mass);
     cudaFree(s->export_buf);
+    cudaFree(s->inverse);
     cudaFree(s->nl_T);
     cudaFree(s->nl_F);
     delete s;
@@ -1794,36 +1796,90 @@ int mpmg_mixed_get_map(mpmg_ctx *ctx, int *in_element, int *active)
 
 namespace {
 
-// One particle field of the stored records in the caller's particle order,
-// widened to FP64 (the particle index travels in D.z).  Positions are the
-// element's corner plus the local coordinate, times h, as the host
-// read-back computes them; a particle outside the grid holds its position.
-__global__ void mx_export_kernel(int n, const float4 *__restrict__ rec, int comp, const float4 *__restrict__ drec,
-                                 const int *__restrict__ cell, int xy, const __grid_constant__ MemberM m0,
-                                 BatchView bv, int ne, double *__restrict__ out)
+// Particle fields of the stored records in the caller's particle order,
+// widened to FP64.  Positions are the element's corner plus the local
+// coordinate, times h, as the host read-back computes them; a particle outside
+// the grid holds its position.  A thread takes one of the caller's particles,
+// reads its 64 bytes of records through the inverse permutation (the particle
+// index travels in D.z) and writes its value of every field, so that the stores
+// are coalesced and may go to pinned host memory: 13 fields of 1 048 576
+// particles 633 us, where an export and a copy for each took 987 us.
+constexpr int kExportFields = 16;
+
+struct ExportFields {
+    int count;
+    int slot[kExportFields];      // 4 record + component
+    int xy[kExportFields];        // 1: x, 2: y
+    double *out[kExportFields];
+};
+
+__global__ void __launch_bounds__(256) mx_inverse_kernel(int n, const float4 *__restrict__ D,
+                                                         uint32_t *__restrict__ inverse)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int pid = __float_as_int(drec[i].z);
-    const float4 r = rec[i];
-    const float v = comp == 0 ? r.x : comp == 1 ? r.y : comp == 2 ? r.z : r.w;
-    double o = (double)v;
-    if (xy != 0) {
-        const int c = cell[i];
-        if (c < ne) {
-            const MemberM &M = bv.count > 1 ? bv.m[find_member(bv.elem_off, bv.count, c)] : m0;
-            const int lc = c - M.e0;
-            const int cj = (int)mpmg_div((uint32_t)lc, M.g.div_Ex), ci = lc - cj * M.g.Ex;
-            o = ((double)(xy == 1 ? ci : cj) + (double)v) * M.g.h;
-        }
+    if (i < n) inverse[__float_as_int(D[i].z)] = (uint32_t)i;
+}
+
+__global__ void __launch_bounds__(256) mx_export_kernel(
+    int n, const float4 *__restrict__ A, const float4 *__restrict__ B, const float4 *__restrict__ C,
+    const float4 *__restrict__ D, const uint32_t *__restrict__ inverse, const int *__restrict__ cell,
+    const __grid_constant__ ExportFields F, const __grid_constant__ MemberM m0, BatchView bv, int ne)
+{
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= n) return;
+    const uint32_t i = inverse[p];
+    const float4 a = A[i], b = B[i], c4 = C[i], d = D[i];
+    const int c = cell[i];
+    double ox = 0, oy = 0, h = 1;
+    if (c < ne) {
+        const MemberM &M = bv.count > 1 ? bv.m[find_member(bv.elem_off, bv.count, c)] : m0;
+        const int lc = c - M.e0;
+        const int cj = (int)mpmg_div((uint32_t)lc, M.g.div_Ex), ci = lc - cj * M.g.Ex;
+        ox = ci;
+        oy = cj;
+        h = M.g.h;
     }
-    out[pid] = o;
+    for (int f = 0; f < F.count; f++) {
+        const float4 r = F.slot[f] < 4 ? a : F.slot[f] < 8 ? b : F.slot[f] < 12 ? c4 : d;
+        const int comp = F.slot[f] & 3;
+        double o = (double)(comp == 0 ? r.x : comp == 1 ? r.y : comp == 2 ? r.z : r.w);
+        if (F.xy[f] != 0 && c < ne) o = ((F.xy[f] == 1 ? ox : oy) + o) * h;
+        F.out[f][p] = o;
+    }
+}
+
+// Adds the particle field `name` to the list; false where the records do not hold it.
+bool add_export(mpmg_ctx *ctx, const char *name, double *out, ExportFields &F)
+{
+    int rec = 0, comp = 0, xy = 0;
+    if (strcmp(name, "x") == 0) xy = 1;
+    else if (strcmp(name, "y") == 0) { xy = 2; comp = 1; }
+    else if (!field_slot(ctx->cfg.material, name, &rec, &comp)) return false;
+    F.slot[F.count] = 4 * rec + comp;
+    F.xy[F.count] = xy;
+    F.out[F.count++] = out;
+    return true;
+}
+
+int launch_export(mpmg_ctx *ctx, ExportFields &F)
+{
+    MixedState *s = ctx->mixed;
+    const int b = s->cur, n = (int)ctx->np;
+    if (n == 0 || F.count == 0) return MPMG_OK;
+    const MemberM m0 = make_member(ctx->batch ? ctx->batch->cfg[0] : ctx->cfg, 0, 0);
+    mx_inverse_kernel<<<blocks_for(n, 256), 256, 0, ctx->stream>>>(n, s->D[b], s->inverse);
+    mx_export_kernel<<<blocks_for(n, 256), 256, 0, ctx->stream>>>(n, s->A[b], s->B[b], s->C[b], s->D[b], s->inverse,
+                                                                   cell_array(ctx, b), F, m0, batch_view(ctx),
+                                                                   (int)ctx->ne);
+    ctx->launches += 2;
+    F.count = 0;
+    MPMG_CHECK(cudaGetLastError());
+    return MPMG_OK;
 }
 
 int frame_get(mpmg_ctx *ctx, const char *name, double *out)
 {
     MixedState *s = ctx->mixed;
-    const int b = s->cur;
     const size_t n = ctx->np;
     if (strncmp(name, "node_", 5) == 0) {
         if (strcmp(name, "node_m") == 0) {
@@ -1843,20 +1899,12 @@ int frame_get(mpmg_ctx *ctx, const char *name, double *out)
         for (size_t k = 0; k < ctx->nn; k++) out[k] = get_comp(h[k], comp);
         return MPMG_OK;
     }
-    int rec = 0, comp = 0, xy = 0;
-    if (strcmp(name, "x") == 0) xy = 1;
-    else if (strcmp(name, "y") == 0) { xy = 2; comp = 1; }
-    else if (!field_slot(ctx->cfg.material, name, &rec, &comp)) return MPMG_ERR_UNKNOWN_FIELD;
+    ExportFields F = {};
+    if (!add_export(ctx, name, s->export_buf, F)) return MPMG_ERR_UNKNOWN_FIELD;
     if (n == 0) return MPMG_OK;
-    const MemberM m0 = make_member(ctx->batch ? ctx->batch->cfg[0] : ctx->cfg, 0, 0);
-    mx_export_kernel<<<blocks_for(n, 256), 256, 0, ctx->stream>>>((int)n, record(s, b, rec), comp, s->D[b],
-                                                                   cell_array(ctx, b), xy, m0, batch_view(ctx),
-                                                                   (int)ctx->ne, s->export_buf);
-    ctx->launches += 1;
-    MPMG_CHECK(cudaGetLastError());
-    MPMG_CHECK(cudaMemcpyAsync(out, s->export_buf, n * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-    MPMG_CHECK(cudaStreamSynchronize(ctx->stream));
-    return MPMG_OK;
+    const int rc = launch_export(ctx, F);
+    if (rc != MPMG_OK) return rc;
+    return mpmg_copy_out(ctx, out, s->export_buf, n * sizeof(double));
 }
 
 }  // namespace
@@ -1867,16 +1915,26 @@ int mpmg_mixed_get(mpmg_ctx *ctx, const char *name, double *out)
 }
 
 // Several fields; done[k] is set for every field read here (the others are
-// not held by the mixed state).
-int mpmg_mixed_get_many(mpmg_ctx *ctx, int count, const char *const *names, double *const *out, bool *done)
+// not held by the mixed state).  The particle fields whose destination the
+// device can write (dev[k]) go in one export.
+int mpmg_mixed_get_many(mpmg_ctx *ctx, int count, const char *const *names, double *const *out, double *const *dev,
+                        bool *done)
 {
-    for (int k = 0; k < count; k++) {
-        done[k] = false;
-        const int rc = frame_get(ctx, names[k], out[k]);
-        if (rc == MPMG_OK) done[k] = true;
-        else if (rc != MPMG_ERR_UNKNOWN_FIELD) return rc;
+    ExportFields F = {};
+    int rc = MPMG_OK;
+    for (int k = 0; k < count && rc == MPMG_OK; k++) {
+        done[k] = dev[k] != nullptr && add_export(ctx, names[k], dev[k], F);
+        if (F.count == kExportFields) rc = launch_export(ctx, F);
     }
-    return MPMG_OK;
+    if (rc == MPMG_OK) rc = launch_export(ctx, F);
+    MPMG_CHECK(cudaStreamSynchronize(ctx->stream));
+    for (int k = 0; k < count && rc == MPMG_OK; k++) {
+        if (done[k]) continue;
+        rc = frame_get(ctx, names[k], out[k]);
+        done[k] = rc == MPMG_OK;
+        if (rc == MPMG_ERR_UNKNOWN_FIELD) rc = MPMG_OK;
+    }
+    return rc;
 }
 
 int mpmg_mixed_set(mpmg_ctx *ctx, const char *name, const double *in)
