@@ -47,12 +47,11 @@ enum Phase {
 };
 
 struct SortScratch {
+    uint32_t *keys;        // the clamped keys
     uint32_t *keys_alt;
     uint32_t *vals_alt;
     uint32_t *tile_hist;   // [1024 digits][num tiles], digit-major
     uint32_t *digit_total; // [1024]
-    int num_tiles;
-    int capacity;          // particles
 };
 
 // Mixed-precision particle storage: four float4 records per particle, kept
@@ -278,11 +277,8 @@ int mpmg_cuda_status(cudaError_t e, const char *what);
 
 // Kernel launch helpers implemented per translation unit.
 // Scratch words (uint32) a sort of n keys needs, and its tile count.
-size_t mpmg_sort_scratch_words(size_t n, int key_bits, int *num_tiles_out);
-// Sort with caller-provided scratch; returns the number of launches issued.
-int mpmg_sort_run(const uint32_t *keys, const uint32_t *vals, int n, int ne, int key_bits,
-                  const SortScratch &sc, uint32_t *sorted_keys, uint32_t *perm, int *cell_start,
-                  cudaStream_t s);
+cudaError_t mpmg_sort_run(const uint32_t *keys, int n, int ne, int key_bits, int sms, const SortScratch &sc,
+                          uint32_t *sorted_keys, uint32_t *perm, int *cell_start, cudaStream_t s);
 int mpmg_launch_step(mpmg_ctx *ctx);             // one full FP64 step
 // FP64 form: the element rows of the current positions, where they are not
 // ready (a no-op otherwise); the steps' launches assume them.

@@ -12,7 +12,8 @@
 //
 // Keys need ceil(log2(num_elements + 1)) bits (18 for 512^2 elements); they
 // are sorted in ceil(bits / 10) passes of at most 10 bits.  Each pass:
-//   upsweep    per-tile digit histogram (tile = 2048 keys, shared atomics)
+//   upsweep    per-tile digit histogram (shared atomics); the first pass's also
+//              clamps the caller's keys into the scratch
 //   scan       one warp per digit: exclusive prefix of that digit's counts
 //              over the tiles, and the digit's total
 //   downsweep  every warp ranks its 256 contiguous keys stably (match_any +
@@ -20,19 +21,28 @@
 //              counts into offsets (digit prefix over the whole input + this
 //              tile's prefix + earlier warps), and keys and values scatter
 // Integer-only and deterministic for any launch order.
+//
+// Bound by latency: 125k keys are seven short kernels.  So each is launched
+// before its predecessor has finished (programmatic dependent launch), a tile
+// is 1024 keys where 2048 would leave SMs without one, and the offsets come
+// from 32-way searches of block ranges: 125k keys of 262 144 elements 49 -> 27
+// us, of 40 000 elements 19.4 (35.0 without the early launches).
 #include "mpmg_internal.cuh"
 
 namespace {
 
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
-constexpr int kRounds = 8;                       // keys per lane
-constexpr int kTile = kThreads * kRounds;        // 2048 keys per block
+constexpr int kMaxRounds = 8;                    // keys per lane: 4 or 8, 1024 or 2048 a block
 constexpr int kMaxBits = 10;
 constexpr int kMaxRadix = 1 << kMaxBits;
 
-__global__ void __launch_bounds__(kThreads) upsweep_kernel(const uint32_t *__restrict__ keys, int n,
+// FIRST: the keys are the caller's; a key outside [0, ne] becomes ne, and the
+// clamped keys go to `clamped` for the rest of the sort.
+template <int ROUNDS, bool FIRST>
+__global__ void __launch_bounds__(kThreads) upsweep_kernel(const uint32_t *__restrict__ keys, int n, uint32_t ne,
                                                            int shift, int bits, int num_tiles,
+                                                           uint32_t *__restrict__ clamped,
                                                            uint32_t *__restrict__ tile_hist)
 {
     __shared__ uint32_t hist[kMaxRadix];
@@ -40,11 +50,19 @@ __global__ void __launch_bounds__(kThreads) upsweep_kernel(const uint32_t *__res
     for (int d = threadIdx.x; d < radix; d += kThreads) hist[d] = 0;
     __syncthreads();
     const uint32_t mask = (uint32_t)radix - 1u;
-    const int base = blockIdx.x * kTile;
+    const int base = blockIdx.x * (kThreads * ROUNDS);
+    mpmg_pdl_wait();
+    mpmg_pdl_trigger();
 #pragma unroll
-    for (int k = 0; k < kRounds; k++) {
+    for (int k = 0; k < ROUNDS; k++) {
         int idx = base + k * kThreads + threadIdx.x;
-        if (idx < n) atomicAdd(&hist[(keys[idx] >> shift) & mask], 1u);
+        if (idx >= n) continue;
+        uint32_t key = keys[idx];
+        if (FIRST) {
+            if (key > ne) key = ne;             // a negative key is above every element
+            clamped[idx] = key;
+        }
+        atomicAdd(&hist[(key >> shift) & mask], 1u);
     }
     __syncthreads();
     for (int d = threadIdx.x; d < radix; d += kThreads)
@@ -62,6 +80,8 @@ __global__ void __launch_bounds__(kThreads) scan_tiles_kernel(uint32_t *__restri
     if (d >= radix) return;
     uint32_t *row = tile_hist + (size_t)d * num_tiles;
     uint32_t run = 0;
+    mpmg_pdl_wait();
+    mpmg_pdl_trigger();
     for (int base = 0; base < num_tiles; base += 32) {
         int t = base + lane;
         uint32_t v = (t < num_tiles) ? row[t] : 0u;
@@ -77,6 +97,8 @@ __global__ void __launch_bounds__(kThreads) scan_tiles_kernel(uint32_t *__restri
     if (lane == 0) digit_total[d] = run;
 }
 
+// FIRST: the values are the index sequence.
+template <int ROUNDS, bool FIRST>
 __global__ void __launch_bounds__(kThreads) downsweep_kernel(
     const uint32_t *__restrict__ keys_in, const uint32_t *__restrict__ vals_in, int n, int shift,
     int bits, int num_tiles, const uint32_t *__restrict__ tile_prefix,
@@ -93,6 +115,8 @@ __global__ void __launch_bounds__(kThreads) downsweep_kernel(
     const uint32_t lt_mask = (1u << lane) - 1u;
 
     for (int k = threadIdx.x; k < kWarps * kMaxRadix; k += kThreads) (&warp_hist[0][0])[k] = 0;
+    mpmg_pdl_wait();
+    mpmg_pdl_trigger();
 
     // Exclusive prefix of the digit totals (the digit's start in the output).
     {
@@ -125,15 +149,18 @@ __global__ void __launch_bounds__(kThreads) downsweep_kernel(
     }
     __syncthreads();
 
-    // Each warp ranks its contiguous 256 keys in order (stable).
-    const int wbase_idx = blockIdx.x * kTile + warp * (kRounds * 32);
-    uint32_t key[kRounds], val[kRounds], rank[kRounds];
+    // Each warp ranks its contiguous keys in order (stable).
+    const int wbase_idx = blockIdx.x * (kThreads * ROUNDS) + warp * (ROUNDS * 32);
+    uint32_t key[ROUNDS], val[ROUNDS], rank[ROUNDS];
 #pragma unroll
-    for (int r = 0; r < kRounds; r++) {
+    for (int r = 0; r < ROUNDS; r++) {
         const int idx = wbase_idx + r * 32 + lane;
-        const bool valid = idx < n;
-        key[r] = valid ? keys_in[idx] : 0xffffffffu;
-        val[r] = valid ? vals_in[idx] : 0u;
+        key[r] = idx < n ? keys_in[idx] : 0xffffffffu;
+        val[r] = FIRST ? (uint32_t)idx : idx < n ? vals_in[idx] : 0u;
+    }
+#pragma unroll
+    for (int r = 0; r < ROUNDS; r++) {
+        const bool valid = wbase_idx + r * 32 + lane < n;
         const uint32_t d = (key[r] >> shift) & mask;
         const uint32_t vmask = __ballot_sync(0xffffffffu, valid);
         const uint32_t peers = __match_any_sync(0xffffffffu, valid ? d : 0xffffffffu) & vmask;
@@ -157,7 +184,7 @@ __global__ void __launch_bounds__(kThreads) downsweep_kernel(
     }
     __syncthreads();
 #pragma unroll
-    for (int r = 0; r < kRounds; r++) {
+    for (int r = 0; r < ROUNDS; r++) {
         const int idx = wbase_idx + r * 32 + lane;
         if (idx < n) {
             const uint32_t d = (key[r] >> shift) & mask;
@@ -168,63 +195,99 @@ __global__ void __launch_bounds__(kThreads) downsweep_kernel(
     }
 }
 
-// cell_start[e] = first sorted position whose key is >= e, for e in [0, ne].
-__global__ void cell_start_kernel(const uint32_t *__restrict__ sorted_keys, int n, int ne,
-                                  int *__restrict__ cell_start)
+// The first sorted position whose key is >= e, by a whole warp: 31 probes a
+// round, so that a million keys take four dependent loads.
+__device__ __forceinline__ int lower_bound_warp(const uint32_t *__restrict__ keys, int n, uint32_t e)
 {
-    int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e > ne) return;
-    int lo = 0, hi = n;
+    const int lane = threadIdx.x & 31;
+    int lo = 0, hi = n;                      // the answer is in [lo, hi]
     while (lo < hi) {
-        int mid = (lo + hi) >> 1;
-        if (sorted_keys[mid] < (uint32_t)e) lo = mid + 1;
-        else hi = mid;
+        const int step = (hi - lo + 31) / 32;
+        const int at = lo + (lane + 1) * step - 1;
+        const uint32_t below = __ballot_sync(0xffffffffu, at < hi && keys[at] < e);
+        const int count = __popc(below);     // the probes are ordered: lanes 0 .. count - 1
+        const int next = lo + (count + 1) * step - 1;
+        lo += count * step;
+        if (next < hi) hi = next;
     }
-    cell_start[e] = lo;
+    return lo;
+}
+
+// cell_start[e] = first sorted position whose key is >= e, for e in [0, ne].  A
+// block of kStartElems elements finds its range of the sorted keys, and each
+// thread the first entries there of the elements between its key and the one
+// before.
+constexpr int kStartElems = 256;            // 1024: 125k keys of 40 000 elements 23.2 us instead of 19.4
+
+__global__ void __launch_bounds__(kThreads) cell_start_kernel(const uint32_t *__restrict__ sorted_keys, int n, int ne,
+                                                              int *__restrict__ cell_start)
+{
+    __shared__ int range[2];
+    __shared__ int first[kStartElems];
+    const long long e0 = (long long)blockIdx.x * kStartElems;
+    const int w = threadIdx.x >> 5;
+    mpmg_pdl_wait();
+    if (w < 2) {
+        const int at = lower_bound_warp(sorted_keys, n, (uint32_t)(e0 + (w == 0 ? 0 : kStartElems)));
+        if ((threadIdx.x & 31) == 0) range[w] = at;
+    }
+    __syncthreads();
+    const int lo = range[0], hi = range[1];
+    for (int t = threadIdx.x; t < kStartElems; t += kThreads) first[t] = hi;
+    __syncthreads();
+    for (int i = lo + threadIdx.x; i < hi; i += kThreads) {
+        const int k = (int)((long long)sorted_keys[i] - e0);
+        const int before = i > lo ? (int)((long long)sorted_keys[i - 1] - e0) : -1;
+        for (int e = before + 1; e <= k; e++) first[e] = i;
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < kStartElems; t += kThreads)
+        if (e0 + t <= ne) cell_start[e0 + t] = first[t];
 }
 
 }  // namespace
 
-size_t mpmg_sort_scratch_words(size_t n, int key_bits, int *num_tiles_out)
+// Sorts the caller's n keys (clamped to [0, ne], ne < 2^key_bits) with their
+// indices into sorted_keys and perm using the given scratch, then fills
+// cell_start[0..ne].  A tile is 1024 keys up to 1024 a multiprocessor (a tile
+// of 2048 leaves half of them idle: 125k keys 19.4 us, 22.3 with it) and 2048
+// beyond (300k keys 29.4 us, 31.3 with tiles of 1024, and the scratch holds 512
+// tiles).
+cudaError_t mpmg_sort_run(const uint32_t *keys, int n, int ne, int key_bits, int sms, const SortScratch &sc,
+                          uint32_t *sorted_keys, uint32_t *perm, int *cell_start, cudaStream_t s)
 {
-    int tiles = (int)((n + kTile - 1) / kTile);
-    if (tiles < 1) tiles = 1;
-    if (num_tiles_out) *num_tiles_out = tiles;
-    (void)key_bits;
-    // keys_alt + vals_alt + tile histogram + digit totals
-    return 2 * (n > 0 ? n : 1) + (size_t)kMaxRadix * tiles + kMaxRadix;
-}
-
-// Sorts keys/vals (n entries, keys < 2^key_bits) into sorted_keys/perm using
-// the given scratch, then fills cell_start[0..ne].  Returns launches issued.
-int mpmg_sort_run(const uint32_t *keys, const uint32_t *vals, int n, int ne, int key_bits,
-                  const SortScratch &sc, uint32_t *sorted_keys, uint32_t *perm, int *cell_start,
-                  cudaStream_t s)
-{
-    int launches = 0;
+    const dim3 block(kThreads);
     if (n > 0) {
+        const bool small = n <= sms * kThreads * 4;
         const int passes = (key_bits + kMaxBits - 1) / kMaxBits;
         const int base_bits = key_bits / passes, extra = key_bits % passes;
-        const int tiles = (n + kTile - 1) / kTile;
-        const uint32_t *src_k = keys, *src_v = vals;
+        const int tile = kThreads * (small ? 4 : kMaxRounds), tiles = (n + tile - 1) / tile;
+        const uint32_t *src_k = sc.keys, *src_v = nullptr;
         int shift = 0;
         for (int p = 0; p < passes; p++) {
             const int bits = base_bits + (p < extra ? 1 : 0);
             const int radix = 1 << bits;
-            const bool to_out = ((passes - 1 - p) % 2) == 0;
+            const bool to_out = ((passes - 1 - p) % 2) == 0, first = p == 0;
             uint32_t *dst_k = to_out ? sorted_keys : sc.keys_alt;
             uint32_t *dst_v = to_out ? perm : sc.vals_alt;
-            upsweep_kernel<<<tiles, kThreads, 0, s>>>(src_k, n, shift, bits, tiles, sc.tile_hist);
-            scan_tiles_kernel<<<(radix + kWarps - 1) / kWarps, kThreads, 0, s>>>(sc.tile_hist, tiles, radix,
-                                                                                sc.digit_total);
-            downsweep_kernel<<<tiles, kThreads, 0, s>>>(src_k, src_v, n, shift, bits, tiles, sc.tile_hist,
-                                                        sc.digit_total, dst_k, dst_v);
-            launches += 3;
+            cudaError_t e = mpmg_launch_pdl(
+                true, first ? (small ? upsweep_kernel<4, true> : upsweep_kernel<8, true>)
+                            : (small ? upsweep_kernel<4, false> : upsweep_kernel<8, false>),
+                dim3(tiles), block, 0, s, first ? keys : src_k, n, (uint32_t)ne, shift, bits, tiles, sc.keys, sc.tile_hist);
+            if (e == cudaSuccess)
+                e = mpmg_launch_pdl(true, scan_tiles_kernel, dim3((radix + kWarps - 1) / kWarps), block, 0, s,
+                                    sc.tile_hist, tiles, radix, sc.digit_total);
+            if (e == cudaSuccess)
+                e = mpmg_launch_pdl(true, first ? (small ? downsweep_kernel<4, true> : downsweep_kernel<8, true>)
+                                                : (small ? downsweep_kernel<4, false> : downsweep_kernel<8, false>),
+                                    dim3(tiles), block, 0, s, src_k, src_v, n, shift, bits, tiles,
+                                    (const uint32_t *)sc.tile_hist, (const uint32_t *)sc.digit_total, dst_k, dst_v);
+            if (e != cudaSuccess) return e;
             src_k = dst_k;
             src_v = dst_v;
             shift += bits;
         }
     }
-    cell_start_kernel<<<(ne + 1 + 255) / 256, 256, 0, s>>>(sorted_keys, n, ne, cell_start);
-    return launches + 1;
+    return mpmg_launch_pdl(true, cell_start_kernel, dim3(ne / kStartElems + 1), block, 0, s,
+                           (const uint32_t *)sorted_keys, n, ne, cell_start);
 }

@@ -11,12 +11,12 @@
 //
 // The scratch array below is held by every GPU that loads this library, for
 // the life of the process.  Its capacity is MPMG_NOALLOC_MAX_PARTICLES keys
-// (2^20, the 1 048 576-particle workload; about 19 MB); larger inputs are
+// (2^20, the 1 048 576-particle workload; about 15 MB); larger inputs are
 // rejected with MPMG_ERR_SCRATCH_LIMIT.  All calls share the one array, so
 // calls that overlap on the GPU (different streams, or different host threads
 // on the same device) race and must be serialised by the caller.  Nothing in
-// the array must start at zero: every call rewrites the keys it sorts, the
-// index sequence and the histograms it reads.
+// the array must start at zero: every call rewrites the keys it sorts and the
+// histograms it reads.
 //
 // Keys outside [0, num_elements] (the reference marks a particle outside the
 // grid with -1) are clamped to num_elements, the outside marker, while they
@@ -34,9 +34,8 @@ constexpr size_t kMaxKeys = MPMG_NOALLOC_MAX_PARTICLES;
 constexpr size_t kMaxRadix = 1024;
 constexpr size_t kTileKeys = 2048;
 constexpr size_t kMaxTiles = (kMaxKeys + kTileKeys - 1) / kTileKeys;
-// clamped keys + keys_alt + vals_alt + index sequence + per-tile histograms
-// + digit totals
-constexpr size_t kWords = 4 * kMaxKeys + kMaxRadix * kMaxTiles + kMaxRadix;
+// clamped keys + keys_alt + vals_alt + per-tile histograms + digit totals
+constexpr size_t kWords = 3 * kMaxKeys + kMaxRadix * kMaxTiles + kMaxRadix;
 
 // In host code this name is only a host-side stand-in for the array, not a
 // device address: the host passes the address cudaGetSymbolAddress returns.
@@ -45,23 +44,12 @@ static __device__ __align__(256) uint32_t g_sort_scratch[kWords];
 constexpr int kMaxDevices = 64;
 std::mutex g_setup_mutex;
 uint32_t *g_scratch_addr[kMaxDevices] = {nullptr};
+int g_sms[kMaxDevices] = {0};
 
-// The keys the sort reads: d_keys with every key outside [0, ne] replaced by
-// ne; and the index sequence 0..n-1 the permutation starts from.
-__global__ void clamp_iota_kernel(const int *__restrict__ keys, int n, int ne, uint32_t *__restrict__ keys_in,
-                                  uint32_t *__restrict__ index)
-{
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) {
-        const int k = keys[i];
-        keys_in[i] = (k < 0 || k > ne) ? (uint32_t)ne : (uint32_t)k;
-        index[i] = (uint32_t)i;
-    }
-}
-
-// Device address of the scratch array on the current device, looked up once
+// Device address of the scratch array on the current device and the device's
+// multiprocessors, looked up once
 // per device with that device current.
-int scratch_address(uint32_t **out)
+int scratch_address(uint32_t **out, int *sms)
 {
     int dev = 0;
     MPMG_CHECK(cudaGetDevice(&dev));
@@ -74,9 +62,11 @@ int scratch_address(uint32_t **out)
         void *p = nullptr;
         cudaError_t e = cudaGetSymbolAddress(&p, g_sort_scratch);
         if (e != cudaSuccess) return mpmg_cuda_status(e, "cudaGetSymbolAddress(sort scratch)");
+        MPMG_CHECK(cudaDeviceGetAttribute(&g_sms[dev], cudaDevAttrMultiProcessorCount, dev));
         g_scratch_addr[dev] = (uint32_t *)p;
     }
     *out = g_scratch_addr[dev];
+    *sms = g_sms[dev];
     return MPMG_OK;
 }
 
@@ -99,23 +89,18 @@ extern "C" int mpmg_sort_cells_noalloc(const int *d_keys, int n, int num_element
         return MPMG_ERR_INVALID;
     }
     uint32_t *base = nullptr;
-    int rc = scratch_address(&base);
+    int sms = 0;
+    int rc = scratch_address(&base, &sms);
     if (rc != MPMG_OK) return rc;
     SortScratch sc;
-    uint32_t *keys_in = base;
+    sc.keys = base;
     sc.keys_alt = base + kMaxKeys;
     sc.vals_alt = base + 2 * kMaxKeys;
-    uint32_t *index = base + 3 * kMaxKeys;
-    sc.tile_hist = base + 4 * kMaxKeys;
+    sc.tile_hist = base + 3 * kMaxKeys;
     sc.digit_total = sc.tile_hist + kMaxRadix * kMaxTiles;
-    sc.num_tiles = (int)((n + kTileKeys - 1) / kTileKeys);
-    sc.capacity = (int)kMaxKeys;
     int bits = 1;
     while ((1ll << bits) <= (long long)num_elements) bits++;
-    cudaStream_t s = (cudaStream_t)stream;
-    if (n > 0) clamp_iota_kernel<<<(n + 255) / 256, 256, 0, s>>>(d_keys, n, num_elements, keys_in, index);
-    mpmg_sort_run(keys_in, index, n, num_elements, bits, sc, (uint32_t *)d_sorted_keys,
-                  (uint32_t *)d_perm, d_cell_start, s);
-    MPMG_CHECK(cudaGetLastError());
+    MPMG_CHECK(mpmg_sort_run((const uint32_t *)d_keys, n, num_elements, bits, sms, sc, (uint32_t *)d_sorted_keys,
+                             (uint32_t *)d_perm, d_cell_start, (cudaStream_t)stream));
     return MPMG_OK;
 }
