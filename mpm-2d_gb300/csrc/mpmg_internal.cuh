@@ -63,15 +63,18 @@ struct SortScratch {
 struct MixedState {
     float4 *A[2], *B[2], *C[2], *D[2];
     int cur;
-    float *cell_sums;      // batches: 20 FP32 corner sums per element, value-major
-    uint32_t *halo_perm;   // single simulations: 3 x np scratch orders of oversized shared tile elements
+    uint32_t *halo_perm;   // 3 x np scratch orders of oversized shared tile elements
+    uint2 *tile_map[3];    // batches: member and tile (row << 16 | column) of each P2G block, for each tile variant
+    int tiles[3];          // P2G tiles of each variant
+    int max_tiles;
+    int *tile_zero;        // per P2G tile: its nodes are known to be zero
     float4 *node4;         // per node: ax, ay, vx, vy (FP32) for the gathers
     float2 *node_mass;     // per node: mass as float-float (hi, lo)
     int g2p_blocks;        // persistent G2P grid size
     int g2p_per_sm_max;    // G2P blocks of the current tile that fit on one SM
     int sms;
     int g2p_tile;          // particles a G2P tile (256 or 128)
-    int p2g_variant;       // batched P2G tile (kP2GElems / kP2GStage index)
+    int p2g_variant;       // a batch's P2G tile (kP2GElems / kP2GStage index)
     double *export_buf;    // one FP64 particle field in caller order, for read-back
     uint32_t *inverse;     // stored position of each of the caller's particles, for read-back
     float4 *nl_T, *nl_F;   // g_nonlocal_mu2: trial stress and bulk fluidity per stored particle

@@ -322,42 +322,27 @@ __device__ __forceinline__ int find_member(const int *__restrict__ off, int coun
 
 // ---------------------------------------------------------------------------
 
-// P2G of a batch (a single simulation runs mx_p2g_grid_kernel, which sums
-// the same way over element tiles and finishes the nodes itself): a block
-// takes 256 consecutive elements, one thread each, and works
-// through them in passes of whole elements whose particles (a contiguous
-// range of the binned order) fit a 1024-particle shared-memory stage.  Each
-// pass loads the range's slots (coalesced) and copies the particle records
-// they point to into shared memory with asynchronous copies (cp.async; the
-// slots are close to the identity because the storage is kept in element
-// order, so the copies are nearly sequential); then every thread orders its
-// element's stage indices by storage position (insertion sort in shared
-// memory: the deterministic, launch-order-independent order), writes perm
-// and rank, and sums its particles in that order: 4 corners x (m, mvx, mvy,
-// fx, fy) in FP32 (process_usl.c:491-522 per particle, regrouped per
-// element).  An element with more particles than the stage is summed alone
-// from global memory.
-//
 // The stage is padded: with about four particles an element, the threads of
 // a warp read entries about four apart, which in an unpadded array land on
 // the same few banks (16-byte records 64 bytes apart, 4-byte words 16 bytes
 // apart).  One pad record after every 8 records, one pad word after every 32
 // words and two pad halves after every 64 halves spread them over all banks.
 //
-// The batched kernel's tile (elements per block = threads, particles staged
-// per pass) is a template: mpmg_autotune picks one of kP2GVariants at run
-// time.  The fused single-simulation kernel stages 4 entries a thread.
-constexpr int kP2GPer = 4;   // stage entries per thread of the fused kernel
+// A batch's tile (elements a block = threads, particles staged a pass) is a
+// template: mpmg_autotune picks one of kP2GVariants at run time.
+constexpr int kP2GPer = 4;   // staged entries a lane has in flight
 
 __device__ __forceinline__ int pad16b(int j) { return j + (j >> 3); }
 __device__ __forceinline__ int pad4b(int j) { return j + (j >> 5); }
 __device__ __forceinline__ int pad2b(int j) { return j + ((j >> 6) << 1); }
 
-// (elements a block, staged particles) of the batched P2G; variant 0 is the
-// default
+// (elements a block, staged particles) of a batch's tiles; variant 0 is the
+// default and a single simulation's
 constexpr int kP2GVariants = 3;
 constexpr int kP2GElems[kP2GVariants] = {256, 128, 512};
 constexpr int kP2GStage[kP2GVariants] = {1024, 512, 1024};
+constexpr int kTileX[kP2GVariants] = {16, 16, 32};
+constexpr int kTileY[kP2GVariants] = {16, 8, 16};
 
 __device__ __forceinline__ void p2g_accumulate(float (&acc)[4][5], float ih, float grav, float4 a4, float4 b4,
                                                float syy)
@@ -379,116 +364,6 @@ __device__ __forceinline__ void p2g_accumulate(float (&acc)[4][5], float ih, flo
         acc[a][3] = __fadd_rn(acc[a][3], __fmaf_rn(gy[a], s1, __fmul_rn(gx[a], s0)));
         acc[a][4] = __fadd_rn(acc[a][4], __fmaf_rn(gy[a], s2, __fmaf_rn(gx[a], s1, __fmul_rn(s[a], pby))));
     }
-}
-
-template <int kP2GThreads, int kP2GChunk, bool BATCH>
-__global__ void __launch_bounds__(kP2GThreads, 1024 / kP2GThreads) mx_p2g_kernel(
-    const __grid_constant__ MemberM m0, BatchView bv, int ne_total, const int *__restrict__ cell_start,
-    const uint32_t *__restrict__ slots, uint32_t *__restrict__ perm, uint32_t *__restrict__ rank, Buf P,
-    const StepParams *__restrict__ sp, float *__restrict__ cell_sums)
-{
-    constexpr int kP2GPer = kP2GChunk / kP2GThreads;   // stage entries per thread
-    constexpr int kP2GChunk16 = kP2GChunk + kP2GChunk / 8;
-    constexpr int kP2GChunk4 = kP2GChunk + kP2GChunk / 32;
-    constexpr int kP2GChunk2 = kP2GChunk + kP2GChunk / 32;
-    __shared__ float4 sh_a[kP2GChunk16];
-    __shared__ float4 sh_b[kP2GChunk16];
-    __shared__ float sh_syy[kP2GChunk4];
-    __shared__ uint32_t sh_slot[kP2GChunk4];
-    __shared__ uint16_t sh_ord[kP2GChunk2];
-    __shared__ int sh_cs[kP2GThreads + 1];
-    const int e0 = blockIdx.x * kP2GThreads;
-    const int ne_blk = min(kP2GThreads, ne_total - e0);
-    // element offsets come from the scan, two kernels back; the slots from
-    // the scatter, the kernel just before
-    for (int t = threadIdx.x; t <= ne_blk; t += kP2GThreads) sh_cs[t] = cell_start[e0 + t];
-    mpmg_pdl_wait();
-    __syncthreads();
-    const int me = threadIdx.x;
-    const int k0 = me < ne_blk ? sh_cs[me] : 0, k1 = me < ne_blk ? sh_cs[me + 1] : 0;
-    float grav, ih;
-    if (BATCH) {
-        const int k = find_member(bv.elem_off, bv.count, min(e0 + me, ne_total - 1));
-        grav = (float)sp[k].gravity;
-        ih = bv.m[k].g.inv_hf;
-    } else {
-        grav = (float)sp->gravity;
-        ih = m0.g.inv_hf;
-    }
-    int ea = 0;
-    while (ea < ne_blk) {
-        // elements [ea, eb) of this pass: the most whose particles fit the stage
-        const int limit = sh_cs[ea] + kP2GChunk;
-        int lo = ea + 1, hi = ne_blk;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (sh_cs[mid] <= limit) lo = mid;
-            else hi = mid - 1;
-        }
-        const int eb = lo;
-        const int base = sh_cs[ea], end = sh_cs[eb];
-        const bool mine = me >= ea && me < eb && k1 > k0;
-        float acc[4][5];
-#pragma unroll
-        for (int a = 0; a < 4; a++)
-#pragma unroll
-            for (int f = 0; f < 5; f++) acc[a][f] = 0.0f;
-        if (end - base <= kP2GChunk) {
-            uint32_t sl[kP2GPer];
-#pragma unroll
-            for (int u = 0; u < kP2GPer; u++) {
-                const int k = base + (int)threadIdx.x + u * kP2GThreads;
-                sl[u] = k < end ? slots[k] : 0u;
-            }
-#pragma unroll
-            for (int u = 0; u < kP2GPer; u++) {
-                const int j = (int)threadIdx.x + u * kP2GThreads;
-                if (base + j < end) {
-                    sh_slot[pad4b(j)] = sl[u];
-                    mpmg_cp_async16(&sh_a[pad16b(j)], P.A + sl[u]);
-                    mpmg_cp_async16(&sh_b[pad16b(j)], P.B + sl[u]);
-                    mpmg_cp_async4(&sh_syy[pad4b(j)], &P.C[sl[u]].x);
-                }
-            }
-            mpmg_cp_async_wait_all();
-            __syncthreads();
-            if (mine) {
-                const int j0 = k0 - base, j1 = k1 - base;
-                for (int j = j0; j < j1; j++) {
-                    const uint32_t x = sh_slot[pad4b(j)];
-                    int t = j - 1;
-                    while (t >= j0 && sh_slot[pad4b(sh_ord[pad2b(t)])] > x) {
-                        sh_ord[pad2b(t + 1)] = sh_ord[pad2b(t)];
-                        t--;
-                    }
-                    sh_ord[pad2b(t + 1)] = (uint16_t)j;
-                }
-                for (int j = j0; j < j1; j++) {
-                    const int q = sh_ord[pad2b(j)];
-                    const uint32_t i = sh_slot[pad4b(q)];
-                    perm[base + j] = i;
-                    rank[i] = (uint32_t)(base + j);
-                    p2g_accumulate(acc, ih, grav, sh_a[pad16b(q)], sh_b[pad16b(q)], sh_syy[pad4b(q)]);
-                }
-            }
-            __syncthreads();
-        } else if (mine) {
-            // a single element larger than the stage
-            mpmg_order_segment(slots, perm, rank, k0, k1);
-            for (int k = k0; k < k1; k++) {
-                const uint32_t i = perm[k];
-                p2g_accumulate(acc, ih, grav, P.A[i], P.B[i], P.C[i].x);
-            }
-        }
-        if (mine) {
-#pragma unroll
-            for (int a = 0; a < 4; a++)
-#pragma unroll
-                for (int f = 0; f < 5; f++) cell_sums[(size_t)(a * 5 + f) * ne_total + e0 + me] = acc[a][f];
-        }
-        ea = eb;
-    }
-    mpmg_pdl_trigger();
 }
 
 // Double-FP32 ("float-float") helpers: a value is hi + lo with |lo| <= ulp(hi)/2,
@@ -621,61 +496,29 @@ __device__ __forceinline__ void node_finish(const MemberM &M, double t_next, flo
     }
 }
 
-// Grid update of a batch, one thread per node, from the corner sums
-// mx_p2g_kernel left in global memory.
-template <bool F64NODE, bool BATCH>
-__global__ void __launch_bounds__(256) mx_grid_kernel(const __grid_constant__ MemberM m0, BatchView bv, int ne_total,
-                                                      int nn_total, const int *__restrict__ cell_start,
-                                                      const float *__restrict__ cell_sums,
-                                                      const StepParams *__restrict__ sp, float tol,
-                                                      float2 *__restrict__ node_mass, float4 *__restrict__ node4,
-                                                      double *__restrict__ node_mx,
-                                                      double *__restrict__ node_my, double *__restrict__ node_fx,
-                                                      double *__restrict__ node_fy, double *__restrict__ node_m64)
-{
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= nn_total) return;
-    const int k = BATCH ? find_member(bv.node_off, bv.count, n) : 0;
-    const MemberM &M = BATCH ? bv.m[k] : m0;
-    const GeomM &g = M.g;
-    const int ln = n - M.nd0;
-    const int j = (int)mpmg_div((uint32_t)ln, g.div_Nx), i = ln - j * g.Nx;
-    // the four elements in colour order, where they hold particles
-    // (cell_start is from the scan, three kernels back)
-    long long off[4];
-#pragma unroll
-    for (int c = 0; c < 4; c++) {
-        const int ci = ((i & 1) == (c & 1)) ? i : i - 1;
-        const int cj = ((j & 1) == (c >> 1)) ? j : j - 1;
-        off[c] = -1;
-        if (ci < 0 || cj < 0 || ci >= g.Ex || cj >= g.Ey) continue;
-        const int e = M.e0 + cj * g.Ex + ci;
-        const int a = (ci == i) ? ((cj == j) ? 0 : 3) : ((cj == j) ? 1 : 2);
-        if (cell_start[e] != cell_start[e + 1]) off[c] = (long long)(a * 5) * ne_total + e;
-    }
-    const double t_next = sp[k].t + M.dt;
-    mpmg_pdl_wait();        // the corner sums come from the P2G just before
-    mpmg_pdl_trigger();
-    node_finish<F64NODE>(M, t_next, tol, i, j, n, cell_sums, off, (long long)ne_total, node_mass, node4, node_mx,
-                         node_my, node_fx, node_fy, node_m64);
-}
-
-// P2G and grid update in one kernel, for a single simulation.  A block takes
-// a TX x TY tile of elements, one thread each, sums them exactly as
-// mx_p2g_kernel does (the same staging, order and arithmetic), leaves the 20
-// corner sums in shared memory and finishes the (TX - 1) x (TY - 1) nodes
-// whose four elements all lie in the tile exactly as mx_grid_kernel does.
-// Neighbouring tiles share one column or row of elements, which both sum to
-// the same values; perm and rank of an element are written by the one tile
-// where it is not in the first column or row.  An element with more
-// particles than the stage is ordered in global memory: by its owner in
-// perm, by the other tiles in a scratch copy of their own (one per kind of
-// overlap).  The corner sums never reach global memory and the grid update
-// needs no launch.
-template <int TX, int TY>
+// P2G and grid update in one kernel.  A block takes a TX x TY tile of a
+// member's elements, one thread each.  It works through them in passes of
+// whole elements whose particles fit the shared-memory stage: a pass copies
+// the particle records the slots point to with asynchronous copies (cp.async;
+// the storage is kept in element order, so a tile row's are nearly sequential),
+// then every thread orders its element's stage indices by storage position
+// (insertion sort in shared memory: the deterministic, launch-order-independent
+// order), writes perm and rank, and sums its particles in that order: 4 corners
+// x (m, mvx, mvy, fx, fy) in FP32 (process_usl.c:491-522 per particle, regrouped
+// per element).  The 20 corner sums stay in shared memory, from which the block
+// finishes the (TX - 1) x (TY - 1) nodes whose four elements all lie in the
+// tile.  Neighbouring tiles share one column or row of elements, which both sum
+// to the same values; perm and rank of an element are written by the one tile
+// where it is not in the first column or row.  An element with more particles
+// than the stage is ordered in global memory: by its owner in perm, by the
+// other tiles in a scratch copy of their own (one per kind of overlap).
+// A batch's tiles are its members' one after another (tile_map).  One kernel
+// instead of sums in global memory and a node kernel: 32 members with 1.4 M
+// particles 92 -> 58 us.
+template <int TX, int TY, int CHUNK>
 struct FusedTile {
     static constexpr int threads = TX * TY;
-    static constexpr int chunk = 4 * threads;                  // staged particles a pass
+    static constexpr int chunk = CHUNK;                        // staged particles a pass
     static constexpr int c16 = chunk + chunk / 8, c4 = chunk + chunk / 32, c2 = chunk + chunk / 32;
     static constexpr int sum_stride = threads + 1;             // corner-sum row in shared memory
     static constexpr int rows_per_warp = 32 / TX;
@@ -683,19 +526,19 @@ struct FusedTile {
     static_assert(TX * (32 / TX) == 32 && rows_per_warp <= 2 && threads % 32 == 0, "a warp stages one or two whole tile rows");
     static_assert(sizeof(float) * 20 * sum_stride <= smem, "the corner sums overlay the stage");
 };
-constexpr int kFusedTX = 16, kFusedTY = 16;
-using FusedT = FusedTile<kFusedTX, kFusedTY>;
 
-template <bool F64NODE, int TX, int TY>
+template <bool F64NODE, bool BATCH, int TX, int TY, int CHUNK>
 __global__ void __launch_bounds__(TX * TY, 1024 / (TX * TY)) mx_p2g_grid_kernel(
-    const __grid_constant__ MemberM M, int np, int tiles_x, const int *__restrict__ cell_start,
+    const __grid_constant__ MemberM m0, BatchView bv, const uint2 *__restrict__ tile_map,
+    int *__restrict__ tile_zero, int np,
+    const int *__restrict__ cell_start,
     const uint32_t *__restrict__ slots, uint32_t *__restrict__ perm, uint32_t *__restrict__ rank,
     uint32_t *__restrict__ halo_perm, Buf P, const StepParams *__restrict__ sp, float tol,
     float2 *__restrict__ node_mass, float4 *__restrict__ node4, double *__restrict__ node_mx,
     double *__restrict__ node_my, double *__restrict__ node_fx, double *__restrict__ node_fy,
     double *__restrict__ node_m64)
 {
-    using T = FusedTile<TX, TY>;
+    using T = FusedTile<TX, TY, CHUNK>;
     constexpr int NT = T::threads, CH = T::chunk, SS = T::sum_stride;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int sh_off[NT + 1];     // stage offsets of the tile's elements
@@ -709,19 +552,51 @@ __global__ void __launch_bounds__(TX * TY, 1024 / (TX * TY)) mx_p2g_grid_kernel(
     float *sh_sum = reinterpret_cast<float *>(smem);
 
     const int me = threadIdx.x, lane = me & 31, warp = me >> 5;
-    const int tx = blockIdx.x % tiles_x, ty = blockIdx.x / tiles_x;
+    // the block's member and tile: from the table, in one load
+    uint2 at = make_uint2(0, 0);
+    if (BATCH) at = tile_map[blockIdx.x];
+    const int zero = tile_zero[blockIdx.x];      // of this kernel's last launch
+    const int member = BATCH ? (int)at.x : 0;
+    const MemberM &M = BATCH ? bv.m[member] : m0;
+    const int Ex = M.g.Ex, Ey = M.g.Ey, Nx = M.g.Nx, Ny = M.g.Ny;
+    if (!BATCH) {
+        const unsigned tiles_x = (unsigned)(Nx + TX - 2) / (TX - 1);
+        at.y = (blockIdx.x / tiles_x) << 16 | (blockIdx.x % tiles_x);
+    }
+    const int tx = (int)(at.y & 0xffffu), ty = (int)(at.y >> 16);
     const int lx = me % TX, ly = me / TX;
     const int ei = tx * (TX - 1) - 1 + lx, ej = ty * (TY - 1) - 1 + ly;
-    const bool exists = ei >= 0 && ej >= 0 && ei < M.g.Ex && ej < M.g.Ey;
+    const bool exists = ei >= 0 && ej >= 0 && ei < Ex && ej < Ey;
+    sp += member;
     const bool owner = lx > 0 && ly > 0;
     // element offsets come from the scan, two kernels back
     int k0 = 0, k1 = 0;
     if (exists) {
-        const int e = ej * M.g.Ex + ei;
+        const int e = M.e0 + ej * Ex + ei;
         k0 = cell_start[e];
         k1 = cell_start[e + 1];
     }
     const int cnt = k1 - k0;
+    // no particles around (most of the tiles of a heap or an emptying silo):
+    // the nodes are zero, and written only where the tile's last step left
+    // something else (1.85 M nodes of 32 members: 119 -> 113 us a step)
+    if (!__syncthreads_or(cnt)) {
+        mpmg_pdl_wait();
+        if (!zero) {
+            const int i = tx * (TX - 1) + me % (TX - 1), j = ty * (TY - 1) + me / (TX - 1);
+            if (me < (TX - 1) * (TY - 1) && i < Nx && j < Ny) {
+                const int n = M.nd0 + j * Nx + i;
+                node_mass[n] = make_float2(0.0f, 0.0f);
+                node4[n] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if (node_m64 != nullptr) node_m64[n] = 0.0;
+                if (node_mx != nullptr) node_mx[n] = node_my[n] = node_fx[n] = node_fy[n] = 0.0;
+            }
+            if (me == 0) tile_zero[blockIdx.x] = 1;
+        }
+        mpmg_pdl_trigger();
+        return;
+    }
+    if (zero && me == 0) tile_zero[blockIdx.x] = 0;
     // stage offsets: exclusive prefix of the counts in tile order
     int incl = cnt;
 #pragma unroll
@@ -843,9 +718,10 @@ __global__ void __launch_bounds__(TX * TY, 1024 / (TX * TY)) mx_p2g_grid_kernel(
 #pragma unroll
         for (int f = 0; f < 5; f++) sh_sum[(a * 5 + f) * SS + me] = acc[a][f];
     __syncthreads();
+    static_assert((TX - 1) * (TY - 1) <= TX * TY, "a thread a node");
     if (me < (TX - 1) * (TY - 1)) {
         const int i = tx * (TX - 1) + me % (TX - 1), j = ty * (TY - 1) + me / (TX - 1);
-        if (i < M.g.Nx && j < M.g.Ny) {
+        if (i < Nx && j < Ny) {
             // the node's elements lie in the tile (local column and row
             // nx or nx + 1, ny or ny + 1); one outside the grid has no
             // particles, so the count test alone skips it
@@ -859,7 +735,7 @@ __global__ void __launch_bounds__(TX * TY, 1024 / (TX * TY)) mx_p2g_grid_kernel(
                 const int a = dx ? (dy ? 0 : 3) : (dy ? 1 : 2);
                 off[c] = sh_off[le + 1] != sh_off[le] ? (a * 5) * SS + le : -1;
             }
-            node_finish<F64NODE>(M, sp->t + M.dt, tol, i, j, j * M.g.Nx + i, sh_sum, off, SS, node_mass, node4,
+            node_finish<F64NODE>(M, sp->t + M.dt, tol, i, j, M.nd0 + j * Nx + i, sh_sum, off, SS, node_mass, node4,
                                  node_mx, node_my, node_fx, node_fy, node_m64);
         }
     }
@@ -1380,15 +1256,39 @@ size_t g2p_smem_size(int tile)
     return tile == 128 ? g2p_smem_bytes<128>() : g2p_smem_bytes<256>();
 }
 
-using P2GKernel = void (*)(MemberM, BatchView, int, const int *, const uint32_t *, uint32_t *, uint32_t *, Buf,
-                          const StepParams *, float *);
+using P2GKernel = void (*)(MemberM, BatchView, const uint2 *, int *, int, const int *, const uint32_t *, uint32_t *,
+                           uint32_t *, uint32_t *, Buf, const StepParams *, float, float2 *, float4 *, double *,
+                           double *, double *, double *, double *);
 
-// The batched P2G of variant v (kP2GElems[v] elements a block).
-P2GKernel p2g_variant(int v)
+// The P2G and grid update with tile variant v.
+template <int V>
+P2GKernel p2g_variant_t(bool f64, bool batch)
 {
-    if (v == 1) return mx_p2g_kernel<kP2GElems[1], kP2GStage[1], true>;
-    if (v == 2) return mx_p2g_kernel<kP2GElems[2], kP2GStage[2], true>;
-    return mx_p2g_kernel<kP2GElems[0], kP2GStage[0], true>;
+    if (f64)
+        return batch ? mx_p2g_grid_kernel<true, true, kTileX[V], kTileY[V], kP2GStage[V]>
+                     : mx_p2g_grid_kernel<true, false, kTileX[0], kTileY[0], kP2GStage[0]>;
+    return batch ? mx_p2g_grid_kernel<false, true, kTileX[V], kTileY[V], kP2GStage[V]>
+                 : mx_p2g_grid_kernel<false, false, kTileX[0], kTileY[0], kP2GStage[0]>;
+}
+
+P2GKernel p2g_variant(int v, bool f64, bool batch)
+{
+    return v == 1 ? p2g_variant_t<1>(f64, batch) : v == 2 ? p2g_variant_t<2>(f64, batch) : p2g_variant_t<0>(f64, batch);
+}
+
+size_t p2g_smem_size(int v)
+{
+    return v == 1   ? FusedTile<kTileX[1], kTileY[1], kP2GStage[1]>::smem
+           : v == 2 ? FusedTile<kTileX[2], kTileY[2], kP2GStage[2]>::smem
+                    : FusedTile<kTileX[0], kTileY[0], kP2GStage[0]>::smem;
+}
+
+// Tiles of a simulation with variant v.
+int p2g_tiles(const mpmg_config &c, int v, int *tiles_x, int *tiles_y)
+{
+    *tiles_x = (int)((c.Nx + kTileX[v] - 2) / (kTileX[v] - 1));
+    *tiles_y = (int)((c.Ny + kTileY[v] - 2) / (kTileY[v] - 1));
+    return *tiles_x * *tiles_y;
 }
 
 }  // namespace
@@ -1412,11 +1312,7 @@ int mpmg_mixed_init(mpmg_ctx *ctx, const double *m, const double *v, const doubl
         for (float4 **p : f)
             if ((rc = dalloc(p, n)) != MPMG_OK) return rc;
     }
-    if (ctx->batch != nullptr) {
-        if ((rc = dalloc(&s->cell_sums, 20 * ctx->ne)) != MPMG_OK) return rc;
-    } else if ((rc = dalloc(&s->halo_perm, 3 * n)) != MPMG_OK) {
-        return rc;
-    }
+    if ((rc = dalloc(&s->halo_perm, 3 * n)) != MPMG_OK) return rc;
     if ((rc = dalloc(&s->node4, ctx->nn)) != MPMG_OK) return rc;
     if ((rc = dalloc(&s->node_mass, ctx->nn)) != MPMG_OK) return rc;
     if ((rc = dalloc(&s->export_buf, n)) != MPMG_OK) return rc;
@@ -1449,10 +1345,30 @@ int mpmg_mixed_init(mpmg_ctx *ctx, const double *m, const double *v, const doubl
         bt->d_members = dm;
         if ((rc = dalloc(&bt->d_elem_off, count + 1)) != MPMG_OK) return rc;
         if ((rc = dalloc(&bt->d_node_off, count + 1)) != MPMG_OK) return rc;
+        for (int v = 0; v < kP2GVariants; v++) {
+            std::vector<uint2> map;
+            for (int k = 0; k < count; k++) {
+                int nx, ny;
+                p2g_tiles(bt->cfg[k], v, &nx, &ny);
+                for (int j = 0; j < ny; j++)
+                    for (int i = 0; i < nx; i++) map.push_back(make_uint2((unsigned)k, (unsigned)j << 16 | (unsigned)i));
+            }
+            if ((rc = dalloc(&s->tile_map[v], map.size())) != MPMG_OK) return rc;
+            s->tiles[v] = (int)map.size();
+            MPMG_CHECK(cudaMemcpy(s->tile_map[v], map.data(), map.size() * sizeof(uint2), cudaMemcpyHostToDevice));
+        }
         MPMG_CHECK(cudaMemcpy(dm, hm.data(), count * sizeof(MemberM), cudaMemcpyHostToDevice));
         MPMG_CHECK(cudaMemcpy(bt->d_elem_off, eo.data(), (count + 1) * sizeof(int), cudaMemcpyHostToDevice));
         MPMG_CHECK(cudaMemcpy(bt->d_node_off, no.data(), (count + 1) * sizeof(int), cudaMemcpyHostToDevice));
     }
+
+    if (!bt) {
+        int nx, ny;
+        s->tiles[0] = p2g_tiles(ctx->cfg, 0, &nx, &ny);
+    }
+    s->max_tiles = s->tiles[0];
+    for (int t : s->tiles) s->max_tiles = t > s->max_tiles ? t : s->max_tiles;
+    if ((rc = dalloc(&s->tile_zero, s->max_tiles)) != MPMG_OK) return rc;
 
     // The caller's FP64 arrays go to the device as they are, into buffer 1's
     // records and the export buffer (64 + 8 bytes a particle: the nine
@@ -1516,10 +1432,10 @@ int mpmg_mixed_init(mpmg_ctx *ctx, const double *m, const double *v, const doubl
         MPMG_CHECK(cudaFuncSetAttribute(g2p_variant(ctx->cfg.material, bt != nullptr, tile),
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g2p_smem_size(tile)));
     }
-    MPMG_CHECK(cudaFuncSetAttribute(mx_p2g_grid_kernel<false, kFusedTX, kFusedTY>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FusedT::smem));
-    MPMG_CHECK(cudaFuncSetAttribute(mx_p2g_grid_kernel<true, kFusedTX, kFusedTY>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FusedT::smem));
+    const bool f64 = ctx->cfg.precision == MPMG_PRECISION_MIXED_F64NODE;
+    for (int v = 0; v < (bt ? kP2GVariants : 1); v++)
+        MPMG_CHECK(cudaFuncSetAttribute(p2g_variant(v, f64, bt != nullptr), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)p2g_smem_size(v)));
     s->sms = sms > 0 ? sms : 1;
     s->p2g_variant = 0;
     rc = mpmg_mixed_set_tiles(ctx, 0, kG2PTileSizes[0]);
@@ -1543,9 +1459,9 @@ int mpmg_mixed_set_g2p_per_sm(mpmg_ctx *ctx, int per_sm)
     return per_sm;
 }
 
-// The tiles of the mixed step: the batched P2G's variant (elements a block
-// and staged particles, kP2GElems / kP2GStage; single simulations run the
-// fused kernel and ignore it) and the G2P tile (kG2PTileSizes).  The G2P
+// The tiles of the mixed step: a batch's P2G variant (elements a block and
+// staged particles, kP2GElems / kP2GStage; single simulations run variant 0)
+// and the G2P tile (kG2PTileSizes).  The G2P
 // grid goes back to all the blocks of the new tile that fit.  Tiles change
 // which block handles which elements or particles, never a result.
 int mpmg_mixed_set_tiles(mpmg_ctx *ctx, int p2g_variant, int g2p_tile)
@@ -1556,6 +1472,8 @@ int mpmg_mixed_set_tiles(mpmg_ctx *ctx, int p2g_variant, int g2p_tile)
     int per_sm = 0;
     MPMG_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
         &per_sm, g2p_variant(ctx->cfg.material, ctx->batch != nullptr, g2p_tile), g2p_tile, g2p_smem_size(g2p_tile)));
+    // no tile of another variant is known to be zero
+    MPMG_CHECK(cudaMemsetAsync(s->tile_zero, 0, (size_t)s->max_tiles * sizeof(int), ctx->stream));
     s->p2g_variant = p2g_variant;
     s->g2p_tile = g2p_tile;
     s->g2p_per_sm_max = per_sm > 0 ? per_sm : 1;
@@ -1584,8 +1502,9 @@ void mpmg_mixed_free(mpmg_ctx *ctx)
         cudaFree(s->C[b]);
         cudaFree(s->D[b]);
     }
-    cudaFree(s->cell_sums);
     cudaFree(s->halo_perm);
+    for (uint2 *t : s->tile_map) cudaFree(t);
+    cudaFree(s->tile_zero);
     cudaFree(s->node4);
     cudaFree(s->node_mass);
     cudaFree(s->export_buf);
@@ -1625,7 +1544,7 @@ int mpmg_mixed_step(mpmg_ctx *ctx)
     const bool batch = ctx->batch != nullptr;
     const MemberM m0 = make_member(batch ? ctx->batch->cfg[0] : c, 0, 0);
     const BatchView bv = batch_view(ctx);
-    const int n = (int)ctx->np, ne = (int)ctx->ne, nn = (int)ctx->nn;
+    const int n = (int)ctx->np, ne = (int)ctx->ne;
     const int cur = s->cur, nxt = 1 - cur;
 
     mpmg_phase_begin(ctx, PH_SORT);
@@ -1637,36 +1556,14 @@ int mpmg_mixed_step(mpmg_ctx *ctx)
     const bool f64 = c.precision == MPMG_PRECISION_MIXED_F64NODE;
     const bool nonlocal = c.material == MPMG_G_NONLOCAL_MU2;
     double *node_m64 = nonlocal ? ctx->node_m : (double *)nullptr;
-    if (!batch) {
-        // P2G and grid update fused over element tiles
-        mpmg_phase_begin(ctx, PH_P2G);
-        const int tiles_x = (m0.g.Nx + kFusedTX - 2) / (kFusedTX - 1);
-        const int tiles_y = (m0.g.Ny + kFusedTY - 2) / (kFusedTY - 1);
-        MPMG_CHECK(mpmg_launch_pdl(true, f64 ? mx_p2g_grid_kernel<true, kFusedTX, kFusedTY>
-                                             : mx_p2g_grid_kernel<false, kFusedTX, kFusedTY>,
-                                   dim3(tiles_x * tiles_y), dim3(FusedT::threads), FusedT::smem, st, m0, n,
-                                   tiles_x, (const int *)ctx->cell_start, (const uint32_t *)ctx->bin.slots,
-                                   ctx->perm, ctx->bin.rank, s->halo_perm, S, (const StepParams *)ctx->d_params,
-                                   (float)MPMG_TOL, s->node_mass, s->node4, ctx->node_mx, ctx->node_my,
-                                   ctx->node_fx, ctx->node_fy, node_m64));
-        mpmg_phase_end(ctx, PH_P2G);
-    } else {
-        mpmg_phase_begin(ctx, PH_P2G);
-        const int pe = kP2GElems[s->p2g_variant];
-        MPMG_CHECK(mpmg_launch_pdl(true, p2g_variant(s->p2g_variant), dim3(blocks_for(ctx->ne, pe)), dim3(pe), 0,
-                                   st, m0, bv, ne, (const int *)ctx->cell_start,
-                                   (const uint32_t *)ctx->bin.slots, ctx->perm, ctx->bin.rank, S,
-                                   (const StepParams *)ctx->d_params, s->cell_sums));
-        mpmg_phase_end(ctx, PH_P2G);
-
-        mpmg_phase_begin(ctx, PH_GRID);
-        MPMG_CHECK(mpmg_launch_pdl(true, f64 ? mx_grid_kernel<true, true> : mx_grid_kernel<false, true>,
-                                   dim3(blocks_for(ctx->nn, 256)), dim3(256), 0, st, m0, bv, ne, nn,
-                                   (const int *)ctx->cell_start, (const float *)s->cell_sums,
-                                   (const StepParams *)ctx->d_params, (float)MPMG_TOL, s->node_mass, s->node4,
-                                   ctx->node_mx, ctx->node_my, ctx->node_fx, ctx->node_fy, node_m64));
-        mpmg_phase_end(ctx, PH_GRID);
-    }
+    mpmg_phase_begin(ctx, PH_P2G);
+    const int v = batch ? s->p2g_variant : 0;
+    MPMG_CHECK(mpmg_launch_pdl(true, p2g_variant(v, f64, batch), dim3(s->tiles[v]), dim3(kP2GElems[v]), p2g_smem_size(v),
+                               st, m0, bv, (const uint2 *)s->tile_map[v], s->tile_zero, n, (const int *)ctx->cell_start,
+                               (const uint32_t *)ctx->bin.slots, ctx->perm, ctx->bin.rank, s->halo_perm, S,
+                               (const StepParams *)ctx->d_params, (float)MPMG_TOL, s->node_mass, s->node4,
+                               ctx->node_mx, ctx->node_my, ctx->node_fx, ctx->node_fy, node_m64));
+    mpmg_phase_end(ctx, PH_P2G);
 
     mpmg_phase_begin(ctx, PH_G2P);
     MPMG_CHECK(mpmg_launch_pdl(true, g2p_variant(c.material, batch, s->g2p_tile), dim3(s->g2p_blocks),
@@ -1674,7 +1571,7 @@ int mpmg_mixed_step(mpmg_ctx *ctx)
                                (const int *)cell_array(ctx, cur), cell_array(ctx, nxt), (const float4 *)s->node4,
                                ctx->bin.counts, ctx->d_params, ctx->d_status, NLOut{s->nl_T, s->nl_F}));
     mpmg_phase_end(ctx, PH_G2P);
-    ctx->launches += batch ? 3 : 2;
+    ctx->launches += 2;
     if (nonlocal) {
         // the fluidity solve (FP64 Krylov) and the stress update
         mpmg_phase_begin(ctx, PH_FLUIDITY);
