@@ -549,7 +549,7 @@ int mpmg_destroy(mpmg_ctx *ctx)
     if (ctx->batch) {
         cudaFree(ctx->batch->d_members);
         cudaFree(ctx->batch->d_elem_off);
-        cudaFree(ctx->batch->d_node_off);
+        cudaFree(ctx->batch->d_first);
         delete ctx->batch;
         ctx->batch = nullptr;
     }

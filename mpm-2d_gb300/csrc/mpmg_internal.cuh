@@ -91,7 +91,7 @@ struct BatchInfo {
     std::vector<size_t> poff, eoff, noff;
     void *d_members;       // device table of per-member constants (mpmg_mixed.cu)
     int *d_elem_off;       // eoff as int32, count + 1
-    int *d_node_off;       // noff as int32, count + 1
+    int *d_first;          // the member of every 256th element
 };
 
 // Counting-sort binning scratch (mpmg_bin.cu).  Bins 0..ne-1 count the keys

@@ -304,7 +304,7 @@ struct MemberM {
 struct BatchView {
     const MemberM *m;
     const int *elem_off;   // first global element of each member, then the total
-    const int *node_off;   // first global node of each member, then the total
+    const int *first;      // the member of every 256th global element
     int count;
 };
 
@@ -318,6 +318,16 @@ __device__ __forceinline__ int find_member(const int *__restrict__ off, int coun
         else hi = mid - 1;
     }
     return lo;
+}
+
+// The member of global element e: from the 256-element table, on to the next
+// ones where a member begins in between (a search of the offsets is five
+// dependent loads for 32 members).
+__device__ __forceinline__ int element_member(const BatchView &bv, int e)
+{
+    int k = __ldg(bv.first + (e >> 8));
+    while (e >= __ldg(bv.elem_off + k + 1)) k++;
+    return k;
 }
 
 // ---------------------------------------------------------------------------
@@ -396,6 +406,14 @@ __device__ __forceinline__ float ff_div(float nh, float nl, float dh, float dl, 
     return __fmaf_rn(res, r, q);
 }
 
+// A float as a double without the conversion, which runs on the FP64 pipe.
+__device__ __forceinline__ double widen_f(float f)
+{
+    const unsigned b = __float_as_uint(f), e = b & 0x7f800000u;
+    if (e == 0u || e == 0x7f800000u) return (b << 1) == 0u ? __hiloint2double((int)b, 0) : (double)f;   // zero; the rest
+    return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + (896u << 20))), (int)(b << 29));
+}
+
 // One node of the grid update: the four elements' corner sums in colour
 // order (process_usl.c:524-540), float-float for mass and momentum; boundary
 // masks; momentum update and nodal velocity / acceleration
@@ -403,7 +421,7 @@ __device__ __forceinline__ float ff_div(float nh, float nl, float dh, float dl, 
 // colour element c (off[c] < 0 when that element is absent or holds no
 // particle); the corner's other four sums follow at stride fs.
 template <bool F64NODE, typename Off>
-__device__ __forceinline__ void node_finish(const MemberM &M, double t_next, float tol, int i, int j, int n,
+__device__ __forceinline__ void node_finish(const MemberM &M, double t_next, float tol, double one, int i, int j, int n,
                                             const float *__restrict__ cs, const Off (&off)[4], Off fs,
                                             float2 *__restrict__ node_mass, float4 *__restrict__ node4,
                                             double *__restrict__ node_mx, double *__restrict__ node_my,
@@ -420,9 +438,9 @@ __device__ __forceinline__ void node_finish(const MemberM &M, double t_next, flo
         if (off[c] < 0) continue;
         const float *p = cs + off[c];
         if (F64NODE) {
-            m64 += (double)p[0];
-            mx64 += (double)p[fs];
-            my64 += (double)p[2 * fs];
+            m64 = __fma_rn(m64, one, widen_f(p[0]));
+            mx64 = __fma_rn(mx64, one, widen_f(p[fs]));
+            my64 = __fma_rn(my64, one, widen_f(p[2 * fs]));
         } else {
             ff_add(mh, ml, p[0]);
             ff_add(xh, xl, p[fs]);
@@ -437,13 +455,14 @@ __device__ __forceinline__ void node_finish(const MemberM &M, double t_next, flo
         if (bx) { mx64 = 0; fx = 0; }
         if (by) { my64 = 0; fy = 0; }
         float4 nd = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (m64 > (double)MPMG_TOL) {
+        // m64 > MPMG_TOL on the bit patterns (masses are not negative)
+        if (__double_as_longlong(m64) > __double_as_longlong(MPMG_TOL) && __double_as_longlong(m64) <= 0x7ff0000000000000LL) {
             // FP64 momentum update and division (1 / m: the FP32 reciprocal
             // refined by one Newton step, ~2^-46 relative)
-            double r = (double)__frcp_rn((float)m64);
-            r = fma(r, fma(-m64, r, 1.0), r);
-            mx64 += dt * (double)fx;
-            my64 += dt * (double)fy;
+            double r = widen_f(__frcp_rn((float)m64));
+            r = fma(r, fma(-m64, r, one), r);
+            mx64 = fma(dt, widen_f(fx), mx64);
+            my64 = fma(dt, widen_f(fy), my64);
             const float rf = (float)r;
             nd.x = fx * rf;
             nd.y = fy * rf;
@@ -451,7 +470,7 @@ __device__ __forceinline__ void node_finish(const MemberM &M, double t_next, flo
             nd.w = (float)(my64 * r);
         }
         const float mhi = (float)m64;
-        node_mass[n] = make_float2(mhi, (float)(m64 - (double)mhi));
+        node_mass[n] = make_float2(mhi, (float)(m64 - widen_f(mhi)));
         if (node_m64 != nullptr) node_m64[n] = m64;
         node4[n] = nd;
         if (node_mx != nullptr) {
@@ -544,6 +563,8 @@ __global__ void __launch_bounds__(TX * TY, 1024 / (TX * TY)) mx_p2g_grid_kernel(
     __shared__ int sh_off[NT + 1];     // stage offsets of the tile's elements
     __shared__ int sh_gs[TY];          // storage position of each tile row's first particle
     __shared__ int sh_wsum[NT / 32];
+    __shared__ double sh_one;          // 1 as a register operand (mat::Unit)
+    if (threadIdx.x == 0) sh_one = 1.0;
     float4 *sh_a = reinterpret_cast<float4 *>(smem);
     float4 *sh_b = sh_a + T::c16;
     float *sh_syy = reinterpret_cast<float *>(sh_b + T::c16);
@@ -735,7 +756,7 @@ __global__ void __launch_bounds__(TX * TY, 1024 / (TX * TY)) mx_p2g_grid_kernel(
                 const int a = dx ? (dy ? 0 : 3) : (dy ? 1 : 2);
                 off[c] = sh_off[le + 1] != sh_off[le] ? (a * 5) * SS + le : -1;
             }
-            node_finish<F64NODE>(M, sp->t + M.dt, tol, i, j, M.nd0 + j * Nx + i, sh_sum, off, SS, node_mass, node4,
+            node_finish<F64NODE>(M, sp->t + M.dt, tol, sh_one, i, j, M.nd0 + j * Nx + i, sh_sum, off, SS, node_mass, node4,
                                  node_mx, node_my, node_fx, node_fy, node_m64);
         }
     }
@@ -958,7 +979,7 @@ __global__ void __launch_bounds__(kG2PTile, 768 / kG2PTile) mx_g2p_kernel(
                 D.D[dst] = d4;
                 cell_dst[dst] = ne_total;
             } else {
-                const int mk = BATCH ? find_member(bv.elem_off, bv.count, e) : 0;
+                const int mk = BATCH ? element_member(bv, e) : 0;
                 const MemberM &M = BATCH ? bv.m[mk] : m0;
                 new_key = g2p_particle<MATERIAL>(M, sentinel, node4, e - M.e0, a4, b4, c4, d4, dst, D, cell_dst,
                                                  i, nl);
@@ -1334,17 +1355,20 @@ int mpmg_mixed_init(mpmg_ctx *ctx, const double *m, const double *v, const doubl
     const int count = bt ? bt->count : 1;
     if (bt) {
         std::vector<MemberM> hm(count);
-        std::vector<int> eo(count + 1), no(count + 1);
+        std::vector<int> eo(count + 1);
         for (int k = 0; k < count; k++) hm[k] = make_member(bt->cfg[k], bt->eoff[k], bt->noff[k]);
-        for (int k = 0; k <= count; k++) {
-            eo[k] = (int)bt->eoff[k];
-            no[k] = (int)bt->noff[k];
-        }
+        for (int k = 0; k <= count; k++) eo[k] = (int)bt->eoff[k];
         MemberM *dm = nullptr;
         if ((rc = dalloc(&dm, count)) != MPMG_OK) return rc;
         bt->d_members = dm;
         if ((rc = dalloc(&bt->d_elem_off, count + 1)) != MPMG_OK) return rc;
-        if ((rc = dalloc(&bt->d_node_off, count + 1)) != MPMG_OK) return rc;
+        std::vector<int> first(ctx->ne / 256 + 1);
+        for (int e = 0, k = 0; (size_t)e * 256 < ctx->ne; e++) {
+            while (k + 1 < count && (size_t)e * 256 >= bt->eoff[k + 1]) k++;
+            first[e] = k;
+        }
+        if ((rc = dalloc(&bt->d_first, first.size())) != MPMG_OK) return rc;
+        MPMG_CHECK(cudaMemcpy(bt->d_first, first.data(), first.size() * sizeof(int), cudaMemcpyHostToDevice));
         for (int v = 0; v < kP2GVariants; v++) {
             std::vector<uint2> map;
             for (int k = 0; k < count; k++) {
@@ -1359,7 +1383,6 @@ int mpmg_mixed_init(mpmg_ctx *ctx, const double *m, const double *v, const doubl
         }
         MPMG_CHECK(cudaMemcpy(dm, hm.data(), count * sizeof(MemberM), cudaMemcpyHostToDevice));
         MPMG_CHECK(cudaMemcpy(bt->d_elem_off, eo.data(), (count + 1) * sizeof(int), cudaMemcpyHostToDevice));
-        MPMG_CHECK(cudaMemcpy(bt->d_node_off, no.data(), (count + 1) * sizeof(int), cudaMemcpyHostToDevice));
     }
 
     if (!bt) {
@@ -1530,7 +1553,7 @@ static BatchView batch_view(const mpmg_ctx *ctx)
     if (ctx->batch) {
         bv.m = (const MemberM *)ctx->batch->d_members;
         bv.elem_off = ctx->batch->d_elem_off;
-        bv.node_off = ctx->batch->d_node_off;
+        bv.first = ctx->batch->d_first;
         bv.count = ctx->batch->count;
     }
     return bv;
@@ -1729,7 +1752,7 @@ __global__ void __launch_bounds__(256) mx_export_kernel(
     const int c = cell[i];
     double ox = 0, oy = 0, h = 1;
     if (c < ne) {
-        const MemberM &M = bv.count > 1 ? bv.m[find_member(bv.elem_off, bv.count, c)] : m0;
+        const MemberM &M = bv.count > 1 ? bv.m[element_member(bv, c)] : m0;
         const int lc = c - M.e0;
         const int cj = (int)mpmg_div((uint32_t)lc, M.g.div_Ex), ci = lc - cj * M.g.Ex;
         ox = ci;
