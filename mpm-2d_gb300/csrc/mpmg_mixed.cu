@@ -904,8 +904,10 @@ __global__ void __launch_bounds__(kG2PTile, 768 / kG2PTile) mx_g2p_kernel(
         mpmg_bulk_g2s(stage[k].C, S.C + base, kG2PTile * 16, &full[k]);
         mpmg_bulk_g2s(stage[k].D, S.D + base, kG2PTile * 16, &full[k]);
         mpmg_bulk_g2s(stage[k].src, cell_src + base, kG2PTile * 4, &full[k]);
-        mpmg_bulk_g2s(stage[k].rank, rank + base, kG2PTile * 4, &full[k]);
         inflight |= 1u << k;
+    };
+    auto issue_rank = [&](int tile, int k) {
+        mpmg_bulk_g2s(stage[k].rank, rank + (size_t)tile * kG2PTile, kG2PTile * 4, &full[k]);
     };
     if (tid == 0) {
         for (int k = 0; k < kG2PStages; k++) {
@@ -913,11 +915,14 @@ __global__ void __launch_bounds__(kG2PTile, 768 / kG2PTile) mx_g2p_kernel(
             if (tile < num_tiles && (tile + 1) * kG2PTile <= n) issue(tile, k);
         }
     }
-    // The stored records and elements come from the previous step's G2P and
-    // the ranks from this step's P2G, two kernels back: the first copies are
-    // in flight before the wait.  The nodal values come from the grid
-    // update just before.
+    // The stored records and elements come from the previous step's G2P: their
+    // first copies are in flight before the wait.  The ranks and the nodal
+    // values come from the kernel just before.
     mpmg_pdl_wait();
+    if (tid == 0) {
+        for (int k = 0; k < kG2PStages; k++)
+            if (inflight & (1u << k)) issue_rank(blockIdx.x + k * gridDim.x, k);
+    }
     if (blockIdx.x == 0) {
         // Advance t and compute the next step's body force (the driver's
         // time_varying_loads, loading.c:34-54), one thread per member.  No
@@ -999,6 +1004,7 @@ __global__ void __launch_bounds__(kG2PTile, 768 / kG2PTile) mx_g2p_kernel(
             if (next < num_tiles && (next + 1) * kG2PTile <= n) {
                 mpmg_fence_proxy_async();
                 issue(next, k);
+                issue_rank(next, k);
             }
         }
         k = (k + 1 == kG2PStages) ? 0 : k + 1;
