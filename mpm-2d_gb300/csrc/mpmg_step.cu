@@ -402,10 +402,12 @@ __global__ void __launch_bounds__(EB * SPLIT) p2g_cells_kernel(
 // c3 = (q2 - q3) - c1: four FP64 operations per element and field here save
 // the G2P about six per particle, and an element's sixteen doubles are one
 // 128-byte line for its gathers instead of sixteen loads from eight lines.
-// TY = 16 recomputes 10 % of the nodes; TY = 4 (39 %) where the grid is too
-// small to give every SM a tall tile, so that its chain is spread out.
+// Flat tiles: TY = 4 recomputes 39 % of the nodes (16: 10 %), but a block is one
+// warp a sub-partition, and a sparse grid's filled tiles spread over all SMs
+// (125k particles on 261k nodes: 54.0 us a step, 56.3 with TY = 8, 58.2 with 16;
+// 1 048 576 particles on 263k: 253.3, 252.3, 253.8).
 
-constexpr int kGridTX = 32;
+constexpr int kGridTX = 32, kGridTY = 4;
 
 // The corner (BL, BR, TR, TL) that node (i, j) is of its colour-c element.
 __device__ __forceinline__ int c_corner(int c, int i, int j)
@@ -414,8 +416,7 @@ __device__ __forceinline__ int c_corner(int c, int i, int j)
     return right ? (up ? 0 : 3) : (up ? 1 : 2);
 }
 
-template <int TY>
-__global__ void __launch_bounds__(kGridTX * TY) grid_kernel(
+__global__ void __launch_bounds__(kGridTX * kGridTY) grid_kernel(
     GridGeom g, BcParams bc, int tiles_x, const uint32_t *__restrict__ count, uint32_t *__restrict__ count_next,
     uint32_t *__restrict__ n_over_next, uint32_t *__restrict__ n_filled_next, uint32_t *__restrict__ cursor,
     const double *__restrict__ cell_sums, const StepParams *__restrict__ sp, double dt,
@@ -424,7 +425,7 @@ __global__ void __launch_bounds__(kGridTX * TY) grid_kernel(
     double *__restrict__ node_my, double *__restrict__ node_fx, double *__restrict__ node_fy,
     double2 *__restrict__ coef, int early)
 {
-    __shared__ double sh[4][TY][kGridTX];
+    __shared__ double sh[4][kGridTY][kGridTX];
     __shared__ double sh_const[4];         // constants as registers (mat::Unit)
     if (threadIdx.x == 0) {
         sh_const[0] = 1.0;
@@ -433,7 +434,7 @@ __global__ void __launch_bounds__(kGridTX * TY) grid_kernel(
         sh_const[3] = dt;
     }
     const int tx = threadIdx.x % kGridTX, ty = threadIdx.x / kGridTX;
-    const int i = (int)(blockIdx.x % tiles_x) * (kGridTX - 1) + tx, j = (int)(blockIdx.x / tiles_x) * (TY - 1) + ty;
+    const int i = (int)(blockIdx.x % tiles_x) * (kGridTX - 1) + tx, j = (int)(blockIdx.x / tiles_x) * (kGridTY - 1) + ty;
     const bool node = i < g.Nx && j < g.Ny;
     // Colour c = 2 * (row % 2) + (col % 2) (process_usl.c:158); the four
     // elements around a node have the four colours, summed in order 0..3.
@@ -454,7 +455,7 @@ __global__ void __launch_bounds__(kGridTX * TY) grid_kernel(
             src[c] = cell_sums + (size_t)e * kCell + corner * 4;
         }
     }
-    const bool own = node && (tx < kGridTX - 1 || i == g.Nx - 1) && (ty < TY - 1 || j == g.Ny - 1);
+    const bool own = node && (tx < kGridTX - 1 || i == g.Nx - 1) && (ty < kGridTY - 1 || j == g.Ny - 1);
     mpmg_pdl_wait();
     if (early) mpmg_pdl_trigger();
     __syncthreads();
@@ -538,7 +539,7 @@ __global__ void __launch_bounds__(kGridTX * TY) grid_kernel(
     sh[2][ty][tx] = vxn;
     sh[3][ty][tx] = vyn;
     __syncthreads();
-    if (filled && tx < kGridTX - 1 && ty < TY - 1) {
+    if (filled && tx < kGridTX - 1 && ty < kGridTY - 1) {
         double2 *out = coef + (size_t)(j * g.Ex + i) * 8;
 #pragma unroll
         for (int f = 0; f < 4; f++) {
@@ -551,12 +552,11 @@ __global__ void __launch_bounds__(kGridTX * TY) grid_kernel(
     mpmg_pdl_trigger();
 }
 
-template <int TY>
 cudaError_t launch_grid(mpmg_ctx *ctx, const GridGeom &g)
 {
     const RowBins &r = ctx->row;
-    const int tiles_x = (g.Nx + kGridTX - 2) / (kGridTX - 1), tiles_y = (g.Ny + TY - 2) / (TY - 1);
-    return mpmg_launch_pdl(true, grid_kernel<TY>, dim3(tiles_x * tiles_y), dim3(kGridTX * TY), 0, ctx->stream, g,
+    const int tiles_x = (g.Nx + kGridTX - 2) / (kGridTX - 1), tiles_y = (g.Ny + kGridTY - 2) / (kGridTY - 1);
+    return mpmg_launch_pdl(true, grid_kernel, dim3(tiles_x * tiles_y), dim3(kGridTX * kGridTY), 0, ctx->stream, g,
                            make_bc(ctx), tiles_x, (const uint32_t *)r.count[r.cur], r.count[1 - r.cur],
                            r.n_over + (1 - r.cur), r.n_filled + (1 - r.cur), r.cursor, (const double *)ctx->cell_sums,
                            (const StepParams *)ctx->d_params, ctx->cfg.dt,
@@ -1156,7 +1156,7 @@ inline int blocks_for(size_t n, int threads)
 }  // namespace
 
 // More than two warps of particles a sub-partition: the G2P is then bound by
-// the FP64 pipe and takes blocks of four warps and integer products
+// the FP64 pipe and takes larger blocks and integer products
 // (mat::SoftElastic; g_local_mu2, 1 048 576 particles: 287 -> 254 us a step,
 // 125k: 67 -> 62; isolin, 65k: 40.5 -> 38.8).  Up to there a sub-partition's
 // one or two warps run a serial chain, through an instruction cache that the
@@ -1182,7 +1182,10 @@ template <int MATERIAL, int PHASE>
 static cudaError_t launch_g2p(mpmg_ctx *ctx, const G2PArgs &A)
 {
     const bool bound = g2p_pipe_bound(ctx);
-    const int t = bound ? 128 : 32;
+    // blocks of two warps up to sixteen warps a sub-partition, where a block of
+    // four more or less on an SM still shows (125k: 58.2 us with four, 56.4 with
+    // two; 1 048 576: 253.8 and 255.6)
+    const int t = !bound ? 32 : ctx->np <= (size_t)ctx->sms * 4 * 32 * 16 ? 64 : 128;
     ctx->launches += 1;
     return mpmg_launch_pdl(true,
                            bound ? g2p_kernel<typename BoundArith<PHASE>::E, MATERIAL, PHASE>
@@ -1265,8 +1268,7 @@ int mpmg_launch_step(mpmg_ctx *ctx)
     mpmg_phase_end(ctx, PH_P2G);
 
     mpmg_phase_begin(ctx, PH_GRID);
-    // a tall tile for every SM, or flat ones
-    MPMG_CHECK(ctx->nn >= (size_t)ctx->sms * 31 * 15 ? launch_grid<16>(ctx, g) : launch_grid<4>(ctx, g));
+    MPMG_CHECK(launch_grid(ctx, g));
     ctx->launches += 1;
     mpmg_phase_end(ctx, PH_GRID);
 
