@@ -839,18 +839,19 @@ __device__ __forceinline__ void nonlocal_mu2_stress(const E &el, double gf, doub
         nup_tau = 0;
         sxx = 0; sxy = 0; syy = 0;
     } else if (is_pos(p_tr)) {
-        const double scale_factor = quot(p_tr, __fma_rn(el.Gdt, gf, p_tr));
+        const double scale_factor = quot(p_tr, el.add(el.mul(el.Gdt, gf), p_tr));
+        const double tau_tau = el.mul(tau_tr, scale_factor);
         // ((tau - tau_tau) / G) / dt as one quotient by G dt (the fluidity
         // comes from an iterative solve, so this value is not bit-exact
         // with the reference's anyway)
-        nup_tau = dvd_const(__fma_rn(-tau_tr, scale_factor, tau_tr), el.kGdt);
-        sxx = __fma_rn(scale_factor, t0xx, -p_tr);
+        nup_tau = dvd_const(el.sub(tau_tr, tau_tau), el.kGdt);
+        sxx = el.sub(el.mul(scale_factor, t0xx), p_tr);
         sxy = el.mul(scale_factor, t0xy);
-        syy = __fma_rn(scale_factor, t0yy, -p_tr);
+        syy = el.sub(el.mul(scale_factor, t0yy), p_tr);
     } else {
         nup_tau = 0;
     }
-    gammap = __fma_rn(nup_tau, el.dt, gammap);
+    gammap = el.add(gammap, el.mul(nup_tau, el.dt));
     gammadotp = nup_tau;
 }
 

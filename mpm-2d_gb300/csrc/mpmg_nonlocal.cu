@@ -169,12 +169,13 @@ __global__ void __launch_bounds__(128) assemble_kernel(
         mbb = fma(vb, b, mbb);
     }
     // sum v grad s_r . grad s_c h^2 from the moments, rows (0,0..3),
-    // (1,1..3), (2,2..3), (3,3); oxx = sum v ox^2, oyy = sum v oy^2
-    const double oxx = u.add(u.sub(m0, u.add(ma, ma)), maa), oyy = u.add(u.sub(m0, u.add(mb, mb)), mbb);
+    // (1,1..3), (2,2..3), (3,3); doublings are exact
+    const double m2 = u.add(m0, m0), ma2 = u.add(ma, ma), mb2 = u.add(mb, mb);
+    const double oxx = u.add(u.sub(m0, ma2), maa), oyy = u.add(u.sub(m0, mb2), mbb);
     const double xa = u.sub(ma, maa), yb = u.sub(mb, mbb);
-    const double g02 = -u.add(xa, yb);
+    const double g02 = u.add(u.sub(maa, ma), u.sub(mbb, mb));
     const double gg[10] = {
-        u.add(oxx, oyy),                                // oy^2 + ox^2
+        u.add(u.add(u.sub(m2, ma2), maa), u.sub(mbb, mb2)),   // oy^2 + ox^2
         u.sub(xa, oyy),                                 // ox a - oy^2
         g02,                                            // -oy b - ox a
         u.sub(yb, oxx),                                 // oy b - ox^2
@@ -2384,8 +2385,8 @@ __global__ void __launch_bounds__(kMgThreads, 1) pcg_mg_kernel(SolveArgs S, cons
 
 // Nodal fluidity back to the particles, then the stress update
 // (g_nonlocal_mu2.c:545-564 and :160-218; g_nonlocal.c:559-578, :154-298).
-// Bound by the FP64 pipe: the nodal field as a bilinear form, compares on bit
-// patterns, integer products (835 996 particles: 62 -> 37 us).
+// Bound by the FP64 pipe: integer products, compares on bit patterns, register
+// operands (835 996 particles: 62 -> 37 us).
 // AVG: the element average of the four nodal values instead of the shape
 // functions (g_nonlocal_avg.c:575-578). MU2 reads the trial stress the G2P
 // kept (trial: p_d, t0xx, t0xy, t0yy, tau, value-major) in place of the
@@ -2418,10 +2419,11 @@ __global__ void __launch_bounds__(256) fluidity_stress_kernel(
             g += 0.25 * node_gf[n0 + 1 + Nx];
             g += 0.25 * node_gf[n0 + Nx];
         } else {
-            // the bilinear form c0 + c1 a + b (c2 + c3 a)
-            const double c0 = node_gf[n0], n3 = node_gf[n0 + Nx], c1 = el.sub(node_gf[n0 + 1], c0);
-            const double c3 = el.sub(el.sub(node_gf[n0 + 1 + Nx], n3), c1);
-            g = fma(b, fma(a, c3, el.sub(n3, c0)), fma(a, c1, c0));
+            const double ox = el.sub(el.one, a), oy = el.sub(el.one, b);
+            g = fma(node_gf[n0], el.mul(ox, oy), g);
+            g = fma(node_gf[n0 + 1], el.mul(a, oy), g);
+            g = fma(node_gf[n0 + 1 + Nx], el.mul(a, b), g);
+            g = fma(node_gf[n0 + Nx], el.mul(ox, b), g);
         }
         gf[i] = g;
     }
