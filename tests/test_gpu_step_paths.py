@@ -6,7 +6,7 @@ products (2 and 16 warps a sub-partition) and filled-element counts either side
 of the P2G's two forms, against the oracle.  Criterion as for one step from a
 reference state: 1e-10 of each field's largest value.
 
-Mixed: grids of one to a few elements either side of the P2G's 16 x 16 tiles, as
+Mixed: grids of one to a few elements either side of the P2G's tiles, as
 batch members and alone, against the FP64 form; and tiles that particles leave.
 Criterion: FP32 state, a few steps: 1e-5 of the field's norm.
 
@@ -96,7 +96,7 @@ def small_grid(nx, ny, seed):
 
 @pytest.mark.parametrize("precision", ["mixed", "mixed_f64node"])
 def test_mixed_tiles_vs_fp64(precision):
-    grids = [(2, 2), (16, 17), (17, 16), (15, 31), (31, 32), (47, 3)]
+    grids = [(2, 2), (16, 17), (17, 16), (15, 31), (31, 32), (47, 3), (32, 8), (33, 7)]
     members = [small_grid(nx, ny, k) for k, (nx, ny) in enumerate(grids)]
     batch = mpm2d.Batch(members, precision=precision)
     batch.step(5)
