@@ -273,7 +273,14 @@ __device__ __forceinline__ double quot(double a, double b)
 // a b as a b + (-0) and a + b as a 1 + b (the same results bit for bit), and
 // keep 1, -0 and every other constant in shared memory, from where they load
 // into registers; as literals or kernel parameters the compiler would fold
-// them back.
+// them back.  (It also folds a shared variable that only ever holds one
+// constant: those are stored through opaque().)
+__device__ __forceinline__ double opaque(double x)
+{
+    asm volatile("" : "+d"(x));
+    return x;
+}
+
 struct Unit {
     double one, nz;         // 1, -0
     __device__ __forceinline__ double mul(double a, double b) const { return __fma_rn(a, b, nz); }

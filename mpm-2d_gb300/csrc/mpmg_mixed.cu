@@ -30,6 +30,7 @@
 #include <vector>
 
 #include "mpmg_internal.cuh"
+#include "mpmg_materials.cuh"
 
 namespace {
 
@@ -567,7 +568,7 @@ __global__ void __launch_bounds__(TX * TY, 1024 / (TX * TY)) mx_p2g_grid_kernel(
     __shared__ int sh_gs[TY];          // storage position of each tile row's first particle
     __shared__ int sh_wsum[NT / 32];
     __shared__ double sh_one;          // 1 as a register operand (mat::Unit)
-    if (threadIdx.x == 0) sh_one = 1.0;
+    if (threadIdx.x == 0) sh_one = mat::opaque(1.0);
     float4 *sh_a = reinterpret_cast<float4 *>(smem);
     float4 *sh_b = sh_a + T::c16;
     float *sh_syy = reinterpret_cast<float *>(sh_b + T::c16);

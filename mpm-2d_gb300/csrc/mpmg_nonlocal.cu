@@ -113,8 +113,8 @@ __global__ void __launch_bounds__(128) assemble_kernel(
 {
     __shared__ double sh_const[2];         // constants as registers (mat::Unit)
     if (threadIdx.x == 0) {
-        sh_const[0] = 1.0;
-        sh_const[1] = -0.0;
+        sh_const[0] = mat::opaque(1.0);
+        sh_const[1] = mat::opaque(-0.0);
     }
     __syncthreads();
     int e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2017,8 +2017,8 @@ __global__ void __launch_bounds__(kMgThreads, 1) pcg_mg_kernel(SolveArgs S, cons
     for (int e = threadIdx.x; e < (int)(sizeof(MgPlan) / sizeof(int)); e += blockDim.x)
         reinterpret_cast<int *>(&P)[e] = __ldg(reinterpret_cast<const int *>(plan) + e);
     if (threadIdx.x == 0) {
-        sh_unit[0] = 1.0;
-        sh_unit[1] = -0.0;
+        sh_unit[0] = mat::opaque(1.0);
+        sh_unit[1] = mat::opaque(-0.0);
     }
     __syncthreads();
     const mat::Unit u{sh_unit[0], sh_unit[1]};

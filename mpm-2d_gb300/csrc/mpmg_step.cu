@@ -163,8 +163,8 @@ __global__ void __launch_bounds__(EB * SPLIT) p2g_cells_kernel(
     __shared__ double sh_const[3];         // constants as registers (mat::Unit)
     const int tid = threadIdx.x;
     if (tid == 0) {
-        sh_const[0] = 1.0;
-        sh_const[1] = -0.0;
+        sh_const[0] = mat::opaque(1.0);
+        sh_const[1] = mat::opaque(-0.0);
         sh_const[2] = g.inv_h;
     }
     if (tid < NB) sh_bin[tid] = 0;
@@ -428,8 +428,8 @@ __global__ void __launch_bounds__(kGridTX * kGridTY) grid_kernel(
     __shared__ double sh[4][kGridTY][kGridTX];
     __shared__ double sh_const[4];         // constants as registers (mat::Unit)
     if (threadIdx.x == 0) {
-        sh_const[0] = 1.0;
-        sh_const[1] = -0.0;
+        sh_const[0] = mat::opaque(1.0);
+        sh_const[1] = mat::opaque(-0.0);
         sh_const[2] = g.inv_h;
         sh_const[3] = dt;
     }
