@@ -61,20 +61,15 @@ WORKLOAD = "box_fill_1M_g_local_mu2"
 # once per use; node gathers counted once per node), as (per particle, per
 # element, per node).
 #
-# FP64 form, g_local_mu2: keys read x y active (20 B) and write element,
-# active, key (12 B) per particle; the sort's scatter reads the key and writes
-# slot + sorted key, the P2G's ordering reads the slot and writes perm (20 B
-# per particle; bins read, cursor and offsets written, 16 B per element); the
-# P2G reads perm and 9 particle doubles and writes 4 corners x 5 sums; the
-# grid update reads them back and writes 5 doubles per node; the G2P reads
-# element + 13 doubles and writes 13 doubles per particle and gathers 4
-# doubles per node.
+# FP64 form, g_local_mu2: the P2G reads a row entry (4 B) and 9 particle doubles
+# and writes 20 corner sums per element; the grid update reads them back and
+# writes 16 element coefficients and 5 doubles per node; the G2P reads key + 13
+# doubles and writes 13 doubles, element, key and the next step's row entry per
+# particle, and reads the coefficients.
 FP64_BYTES = {
-    "keys": (32, 0, 0),
-    "sort": (20, 16, 0),
     "p2g": (4 + 9 * 8, 160, 0),
-    "grid": (0, 160, 40),
-    "g2p": (13 * 8 + 8 + 13 * 8, 0, 32),
+    "grid": (0, 288, 40),
+    "g2p": (4 + 13 * 8 + 13 * 8 + 12, 128, 0),
 }
 # The compulsory bytes of the FP64 step (each persistent field read
 # and written once, sort scratch and transients excluded): 216 B per
@@ -103,33 +98,23 @@ MIXED_BYTES = {
 # g_local_mu2, 64 B per node-step; of those the G2P moves the particle state
 # (13 floats read, 13 written = 104 B) and the node gathers (16 B per node).
 MIXED_STEP_SURVEY_BYTES = (112, 0, 64)
-# A batch runs P2G and grid update as two kernels, so the element corner sums
-# (5 floats x 4 corners) are written and read back: 80 B per element each.
-BATCH_BYTES = {
-    "sort": (20, 16, 0),
-    "p2g": (40, 80, 0),
-    "grid": (0, 80, 24),
-    "g2p": (128, 0, 16),
-}
 MIXED_G2P_SURVEY_BYTES = (104, 0, 16)
 
-# FP64 work per particle of the FP64 G2P + g_local_mu2 after the warm-up
-# steps, from one ncu capture of g2p_kernel<1,0> (the same fill at 256^2
-# elements, 262 144 particles, step 27; per-particle counts do not depend on
-# the size): operations (DADD + DMUL + 2 DFMA: 48.4 + 48.4 + 2 x 54.6) and
-# FP64 pipe instructions (pipe-active cycles x 2 per SM, compares and
-# conversions included).
-G2P64_FLOPS_PER_PARTICLE = 206.0
-G2P64_PIPE_INSTR_PER_PARTICLE = 210.8
+# FP64 work per particle of the FP64 G2P + g_local_mu2, from one ncu capture of
+# its kernel at 1 048 576 particles: operations the FP64 pipe executes (DADD +
+# DMUL + 2 DFMA: 6.0 + 0.1 + 2 x 60.1; the law's plain products, quotients by
+# constants and the exponential run on the integer pipe) and FP64 pipe
+# instructions.
+G2P64_FLOPS_PER_PARTICLE = 126.3
+G2P64_PIPE_INSTR_PER_PARTICLE = 72.2
 
 # DRAM bytes (read + write) of one mx_g2p_kernel launch on this workload from
 # one ncu capture: 80.8 MB read + 17.0 MB written; writes still in L2 at the
 # kernel's end are not in the figure.
 G2P_TRAFFIC_BYTES = 97.8e6
-# dram__bytes_read.sum + dram__bytes_write.sum of one g2p_kernel<1,0> launch
-# on the 1 048 576-particle workload (126.1 + 49.1 MB, the FP64 step's ncu
-# capture)
-G2P64_TRAFFIC_BYTES = 175.2e6
+# dram__bytes_read.sum + dram__bytes_write.sum of one FP64 G2P launch on the
+# 1 048 576-particle workload (151.8 + 71.5 MB, the same capture)
+G2P64_TRAFFIC_BYTES = 223.3e6
 
 # The compiled reference against the oracle port on this workload, same host
 # and thread count (oracle/time_reference.py, 8-core x86-64 development host,
@@ -465,7 +450,7 @@ def run_gpu(args):
     g2p64 = phases64["g2p"]
     fp64_peak = mpm2d.fp64_rate(dev)
     step64_survey = phase_bytes({"s": FP64_STEP_SURVEY_BYTES}, "s", n, ne, nn)
-    roofline = {"bound": "hbm", "kernel": "g2p (FP64 G2P + g_local_mu2, g2p_kernel<1,0>)",
+    roofline = {"bound": "hbm", "kernel": "g2p (FP64 G2P + g_local_mu2, g2p_kernel<SoftElastic,1,0>)",
                 "achieved": g2p64["gbs"], "peak": peak, "peak_kind": peak_kind, "unit": "GB/s",
                 "frac": g2p64["gbs"] / peak,
                 "traffic": G2P64_TRAFFIC_BYTES if n == 1048576 else None,
@@ -601,7 +586,7 @@ def run_gpu(args):
         bn = nb
         be = int(sum((sc["Nx"] - 1) * (sc["Ny"] - 1) for sc in ens))
         bnn = int(sum(sc["Nx"] * sc["Ny"] for sc in ens))
-        b_builder = sum(phase_bytes(BATCH_BYTES, k, bn, be, bnn) for k in BATCH_BYTES)
+        b_builder = sum(phase_bytes(MIXED_BYTES, k, bn, be, bnn) for k in MIXED_BYTES)
         b_survey = phase_bytes({"s": MIXED_STEP_SURVEY_BYTES}, "s", bn, be, bnn)
         b_step_s = msb / bsteps / 1e3
         # the same members one at a time (each its own context and step graphs)
