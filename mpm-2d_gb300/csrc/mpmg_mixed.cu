@@ -198,6 +198,8 @@ __device__ __forceinline__ void g_local_mu2_f(const MatF &p, float m, float v, f
 // fluidity p / (G dt) (1 / scale - 1) cancels near yield, and in FP32 that
 // cancellation biased the flow (an 8 % faster silo discharge than the FP64
 // form; within the FP64 form's own round-off spread once evaluated in FP64).
+// Roots and quotients are mat::root and mat::quot: the same values in one FP64
+// operation each.
 __device__ __forceinline__ void nonlocal_mu2_trial_f(const MatF &p, float exx, float exy, float eyy, float wxy,
                                                      float sxx, float sxy, float syy, float &p_tr, float &t0xx,
                                                      float &t0xy, float &t0yy, float &tau_tr)
@@ -210,7 +212,7 @@ __device__ __forceinline__ void nonlocal_mu2_trial_f(const MatF &p, float exx, f
     const double pt = -0.5 * (sxx_tr + syy_tr);
     const double a = sxx_tr + pt, b = sxy_tr, c = syy_tr + pt;
     p_tr = (float)pt; t0xx = (float)a; t0xy = (float)b; t0yy = (float)c;
-    tau_tr = (float)sqrt(0.5 * (a * a + 2.0 * b * b + c * c));
+    tau_tr = (float)mat::root(0.5 * (a * a + 2.0 * b * b + c * c));
 }
 
 __device__ __forceinline__ void nonlocal_mu2_bulk_f(const MatF &p, float m, float v, float p_tr, float tau_tr,
@@ -225,15 +227,15 @@ __device__ __forceinline__ void nonlocal_mu2_bulk_f(const MatF &p, float m, floa
         double tau_tau = tau;
         if (tau > S0) {
             const double S2 = (double)p.mu_2 * pr;
-            const double alpha = (double)p.alpha_coef * sqrt(pr * (double)p.inv_grains_rho);
+            const double alpha = (double)p.alpha_coef * mat::root(pr * (double)p.inv_grains_rho);
             const double B = -(S2 + tau + alpha);
             const double H = S2 * tau + S0 * alpha;
-            const double disc = sqrt(B * B - 4.0 * H);
-            tau_tau = (B > 0.0) ? (-B - disc) * 0.5 : (2.0 * H) / (-B + disc);
+            const double disc = mat::root(B * B - 4.0 * H);
+            tau_tau = (B > 0.0) ? (-B - disc) * 0.5 : mat::quot(2.0 * H, -B + disc);
             // (1 / scale - 1) with scale = tau_tau / tau, as one quotient
-            gf_local = (float)(pr * (double)p.inv_G_dt * ((tau - tau_tau) / tau_tau));
+            gf_local = (float)(pr * (double)p.inv_G_dt * mat::quot(tau - tau_tau, tau_tau));
         }
-        xisq_inv = (float)(fabs(tau_tau / pr - (double)p.mu_s) * (double)p.inv_A2d2);
+        xisq_inv = (float)(fabs(mat::quot(tau_tau, pr) - (double)p.mu_s) * (double)p.inv_A2d2);
     }
 }
 
@@ -247,7 +249,7 @@ __device__ __forceinline__ void nonlocal_mu2_stress_f(const MatF &p, float gf, f
     if (!(p_tr > 0.0f)) {
         sxx = sxy = syy = 0.0f;
     } else {
-        const double scale = (double)p_tr / ((double)p.G * p.dt * gf + p_tr);
+        const double scale = mat::quot((double)p_tr, (double)p.G * p.dt * gf + p_tr);
         nup = (float)((tau_tr - tau_tr * scale) * (double)p.inv_G_dt);
         sxx = (float)(scale * t0xx - p_tr);
         sxy = (float)(scale * t0xy);
