@@ -194,11 +194,12 @@ MPMG_API int mpmg_synchronize(mpmg_ctx *ctx);
    Tyy Tzz state0..state10.  Node fields: node_m node_mx node_my node_fx
    node_fy node_vx node_vy node_ax node_ay node_gf. */
 MPMG_API int mpmg_get_field(mpmg_ctx *ctx, const char *name, double *host_out);
-/* Reads count fields at once, each device array behind them downloaded
-   once: a whole output frame, as the driver's write_frame
+/* Reads count fields at once, behind the steps and with one wait: a whole
+   output frame, as the driver's write_frame
    (src/writer.c:190-201, called from src/main.c:957) reads the particles'
    m v x y x_t y_t sxx sxy syy ux uy state[9] state[10].  host_out[k]
-   receives names[k]. */
+   receives names[k].  Pinned destinations are written by the device in one
+   launch; pageable ones are copied one by one through pinned chunks. */
 MPMG_API int mpmg_get_fields(mpmg_ctx *ctx, int count, const char *const *names, double *const *host_out);
 
 /* The driver's output files.  mpmg_write_frame writes one write_frame block
@@ -228,14 +229,15 @@ MPMG_API int mpmg_set_map(mpmg_ctx *ctx, const int *in_element, const int *activ
 
 /* The last step's cell sort: sorted keys (element, or num_elements for
    inactive particles), the permutation (sorted position -> particle index)
-   and per-element start offsets (num_elements + 1 entries). */
+   and per-element start offsets (num_elements + 1 entries).  The FP64 step
+   bins without a sort; for it the sort is formed here. */
 MPMG_API int mpmg_get_sort(mpmg_ctx *ctx, int *sorted_keys, int *perm, int *cell_start);
 
 /* Online tuning of a mixed-form context's tiles and launch shape (no
    counterpart in the reference).  First the tiles, at the default launch
    shape: a batch's P2G tile (256 elements a block staging 1024 particles a
    pass, 128 staging 512, or 512 staging 1024; a single simulation runs the
-   fused P2G and grid update) with the G2P tile (256 or 128 particles).  Then,
+   first) with the G2P tile (256 or 128 particles).  Then,
    with the fastest tiles, the persistent G2P grid (1 up to as many blocks per
    SM as fit) and the steps per replayed CUDA graph (4, 8, 16).  Every
    candidate runs the simulation itself (a warm-up graph, then steps_per_trial

@@ -105,7 +105,7 @@ __global__ void nonlocal_bulk_kernel(int n, mat::NonlocalParams np, const double
 // them once, instead of per particle; the mass part stays per particle.  The
 // kernel is bound by the FP64 pipe (1/64 of the FP32 rate on GB300): products
 // run in integer arithmetic (mat::imul), sums with register operands, 34 -> 21
-// FP64 instructions a particle (835 996 particles: 76 -> 63 us).
+// FP64 instructions a particle (835 996 particles: 76 -> 65 us).
 __global__ void __launch_bounds__(128) assemble_kernel(
     int ne, int Ex, double inv_h, int dense_only, RowView rv, const double *__restrict__ xl, const double *__restrict__ yl,
     const double *__restrict__ v, const double *__restrict__ dense, const double *__restrict__ gfl,
