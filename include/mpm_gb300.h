@@ -393,7 +393,7 @@ MPMG_API int mpmg_measure_fp64_rate(int device, double *flops_per_s);
  * complete when the stream is.  num_elements must lie in [1, 2^30)
  * (MPMG_ERR_INVALID otherwise).
  *
- * Scratch is a fixed device array inside this library (about 19 MB), held by
+ * Scratch is a fixed device array inside this library (about 15 MB), held by
  * every GPU that loads it until the process exits; n above
  * MPMG_NOALLOC_MAX_PARTICLES is rejected with MPMG_ERR_SCRATCH_LIMIT.  The
  * first call on a device looks up that array's device address and keeps it

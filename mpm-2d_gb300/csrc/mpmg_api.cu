@@ -1303,7 +1303,7 @@ int mpmg_get_fields(mpmg_ctx *ctx, int count, const char *const *names, double *
         if (names[k] == nullptr || host_out[k] == nullptr) return MPMG_ERR_INVALID;
     MPMG_CHECK(cudaSetDevice(ctx->dev));
     // destinations the device writes itself (null: a copy); none where two of
-    // them overlap, so that the later field's values stay as they were
+    // them overlap: there the fields are read in turn, the later over the earlier
     std::vector<double *> dev(count > 0 ? count : 1, nullptr);
     std::vector<FieldRef> ref(count > 0 ? count : 1);
     std::vector<char> done(count > 0 ? count : 1, 0);
@@ -1332,6 +1332,11 @@ int mpmg_get_fields(mpmg_ctx *ctx, int count, const char *const *names, double *
     // every array's copy and the step record behind the steps, then one wait
     for (int k = 0; k < count; k++)
         if ((rc = find_field(ctx, names[k], &ref[k], false)) != MPMG_OK) return rc;
+    if (!apart) {
+        for (int k = 0; k < count; k++)
+            if ((rc = mpmg_get_field(ctx, names[k], host_out[k])) != MPMG_OK) return rc;
+        return MPMG_OK;
+    }
     MPMG_CHECK(cudaMemcpyAsync(ctx->h_record, ctx->d_params, step_record_bytes(ctx), cudaMemcpyDeviceToHost,
                                ctx->stream));
     FrameJobs jobs;
@@ -1339,7 +1344,7 @@ int mpmg_get_fields(mpmg_ctx *ctx, int count, const char *const *names, double *
     for (int k = 0; k < count; k++) {
         const size_t bytes = ref[k].count * sizeof(double);
         if (ref[k].kind != 0 || bytes == 0) continue;
-        if (apart) dev[k] = mpmg_device_view(host_out[k], bytes);
+        dev[k] = mpmg_device_view(host_out[k], bytes);
         if (dev[k] == nullptr) {
             if ((rc = mpmg_copy_out(ctx, host_out[k], ref[k].ptr, bytes)) != MPMG_OK) return rc;
             continue;

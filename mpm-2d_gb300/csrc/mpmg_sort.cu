@@ -213,11 +213,28 @@ __device__ __forceinline__ int lower_bound_warp(const uint32_t *__restrict__ key
     return lo;
 }
 
+// The first position in [lo, hi) whose key is >= e (hi if none), by one thread:
+// three probes a round.
+__device__ __forceinline__ int lower_bound_in(const uint32_t *__restrict__ keys, int lo, int hi, uint32_t e)
+{
+    while (lo < hi) {
+        const int q = (hi - lo) >> 2, a = lo + q, b = a + q, c = b + q;    // c < hi
+        const bool ka = keys[a] < e, kb = keys[b] < e, kc = keys[c] < e;
+        if (kc) lo = c + 1;
+        else if (kb) { lo = b + 1; hi = c; }
+        else if (ka) { lo = a + 1; hi = b; }
+        else hi = a;
+    }
+    return lo;
+}
+
 // cell_start[e] = first sorted position whose key is >= e, for e in [0, ne].  A
 // block of kStartElems elements finds its range of the sorted keys, and each
 // thread the first entries there of the elements between its key and the one
-// before.
+// before; or, where the range is long, each thread its element's by a search in
+// it (full elements: a few blocks would read nearly all of the keys).
 constexpr int kStartElems = 256;            // 1024: 125k keys of 40 000 elements 23.2 us instead of 19.4
+constexpr int kSweepKeys = 8 * kThreads;     // eight keys a thread, about a search's ten dependent loads
 
 __global__ void __launch_bounds__(kThreads) cell_start_kernel(const uint32_t *__restrict__ sorted_keys, int n, int ne,
                                                               int *__restrict__ cell_start)
@@ -228,11 +245,18 @@ __global__ void __launch_bounds__(kThreads) cell_start_kernel(const uint32_t *__
     const int w = threadIdx.x >> 5;
     mpmg_pdl_wait();
     if (w < 2) {
-        const int at = lower_bound_warp(sorted_keys, n, (uint32_t)(e0 + (w == 0 ? 0 : kStartElems)));
+        // up to the keys outside the grid, in the last block
+        const long long e = w == 0 ? e0 : e0 + kStartElems < ne ? e0 + kStartElems : ne;
+        const int at = lower_bound_warp(sorted_keys, n, (uint32_t)e);
         if ((threadIdx.x & 31) == 0) range[w] = at;
     }
     __syncthreads();
     const int lo = range[0], hi = range[1];
+    if (hi - lo > kSweepKeys) {
+        for (int t = threadIdx.x; t < kStartElems; t += kThreads)
+            if (e0 + t <= ne) cell_start[e0 + t] = lower_bound_in(sorted_keys, lo, hi, (uint32_t)(e0 + t));
+        return;
+    }
     for (int t = threadIdx.x; t < kStartElems; t += kThreads) first[t] = hi;
     __syncthreads();
     for (int i = lo + threadIdx.x; i < hi; i += kThreads) {
