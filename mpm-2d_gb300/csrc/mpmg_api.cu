@@ -106,8 +106,10 @@ int alloc_step_record(mpmg_ctx *ctx, int count)
 }
 
 // The element rows of the FP64 step: a row holds at least twice the mean
-// count of the filled elements (a power of two, 16 to 64), since a flow packs
-// elements unevenly; what a row cannot hold goes to the overflow list.
+// count of the filled elements (a power of two from 16), since a flow packs
+// elements unevenly; what a row cannot hold goes to the overflow list.  Rows
+// above 64 slots take no more memory than 128 slots a particle: a crowd on a
+// large empty grid goes through the list.
 int alloc_rows(mpmg_ctx *ctx, const int *emap, size_t n)
 {
     RowBins &r = ctx->row;
@@ -122,7 +124,8 @@ int alloc_rows(mpmg_ctx *ctx, const int *emap, size_t n)
         }
     }
     r.cap = 16;
-    while (r.cap < 64 && filled > 0 && (size_t)r.cap * filled < 2 * inside) r.cap *= 2;
+    while (filled > 0 && (size_t)r.cap * filled < 2 * inside && (r.cap < 64 || 2 * (size_t)r.cap * ctx->ne <= 128 * n))
+        r.cap *= 2;
     r.cur = 0;
     r.ready = false;
     r.record = false;

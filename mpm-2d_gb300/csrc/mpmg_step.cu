@@ -141,6 +141,87 @@ __global__ void __launch_bounds__(256) keys_kernel(GridGeom g, float inv_hf, int
 // element: 4 corners x (m, mx, my, h fx), then 4 x h fy.
 
 constexpr int kCell = 20;                  // doubles an element
+constexpr int kStage = 16;                 // staged row entries an element, at most a row's slots
+
+// Puts the lists of a block's elements with more than kStage particles in
+// ascending order, a warp to a list: by rank in registers up to 128 particles,
+// beyond by a bitonic network in place whose pairs past the end are left out
+// (all of its exchanges put the larger entry last).  A list longer than its row
+// is first gathered in over_list from the row and the overflow entries, and its
+// place left in row[0] and sh_base.  In a thread's insertion sort instead, the
+// random order of 64 entries took most of the P2G (1 048 576 particles, 64 to
+// an element: ORDERED us a step).
+__device__ __noinline__ void order_long_lists(RowView rv, int lists, const int *sh_elem, const int *sh_count,
+                                              uint32_t *sh_base, const uint32_t *n_over, const uint2 *over,
+                                              uint32_t *cursor)
+{
+    const unsigned all = 0xffffffffu;
+    const int lane = threadIdx.x & 31, warps = blockDim.x / 32;
+    for (int le = threadIdx.x / 32; le < lists; le += warps) {
+        const int cnt = sh_count[le], e = sh_elem[le];
+        if (cnt <= kStage) continue;
+        uint32_t *lst = rv.rows + (size_t)e * rv.cap;
+        if (cnt > rv.cap) {
+            uint32_t *row = lst, base = 0;
+            if (lane == 0) base = atomicAdd(cursor, (uint32_t)cnt);
+            base = __shfl_sync(all, base, 0);
+            lst = rv.over_list + base;
+            for (int j = lane; j < rv.cap; j += 32) lst[j] = row[j];
+            __syncwarp();
+            if (lane == 0) row[0] = sh_base[le] = base;
+            const int extra = (int)*n_over;
+            int have = rv.cap;
+#pragma unroll 4
+            for (int j = 0; j < extra; j += 32) {
+                const uint2 o = j + lane < extra ? over[j + lane] : make_uint2(0xffffffffu, 0u);
+                const bool mine = o.x == (uint32_t)e;
+                const unsigned who = __ballot_sync(all, mine);
+                if (mine) lst[have + __popc(who & ((1u << lane) - 1u))] = o.y;
+                have += __popc(who);
+            }
+            __syncwarp();
+        }
+        if (cnt <= 128) {
+            uint32_t q[4];
+            int rank[4] = {0, 0, 0, 0};
+#pragma unroll
+            for (int r = 0; r < 4; r++) q[r] = lane + 32 * r < cnt ? lst[lane + 32 * r] : 0xffffffffu;
+#pragma unroll
+            for (int b = 0; b < 4; b++) {
+                if (32 * b >= cnt) break;
+#pragma unroll 8
+                for (int k = 0; k < 32; k++) {
+                    const uint32_t w = __shfl_sync(all, q[b], k);
+#pragma unroll
+                    for (int r = 0; r < 4; r++) rank[r] += w < q[r] ? 1 : 0;
+                }
+            }
+            __syncwarp();
+#pragma unroll
+            for (int r = 0; r < 4; r++)
+                if (lane + 32 * r < cnt) lst[rank[r]] = q[r];
+        } else {
+            for (long long size = 2; size < 2ll * cnt; size *= 2) {
+                for (long long d = size / 2; d > 0; d /= 2) {
+                    const bool flip = d == size / 2;      // the first pass of a size pairs mirrored places
+                    for (long long i = lane;; i += 32) {
+                        const long long a0 = i / d * (2 * d), t = i % d, a = a0 + t;
+                        if (a >= cnt) break;
+                        const long long b = flip ? a0 + 2 * d - 1 - t : a + d;
+                        if (b >= cnt) continue;
+                        const uint32_t u = lst[a], w = lst[b];
+                        if (u > w) {
+                            lst[a] = w;
+                            lst[b] = u;
+                        }
+                    }
+                    __syncwarp();
+                }
+            }
+        }
+        __syncwarp();
+    }
+}
 
 template <int EB, int SPLIT>
 __global__ void __launch_bounds__(EB * SPLIT) p2g_cells_kernel(
@@ -153,7 +234,6 @@ __global__ void __launch_bounds__(EB * SPLIT) p2g_cells_kernel(
     double dt, int gravity_mode, double gravity_const, double *__restrict__ cell_sums)
 {
     constexpr int NB = 17;                 // count classes 0..15 and 16 or more
-    constexpr int kStage = 16;             // staged row entries an element
     constexpr int kSumStride = kCell + 1;
     __shared__ double sh_sum[EB * kSumStride];
     __shared__ uint32_t sh_idx[kStage * EB];
@@ -198,7 +278,10 @@ __global__ void __launch_bounds__(EB * SPLIT) p2g_cells_kernel(
         sh_elem[tid] = e0;
         sh_count[tid] = e0 >= 0 ? (int)rv.count[e0] : 0;
     }
-    __syncthreads();
+    if (__syncthreads_or(tid < EB && sh_count[tid] > kStage)) {
+        order_long_lists(rv, EB, sh_elem, sh_count, sh_base, n_over, over, cursor);
+        __syncthreads();
+    }
     constexpr int WB = EB / 32;            // warps an element set
     const int half = SPLIT == 2 ? tid / EB : 0;
     if (WB > 1) {
@@ -225,70 +308,32 @@ __global__ void __launch_bounds__(EB * SPLIT) p2g_cells_kernel(
     }
     const int cnt = sh_count[le], e = sh_elem[le];
     const uint32_t *list = nullptr;        // a long element's list in global memory
-    if (half == 0 && cnt > 0) {
+    if (half == 0 && cnt > 0 && cnt <= kStage) {
         uint32_t *row = rv.rows + (size_t)e * rv.cap;
-        if (cnt <= kStage && cnt <= rv.cap) {
-            // ascending particle index, as the reference's lists (insertion
-            // sort of a handful of entries in this thread's shared column)
-            uint32_t *col = sh_idx + le;
-            uint4 r4[kStage / 4];              // all of the row's loads in flight
+        // ascending particle index, as the reference's lists (insertion
+        // sort of a handful of entries in this thread's shared column)
+        uint32_t *col = sh_idx + le;
+        uint4 r4[kStage / 4];              // all of the row's loads in flight
 #pragma unroll
-            for (int j = 0; j < kStage / 4; j++)
-                if (4 * j < cnt) r4[j] = reinterpret_cast<const uint4 *>(row)[j];
+        for (int j = 0; j < kStage / 4; j++)
+            if (4 * j < cnt) r4[j] = reinterpret_cast<const uint4 *>(row)[j];
 #pragma unroll
-            for (int j = 0; j < kStage; j++) {
-                if (j >= cnt) break;
-                const uint4 v4 = r4[j / 4];
-                const uint32_t q = j % 4 == 0 ? v4.x : j % 4 == 1 ? v4.y : j % 4 == 2 ? v4.z : v4.w;
-                int t = j - 1;
-                while (t >= 0 && col[t * EB] > q) {
-                    col[(t + 1) * EB] = col[t * EB];
-                    t--;
-                }
-                col[(t + 1) * EB] = q;
+        for (int j = 0; j < kStage; j++) {
+            if (j >= cnt) break;
+            const uint4 v4 = r4[j / 4];
+            const uint32_t q = j % 4 == 0 ? v4.x : j % 4 == 1 ? v4.y : j % 4 == 2 ? v4.z : v4.w;
+            int t = j - 1;
+            while (t >= 0 && col[t * EB] > q) {
+                col[(t + 1) * EB] = col[t * EB];
+                t--;
             }
-            if (keep_order)
-                for (int j = 0; j < cnt; j++) row[j] = col[j * EB];
-        } else if (cnt <= rv.cap) {
-            for (int j = 1; j < cnt; j++) {
-                const uint32_t q = row[j];
-                int t = j - 1;
-                while (t >= 0 && row[t] > q) {
-                    row[t + 1] = row[t];
-                    t--;
-                }
-                row[t + 1] = q;
-            }
-        } else {
-            // more particles than the row holds: the row and the element's
-            // entries of the overflow list, ordered in over_list
-            const uint32_t base = atomicAdd(cursor, (uint32_t)cnt);
-            uint32_t *lst = rv.over_list + base;
-            int have = 0;
-            const int extra = (int)*n_over;
-            for (int j = 0; j < rv.cap + extra; j++) {
-                uint32_t q;
-                if (j < rv.cap) {
-                    q = row[j];
-                } else {
-                    const uint2 o = over[j - rv.cap];
-                    if (o.x != (uint32_t)e) continue;
-                    q = o.y;
-                }
-                int t = have - 1;
-                while (t >= 0 && lst[t] > q) {
-                    lst[t + 1] = lst[t];
-                    t--;
-                }
-                lst[t + 1] = q;
-                have++;
-            }
-            row[0] = base;
-            sh_base[le] = base;
+            col[(t + 1) * EB] = q;
         }
+        if (keep_order)
+            for (int j = 0; j < cnt; j++) row[j] = col[j * EB];
     }
     if (SPLIT == 2) __syncthreads();
-    if (cnt > kStage || cnt > rv.cap)
+    if (cnt > kStage)
         list = cnt <= rv.cap ? rv.rows + (size_t)e * rv.cap : rv.over_list + sh_base[le];
     const int ci = e % g.Ex, cj = e / g.Ex;
     const double cx = mat::small_int(ci), cy = mat::small_int(cj);   // the element's column and row (element.c:10-19)

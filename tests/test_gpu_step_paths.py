@@ -83,6 +83,28 @@ def test_fp64_step_paths_vs_oracle(case):
             assert field_err(sim.get(f), orc.get, f) <= 1e-10, (f, field_err(sim.get(f), orc.get, f))
 
 
+@pytest.mark.parametrize("ppc, crowds", [(2, (127, 128, 129)), (2, (256, 257, 1025)), (12, ()), (8, (900,))])
+def test_long_element_lists_vs_oracle(ppc, crowds):
+    """Elements whose lists whole warps order: up to 128 particles and beyond, in rows and past them."""
+    sc = scenes.box_fill(cells=9, ppc_1d=ppc, material="g_local_mu2", dt=1e-6)
+    rng = np.random.default_rng(6)
+    p = sc["particles"]
+    more = {k: [np.full(n, p[k][0]) for n in crowds] for k in p}
+    more["x"] = [(2 * j + rng.uniform(0, 1, n)) * sc["h"] for j, n in enumerate(crowds)]
+    more["y"] = [(3 + j + rng.uniform(0, 1, n)) * sc["h"] for j, n in enumerate(crowds)]
+    p = {k: np.concatenate([p[k]] + more[k]) for k in p}
+    mixed = rng.permutation(p["x"].size)
+    sc = stirred(dict(sc, particles={k: a[mixed] for k, a in p.items()}))
+    sim = mpm2d.Simulation(sc, store_transients=True)
+    orc = O.Oracle(sc, nthreads=4)
+    for _ in range(2):
+        sim.step(1)
+        orc.step(1)
+        np.testing.assert_array_equal(sim.get_map()[0], orc.get_map()[0])
+        for f in FIELDS + ("node_m", "node_mx", "node_my", "node_fx", "node_fy"):
+            assert field_err(sim.get(f), orc.get, f) <= 1e-10, (f, field_err(sim.get(f), orc.get, f))
+
+
 def small_grid(nx, ny, seed):
     h = 1.0 / 64
     n = 4 * (nx - 1) * (ny - 1)
