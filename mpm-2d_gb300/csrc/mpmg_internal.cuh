@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "../../include/mpm_gb300.h"
+#include "mpmg_tiles.h"
 
 #define MPMG_TOL 1e-10          // process_usl.c:25
 #define MPMG_NCOLORS 4
@@ -64,7 +65,7 @@ struct MixedState {
     float4 *A[2], *B[2], *C[2], *D[2];
     int cur;
     uint32_t *halo_perm;   // 3 x np scratch orders of oversized shared tile elements
-    uint2 *tile_map[3];    // batches: member and tile (row << 16 | column) of each P2G block, for each tile variant
+    MpmgTile *tile_map[3]; // batches: the tile of each P2G block, for each tile variant
     int tiles[3];          // P2G tiles of each variant
     int max_tiles;
     int *tile_zero;        // per P2G tile: its nodes are known to be zero

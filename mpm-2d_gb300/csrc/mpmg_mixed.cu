@@ -554,7 +554,7 @@ struct FusedTile {
 
 template <bool F64NODE, bool BATCH, int TX, int TY, int CHUNK>
 __global__ void __launch_bounds__(TX * TY, 1024 / (TX * TY)) mx_p2g_grid_kernel(
-    const __grid_constant__ MemberM m0, BatchView bv, const uint2 *__restrict__ tile_map,
+    const __grid_constant__ MemberM m0, BatchView bv, const MpmgTile *__restrict__ tile_map,
     int *__restrict__ tile_zero, int np,
     const int *__restrict__ cell_start,
     const uint32_t *__restrict__ slots, uint32_t *__restrict__ perm, uint32_t *__restrict__ rank,
@@ -580,17 +580,15 @@ __global__ void __launch_bounds__(TX * TY, 1024 / (TX * TY)) mx_p2g_grid_kernel(
 
     const int me = threadIdx.x, lane = me & 31, warp = me >> 5;
     // the block's member and tile: from the table, in one load
-    uint2 at = make_uint2(0, 0);
-    if (BATCH) at = tile_map[blockIdx.x];
+    uint4 at = make_uint4(0, 0, 0, 0);
+    if (BATCH) at = reinterpret_cast<const uint4 *>(tile_map)[blockIdx.x];
     const int zero = tile_zero[blockIdx.x];      // of this kernel's last launch
     const int member = BATCH ? (int)at.x : 0;
     const MemberM &M = BATCH ? bv.m[member] : m0;
     const int Ex = M.g.Ex, Ey = M.g.Ey, Nx = M.g.Nx, Ny = M.g.Ny;
-    if (!BATCH) {
-        const unsigned tiles_x = (unsigned)(Nx + TX - 2) / (TX - 1);
-        at.y = (blockIdx.x / tiles_x) << 16 | (blockIdx.x % tiles_x);
-    }
-    const int tx = (int)(at.y & 0xffffu), ty = (int)(at.y >> 16);
+    const MpmgTile tile = BATCH ? MpmgTile{at.x, at.y, at.z, 0}
+                                : mpmg_tile_at(0, blockIdx.x, mpmg_tiles_along((uint32_t)Nx, TX));
+    const int tx = (int)tile.col, ty = (int)tile.row;
     const int lx = me % TX, ly = me / TX;
     const int ei = tx * (TX - 1) - 1 + lx, ej = ty * (TY - 1) - 1 + ly;
     const bool exists = ei >= 0 && ej >= 0 && ei < Ex && ej < Ey;
@@ -1289,7 +1287,7 @@ size_t g2p_smem_size(int tile)
     return tile == 128 ? g2p_smem_bytes<128>() : g2p_smem_bytes<256>();
 }
 
-using P2GKernel = void (*)(MemberM, BatchView, const uint2 *, int *, int, const int *, const uint32_t *, uint32_t *,
+using P2GKernel = void (*)(MemberM, BatchView, const MpmgTile *, int *, int, const int *, const uint32_t *, uint32_t *,
                            uint32_t *, uint32_t *, Buf, const StepParams *, float, float2 *, float4 *, double *,
                            double *, double *, double *, double *);
 
@@ -1317,11 +1315,9 @@ size_t p2g_smem_size(int v)
 }
 
 // Tiles of a simulation with variant v.
-int p2g_tiles(const mpmg_config &c, int v, int *tiles_x, int *tiles_y)
+int p2g_tiles(const mpmg_config &c, int v)
 {
-    *tiles_x = (int)((c.Nx + kTileX[v] - 2) / (kTileX[v] - 1));
-    *tiles_y = (int)((c.Ny + kTileY[v] - 2) / (kTileY[v] - 1));
-    return *tiles_x * *tiles_y;
+    return (int)(mpmg_tiles_along((uint32_t)c.Nx, kTileX[v]) * mpmg_tiles_along((uint32_t)c.Ny, kTileY[v]));
 }
 
 }  // namespace
@@ -1382,25 +1378,18 @@ int mpmg_mixed_init(mpmg_ctx *ctx, const double *m, const double *v, const doubl
         if ((rc = dalloc(&bt->d_first, first.size())) != MPMG_OK) return rc;
         MPMG_CHECK(cudaMemcpy(bt->d_first, first.data(), first.size() * sizeof(int), cudaMemcpyHostToDevice));
         for (int v = 0; v < kP2GVariants; v++) {
-            std::vector<uint2> map;
-            for (int k = 0; k < count; k++) {
-                int nx, ny;
-                p2g_tiles(bt->cfg[k], v, &nx, &ny);
-                for (int j = 0; j < ny; j++)
-                    for (int i = 0; i < nx; i++) map.push_back(make_uint2((unsigned)k, (unsigned)j << 16 | (unsigned)i));
-            }
+            std::vector<MpmgTile> map;
+            for (int k = 0; k < count; k++)
+                mpmg_append_tiles(map, (uint32_t)k, (uint32_t)bt->cfg[k].Nx, (uint32_t)bt->cfg[k].Ny, kTileX[v], kTileY[v]);
             if ((rc = dalloc(&s->tile_map[v], map.size())) != MPMG_OK) return rc;
             s->tiles[v] = (int)map.size();
-            MPMG_CHECK(cudaMemcpy(s->tile_map[v], map.data(), map.size() * sizeof(uint2), cudaMemcpyHostToDevice));
+            MPMG_CHECK(cudaMemcpy(s->tile_map[v], map.data(), map.size() * sizeof(MpmgTile), cudaMemcpyHostToDevice));
         }
         MPMG_CHECK(cudaMemcpy(dm, hm.data(), count * sizeof(MemberM), cudaMemcpyHostToDevice));
         MPMG_CHECK(cudaMemcpy(bt->d_elem_off, eo.data(), (count + 1) * sizeof(int), cudaMemcpyHostToDevice));
     }
 
-    if (!bt) {
-        int nx, ny;
-        s->tiles[0] = p2g_tiles(ctx->cfg, 0, &nx, &ny);
-    }
+    if (!bt) s->tiles[0] = p2g_tiles(ctx->cfg, 0);
     s->max_tiles = s->tiles[0];
     for (int t : s->tiles) s->max_tiles = t > s->max_tiles ? t : s->max_tiles;
     if ((rc = dalloc(&s->tile_zero, s->max_tiles)) != MPMG_OK) return rc;
@@ -1538,7 +1527,7 @@ void mpmg_mixed_free(mpmg_ctx *ctx)
         cudaFree(s->D[b]);
     }
     cudaFree(s->halo_perm);
-    for (uint2 *t : s->tile_map) cudaFree(t);
+    for (MpmgTile *t : s->tile_map) cudaFree(t);
     cudaFree(s->tile_zero);
     cudaFree(s->node4);
     cudaFree(s->node_mass);
@@ -1594,7 +1583,7 @@ int mpmg_mixed_step(mpmg_ctx *ctx)
     mpmg_phase_begin(ctx, PH_P2G);
     const int v = batch ? s->p2g_variant : 0;
     MPMG_CHECK(mpmg_launch_pdl(true, p2g_variant(v, f64, batch), dim3(s->tiles[v]), dim3(kP2GElems[v]), p2g_smem_size(v),
-                               st, m0, bv, (const uint2 *)s->tile_map[v], s->tile_zero, n, (const int *)ctx->cell_start,
+                               st, m0, bv, (const MpmgTile *)s->tile_map[v], s->tile_zero, n, (const int *)ctx->cell_start,
                                (const uint32_t *)ctx->bin.slots, ctx->perm, ctx->bin.rank, s->halo_perm, S,
                                (const StepParams *)ctx->d_params, (float)MPMG_TOL, s->node_mass, s->node4,
                                ctx->node_mx, ctx->node_my, ctx->node_fx, ctx->node_fy, node_m64));
