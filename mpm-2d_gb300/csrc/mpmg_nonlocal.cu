@@ -19,6 +19,7 @@
 // stopping test is the same relative residual either way.
 #include "mpmg_internal.cuh"
 #include "mpmg_materials.cuh"
+#include "mpmg_mg_words.cuh"
 
 // Level table of the multigrid preconditioner (pcg_mg_kernel), built at
 // set-up: level l has Nx x Ny nodes, C of them per block; its node arrays
@@ -1413,28 +1414,6 @@ __device__ __forceinline__ void mg_totals4(const mat::Unit &u, const double *par
 #pragma unroll
     for (int c = 0; c < 4; c++) v[c] = scratch[4 * nt + c];
     __syncthreads();
-}
-
-// 2^e times an FP32 value (subnormals as zero) as a double, and 2^e times a
-// double rounded to FP32 (below FP32's normal range: zero), in integer
-// arithmetic: the conversion instructions run on the FP64 pipe.  Both are for
-// vectors of order one and |e| < 800.
-__device__ __forceinline__ double mg_wide(float f, int e)
-{
-    const unsigned b = __float_as_uint(f), m = b & 0x7fffffffu;
-    if (m < 0x00800000u) return 0.0;
-    return __hiloint2double((int)((b & 0x80000000u) | ((m >> 3) + ((unsigned)(896 + e) << 20))), (int)(b << 29));
-}
-
-__device__ __forceinline__ float mg_narrow(double x, int e)
-{
-    const long long b = __double_as_longlong(x);
-    const unsigned long long m = (unsigned long long)b & 0x7fffffffffffffffULL;
-    const int f = (int)(m >> 52) + e;       // exponent field, double's bias
-    if (f < 897 || f > 1150) return f > 1150 ? (float)x : 0.0f;
-    const unsigned long long r = (m + 0x0fffffffULL + ((m >> 29) & 1)) >> 29;   // to nearest even
-    return __uint_as_float((unsigned)((unsigned long long)b >> 32 & 0x80000000u) |
-                           ((unsigned)r + ((unsigned)(e - 896) << 23)));
 }
 
 // All-gather of the four per-block inner products of V-cycle `tag`: each block
