@@ -1059,8 +1059,6 @@ inline size_t pcg_tile_smem(int C, int Nx)
 // Where only neighbours read a vector (level 0's smoothing steps and result),
 // only the Nx + 1 nodes at either end of a block's range are published.
 
-constexpr int kMgThreads = 512;
-constexpr int kMgBlocks = 160;         // blocks of the solve at most (mg_gather4: five a lane)
 constexpr int kMgTrips = 4;            // nodes of a level a thread owns at most
 constexpr int kMgLocal = kMgTrips * kMgThreads;   // levels this small are held by block 0
 constexpr int kMgCoarse = 9;           // nodes of the coarsest level at most (3 x 3)
@@ -1076,115 +1074,6 @@ constexpr float cheb_rho(int k)
 }
 constexpr float cheb_a(int k) { return k == 0 ? 0.0f : cheb_rho(k) * cheb_rho(k - 1); }
 constexpr float cheb_b(int k) { return k == 0 ? 1.0f / kChebTheta : 2.0f * cheb_rho(k) / kChebDelta; }
-// polls of one wait before it gives up (a poll is one L2 round trip, about
-// a microsecond: a few seconds in all)
-constexpr long long kMgPollLimit = 1ll << 22;
-// sleep of a waiting warp between its rounds of loads (ns)
-constexpr unsigned kMgNap = 40;
-
-__device__ __forceinline__ unsigned long long mg_ld(const unsigned long long *p)
-{
-    unsigned long long v;
-    asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p));
-    return v;
-}
-
-__device__ __forceinline__ void mg_st(unsigned long long *p, float x, unsigned tag)
-{
-    const unsigned long long v = ((unsigned long long)tag << 32) | (unsigned long long)__float_as_uint(x);
-    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v));
-}
-
-// A word that needs no wait: value 0 with the current tag.
-__device__ __forceinline__ unsigned long long mg_zero(unsigned tag)
-{
-    return (unsigned long long)tag << 32;
-}
-
-__device__ __forceinline__ float mg_f(unsigned long long v)
-{
-    return __uint_as_float((unsigned)v);
-}
-
-__device__ __forceinline__ bool mg_give_up(long long polls, int *status)
-{
-    if ((polls & 15) != 0) return false;
-    if (polls > kMgPollLimit || (*(volatile int *)status & MPMG_DEV_ERR_SPIN) != 0) {
-        atomicOr(status, MPMG_DEV_ERR_SPIN);
-        return true;
-    }
-    return false;
-}
-
-// Waits until every word of v carries `tag` (addr(t, q) is the address of
-// word q of trip t, for T trips of Q words).  Called by whole warps.  While some
-// lane holds stale words, every lane loads its stale words again, kMgNap ns
-// after the last round: the staged phases wait for a thousand words a block at
-// most, so this floods nothing, and a word is in a register one round trip
-// after it is visible (one lane polling one word and the rest reloaded after
-// it cost a second round trip: 0.456 against 0.441 ms a step on the 130^2
-// silo).  Bounded (kMgPollLimit polls, or another block's timeout): then the
-// spin error is set and the words read 0.
-template <int T, int Q, class Addr>
-__device__ __forceinline__ void mg_resolve(unsigned long long (&v)[T][Q], unsigned tag, int *status, Addr addr)
-{
-    for (long long polls = 1;; polls++) {
-        bool stale = false;
-#pragma unroll
-        for (int t = 0; t < T; t++) {
-#pragma unroll
-            for (int q = 0; q < Q; q++) stale |= (unsigned)(v[t][q] >> 32) != tag;
-        }
-        if (!__any_sync(0xffffffffu, stale)) return;
-        if (mg_give_up(polls, status)) {
-#pragma unroll
-            for (int t = 0; t < T; t++) {
-#pragma unroll
-                for (int q = 0; q < Q; q++) v[t][q] = mg_zero(tag);
-            }
-            return;
-        }
-        __nanosleep(kMgNap);
-#pragma unroll
-        for (int t = 0; t < T; t++) {
-#pragma unroll
-            for (int q = 0; q < Q; q++) {
-                if ((unsigned)(v[t][q] >> 32) != tag) v[t][q] = mg_ld(addr(t, q));
-            }
-        }
-    }
-}
-
-// Copies the words of two node ranges of a level vector (nn nodes), [a0, a1)
-// to d0 and [b0, b1) to d1, as floats once they carry `tag`; nodes outside
-// the level read 0.  Called by the whole block; ends with a block barrier.
-__device__ __noinline__ void mg_stage(const unsigned long long *w, int nn, int a0, int a1, float *d0, int b0,
-                                         int b1, float *d1, unsigned tag, int *status)
-{
-    constexpr int T = 4;
-    const int na = max(a1 - a0, 0), nt = na + max(b1 - b0, 0);
-    for (int base = 0; base < nt; base += T * kMgThreads) {
-        unsigned long long v[T][1];
-#pragma unroll
-        for (int t = 0; t < T; t++) {
-            const int u = base + threadIdx.x + t * kMgThreads;
-            const int m = u < na ? a0 + u : b0 + (u - na);
-            v[t][0] = (u < nt && m >= 0 && m < nn) ? mg_ld(w + m) : mg_zero(tag);
-        }
-        mg_resolve(v, tag, status, [&](int t, int) {
-            const int u = base + threadIdx.x + t * kMgThreads;
-            return w + (u < na ? a0 + u : b0 + (u - na));
-        });
-#pragma unroll
-        for (int t = 0; t < T; t++) {
-            const int u = base + threadIdx.x + t * kMgThreads;
-            if (u < na) d0[u] = mg_f(v[t][0]);
-            else if (u < nt) d1[u - na] = mg_f(v[t][0]);
-        }
-    }
-    __syncthreads();
-}
-
 // Per-level arrays in shared memory (floats).  A level spread over the
 // blocks keeps its b, z1, res (C each) at lv.sm and its rows (coef[9][C],
 // l1inv[C]) at lv.smr (level 0: float 0).  A level held by block 0 keeps its
@@ -1406,54 +1295,6 @@ __device__ __forceinline__ void mg_totals4(const mat::Unit &u, const double *par
 #pragma unroll
         for (int q = 0; q < kMax; q++)
             if (32 * q < nblocks) x = u.add(x, p[q]);
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) x = u.add(x, __shfl_down_sync(0xffffffffu, x, off));
-        if (lane == 0) scratch[4 * nt + c] = x;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int c = 0; c < 4; c++) v[c] = scratch[4 * nt + c];
-    __syncthreads();
-}
-
-// All-gather of the four per-block inner products of V-cycle `tag`: each block
-// publishes its values as tagged words (a double as two), and warp c waits for
-// value c of every block and adds them in block order (lane l the blocks l,
-// l + 32, ..., then a shuffle tree).  A block goes on only when every block has
-// published, and every block publishes after its last read of the V-cycle's
-// words: this is the grid barrier between V-cycles too, in one round trip
-// instead of an arrival, a release and a read.  Two buffers, by the V-cycle's
-// parity: a block that runs ahead writes the next but one only after every
-// block has published, hence read, the one between.
-__device__ __forceinline__ void mg_gather4(const mat::Unit &u, unsigned long long *words, double v[4], int nblocks,
-                                           double *scratch, unsigned tag, int *status)
-{
-    const int nt = blockDim.x;
-    if (threadIdx.x < 4) {
-        const unsigned long long b = (unsigned long long)__double_as_longlong(
-            threadIdx.x == 0 ? v[0] : threadIdx.x == 1 ? v[1] : threadIdx.x == 2 ? v[2] : v[3]);
-        unsigned long long *w = words + 2 * ((size_t)threadIdx.x * nblocks + blockIdx.x);
-        const unsigned long long t = (unsigned long long)tag << 32;
-        asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(w), "l"(t | (b & 0xffffffffu)));
-        asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(w + 1), "l"(t | (b >> 32)));
-    }
-    if (threadIdx.x < 128) {
-        const int lane = threadIdx.x & 31, c = threadIdx.x >> 5;
-        constexpr int kMax = kMgBlocks / 32;
-        unsigned long long p[kMax][2];
-        const unsigned long long *base = words + 2 * (size_t)c * nblocks;
-#pragma unroll
-        for (int q = 0; q < kMax; q++) {
-            const int t = lane + 32 * q;
-#pragma unroll
-            for (int h = 0; h < 2; h++) p[q][h] = t < nblocks ? mg_ld(base + 2 * t + h) : mg_zero(tag);
-        }
-        mg_resolve(p, tag, status, [&](int q, int h) { return base + 2 * (lane + 32 * q) + h; });
-        double x = 0;
-#pragma unroll
-        for (int q = 0; q < kMax; q++)
-            if (32 * q < nblocks)
-                x = u.add(x, __longlong_as_double((long long)((p[q][1] << 32) | (p[q][0] & 0xffffffffu))));
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) x = u.add(x, __shfl_down_sync(0xffffffffu, x, off));
         if (lane == 0) scratch[4 * nt + c] = x;
@@ -1998,6 +1839,7 @@ __global__ void __launch_bounds__(kMgThreads, 1) pcg_mg_kernel(SolveArgs S, cons
     if (threadIdx.x == 0) {
         sh_unit[0] = mat::opaque(1.0);
         sh_unit[1] = mat::opaque(-0.0);
+        mg_gave_up() = 0;
     }
     __syncthreads();
     const mat::Unit u{sh_unit[0], sh_unit[1]};
@@ -2313,7 +2155,8 @@ __global__ void __launch_bounds__(kMgThreads, 1) pcg_mg_kernel(SolveArgs S, cons
         }
         __syncthreads();      // the scratch aliases the held levels' vectors (a held level 0's zf)
         mg_sum4(u, part, scratch);
-        mg_gather4(u, P.gather + (size_t)(v & 1) * 8 * nblocks, part, nblocks, scratch, tag, S.status);
+        // a wait that ran out: leave as at the barriers, x and the record untouched
+        if (!mg_gather4(u, P.gather + (size_t)(v & 1) * 8 * nblocks, part, nblocks, scratch, tag, S.status)) return;
         const double gn = part[0], dl = part[1], sg = part[2];
         rr = part[3];
         if (threadIdx.x == 0) {
@@ -2355,6 +2198,8 @@ __global__ void __launch_bounds__(kMgThreads, 1) pcg_mg_kernel(SolveArgs S, cons
         if (k < cnt) S.x[n0 + k] = x[t];
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
+        // a block that gave up on its wait has not written its part of x
+        if ((*(volatile int *)S.status & MPMG_DEV_ERR_SPIN) != 0) converged = false;
         S.sp->solve_iters = it;
         S.sp->solve_converged = converged ? 1 : 0;
         S.sp->solve_rel_resid = (bb > 0) ? sqrt(rr / bb) : 0.0;

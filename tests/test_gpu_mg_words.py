@@ -1,6 +1,8 @@
 """The multigrid solve's conversions between its FP32 V-cycle and the FP64 outer
 iteration (tests/cuda/mg_words_check.cu, built here with nvcc): exact for normal
-values, and infinities and NaN carried through."""
+values, and infinities and NaN carried through.  And its waits for other blocks'
+words: a wait that runs out (words that nothing writes, a poll limit of 1024)
+returns, sets the spin status, and no total of it passes for a converged one."""
 import ctypes as C
 import os
 import shutil
@@ -20,11 +22,12 @@ def words(tmp_path_factory):
     out = str(tmp_path_factory.mktemp("words") / "libmg_words_check.so")
     src = os.path.join(ROOT, "tests", "cuda", "mg_words_check.cu")
     subprocess.run([nvcc, "-gencode", "arch=compute_103a,code=sm_103a", "-O3", "-std=c++17",
-                    "--expt-relaxed-constexpr", "-I", os.path.join(ROOT, "include"), "-shared",
+                    "-DMPMG_MG_POLL_LIMIT=1024", "--expt-relaxed-constexpr", "-I", os.path.join(ROOT, "include"), "-shared",
                     "-Xcompiler", "-fPIC", "-o", out, src], check=True, capture_output=True)
     lib = C.CDLL(out)
     lib.widen.argtypes = [C.c_longlong, C.c_void_p, C.c_int, C.c_void_p]
     lib.narrow.argtypes = [C.c_longlong, C.c_void_p, C.c_int, C.c_void_p]
+    lib.wait_block.argtypes = [C.c_void_p, C.c_int, C.c_void_p, C.c_int, C.c_void_p, C.c_uint, C.c_void_p, C.c_void_p]
     return lib
 
 
@@ -66,3 +69,53 @@ def test_narrow_rounds_once_and_carries_non_finite(words, e):
     assert np.array_equal(np.isnan(got), np.isnan(x))
     ok = ~np.isnan(x)
     assert np.array_equal(got[ok], want[ok])
+
+
+SPIN = 4       # MPMG_DEV_ERR_SPIN
+
+
+def wait_block(words, nblocks, present, staged=0, staged_present=True, tag=77):
+    """One block's gather among nblocks; `present` of the others have published (value c of
+    block b: 100 c + b), the rest, and this one's own before it publishes, hold an older tag."""
+    import torch
+    w = np.zeros((4, nblocks, 2), dtype=np.uint64)
+    val = (100.0 * np.arange(4)[:, None] + np.arange(nblocks)[None, :]).view(np.uint64)
+    b = np.arange(nblocks)
+    tags = np.where((b > 0) & (b <= present), tag, tag - 1).astype(np.uint64)[None, :] << np.uint64(32)
+    w[:, :, 0] = tags | (val & np.uint64(0xffffffff))
+    w[:, :, 1] = tags | (val >> np.uint64(32))
+    s = np.arange(max(staged, 1)).astype(np.float32).view(np.uint32).astype(np.uint64)
+    s |= np.uint64((tag if staged_present else tag - 1) << 32)
+    dw, ds = (torch.as_tensor(a.view(np.int64).ravel(), device="cuda") for a in (w, s))
+    floats = torch.zeros(max(staged, 1), dtype=torch.float32, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    out = torch.zeros(5, dtype=torch.float64, device="cuda")
+    assert words.wait_block(dw.data_ptr(), nblocks, ds.data_ptr(), staged, floats.data_ptr(), tag, status.data_ptr(),
+                            out.data_ptr()) == 0
+    out = out.cpu().numpy()
+    return out[:4], bool(out[4]), int(status.item()), floats.cpu().numpy()
+
+
+@pytest.mark.parametrize("nblocks", [1, 2, 33, 152, 160])
+def test_gather_sums_every_block(words, nblocks):
+    total, ok, status, floats = wait_block(words, nblocks, nblocks - 1, staged=50)
+    others = np.arange(1, nblocks)
+    want = [1.0 + c + np.sum(100.0 * c + others) for c in range(4)]     # whole numbers: any order
+    assert ok and status == 0 and np.array_equal(total, want)
+    assert np.array_equal(floats, np.arange(50))
+
+
+@pytest.mark.parametrize("nblocks,present", [(2, 0), (33, 31), (160, 0)])
+def test_gather_that_runs_out_is_no_result(words, nblocks, present):
+    total, ok, status, _ = wait_block(words, nblocks, present)
+    assert not ok and status == SPIN
+    assert np.isnan(total).all()
+
+
+@pytest.mark.parametrize("nblocks", [1, 152])
+def test_stage_that_runs_out_never_converges(words, nblocks):
+    """The words read NaN, and the residual this block publishes is NaN, though every
+    block's word arrives."""
+    total, ok, status, floats = wait_block(words, nblocks, nblocks - 1, staged=50, staged_present=False)
+    assert ok and status == SPIN
+    assert np.isnan(floats).all() and np.isnan(total[3])
