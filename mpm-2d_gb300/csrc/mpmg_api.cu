@@ -324,6 +324,21 @@ void mpmg_phase_end(mpmg_ctx *ctx, int phase)
     if (ctx->timing) cudaEventRecord(ctx->ev[2 * phase + 1], ctx->stream);
 }
 
+int mpmg_dalloc_all(std::initializer_list<MpmgPiece> pieces)
+{
+    size_t bytes = 0;
+    const bool ok = mpmg_alloc_all(
+        pieces.begin(), pieces.size(),
+        [&](void **p, size_t n) {
+            bytes = n;
+            return cudaMalloc(p, n) == cudaSuccess;
+        },
+        [](void *p) { cudaFree(p); });
+    if (ok) return MPMG_OK;
+    mpmg_set_error("cudaMalloc of %zu bytes failed: %s", bytes, cudaGetErrorString(cudaGetLastError()));
+    return MPMG_ERR_NOMEM;
+}
+
 // The device address of host memory that the device may write over all of its
 // `bytes` bytes: pinned memory of this process whose allocation covers them.
 // Null otherwise (and where the driver does not tell).

@@ -262,15 +262,20 @@ int mpmg_bin_init(mpmg_ctx *ctx)
     const size_t groups = (ctx->np + 31) / 32;
     const size_t m = ctx->ne + (groups ? groups : 1);
     const size_t tiles = (m + kScanTile - 1) / kScanTile;
-    MPMG_CHECK(cudaMalloc(&ctx->bin.counts, m * sizeof(uint32_t)));
-    MPMG_CHECK(cudaMalloc(&ctx->bin.cursor, m * sizeof(uint32_t)));
-    MPMG_CHECK(cudaMalloc(&ctx->bin.tile_state, (tiles ? tiles : 1) * sizeof(unsigned long long) + 16));
-    MPMG_CHECK(cudaMalloc(&ctx->bin.slots, (ctx->np ? ctx->np : 1) * sizeof(uint32_t)));
-    MPMG_CHECK(cudaMalloc(&ctx->bin.rank, (ctx->np ? ctx->np : 1) * sizeof(uint32_t)));
-    MPMG_CHECK(cudaMemsetAsync(ctx->bin.counts, 0, m * sizeof(uint32_t), ctx->stream));
+    const size_t state_bytes = (tiles ? tiles : 1) * sizeof(unsigned long long) + 16;
+    int rc = mpmg_dalloc_all({{(void **)&ctx->bin.counts, m * sizeof(uint32_t)},
+                              {(void **)&ctx->bin.cursor, m * sizeof(uint32_t)},
+                              {(void **)&ctx->bin.tile_state, state_bytes},
+                              {(void **)&ctx->bin.slots, ctx->np * sizeof(uint32_t)},
+                              {(void **)&ctx->bin.rank, ctx->np * sizeof(uint32_t)}});
+    if (rc != MPMG_OK) return rc;
+    cudaError_t e = cudaMemsetAsync(ctx->bin.counts, 0, m * sizeof(uint32_t), ctx->stream);
     // tile states, ticket and epoch start at zero (no tile published)
-    MPMG_CHECK(cudaMemsetAsync(ctx->bin.tile_state, 0, (tiles ? tiles : 1) * sizeof(unsigned long long) + 16,
-                               ctx->stream));
+    if (e == cudaSuccess) e = cudaMemsetAsync(ctx->bin.tile_state, 0, state_bytes, ctx->stream);
+    if (e != cudaSuccess) {
+        mpmg_bin_free(ctx);
+        return mpmg_cuda_status(e, "binning arrays");
+    }
     ctx->bin.bins = (int)m;
     ctx->bin.tiles = (int)tiles;
     return MPMG_OK;

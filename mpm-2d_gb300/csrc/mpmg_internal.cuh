@@ -8,9 +8,11 @@
 #include <stdint.h>
 #include <string.h>
 
+#include <initializer_list>
 #include <vector>
 
 #include "../../include/mpm_gb300.h"
+#include "mpmg_alloc.h"
 #include "mpmg_tiles.h"
 
 #define MPMG_TOL 1e-10          // process_usl.c:25
@@ -272,6 +274,8 @@ static inline float mpmg_bits_float(int i)
 // Error helpers (host).
 void mpmg_set_error(const char *fmt, ...);
 int mpmg_cuda_status(cudaError_t e, const char *what);
+// Device arrays, all or none (mpmg_alloc.h); MPMG_ERR_NOMEM leaves no CUDA error behind.
+int mpmg_dalloc_all(std::initializer_list<MpmgPiece> pieces);
 
 #define MPMG_CHECK(call)                                          \
     do {                                                          \

@@ -1276,10 +1276,13 @@ int mpmg_fp64_sort(mpmg_ctx *ctx)
 {
     const int n = (int)ctx->np, ne = (int)ctx->ne;
     cudaStream_t s = ctx->stream;
-    if (ctx->bin.counts == nullptr) {
+    if (ctx->sort_keys == nullptr) {
         int rc = mpmg_bin_init(ctx);
-        if (rc != MPMG_OK) return rc;
-        MPMG_CHECK(cudaMalloc(&ctx->sort_keys, (ctx->np ? ctx->np : 1) * sizeof(uint32_t)));
+        if (rc == MPMG_OK) rc = mpmg_dalloc_all({{(void **)&ctx->sort_keys, ctx->np * sizeof(uint32_t)}});
+        if (rc != MPMG_OK) {
+            mpmg_bin_free(ctx);       // a later call starts over
+            return rc;
+        }
     }
     map_keys_kernel<<<blocks_for(n, 256), 256, 0, s>>>(n, ctx->in_element, ctx->active, (uint32_t)ne, ctx->sort_keys);
     int rc = mpmg_bin_count(ctx, ctx->sort_keys);
