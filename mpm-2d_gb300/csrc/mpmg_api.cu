@@ -371,6 +371,27 @@ double *mpmg_device_view(const void *p, size_t bytes)
     return d >= begin && d + bytes <= begin + size ? (double *)at.devicePointer : nullptr;
 }
 
+namespace {
+
+// The two pinned chunks and their events, made on first need; false where the
+// host has no pinned memory left.
+bool out_stage(mpmg_ctx *ctx, size_t chunk)
+{
+    if (ctx->out_stage != nullptr) return true;
+    bool ok = true;
+    for (cudaEvent_t &e : ctx->out_event)
+        ok = ok && (e != nullptr || cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess);
+    void *stage = nullptr;
+    if (ok && cudaMallocHost(&stage, 2 * chunk) == cudaSuccess) {
+        ctx->out_stage = (unsigned char *)stage;      // last: it says that all three are there
+        return true;
+    }
+    cudaGetLastError();
+    return false;
+}
+
+}  // namespace
+
 // Device memory to pageable host memory, after the stream's work: chunks through
 // two pinned buffers, one filling while the host copies the other out.  The
 // driver's own copy into pages fresh from the allocator took 170 us for 512 KB
@@ -382,16 +403,10 @@ int mpmg_copy_out(mpmg_ctx *ctx, void *dst, const void *src, size_t bytes)
     cudaPointerAttributes at;
     const bool known = cudaPointerGetAttributes(&at, dst) == cudaSuccess;
     if (!known) cudaGetLastError();
-    if (!known || at.type != cudaMemoryTypeUnregistered) {
+    if (!known || at.type != cudaMemoryTypeUnregistered || !out_stage(ctx, kChunk)) {
         MPMG_CHECK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
         MPMG_CHECK(cudaStreamSynchronize(ctx->stream));
         return MPMG_OK;
-    }
-    if (ctx->out_stage == nullptr) {
-        void *stage = nullptr;
-        MPMG_CHECK(cudaMallocHost(&stage, 2 * kChunk));
-        ctx->out_stage = (unsigned char *)stage;
-        for (cudaEvent_t &e : ctx->out_event) MPMG_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
     const size_t chunks = (bytes + kChunk - 1) / kChunk;
     for (size_t c = 0; c <= chunks; c++) {
