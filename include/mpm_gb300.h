@@ -192,7 +192,10 @@ MPMG_API int mpmg_synchronize(mpmg_ctx *ctx);
    particle order, node fields in node-number order).  Particle fields: x y v
    v0 m vx vy ax ay bx by sxx sxy syy ux uy exx exy eyy wxy xl yl Txx Txy Tyx
    Tyy Tzz state0..state10.  Node fields: node_m node_mx node_my node_fx
-   node_fy node_vx node_vy node_ax node_ay node_gf. */
+   node_fy node_vx node_vy node_ax node_ay node_gf.
+   Several host threads may read one context at once (mpmg_get_field,
+   mpmg_get_fields, mpmg_get_sort, mpmg_adj_state), while none steps or changes
+   it; other calls on a context come one at a time. */
 MPMG_API int mpmg_get_field(mpmg_ctx *ctx, const char *name, double *host_out);
 /* Reads count fields at once, behind the steps and with one wait: a whole
    output frame, as the driver's write_frame

@@ -400,6 +400,7 @@ int mpmg_copy_out(mpmg_ctx *ctx, void *dst, const void *src, size_t bytes)
 {
     constexpr size_t kChunk = 1 << 20;
     if (bytes == 0) return MPMG_OK;
+    std::lock_guard<std::recursive_mutex> lock(ctx->read_lock);   // the chunks are the context's
     cudaPointerAttributes at;
     const bool known = cudaPointerGetAttributes(&at, dst) == cudaSuccess;
     if (!known) cudaGetLastError();
@@ -1462,6 +1463,7 @@ int mpmg_get_sort(mpmg_ctx *ctx, int *sorted_keys, int *perm, int *cell_start)
 {
     if (ctx == nullptr) return MPMG_ERR_INVALID;
     MPMG_CHECK(cudaSetDevice(ctx->dev));
+    std::lock_guard<std::recursive_mutex> lock(ctx->read_lock);   // one sort at a time, until it is read
     if (!ctx->mixed) {
         // the FP64 step bins into element rows; the sort is formed here from
         // the last step's element map

@@ -9,6 +9,7 @@
 #include <string.h>
 
 #include <initializer_list>
+#include <mutex>
 #include <vector>
 
 #include "../../include/mpm_gb300.h"
@@ -175,6 +176,7 @@ struct mpmg_ctx {
     uint32_t *sort_keys;   // input of mpmg_fp64_sort
     unsigned char *out_stage;   // pinned, 2 MB: mpmg_copy_out
     cudaEvent_t out_event[2];
+    std::recursive_mutex read_lock;   // held by a read that goes through the context's own buffers
     int sms;
 
     // Cell sort.

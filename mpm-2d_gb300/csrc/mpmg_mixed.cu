@@ -1823,6 +1823,7 @@ int frame_get(mpmg_ctx *ctx, const char *name, double *out)
     ExportFields F = {};
     if (!add_export(ctx, name, s->export_buf, F)) return MPMG_ERR_UNKNOWN_FIELD;
     if (n == 0) return MPMG_OK;
+    std::lock_guard<std::recursive_mutex> lock(ctx->read_lock);   // export_buf, until it is read
     const int rc = launch_export(ctx, F);
     if (rc != MPMG_OK) return rc;
     return mpmg_copy_out(ctx, out, s->export_buf, n * sizeof(double));
