@@ -105,31 +105,18 @@ int alloc_step_record(mpmg_ctx *ctx, int count)
     return MPMG_OK;
 }
 
-// The element rows of the FP64 step: a row holds at least twice the mean
-// count of the filled elements (a power of two from 16), since a flow packs
-// elements unevenly; what a row cannot hold goes to the overflow list.  Rows
-// above 64 slots take no more memory than 128 slots a particle: a crowd on a
-// large empty grid goes through the list.
+// The element rows of the FP64 step (mpmg_rows.h); what a row cannot hold goes
+// to the overflow list.
 int alloc_rows(mpmg_ctx *ctx, const int *emap, size_t n)
 {
     RowBins &r = ctx->row;
-    std::vector<bool> seen(ctx->ne, false);
-    size_t filled = 0, inside = 0;
-    for (size_t i = 0; i < n; i++) {
-        if (emap[i] < 0) continue;
-        inside++;
-        if (!seen[emap[i]]) {
-            seen[emap[i]] = true;
-            filled++;
-        }
+    if (!mpmg_row_width(emap, n, ctx->ne, &r.cap, &r.filled0)) {
+        mpmg_set_error("no host memory for the element map of %zu elements", ctx->ne);
+        return MPMG_ERR_NOMEM;
     }
-    r.cap = 16;
-    while (filled > 0 && (size_t)r.cap * filled < 2 * inside && (r.cap < 64 || 2 * (size_t)r.cap * ctx->ne <= 128 * n))
-        r.cap *= 2;
     r.cur = 0;
     r.ready = false;
     r.record = false;
-    r.filled0 = filled;
     int rc = dalloc(&r.n_over, 5);
     r.n_filled = r.n_over + 2;
     r.cursor = r.n_over + 4;

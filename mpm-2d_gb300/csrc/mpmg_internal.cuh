@@ -14,6 +14,7 @@
 
 #include "../../include/mpm_gb300.h"
 #include "mpmg_alloc.h"
+#include "mpmg_rows.h"
 #include "mpmg_tiles.h"
 
 #define MPMG_TOL 1e-10          // process_usl.c:25
