@@ -105,8 +105,7 @@ int alloc_step_record(mpmg_ctx *ctx, int count)
     return MPMG_OK;
 }
 
-// The element rows of the FP64 step (mpmg_rows.h); what a row cannot hold goes
-// to the overflow list.
+// The element rows of the FP64 step (mpmg_rows.h).
 int alloc_rows(mpmg_ctx *ctx, const int *emap, size_t n)
 {
     RowBins &r = ctx->row;
@@ -117,14 +116,14 @@ int alloc_rows(mpmg_ctx *ctx, const int *emap, size_t n)
     r.cur = 0;
     r.ready = false;
     r.record = false;
-    int rc = dalloc(&r.n_over, 5);
-    r.n_filled = r.n_over + 2;
-    r.cursor = r.n_over + 4;
+    int rc = dalloc(&r.n_filled, 3);
+    r.cursor = r.n_filled + 2;
     if (rc == MPMG_OK) rc = dalloc(&r.over_list, n);
+    if (rc == MPMG_OK) rc = dalloc(&r.head, ctx->ne);
+    if (rc == MPMG_OK) rc = dalloc(&r.next, n);
     for (int b = 0; b < 2 && rc == MPMG_OK; b++) {
         rc = dalloc(&r.count[b], ctx->ne);
         if (rc == MPMG_OK) rc = dalloc(&r.rows[b], ctx->ne * (size_t)r.cap);
-        if (rc == MPMG_OK) rc = dalloc(&r.over[b], n);
         if (rc == MPMG_OK) rc = dalloc(&r.filled[b], std::min(ctx->ne, n));
     }
     return rc;
@@ -553,10 +552,11 @@ int mpmg_destroy(mpmg_ctx *ctx)
     for (int b = 0; b < 2; b++) {
         cudaFree(ctx->row.count[b]);
         cudaFree(ctx->row.rows[b]);
-        cudaFree(ctx->row.over[b]);
         cudaFree(ctx->row.filled[b]);
     }
-    cudaFree(ctx->row.n_over);   // the counters, one block
+    cudaFree(ctx->row.n_filled);   // the counters, one block
+    cudaFree(ctx->row.head);
+    cudaFree(ctx->row.next);
     cudaFree(ctx->row.over_list);
     cudaFree(ctx->elem_coef);
     cudaFree(ctx->sort_keys);

@@ -114,22 +114,28 @@ struct BinScratch {
 
 // Element rows of the FP64 step (mpmg_step.cu): each element has a row of
 // `cap` slots for its particles' indices, filled in any order with a counter
-// per element; what does not fit goes to an overflow list of (element, index)
-// pairs.  A list names the elements that hold particles, in any order.  Two
+// per element; what does not fit is chained from the element's head through
+// next[particle], count - cap links long (so neither array is ever cleared).  A
+// list names the elements that hold particles, in any order.  Two
 // buffers: while a step works on buffer `cur`, its G2P already
-// bins the moved particles into the other one for the next step.  `ready`
+// bins the moved particles into the other one for the next step; the chains
+// need one, since the P2G has followed them by then.  `ready`
 // says that buffer cur holds the current positions' elements; setting x, y or
 // the element map from outside clears it, and the next step then bins first.
+// cap and filled0 are those of the initial positions, whatever becomes of them.
+// Chains cost a thread an element about what its sums cost it: particles set
+// from 4 to 64 an element, 1 048 576 of them: 354 us a step, 327 where they were
+// created so (and 156 000 with one overflow list that each element searched).
 struct RowBins {
     int cap;
     uint32_t *count[2];    // ne
     uint32_t *rows[2];     // ne x cap
-    uint2 *over[2];        // n
     uint32_t *filled[2];   // min(ne, n): the elements with particles
-    uint32_t *n_over;      // entries in over[0], over[1]
     uint32_t *n_filled;    // entries in filled[0], filled[1]
     uint32_t *cursor;      // entries taken from over_list
     size_t filled0;        // filled elements of the initial positions
+    uint32_t *head;        // ne
+    uint32_t *next;        // n
     uint32_t *over_list;   // n: the ordered lists of elements with more than cap particles
     int cur;
     bool ready;

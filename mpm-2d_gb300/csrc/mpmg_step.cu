@@ -58,8 +58,7 @@ inline int early_launch(const mpmg_ctx *ctx)
 // rows
 
 struct RowsOut {
-    uint32_t *count, *rows, *filled, *n_filled, *n_over;
-    uint2 *over;
+    uint32_t *count, *rows, *filled, *n_filled, *head, *next;
     int cap;
 };
 
@@ -94,7 +93,7 @@ __device__ __forceinline__ void bin_particle(const RowsOut &R, int i, uint32_t k
     if (!valid) return;
     const uint32_t slot = base + (uint32_t)(lane - leader);
     if (slot < (uint32_t)R.cap) R.rows[(size_t)key * R.cap + slot] = (uint32_t)i;
-    else R.over[atomicAdd(R.n_over, 1u)] = make_uint2(key, (uint32_t)i);
+    else R.next[i] = atomicExch(&R.head[key], (uint32_t)i);
 }
 
 // The rows of the current positions, where no G2P has left them: keys[i] is
@@ -147,39 +146,37 @@ constexpr int kStage = 16;                 // staged row entries an element, at 
 // ascending order, a warp to a list: by rank in registers up to 128 particles,
 // beyond by a bitonic network in place whose pairs past the end are left out
 // (all of its exchanges put the larger entry last).  A list longer than its row
-// is first gathered in over_list from the row and the overflow entries, and its
-// place left in row[0] and sh_base.  In a thread's insertion sort instead, the
-// random order of 64 entries took most of the P2G (1 048 576 particles, 64 to
-// an element: 2118 -> 328 us a step).
+// is first gathered in over_list from the row and its chain, a thread to a
+// chain, and its place left in row[0] and sh_base.  In a thread's insertion sort
+// instead, the random order of 64 entries took most of the P2G (1 048 576
+// particles, 64 to an element: 2118 -> 328 us a step).  Called by the whole block.
 __device__ __noinline__ void order_long_lists(RowView rv, int lists, const int *sh_elem, const int *sh_count,
-                                              uint32_t *sh_base, const uint32_t *n_over, const uint2 *over,
+                                              uint32_t *sh_base, const uint32_t *head, const uint32_t *next,
                                               uint32_t *cursor)
 {
     const unsigned all = 0xffffffffu;
     const int lane = threadIdx.x & 31, warps = blockDim.x / 32;
+    if ((int)threadIdx.x < lists && sh_count[threadIdx.x] > rv.cap) {
+        const int cnt = sh_count[threadIdx.x], e = sh_elem[threadIdx.x];
+        const uint32_t base = atomicAdd(cursor, (uint32_t)cnt);
+        sh_base[threadIdx.x] = base;
+        uint32_t i = head[e];
+        for (int j = rv.cap; j < cnt; j++) {
+            rv.over_list[base + j] = i;
+            if (j + 1 < cnt) i = next[i];      // the first one's has no meaning
+        }
+    }
+    __syncthreads();
     for (int le = threadIdx.x / 32; le < lists; le += warps) {
         const int cnt = sh_count[le], e = sh_elem[le];
         if (cnt <= kStage) continue;
         uint32_t *lst = rv.rows + (size_t)e * rv.cap;
         if (cnt > rv.cap) {
-            uint32_t *row = lst, base = 0;
-            if (lane == 0) base = atomicAdd(cursor, (uint32_t)cnt);
-            base = __shfl_sync(all, base, 0);
-            lst = rv.over_list + base;
+            uint32_t *row = lst;
+            lst = rv.over_list + sh_base[le];
             for (int j = lane; j < rv.cap; j += 32) lst[j] = row[j];
             __syncwarp();
-            if (lane == 0) row[0] = sh_base[le] = base;
-            const int extra = (int)*n_over;
-            int have = rv.cap;
-#pragma unroll 4
-            for (int j = 0; j < extra; j += 32) {
-                const uint2 o = j + lane < extra ? over[j + lane] : make_uint2(0xffffffffu, 0u);
-                const bool mine = o.x == (uint32_t)e;
-                const unsigned who = __ballot_sync(all, mine);
-                if (mine) lst[have + __popc(who & ((1u << lane) - 1u))] = o.y;
-                have += __popc(who);
-            }
-            __syncwarp();
+            if (lane == 0) row[0] = sh_base[le];
         }
         if (cnt <= 128) {
             uint32_t q[4];
@@ -226,7 +223,7 @@ __device__ __noinline__ void order_long_lists(RowView rv, int lists, const int *
 template <int EB, int SPLIT>
 __global__ void __launch_bounds__(EB * SPLIT) p2g_cells_kernel(
     GridGeom g, RowView rv, const uint32_t *__restrict__ filled, const uint32_t *__restrict__ n_filled,
-    const uint32_t *__restrict__ n_over, const uint2 *__restrict__ over, uint32_t *__restrict__ cursor,
+    const uint32_t *__restrict__ head, const uint32_t *__restrict__ next, uint32_t *__restrict__ cursor,
     int keep_order, int early, const double *__restrict__ x, const double *__restrict__ y,
     const double *__restrict__ m,
     const double *__restrict__ vx, const double *__restrict__ vy, const double *__restrict__ v,
@@ -279,7 +276,7 @@ __global__ void __launch_bounds__(EB * SPLIT) p2g_cells_kernel(
         sh_count[tid] = e0 >= 0 ? (int)rv.count[e0] : 0;
     }
     if (__syncthreads_or(tid < EB && sh_count[tid] > kStage)) {
-        order_long_lists(rv, EB, sh_elem, sh_count, sh_base, n_over, over, cursor);
+        order_long_lists(rv, EB, sh_elem, sh_count, sh_base, head, next, cursor);
         __syncthreads();
     }
     constexpr int WB = EB / 32;            // warps an element set
@@ -463,7 +460,7 @@ __device__ __forceinline__ int c_corner(int c, int i, int j)
 
 __global__ void __launch_bounds__(kGridTX * kGridTY) grid_kernel(
     GridGeom g, BcParams bc, int tiles_x, const uint32_t *__restrict__ count, uint32_t *__restrict__ count_next,
-    uint32_t *__restrict__ n_over_next, uint32_t *__restrict__ n_filled_next, uint32_t *__restrict__ cursor,
+    uint32_t *__restrict__ n_filled_next, uint32_t *__restrict__ cursor,
     const double *__restrict__ cell_sums, const StepParams *__restrict__ sp, double dt,
     double *__restrict__ node_m, double *__restrict__ node_ax, double *__restrict__ node_ay,
     double *__restrict__ node_vx, double *__restrict__ node_vy, double *__restrict__ node_mx,
@@ -507,7 +504,7 @@ __global__ void __launch_bounds__(kGridTX * kGridTY) grid_kernel(
     const mat::Unit u{sh_const[0], sh_const[1]};
     // the next step's rows start empty (the G2P fills them)
     if (own && i < g.Ex && j < g.Ey) count_next[j * g.Ex + i] = 0;
-    if (blockIdx.x == 0 && threadIdx.x == 0) *n_over_next = *n_filled_next = *cursor = 0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *n_filled_next = *cursor = 0;
     double ax = 0, ay = 0, vxn = 0, vyn = 0;
     double m = 0, mx = 0, my = 0, fx = 0, fy = 0;
     if (node && (src[0] || src[1] || src[2] || src[3])) {
@@ -603,7 +600,7 @@ cudaError_t launch_grid(mpmg_ctx *ctx, const GridGeom &g)
     const int tiles_x = (g.Nx + kGridTX - 2) / (kGridTX - 1), tiles_y = (g.Ny + kGridTY - 2) / (kGridTY - 1);
     return mpmg_launch_pdl(true, grid_kernel, dim3(tiles_x * tiles_y), dim3(kGridTX * kGridTY), 0, ctx->stream, g,
                            make_bc(ctx), tiles_x, (const uint32_t *)r.count[r.cur], r.count[1 - r.cur],
-                           r.n_over + (1 - r.cur), r.n_filled + (1 - r.cur), r.cursor, (const double *)ctx->cell_sums,
+                           r.n_filled + (1 - r.cur), r.cursor, (const double *)ctx->cell_sums,
                            (const StepParams *)ctx->d_params, ctx->cfg.dt,
                            ctx->node_m, ctx->node_ax, ctx->node_ay, ctx->node_vx, ctx->node_vy, ctx->node_mx,
                            ctx->node_my, ctx->node_fx, ctx->node_fy, (double2 *)ctx->elem_coef, early_launch(ctx));
@@ -1129,7 +1126,7 @@ __global__ void __launch_bounds__(128) order_kernel(int ne, const int *__restric
 RowsOut rows_out(const mpmg_ctx *ctx, int b)
 {
     const RowBins &r = ctx->row;
-    return RowsOut{r.count[b], r.rows[b], r.filled[b], r.n_filled + b, r.n_over + b, r.over[b], r.cap};
+    return RowsOut{r.count[b], r.rows[b], r.filled[b], r.n_filled + b, r.head, r.next, r.cap};
 }
 
 RowView row_view(const mpmg_ctx *ctx)
@@ -1248,8 +1245,8 @@ static cudaError_t launch_p2g(mpmg_ctx *ctx, const GridGeom &g, bool keep_order)
     const size_t most = ctx->np < ctx->ne ? ctx->np : ctx->ne;
     return mpmg_launch_pdl(true, p2g_cells_kernel<EB, SPLIT>, dim3(blocks_for(most, EB)), dim3(EB * SPLIT), 0,
                            ctx->stream, g, row_view(ctx), (const uint32_t *)r.filled[r.cur],
-                           (const uint32_t *)(r.n_filled + r.cur), (const uint32_t *)(r.n_over + r.cur),
-                           (const uint2 *)r.over[r.cur], r.cursor, keep_order ? 1 : 0, early_launch(ctx),
+                           (const uint32_t *)(r.n_filled + r.cur), (const uint32_t *)r.head,
+                           (const uint32_t *)r.next, r.cursor, keep_order ? 1 : 0, early_launch(ctx),
                            (const double *)ctx->x, (const double *)ctx->y, (const double *)ctx->m, (const double *)ctx->vx,
                            (const double *)ctx->vy, (const double *)ctx->v, (const double *)ctx->sxx,
                            (const double *)ctx->sxy, (const double *)ctx->syy, ctx->d_params, c.dt, c.gravity_mode,
@@ -1263,7 +1260,7 @@ int mpmg_fp64_ready(mpmg_ctx *ctx)
     cudaStream_t s = ctx->stream;
     const int n = (int)ctx->np;
     MPMG_CHECK(cudaMemsetAsync(r.count[r.cur], 0, ctx->ne * sizeof(uint32_t), s));
-    MPMG_CHECK(cudaMemsetAsync(r.n_over, 0, 5 * sizeof(uint32_t), s));
+    MPMG_CHECK(cudaMemsetAsync(r.n_filled, 0, 3 * sizeof(uint32_t), s));
     keys_kernel<<<blocks_for(n, 256), 256, 0, s>>>(make_geom(ctx), (float)ctx->inv_h, n, ctx->x, ctx->y, ctx->active,
                                                    ctx->keys, (uint32_t)ctx->ne, rows_out(ctx, r.cur));
     ctx->launches += 1;
