@@ -8,9 +8,10 @@
 // Slots a row and filled elements for the initial element map emap[n] (-1:
 // outside the grid) of ne elements.  A row holds at least twice the mean count
 // of the filled elements (a power of two from 16), since a flow packs elements
-// unevenly.  Rows above 64 slots take no more memory than 128 slots a particle:
-// a crowd on a large empty grid goes beyond its rows.  False without the memory
-// to count (a bit an element).
+// unevenly.  Rows above 16 slots have no more than 128 slots a particle in all:
+// a crowd on a large empty grid goes beyond its rows (64 slots on 4096^2 elements
+// are 8.6 GB in the two buffers, 16 are 2.1).  False without the memory to count
+// (a bit an element).
 inline bool mpmg_row_width(const int *emap, size_t n, size_t ne, int *cap, size_t *filled)
 {
     constexpr size_t bits = CHAR_BIT * sizeof(unsigned long);
@@ -30,7 +31,6 @@ inline bool mpmg_row_width(const int *emap, size_t n, size_t ne, int *cap, size_
     }
     delete[] seen;
     *cap = 16;
-    while (*filled > 0 && (size_t)*cap * *filled < 2 * inside && (*cap < 64 || 2 * (size_t)*cap * ne <= 128 * n))
-        *cap *= 2;
+    while (*filled > 0 && (size_t)*cap * *filled < 2 * inside && 2 * (size_t)*cap * ne <= 128 * n) *cap *= 2;
     return true;
 }

@@ -50,3 +50,14 @@ def test_width_and_filled(rows, ne, ppc):
 def test_no_host_memory_is_reported(rows):
     assert width(rows, [0, 1, 1, -1], 4, no_memory=1)[0] == 1
     assert width(rows, [0, 1, 1, -1], 4) == (0, 16, 2)
+
+
+@pytest.mark.parametrize("ppc", [16, 64, 1000])
+def test_crowd_on_a_large_grid_takes_narrow_rows(rows, ppc):
+    """Rows above 16 slots: 128 slots a particle at most, in each of two buffers."""
+    ne = 1 << 22
+    for crowded in (16, 4096):
+        emap = np.repeat(np.arange(crowded) * 7, ppc)
+        rc, cap, filled = width(rows, emap, ne)
+        assert rc == 0 and filled == crowded
+        assert cap == 16 or cap * ne <= 128 * emap.size
