@@ -1804,11 +1804,13 @@ __device__ void mg_vcycle(const MgPlan &P, float *sm, const double *cinv, unsign
 // Shared memory of pcg_mg_kernel (the offsets are in the plan): level 0's
 // rows, the spread levels' vectors, the held levels' rows, level 0's own
 // V-cycle results, the held levels' vectors (at least the reduction
-// scratch), then doubles: the outer vectors r and w, the coarsest inverse
-// and the elimination matrix.
+// scratch), then doubles: the outer vectors r and w and the coarsest inverse
+// (its elimination matrix is in the reduction scratch: a grid of 521^2 nodes, the
+// largest square one, comes within a kilobyte of a block's shared memory).
 inline size_t pcg_mg_smem(const MgPlan &P)
 {
-    const size_t doubles = 2 * (size_t)P.lv[0].C + kMgCoarse * kMgCoarse + 2 * kMgCoarse * kMgCoarse;
+    const size_t doubles = 2 * (size_t)P.lv[0].C + kMgCoarse * kMgCoarse;
+    static_assert(2 * kMgCoarse * kMgCoarse <= 4 * kMgThreads, "the elimination matrix");
     return (size_t)P.sm_fp64 * sizeof(float) + doubles * sizeof(double);
 }
 
@@ -1854,7 +1856,7 @@ __global__ void __launch_bounds__(kMgThreads, 1) pcg_mg_kernel(SolveArgs S, cons
     double *dv = reinterpret_cast<double *>(sm + P.sm_fp64);
     double *r = dv, *w = r + L0.C;                    // outer residual and A u
     double *cinv = w + L0.C;                          // kMgCoarse^2
-    double *gj = cinv + kMgCoarse * kMgCoarse;        // kMgCoarse x 2 kMgCoarse (coarsest inverse)
+    double *gj = scratch;                             // kMgCoarse x 2 kMgCoarse (coarsest inverse)
     __shared__ double sh_scalar[5];
     __shared__ int sh_next;
     unsigned int episode = 0;
