@@ -202,7 +202,7 @@ MPMG_API int mpmg_get_field(mpmg_ctx *ctx, const char *name, double *host_out);
    (src/writer.c:190-201, called from src/main.c:957) reads the particles'
    m v x y x_t y_t sxx sxy syy ux uy state[9] state[10].  host_out[k]
    receives names[k].  Pinned destinations are written by the device in one
-   launch; pageable ones are copied one by one through pinned chunks. */
+   launch; pageable ones are copied one by one. */
 MPMG_API int mpmg_get_fields(mpmg_ctx *ctx, int count, const char *const *names, double *const *host_out);
 
 /* The driver's output files.  mpmg_write_frame writes one write_frame block

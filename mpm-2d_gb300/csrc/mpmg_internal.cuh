@@ -181,8 +181,6 @@ struct mpmg_ctx {
     RowBins row;
     double *elem_coef;
     uint32_t *sort_keys;   // input of mpmg_fp64_sort
-    unsigned char *out_stage;   // pinned, 2 MB: mpmg_copy_out
-    cudaEvent_t out_event[2];
     std::recursive_mutex read_lock;   // held by a read that goes through the context's own buffers
     int sms;
 
