@@ -1769,6 +1769,28 @@ __global__ void __launch_bounds__(256) mx_export_kernel(
     }
 }
 
+// One field into device memory: a thread takes a stored particle and scatters
+// its value (32 bytes read a particle and one launch, where the export above
+// reads 84 in two: a read of one field of 1 048 576 particles 97 -> 84 us).
+__global__ void __launch_bounds__(256) mx_export_one_kernel(int n, const float4 *__restrict__ rec, int comp,
+                                                            const float4 *__restrict__ D, const int *__restrict__ cell,
+                                                            int xy, const __grid_constant__ MemberM m0, BatchView bv,
+                                                            int ne, double *__restrict__ out)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const float4 r = rec[i];
+    double o = (double)(comp == 0 ? r.x : comp == 1 ? r.y : comp == 2 ? r.z : r.w);
+    const int c = xy != 0 ? cell[i] : ne;
+    if (c < ne) {
+        const MemberM &M = bv.count > 1 ? bv.m[element_member(bv, c)] : m0;
+        const int lc = c - M.e0;
+        const int cj = (int)mpmg_div((uint32_t)lc, M.g.div_Ex), ci = lc - cj * M.g.Ex;
+        o = ((double)(xy == 1 ? ci : cj) + o) * M.g.h;
+    }
+    out[__float_as_int(D[i].z)] = o;
+}
+
 // Adds the particle field `name` to the list; false where the records do not hold it.
 bool add_export(mpmg_ctx *ctx, const char *name, double *out, ExportFields &F)
 {
@@ -1824,8 +1846,12 @@ int frame_get(mpmg_ctx *ctx, const char *name, double *out)
     if (!add_export(ctx, name, s->export_buf, F)) return MPMG_ERR_UNKNOWN_FIELD;
     if (n == 0) return MPMG_OK;
     std::lock_guard<std::recursive_mutex> lock(ctx->read_lock);   // export_buf, until it is read
-    const int rc = launch_export(ctx, F);
-    if (rc != MPMG_OK) return rc;
+    const int b = s->cur, slot = F.slot[0];
+    mx_export_one_kernel<<<blocks_for(n, 256), 256, 0, ctx->stream>>>(
+        (int)n, record(s, b, slot >> 2), slot & 3, s->D[b], cell_array(ctx, b), F.xy[0],
+        make_member(ctx->batch ? ctx->batch->cfg[0] : ctx->cfg, 0, 0), batch_view(ctx), (int)ctx->ne, s->export_buf);
+    ctx->launches += 1;
+    MPMG_CHECK(cudaGetLastError());
     return mpmg_copy_out(ctx, out, s->export_buf, n * sizeof(double));
 }
 

@@ -47,3 +47,20 @@ def test_reads_into_fresh_and_partly_mapped_pages():
     fresh = np.frombuffer(mmap.mmap(-1, 8 * sim.n + 8), dtype=np.float64)[1:]   # no page of it mapped
     np.testing.assert_array_equal(sim.get_frame(["x"], out={"x": fresh})["x"], want)
     sim.close()
+
+
+def test_a_mixed_field_is_one_launch():
+    """No permutation formed for a single field, and the values of the frame export (bit for bit)."""
+    for members in (None, 3):
+        sc = scenes.box_fill(cells=40, material="g_local_mu2")
+        sim = mpm2d.Simulation(sc, precision="mixed") if members is None else mpm2d.Batch([sc] * members)
+        sim.step(3)
+        sim.synchronize()
+        names = ["x", "y", "vx", "syy", "v", "Tzz"]
+        out = {k: torch.zeros(sim.n, dtype=torch.float64, pin_memory=True).numpy() for k in names}
+        frame = sim.get_frame(names, out=out)
+        for k in names:
+            before = sim.launch_count()
+            np.testing.assert_array_equal(sim.get(k), frame[k])
+            assert sim.launch_count() - before == 1
+        sim.close()
