@@ -107,28 +107,29 @@ int alloc_step_record(mpmg_ctx *ctx, int count)
     return MPMG_OK;
 }
 
-// The element rows of the FP64 step (mpmg_rows.h).
-int alloc_rows(mpmg_ctx *ctx, const int *emap, size_t n)
+// The element rows of the FP64 step (mpmg_rows.h), in one allocation.
+int alloc_rows(mpmg_ctx *ctx, const MpmgFilled &count, size_t n)
 {
     RowBins &r = ctx->row;
-    if (!mpmg_row_width(emap, n, ctx->ne, &r.cap, &r.filled0)) {
-        mpmg_set_error("no host memory for the element map of %zu elements", ctx->ne);
-        return MPMG_ERR_NOMEM;
-    }
+    r.filled0 = count.filled();
+    r.cap = mpmg_row_slots(count.inside, r.filled0, n, ctx->ne);
     r.cur = 0;
     r.ready = false;
     r.record = false;
-    int rc = dalloc(&r.n_filled, 3);
-    r.cursor = r.n_filled + 2;
-    if (rc == MPMG_OK) rc = dalloc(&r.over_list, n);
-    if (rc == MPMG_OK) rc = dalloc(&r.head, ctx->ne);
-    if (rc == MPMG_OK) rc = dalloc(&r.next, n);
-    for (int b = 0; b < 2 && rc == MPMG_OK; b++) {
-        rc = dalloc(&r.count[b], ctx->ne);
-        if (rc == MPMG_OK) rc = dalloc(&r.rows[b], ctx->ne * (size_t)r.cap);
-        if (rc == MPMG_OK) rc = dalloc(&r.filled[b], std::min(ctx->ne, n));
+    const size_t ne = ctx->ne, most = std::min(ne, n), row_words = ne * (size_t)r.cap;
+    const struct { uint32_t **p; size_t words; } parts[] = {
+        {&r.rows[0], row_words}, {&r.rows[1], row_words}, {&r.count[0], ne}, {&r.count[1], ne}, {&r.head, ne},
+        {&r.filled[0], most}, {&r.filled[1], most}, {&r.next, n}, {&r.over_list, n}, {&r.n_filled, 2}, {&r.cursor, 1}};
+    size_t words = 0;
+    for (auto &q : parts) words += (q.words + 63) & ~(size_t)63;
+    const int rc = dalloc(&r.block, words);
+    if (rc != MPMG_OK) return rc;
+    uint32_t *at = r.block;
+    for (auto &q : parts) {
+        *q.p = at;
+        at += (q.words + 63) & ~(size_t)63;
     }
-    return rc;
+    return MPMG_OK;
 }
 
 // The step parameters and the status word of a read-back step record: the
@@ -530,15 +531,7 @@ int mpmg_destroy(mpmg_ctx *ctx)
         if (ctx->ring_ev[k]) cudaEventDestroy(ctx->ring_ev[k]);
     }
     if (ctx->rring_h) cudaFreeHost(ctx->rring_h);
-    for (int b = 0; b < 2; b++) {
-        cudaFree(ctx->row.count[b]);
-        cudaFree(ctx->row.rows[b]);
-        cudaFree(ctx->row.filled[b]);
-    }
-    cudaFree(ctx->row.n_filled);   // the counters, one block
-    cudaFree(ctx->row.head);
-    cudaFree(ctx->row.next);
-    cudaFree(ctx->row.over_list);
+    cudaFree(ctx->row.block);
     cudaFree(ctx->elem_coef);
     cudaFree(ctx->sort_keys);
     mpmg_bin_free(ctx);
@@ -811,7 +804,9 @@ int mpmg_create(const mpmg_config *cfg, size_t n, const double *m, const double 
         // Initial element map (process_usl.c:236-244) on the host copy of x, y.
         int *emap = new (std::nothrow) int[n > 0 ? n : 1];
         int *act = new (std::nothrow) int[n > 0 ? n : 1];
-        if (emap == nullptr || act == nullptr) {
+        MpmgFilled count;
+        if (emap == nullptr || act == nullptr || !count.begin(ctx->ne)) {
+            mpmg_set_error("no host memory for the element map");
             delete[] emap;
             delete[] act;
             rc = MPMG_ERR_NOMEM;
@@ -826,8 +821,9 @@ int mpmg_create(const mpmg_config *cfg, size_t n, const double *m, const double 
             }
             emap[i] = e;
             act[i] = e < 0 ? 0 : 1;
+            count.add(e);
         }
-        rc = alloc_rows(ctx, emap, n);
+        rc = alloc_rows(ctx, count, n);
         cudaError_t ce = cudaMemcpy(ctx->in_element, emap, n * sizeof(int), cudaMemcpyHostToDevice);
         if (ce == cudaSuccess) ce = cudaMemcpy(ctx->active, act, n * sizeof(int), cudaMemcpyHostToDevice);
         delete[] emap;

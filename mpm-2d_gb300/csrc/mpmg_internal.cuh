@@ -127,6 +127,7 @@ struct BinScratch {
 // from 4 to 64 an element, 1 048 576 of them: 354 us a step, 327 where they were
 // created so (and 156 000 with one overflow list that each element searched).
 struct RowBins {
+    uint32_t *block;       // the one allocation that holds the arrays
     int cap;
     uint32_t *count[2];    // ne
     uint32_t *rows[2];     // ne x cap

@@ -1260,7 +1260,8 @@ int mpmg_fp64_ready(mpmg_ctx *ctx)
     cudaStream_t s = ctx->stream;
     const int n = (int)ctx->np;
     MPMG_CHECK(cudaMemsetAsync(r.count[r.cur], 0, ctx->ne * sizeof(uint32_t), s));
-    MPMG_CHECK(cudaMemsetAsync(r.n_filled, 0, 3 * sizeof(uint32_t), s));
+    MPMG_CHECK(cudaMemsetAsync(r.n_filled, 0, 2 * sizeof(uint32_t), s));
+    MPMG_CHECK(cudaMemsetAsync(r.cursor, 0, sizeof(uint32_t), s));
     keys_kernel<<<blocks_for(n, 256), 256, 0, s>>>(make_geom(ctx), (float)ctx->inv_h, n, ctx->x, ctx->y, ctx->active,
                                                    ctx->keys, (uint32_t)ctx->ne, rows_out(ctx, r.cur));
     ctx->launches += 1;

@@ -1,5 +1,5 @@
-// Test-only: mpmg_row_width (mpmg_rows.h), with a non-throwing operator new[]
-// that can be made to fail.  Built by tests/test_rows.py with g++ into a
+// Test-only: MpmgFilled and mpmg_row_slots (mpmg_rows.h), with a non-throwing
+// operator new[] that can be made to fail.  Built by tests/test_rows.py with g++ into a
 // temporary shared library.
 #include <stdlib.h>
 
@@ -24,7 +24,12 @@ void operator delete[](void *p, size_t) noexcept
 extern "C" int row_width(const int *emap, size_t n, size_t ne, int no_memory, int *cap, size_t *filled)
 {
     out_of_memory = no_memory != 0;
-    const bool ok = mpmg_row_width(emap, n, ne, cap, filled);
+    MpmgFilled count;
+    const bool ok = count.begin(ne);
     out_of_memory = false;
-    return ok ? 0 : 1;
+    if (!ok) return 1;
+    for (size_t i = 0; i < n; i++) count.add(emap[i]);
+    *filled = count.filled();
+    *cap = mpmg_row_slots(count.inside, *filled, n, ne);
+    return 0;
 }
