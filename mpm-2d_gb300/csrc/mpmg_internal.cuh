@@ -583,19 +583,47 @@ __device__ __forceinline__ bool mpmg_mbar_wait(uint64_t *bar, uint32_t parity, l
     return false;
 }
 
+// a[0..n) in ascending order, in place (heap sort).
+static __device__ __noinline__ void mpmg_heap_sort(uint32_t *a, int n)
+{
+    for (int start = n / 2, end = n; end > 1;) {
+        uint32_t x;
+        if (start > 0) {
+            x = a[--start];               // the heap grows down to the front
+        } else {
+            x = a[--end];                 // the largest goes behind it
+            a[end] = a[0];
+        }
+        int hole = start;
+        for (int child = 2 * hole + 1; child < end; child = 2 * hole + 1) {
+            if (child + 1 < end && a[child + 1] > a[child]) child++;
+            if (a[child] <= x) break;
+            a[hole] = a[child];
+            hole = child;
+        }
+        a[hole] = x;
+    }
+}
+
 // perm[k0..k1) = slots[k0..k1) in ascending order (insertion sort: elements
-// hold a handful of particles), and rank[perm[k]] = k when rank is given.
+// hold a handful of particles; beyond 128 a heap sort, since the scatter of a
+// crowded element is in no order), and rank[perm[k]] = k when rank is given.
 __device__ __forceinline__ void mpmg_order_segment(const uint32_t *__restrict__ slots, uint32_t *__restrict__ perm,
                                                    uint32_t *__restrict__ rank, int k0, int k1)
 {
-    for (int j = k0; j < k1; j++) {
-        const uint32_t x = slots[j];
-        int i = j - 1;
-        while (i >= k0 && perm[i] > x) {
-            perm[i + 1] = perm[i];
-            i--;
+    if (k1 - k0 > 128) {
+        for (int j = k0; j < k1; j++) perm[j] = slots[j];
+        mpmg_heap_sort(perm + k0, k1 - k0);
+    } else {
+        for (int j = k0; j < k1; j++) {
+            const uint32_t x = slots[j];
+            int i = j - 1;
+            while (i >= k0 && perm[i] > x) {
+                perm[i + 1] = perm[i];
+                i--;
+            }
+            perm[i + 1] = x;
         }
-        perm[i + 1] = x;
     }
     if (rank != nullptr)
         for (int j = k0; j < k1; j++) rank[perm[j]] = (uint32_t)j;
