@@ -533,7 +533,9 @@ int mpmg_destroy(mpmg_ctx *ctx)
     if (ctx->rring_h) cudaFreeHost(ctx->rring_h);
     cudaFree(ctx->row.block);
     cudaFree(ctx->elem_coef);
-    cudaFree(ctx->sort_keys);
+    for (uint32_t *p : {ctx->sort_scratch.keys, ctx->sort_scratch.keys_alt, ctx->sort_scratch.vals_alt,
+                        ctx->sort_scratch.tile_hist, ctx->sort_scratch.digit_total, ctx->sort_keys})
+        cudaFree(p);
     mpmg_bin_free(ctx);
     mpmg_nonlocal_free(ctx);
     mpmg_mixed_free(ctx);

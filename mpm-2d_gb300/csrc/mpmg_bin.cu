@@ -204,8 +204,7 @@ constexpr int kScatterGroups = 4;
 
 __global__ void __launch_bounds__(256) scatter_kernel(const uint32_t *__restrict__ keys, int n, uint32_t sentinel,
                                                       uint32_t *__restrict__ cursor, uint32_t *__restrict__ slots,
-                                                      uint32_t *__restrict__ perm, uint32_t *__restrict__ rank,
-                                                      uint32_t *__restrict__ sorted_keys)
+                                                      uint32_t *__restrict__ perm, uint32_t *__restrict__ rank)
 {
     const int lane = threadIdx.x & 31;
     const uint32_t lt = (1u << lane) - 1u;
@@ -246,11 +245,9 @@ __global__ void __launch_bounds__(256) scatter_kernel(const uint32_t *__restrict
             const uint32_t pos = cursor[sentinel + group] + __popc(outside[j] & lt);
             perm[pos] = (uint32_t)k;      // final: storage order within the group's run
             rank[k] = pos;
-            if (sorted_keys != nullptr) sorted_keys[pos] = key[j];
         } else if (key[j] < sentinel) {
             const uint32_t pos = b + (uint32_t)(lane - leader);
             slots[pos] = (uint32_t)k;
-            if (sorted_keys != nullptr) sorted_keys[pos] = key[j];
         }
     }
 }
@@ -315,23 +312,23 @@ int mpmg_bin_reset(mpmg_ctx *ctx)
 
 // Scan of the counted bins and scatter of keys[n]: cell_start[ne + 1],
 // perm and rank for keys outside the grid, bin.slots (unordered within each
-// element) for the rest, and sorted_keys[n] unless it is null.
-int mpmg_bin_scan_scatter(mpmg_ctx *ctx, const uint32_t *keys, uint32_t *sorted_keys, bool pdl)
+// element) for the rest.  Both launch before their predecessors have finished.
+int mpmg_bin_scan_scatter(mpmg_ctx *ctx, const uint32_t *keys)
 {
     cudaStream_t s = ctx->stream;
     const int n = (int)ctx->np;
     const int m = ctx->bin.bins;
     const int tiles = ctx->bin.tiles;
     unsigned int *ticket_epoch = (unsigned int *)(ctx->bin.tile_state + tiles);
-    MPMG_CHECK(mpmg_launch_pdl(pdl, scan_kernel, dim3(tiles), dim3(kScanThreads), 0, s, ctx->bin.counts, m,
+    MPMG_CHECK(mpmg_launch_pdl(true, scan_kernel, dim3(tiles), dim3(kScanThreads), 0, s, ctx->bin.counts, m,
                                (int)ctx->ne, ctx->bin.tile_state, ticket_epoch, ctx->cell_start, ctx->bin.cursor,
                                ctx->d_status));
     ctx->launches += 1;
     if (n > 0) {
         const int keys_per_block = 256 * kScatterGroups;
-        MPMG_CHECK(mpmg_launch_pdl(pdl, scatter_kernel, dim3((n + keys_per_block - 1) / keys_per_block), dim3(256),
+        MPMG_CHECK(mpmg_launch_pdl(true, scatter_kernel, dim3((n + keys_per_block - 1) / keys_per_block), dim3(256),
                                    0, s, keys, n, (uint32_t)ctx->ne, ctx->bin.cursor, ctx->bin.slots, ctx->perm,
-                                   ctx->bin.rank, sorted_keys));
+                                   ctx->bin.rank));
         ctx->launches += 1;
     }
     MPMG_CHECK(cudaGetLastError());

@@ -181,7 +181,8 @@ struct mpmg_ctx {
     // the nodal acceleration and velocity (16 doubles, mpmg_step.cu).
     RowBins row;
     double *elem_coef;
-    uint32_t *sort_keys;   // input of mpmg_fp64_sort
+    uint32_t *sort_keys;   // input of mpmg_fp64_sort, allocated last
+    SortScratch sort_scratch;
     std::recursive_mutex read_lock;   // held by a read that goes through the context's own buffers
     int sms;
 
@@ -306,11 +307,11 @@ int mpmg_bin_init(mpmg_ctx *ctx);
 void mpmg_bin_free(mpmg_ctx *ctx);
 // Stand-alone count of keys[n] (<= ne) into the bins.
 int mpmg_bin_count(mpmg_ctx *ctx, const uint32_t *keys);
-// Scan of the counted bins and scatter: cell_start, sorted_keys (unless
-// null), and perm for keys outside the grid; element slots stay unordered in
-// bin.slots until a P2G kernel orders them into perm (mpmg_order_segment).
+// Scan of the counted bins and scatter: cell_start, and perm for keys outside
+// the grid; element slots stay unordered in bin.slots until a P2G kernel orders
+// them into perm (mpmg_order_segment).
 // mpmg_bin_reset restores the look-back state after a timed-out wait.
-int mpmg_bin_scan_scatter(mpmg_ctx *ctx, const uint32_t *keys, uint32_t *sorted_keys, bool pdl = false);
+int mpmg_bin_scan_scatter(mpmg_ctx *ctx, const uint32_t *keys);
 int mpmg_bin_reset(mpmg_ctx *ctx);
 int mpmg_nonlocal_init(mpmg_ctx *ctx);
 void mpmg_nonlocal_free(mpmg_ctx *ctx);

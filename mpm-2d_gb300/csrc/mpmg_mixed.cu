@@ -1572,7 +1572,7 @@ int mpmg_mixed_step(mpmg_ctx *ctx)
     const int cur = s->cur, nxt = 1 - cur;
 
     mpmg_phase_begin(ctx, PH_SORT);
-    int rc = mpmg_bin_scan_scatter(ctx, (const uint32_t *)cell_array(ctx, cur), nullptr, true);
+    int rc = mpmg_bin_scan_scatter(ctx, (const uint32_t *)cell_array(ctx, cur));
     if (rc != MPMG_OK) return rc;
     mpmg_phase_end(ctx, PH_SORT);
 

@@ -1,8 +1,8 @@
 // Stable LSD radix sort of (element key, particle index) pairs, and the
 // per-element start offsets of the sorted order.  The allocation-free entry
-// point (mpmg_sort_noalloc.cu) runs it on its fixed scratch; the step bins
-// particles with the counting sort of mpmg_bin.cu, which gives the same
-// order.
+// point (mpmg_sort_noalloc.cu) runs it on its fixed scratch, mpmg_get_sort of
+// the FP64 form on the context's; the mixed step bins particles with the
+// counting sort of mpmg_bin.cu, which gives the same order.
 //
 // The reference groups particles by element in find_filled_elements
 // (libmpm/process_usl.c:677-723): for each element, its particles in
