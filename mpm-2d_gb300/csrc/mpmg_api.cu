@@ -1226,7 +1226,7 @@ int mpmg_autotune(mpmg_ctx *ctx, int steps_per_trial, mpmg_tuning *best)
     best->default_ms_per_step = default_ms;
     best->candidates = tried;
     best->steps_advanced = advanced;
-    if (ctx->batch) mpmg_mixed_p2g_shape(best_pv, &best->p2g_elements, &best->p2g_stage);
+    if (ctx->batch) mpmg_mixed_p2g_shape(ctx, best_pv, &best->p2g_elements, &best->p2g_stage);
     best->g2p_tile = best_tile;
     return rc;
 }

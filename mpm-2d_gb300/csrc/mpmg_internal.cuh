@@ -80,6 +80,7 @@ struct MixedState {
     int sms;
     int g2p_tile;          // particles a G2P tile (256 or 128)
     int p2g_variant;       // a batch's P2G tile (kP2GElems / kP2GStage index)
+    int p2g_default;       // the shape that stands for variant 0
     double *export_buf;    // one FP64 particle field in caller order, for read-back
     uint32_t *inverse;     // stored position of each of the caller's particles, for read-back
     float4 *nl_T, *nl_F;   // g_nonlocal_mu2: trial stress and bulk fluidity per stored particle
@@ -329,7 +330,7 @@ void mpmg_mixed_free(mpmg_ctx *ctx);
 int mpmg_mixed_set_g2p_per_sm(mpmg_ctx *ctx, int per_sm);   // returns the value set
 int mpmg_mixed_set_tiles(mpmg_ctx *ctx, int p2g_variant, int g2p_tile);
 int mpmg_mixed_p2g_variants();
-void mpmg_mixed_p2g_shape(int v, int *elements, int *stage);
+void mpmg_mixed_p2g_shape(const mpmg_ctx *ctx, int v, int *elements, int *stage);
 int mpmg_mixed_step(mpmg_ctx *ctx);
 // Host read-back / write of a mixed particle or node field; returns
 // MPMG_ERR_UNKNOWN_FIELD for names the mixed state does not hold.

@@ -349,16 +349,18 @@ __device__ __forceinline__ int pad16b(int j) { return j + (j >> 3); }
 __device__ __forceinline__ int pad4b(int j) { return j + (j >> 5); }
 __device__ __forceinline__ int pad2b(int j) { return j + ((j >> 6) << 1); }
 
-// (elements a block, staged particles) of a batch's tiles; variant 0 is the
-// default and a single simulation's.  Rows of 32 elements: a warp stages one run
-// of storage and its threads' records lie together (16 x 16 elements: silo of
-// 474k particles 35.3 us a step, 33.6 with 32 x 8; 1 048 576 in a box 47.2 and
-// 47.5; 32 members 111.3 and 110.4; smaller and larger tiles are slower).
-constexpr int kP2GVariants = 3;
-constexpr int kP2GElems[kP2GVariants] = {256, 128, 512};
-constexpr int kP2GStage[kP2GVariants] = {1024, 512, 1024};
-constexpr int kTileX[kP2GVariants] = {32, 16, 32};
-constexpr int kTileY[kP2GVariants] = {8, 8, 16};
+// Shapes of the tiles, with their elements and staged particles.  Variants 0 to
+// 2 are a batch's choices for mpmg_autotune, variant 0 the default and a single
+// simulation's: shape 0 or the one that p2g_default_shape puts in its place.
+// Rows of 32 elements: a warp stages one run of storage and its threads' records
+// lie together (16 x 16 elements: silo of 474k particles 35.3 us a step, 33.6
+// with 32 x 8; 1 048 576 in a box 47.2 and 47.5; 32 members 111.3 and 110.4;
+// smaller and larger tiles are slower).
+constexpr int kP2GVariants = 3, kP2GShapes = 4;
+constexpr int kP2GElems[kP2GShapes] = {256, 128, 512, 256};
+constexpr int kP2GStage[kP2GShapes] = {1024, 512, 1024, 1024};
+constexpr int kTileX[kP2GShapes] = {32, 16, 32, 16};
+constexpr int kTileY[kP2GShapes] = {8, 8, 16, 16};
 
 __device__ __forceinline__ void p2g_accumulate(float (&acc)[4][5], float ih, float grav, float4 a4, float4 b4,
                                                float syy)
@@ -1291,33 +1293,52 @@ using P2GKernel = void (*)(MemberM, BatchView, const MpmgTile *, int *, int, con
                            uint32_t *, uint32_t *, Buf, const StepParams *, float, float2 *, float4 *, double *,
                            double *, double *, double *, double *);
 
-// The P2G and grid update with tile variant v.
+// The P2G and grid update with tile shape v.
 template <int V>
-P2GKernel p2g_variant_t(bool f64, bool batch)
+P2GKernel p2g_shape_t(bool f64, bool batch)
 {
+    constexpr int W = V == 3 ? 3 : 0;      // a single simulation's shapes
     if (f64)
         return batch ? mx_p2g_grid_kernel<true, true, kTileX[V], kTileY[V], kP2GStage[V]>
-                     : mx_p2g_grid_kernel<true, false, kTileX[0], kTileY[0], kP2GStage[0]>;
+                     : mx_p2g_grid_kernel<true, false, kTileX[W], kTileY[W], kP2GStage[W]>;
     return batch ? mx_p2g_grid_kernel<false, true, kTileX[V], kTileY[V], kP2GStage[V]>
-                 : mx_p2g_grid_kernel<false, false, kTileX[0], kTileY[0], kP2GStage[0]>;
+                 : mx_p2g_grid_kernel<false, false, kTileX[W], kTileY[W], kP2GStage[W]>;
 }
 
-P2GKernel p2g_variant(int v, bool f64, bool batch)
+P2GKernel p2g_shape(int v, bool f64, bool batch)
 {
-    return v == 1 ? p2g_variant_t<1>(f64, batch) : v == 2 ? p2g_variant_t<2>(f64, batch) : p2g_variant_t<0>(f64, batch);
+    return v == 1   ? p2g_shape_t<1>(f64, batch)
+           : v == 2 ? p2g_shape_t<2>(f64, batch)
+           : v == 3 ? p2g_shape_t<3>(f64, batch)
+                    : p2g_shape_t<0>(f64, batch);
 }
 
 size_t p2g_smem_size(int v)
 {
     return v == 1   ? FusedTile<kTileX[1], kTileY[1], kP2GStage[1]>::smem
            : v == 2 ? FusedTile<kTileX[2], kTileY[2], kP2GStage[2]>::smem
+           : v == 3 ? FusedTile<kTileX[3], kTileY[3], kP2GStage[3]>::smem
                     : FusedTile<kTileX[0], kTileY[0], kP2GStage[0]>::smem;
 }
 
-// Tiles of a simulation with variant v.
-int p2g_tiles(const mpmg_config &c, int v)
+// Tiles of a simulation with shape v.
+size_t p2g_tiles(const mpmg_config &c, int v)
 {
-    return (int)(mpmg_tiles_along((uint32_t)c.Nx, kTileX[v]) * mpmg_tiles_along((uint32_t)c.Ny, kTileY[v]));
+    return (size_t)mpmg_tiles_along((uint32_t)c.Nx, kTileX[v]) * mpmg_tiles_along((uint32_t)c.Ny, kTileY[v]);
+}
+
+// The shape that stands for variant 0: rows of 32 elements, or the square where
+// it leaves at most 7/8 of the tiles (us a step with rows and squares: 3 x 20001
+// nodes 40.0 and 26.3, 33 x 4001 33.6 and 31.7, 129 x 1001 30.4 and 28.6; 48 x
+// 3001, at 0.94 of the tiles, 31.9 and 33.0); in a batch the half tile where it
+// takes no more tiles than the square (2000 members of 5 x 5 nodes 38.7 and 32.0).
+int p2g_default_shape(const mpmg_config *cfg, int count, bool batch)
+{
+    size_t tiles[kP2GShapes] = {0, 0, 0, 0};
+    for (int k = 0; k < count; k++)
+        for (int v = 0; v < kP2GShapes; v++) tiles[v] += p2g_tiles(cfg[k], v);
+    if (batch && tiles[1] <= tiles[3] && tiles[1] <= tiles[0]) return 1;
+    return 8 * tiles[3] <= 7 * tiles[0] ? 3 : 0;
 }
 
 }  // namespace
@@ -1361,6 +1382,7 @@ int mpmg_mixed_init(mpmg_ctx *ctx, const double *m, const double *v, const doubl
     // members: one, or the batch's (their constants and first-index tables)
     BatchInfo *bt = ctx->batch;
     const int count = bt ? bt->count : 1;
+    s->p2g_default = p2g_default_shape(bt ? bt->cfg.data() : &ctx->cfg, count, bt != nullptr);
     if (bt) {
         std::vector<MemberM> hm(count);
         std::vector<int> eo(count + 1);
@@ -1378,9 +1400,11 @@ int mpmg_mixed_init(mpmg_ctx *ctx, const double *m, const double *v, const doubl
         if ((rc = dalloc(&bt->d_first, first.size())) != MPMG_OK) return rc;
         MPMG_CHECK(cudaMemcpy(bt->d_first, first.data(), first.size() * sizeof(int), cudaMemcpyHostToDevice));
         for (int v = 0; v < kP2GVariants; v++) {
+            const int shape = v == 0 ? s->p2g_default : v;
             std::vector<MpmgTile> map;
             for (int k = 0; k < count; k++)
-                mpmg_append_tiles(map, (uint32_t)k, (uint32_t)bt->cfg[k].Nx, (uint32_t)bt->cfg[k].Ny, kTileX[v], kTileY[v]);
+                mpmg_append_tiles(map, (uint32_t)k, (uint32_t)bt->cfg[k].Nx, (uint32_t)bt->cfg[k].Ny, kTileX[shape],
+                                  kTileY[shape]);
             if ((rc = dalloc(&s->tile_map[v], map.size())) != MPMG_OK) return rc;
             s->tiles[v] = (int)map.size();
             MPMG_CHECK(cudaMemcpy(s->tile_map[v], map.data(), map.size() * sizeof(MpmgTile), cudaMemcpyHostToDevice));
@@ -1389,7 +1413,7 @@ int mpmg_mixed_init(mpmg_ctx *ctx, const double *m, const double *v, const doubl
         MPMG_CHECK(cudaMemcpy(bt->d_elem_off, eo.data(), (count + 1) * sizeof(int), cudaMemcpyHostToDevice));
     }
 
-    if (!bt) s->tiles[0] = p2g_tiles(ctx->cfg, 0);
+    if (!bt) s->tiles[0] = (int)p2g_tiles(ctx->cfg, s->p2g_default);
     s->max_tiles = s->tiles[0];
     for (int t : s->tiles) s->max_tiles = t > s->max_tiles ? t : s->max_tiles;
     if ((rc = dalloc(&s->tile_zero, s->max_tiles)) != MPMG_OK) return rc;
@@ -1457,9 +1481,11 @@ int mpmg_mixed_init(mpmg_ctx *ctx, const double *m, const double *v, const doubl
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g2p_smem_size(tile)));
     }
     const bool f64 = ctx->cfg.precision == MPMG_PRECISION_MIXED_F64NODE;
-    for (int v = 0; v < (bt ? kP2GVariants : 1); v++)
-        MPMG_CHECK(cudaFuncSetAttribute(p2g_variant(v, f64, bt != nullptr), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)p2g_smem_size(v)));
+    for (int v = 0; v < (bt ? kP2GVariants : 1); v++) {
+        const int shape = v == 0 ? s->p2g_default : v;
+        MPMG_CHECK(cudaFuncSetAttribute(p2g_shape(shape, f64, bt != nullptr),
+                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p2g_smem_size(shape)));
+    }
     s->sms = sms > 0 ? sms : 1;
     s->p2g_variant = 0;
     rc = mpmg_mixed_set_tiles(ctx, 0, kG2PTileSizes[0]);
@@ -1484,7 +1510,7 @@ int mpmg_mixed_set_g2p_per_sm(mpmg_ctx *ctx, int per_sm)
 }
 
 // The tiles of the mixed step: a batch's P2G variant (elements a block and
-// staged particles, kP2GElems / kP2GStage; single simulations run variant 0)
+// staged particles, mpmg_mixed_p2g_shape; single simulations run variant 0)
 // and the G2P tile (kG2PTileSizes).  The G2P
 // grid goes back to all the blocks of the new tile that fit.  Tiles change
 // which block handles which elements or particles, never a result.
@@ -1510,10 +1536,11 @@ int mpmg_mixed_p2g_variants()
     return kP2GVariants;
 }
 
-void mpmg_mixed_p2g_shape(int v, int *elements, int *stage)
+void mpmg_mixed_p2g_shape(const mpmg_ctx *ctx, int v, int *elements, int *stage)
 {
-    *elements = kP2GElems[v];
-    *stage = kP2GStage[v];
+    const int shape = v == 0 ? ctx->mixed->p2g_default : v;
+    *elements = kP2GElems[shape];
+    *stage = kP2GStage[shape];
 }
 
 void mpmg_mixed_free(mpmg_ctx *ctx)
@@ -1581,9 +1608,9 @@ int mpmg_mixed_step(mpmg_ctx *ctx)
     const bool nonlocal = c.material == MPMG_G_NONLOCAL_MU2;
     double *node_m64 = nonlocal ? ctx->node_m : (double *)nullptr;
     mpmg_phase_begin(ctx, PH_P2G);
-    const int v = batch ? s->p2g_variant : 0;
-    MPMG_CHECK(mpmg_launch_pdl(true, p2g_variant(v, f64, batch), dim3(s->tiles[v]), dim3(kP2GElems[v]), p2g_smem_size(v),
-                               st, m0, bv, (const MpmgTile *)s->tile_map[v], s->tile_zero, n, (const int *)ctx->cell_start,
+    const int v = batch ? s->p2g_variant : 0, shape = v == 0 ? s->p2g_default : v;
+    MPMG_CHECK(mpmg_launch_pdl(true, p2g_shape(shape, f64, batch), dim3(s->tiles[v]), dim3(kP2GElems[shape]),
+                               p2g_smem_size(shape), st, m0, bv, (const MpmgTile *)s->tile_map[v], s->tile_zero, n, (const int *)ctx->cell_start,
                                (const uint32_t *)ctx->bin.slots, ctx->perm, ctx->bin.rank, s->halo_perm, S,
                                (const StepParams *)ctx->d_params, (float)MPMG_TOL, s->node_mass, s->node4,
                                ctx->node_mx, ctx->node_my, ctx->node_fx, ctx->node_fy, node_m64));
