@@ -447,9 +447,8 @@ __global__ void __launch_bounds__(EB * SPLIT) p2g_cells_kernel(
 // Flat tiles: TY = 4 recomputes 39 % of the nodes (16: 10 %), but a block is one
 // warp a sub-partition, and a sparse grid's filled tiles spread over all SMs
 // (125k particles on 261k nodes: 54.0 us a step, 56.3 with TY = 8, 58.2 with 16;
-// 1 048 576 particles on 263k: 253.3, 252.3, 253.8).
-
-constexpr int kGridTX = 32, kGridTY = 4;
+// 1 048 576 particles on 263k: 253.3, 252.3, 253.8).  Narrow grids take 8 x 16
+// (launch_grid).
 
 // The corner (BL, BR, TR, TL) that node (i, j) is of its colour-c element.
 __device__ __forceinline__ int c_corner(int c, int i, int j)
@@ -458,7 +457,8 @@ __device__ __forceinline__ int c_corner(int c, int i, int j)
     return right ? (up ? 0 : 3) : (up ? 1 : 2);
 }
 
-__global__ void __launch_bounds__(kGridTX * kGridTY) grid_kernel(
+template <int TX, int TY>
+__global__ void __launch_bounds__(TX * TY) grid_kernel(
     GridGeom g, BcParams bc, int tiles_x, const uint32_t *__restrict__ count, uint32_t *__restrict__ count_next,
     uint32_t *__restrict__ n_filled_next, uint32_t *__restrict__ cursor,
     const double *__restrict__ cell_sums, const StepParams *__restrict__ sp, double dt,
@@ -467,7 +467,7 @@ __global__ void __launch_bounds__(kGridTX * kGridTY) grid_kernel(
     double *__restrict__ node_my, double *__restrict__ node_fx, double *__restrict__ node_fy,
     double2 *__restrict__ coef, int early)
 {
-    __shared__ double sh[4][kGridTY][kGridTX];
+    __shared__ double sh[4][TY][TX];
     __shared__ double sh_const[4];         // constants as registers (mat::Unit)
     if (threadIdx.x == 0) {
         sh_const[0] = mat::opaque(1.0);
@@ -475,8 +475,8 @@ __global__ void __launch_bounds__(kGridTX * kGridTY) grid_kernel(
         sh_const[2] = g.inv_h;
         sh_const[3] = dt;
     }
-    const int tx = threadIdx.x % kGridTX, ty = threadIdx.x / kGridTX;
-    const int i = (int)(blockIdx.x % tiles_x) * (kGridTX - 1) + tx, j = (int)(blockIdx.x / tiles_x) * (kGridTY - 1) + ty;
+    const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
+    const int i = (int)(blockIdx.x % tiles_x) * (TX - 1) + tx, j = (int)(blockIdx.x / tiles_x) * (TY - 1) + ty;
     const bool node = i < g.Nx && j < g.Ny;
     // Colour c = 2 * (row % 2) + (col % 2) (process_usl.c:158); the four
     // elements around a node have the four colours, summed in order 0..3.
@@ -497,7 +497,7 @@ __global__ void __launch_bounds__(kGridTX * kGridTY) grid_kernel(
             src[c] = cell_sums + (size_t)e * kCell + corner * 4;
         }
     }
-    const bool own = node && (tx < kGridTX - 1 || i == g.Nx - 1) && (ty < kGridTY - 1 || j == g.Ny - 1);
+    const bool own = node && (tx < TX - 1 || i == g.Nx - 1) && (ty < TY - 1 || j == g.Ny - 1);
     mpmg_pdl_wait();
     if (early) mpmg_pdl_trigger();
     __syncthreads();
@@ -581,7 +581,7 @@ __global__ void __launch_bounds__(kGridTX * kGridTY) grid_kernel(
     sh[2][ty][tx] = vxn;
     sh[3][ty][tx] = vyn;
     __syncthreads();
-    if (filled && tx < kGridTX - 1 && ty < kGridTY - 1) {
+    if (filled && tx < TX - 1 && ty < TY - 1) {
         double2 *out = coef + (size_t)(j * g.Ex + i) * 8;
 #pragma unroll
         for (int f = 0; f < 4; f++) {
@@ -594,16 +594,24 @@ __global__ void __launch_bounds__(kGridTX * kGridTY) grid_kernel(
     mpmg_pdl_trigger();
 }
 
-cudaError_t launch_grid(mpmg_ctx *ctx, const GridGeom &g)
+template <int TX, int TY>
+cudaError_t launch_grid_t(mpmg_ctx *ctx, const GridGeom &g)
 {
     const RowBins &r = ctx->row;
-    const int tiles_x = (g.Nx + kGridTX - 2) / (kGridTX - 1), tiles_y = (g.Ny + kGridTY - 2) / (kGridTY - 1);
-    return mpmg_launch_pdl(true, grid_kernel, dim3(tiles_x * tiles_y), dim3(kGridTX * kGridTY), 0, ctx->stream, g,
+    const int tiles_x = (g.Nx + TX - 2) / (TX - 1), tiles_y = (g.Ny + TY - 2) / (TY - 1);
+    return mpmg_launch_pdl(true, grid_kernel<TX, TY>, dim3(tiles_x * tiles_y), dim3(TX * TY), 0, ctx->stream, g,
                            make_bc(ctx), tiles_x, (const uint32_t *)r.count[r.cur], r.count[1 - r.cur],
                            r.n_filled + (1 - r.cur), r.cursor, (const double *)ctx->cell_sums,
                            (const StepParams *)ctx->d_params, ctx->cfg.dt,
                            ctx->node_m, ctx->node_ax, ctx->node_ay, ctx->node_vx, ctx->node_vy, ctx->node_mx,
                            ctx->node_my, ctx->node_fx, ctx->node_fy, (double2 *)ctx->elem_coef, early_launch(ctx));
+}
+
+// Tiles of 8 x 16 nodes on a grid of up to 8 columns, where rows of 32 are
+// mostly idle (3 x 20001 nodes: 62 us a step, 126 with rows).
+cudaError_t launch_grid(mpmg_ctx *ctx, const GridGeom &g)
+{
+    return g.Nx <= 8 ? launch_grid_t<8, 16>(ctx, g) : launch_grid_t<32, 4>(ctx, g);
 }
 
 // ---------------------------------------------------------------------------
