@@ -1122,9 +1122,9 @@ int step_with_graphs(mpmg_ctx *ctx, int nsteps)
 extern "C" {
 
 // Online tuning of the mixed step's tiles and launch shape, on the
-// simulation itself.  First the tiles: every batched-P2G tile (elements a
-// block, particles staged a pass; batches only, a single simulation runs the
-// fused P2G) with every G2P tile, at the default launch shape; then, with
+// simulation itself.  First the tiles: every P2G tile a batch may take (a
+// single simulation keeps its own) with every G2P tile, at the default launch
+// shape; then, with
 // the fastest tiles, the launch shape: G2P blocks per SM x steps per graph.
 // Each candidate runs a warm-up graph and then steps_per_trial steps
 // (rounded up to whole graphs) timed with CUDA events.  No knob changes any

@@ -194,7 +194,8 @@ struct mpmg_ctx {
     int *cell_start;       // num_elements + 1
     BinScratch bin;
 
-    // P2G per-element corner sums: 20 values per element, value-major.
+    // P2G corner sums: a run of 20 doubles per element (mpmg_step.cu; MUSL's
+    // and g_local_mu2_ext's own sums lie in it value-major).
     double *cell_sums;
 
     // Grid.

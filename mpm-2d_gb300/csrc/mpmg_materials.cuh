@@ -20,7 +20,9 @@ __device__ __forceinline__ double sub(double a, double b) { return __dadd_rn(a, 
 // elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
 // Dev. 34(1), 1990).  Five FP64 operations in place of a full division; the
 // result equals a / b for normal operands and quotients (a zero quotient
-// comes out +0, and non-finite operands are not carried through).
+// comes out +0, and non-finite operands are not carried through).  The laws
+// divide by dvd_const below, in no FP64 operation; this form is kept as the
+// five-operation alternative that tests/test_gpu_arith.py measures.
 __device__ __forceinline__ double dvd_known(double a, double b, double y)
 {
     double q = __dmul_rn(a, y);

@@ -108,7 +108,7 @@ __global__ void nonlocal_bulk_kernel(int n, mat::NonlocalParams np, const double
 // run in integer arithmetic (mat::imul), sums with register operands, 34 -> 21
 // FP64 instructions a particle (835 996 particles: 76 -> 65 us).
 __global__ void __launch_bounds__(128) assemble_kernel(
-    int ne, int Ex, double inv_h, int dense_only, RowView rv, const double *__restrict__ xl, const double *__restrict__ yl,
+    int ne, double inv_h, int dense_only, RowView rv, const double *__restrict__ xl, const double *__restrict__ yl,
     const double *__restrict__ v, const double *__restrict__ dense, const double *__restrict__ gfl,
     const double *__restrict__ xisq, double *__restrict__ elem_k, double *__restrict__ elem_f)
 {
@@ -191,7 +191,6 @@ __global__ void __launch_bounds__(128) assemble_kernel(
     for (int k = 0; k < 10; k++) elem_k[(size_t)k * ne + e] = fma(gg[k], ih2, K[k]);
 #pragma unroll
     for (int k = 0; k < 4; k++) elem_f[(size_t)k * ne + e] = F[k];
-    (void)Ex;
 }
 
 struct SolveArgs {
@@ -1011,7 +1010,8 @@ inline size_t pcg_tile_smem(int C, int Nx)
 // (only the 1e-10 shift and the xi^-2-weighted mass keep it from being
 // singular) therefore survives FP32 coarsening.
 //
-// Preconditioner: one V(1,1) cycle in FP32 on r / |r|.
+// Preconditioner: one V-cycle in FP32 on r, scaled to order one by a power of
+// two.
 //   * On each coarse level, one l1-Jacobi step (Baker, Falgout, Kolev and
 //     Yang, 2011).  D_l1 is each row's absolute sum, so the smoother converges
 //     without an eigenvalue estimate.  The step size is the Chebyshev step
@@ -1025,8 +1025,7 @@ inline size_t pcg_tile_smem(int C, int Nx)
 //   * Then the residual and its restriction.
 //   * At the coarsest level, an exact solve: an FP64 inverse formed every
 //     solve.
-//   * On the way up, prolongation and one post-smoothing step of the same
-//     size.
+//   * On the way up, prolongation and the level's smoothing again.
 //
 // Outer iteration: FP64 CG in the one-reduction form of Chronopoulos and
 // Gear.  It uses the Polak-Ribiere beta, which tolerates the rounding of an
@@ -1035,13 +1034,12 @@ inline size_t pcg_tile_smem(int C, int Nx)
 //   pi    = delta + 2 beta <s, u> + beta^2 pi_old
 //   alpha = gamma / pi
 // where u = M r, w = A u, gamma = <r, u>, delta = <w, u>, and s = A p by
-// recurrence.  Each iteration needs one grid barrier, for the four inner
-// products.
+// recurrence.  Each iteration gathers the blocks' four inner products once
+// (mg_gather4), which is its only barrier between all blocks.
 //
 // Where the levels live.  A level of more than 2048 nodes is spread over the
-// blocks in contiguous node ranges (level 0 over blocks 1 .. n - 1, so that
-// block 0 has no level-0 work); the coarser levels are held whole by block
-// 0, whose threads meet at block barriers between phases.  All blocks
+// blocks 1 .. n - 1 in contiguous node ranges; the coarser levels are held
+// whole by block 0, which has no other work and whose threads meet at block barriers between phases.  All blocks
 // restrict into the first held level and block 0 stages it.
 //
 // Synchronisation between blocks.  Each phase writes its level vector to
@@ -2623,7 +2621,7 @@ int mpmg_launch_fluidity(mpmg_ctx *ctx)
         ctx->launches += 1;
     }
     const double *xisq = mu2 ? ctx->state[6] : ctx->state[10];
-    assemble_kernel<<<blocks_for(ne, 128), 128, 0, s>>>(ne, ctx->Ex, ctx->inv_h, mu2 ? 1 : 0,
+    assemble_kernel<<<blocks_for(ne, 128), 128, 0, s>>>(ne, ctx->inv_h, mu2 ? 1 : 0,
                                                         RowView{ctx->row.count[ctx->row.cur],
                                                                 ctx->row.rows[ctx->row.cur], ctx->row.over_list,
                                                                 ctx->row.cap},

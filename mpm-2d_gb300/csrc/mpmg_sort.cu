@@ -16,7 +16,7 @@
 //              clamps the caller's keys into the scratch
 //   scan       one warp per digit: exclusive prefix of that digit's counts
 //              over the tiles, and the digit's total
-//   downsweep  every warp ranks its 256 contiguous keys stably (match_any +
+//   downsweep  every warp ranks its 128 or 256 contiguous keys stably (match_any +
 //              a warp-private digit histogram), the block turns the per-warp
 //              counts into offsets (digit prefix over the whole input + this
 //              tile's prefix + earlier warps), and keys and values scatter
@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(kThreads) downsweep_kernel(
     }
 }
 
-// The first sorted position whose key is >= e, by a whole warp: 31 probes a
+// The first sorted position whose key is >= e, by a whole warp: 32 probes a
 // round, so that a million keys take four dependent loads.
 __device__ __forceinline__ int lower_bound_warp(const uint32_t *__restrict__ keys, int n, uint32_t e)
 {

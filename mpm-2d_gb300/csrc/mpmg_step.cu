@@ -1314,7 +1314,9 @@ int mpmg_launch_step(mpmg_ctx *ctx)
     // later phases of these read the ordered rows
     const bool keep_order = nonlocal || musl || c.material == MPMG_G_LOCAL_MU2_EXT || ctx->row.record;
     // two threads an element in single-warp sets, where that leaves every
-    // sub-partition at most one warp
+    // sub-partition at most one warp (of the initial positions: a run that
+    // spreads from one form's range into the other's keeps its form, 262 144
+    // particles 87.7 us a step where they began packed, 83.5 where spread)
     MPMG_CHECK((ctx->row.filled0 <= (size_t)ctx->sms * 4 * 16 ? launch_p2g<32, 2>(ctx, g, keep_order)
                                                               : launch_p2g<64, 1>(ctx, g, keep_order)));
     mpmg_phase_end(ctx, PH_P2G);
