@@ -175,7 +175,10 @@ MPMG_API int mpmg_config_init(mpmg_config *cfg);
  * Creates a simulation from host arrays of n particles: mass, volume,
  * position, velocity and in-plane stress, the columns of the reference's
  * particle file (src/reader.c:66-99).  The arrays are copied; the caller keeps
- * them.  On success *out holds the context.
+ * them.  On success *out holds the context.  Device memory of the FP64 form:
+ * about 480 bytes an element with its node where few particles lie in it (its
+ * row of particle indices widens with the initial filling), and about 150 a
+ * particle; of the mixed form about 36 and 180.
  */
 MPMG_API int mpmg_create(const mpmg_config *cfg, size_t n, const double *m, const double *v,
                 const double *x, const double *y, const double *vx, const double *vy,
