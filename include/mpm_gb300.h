@@ -176,9 +176,10 @@ MPMG_API int mpmg_config_init(mpmg_config *cfg);
  * position, velocity and in-plane stress, the columns of the reference's
  * particle file (src/reader.c:66-99).  The arrays are copied; the caller keeps
  * them.  On success *out holds the context.  Device memory of the FP64 form:
- * about 480 bytes an element with its node where few particles lie in it (its
- * row of particle indices widens with the initial filling), and about 150 a
- * particle; of the mixed form about 36 and 180.
+ * about 480 bytes an element with its node (its row of particle indices widens
+ * with the initial filling; 200 where the grid has 2^24 elements or more and
+ * the particles are fewer than half as many, with 290 more a particle then),
+ * and about 150 a particle; of the mixed form about 36 and 180.
  */
 MPMG_API int mpmg_create(const mpmg_config *cfg, size_t n, const double *m, const double *v,
                 const double *x, const double *y, const double *vx, const double *vy,

@@ -117,9 +117,11 @@ int alloc_rows(mpmg_ctx *ctx, const MpmgFilled &count, size_t n)
     r.ready = false;
     r.record = false;
     const size_t ne = ctx->ne, most = std::min(ne, n), row_words = ne * (size_t)r.cap;
+    const bool by_list = mpmg_sums_by_list(n, ne);
     const struct { uint32_t **p; size_t words; } parts[] = {
         {&r.rows[0], row_words}, {&r.rows[1], row_words}, {&r.count[0], ne}, {&r.count[1], ne}, {&r.head, ne},
-        {&r.filled[0], most}, {&r.filled[1], most}, {&r.next, n}, {&r.over_list, n}, {&r.n_filled, 2}, {&r.cursor, 1}};
+        {&r.filled[0], most}, {&r.filled[1], most}, {&r.pos[0], by_list ? ne : 0},
+        {&r.pos[1], by_list ? ne : 0}, {&r.next, n}, {&r.over_list, n}, {&r.n_filled, 2}, {&r.cursor, 1}};
     size_t words = 0;
     for (auto &q : parts) words += (q.words + 63) & ~(size_t)63;
     const int rc = dalloc(&r.block, words);
@@ -129,6 +131,7 @@ int alloc_rows(mpmg_ctx *ctx, const MpmgFilled &count, size_t n)
         *q.p = at;
         at += (q.words + 63) & ~(size_t)63;
     }
+    if (!by_list) r.pos[0] = r.pos[1] = nullptr;
     return MPMG_OK;
 }
 
@@ -763,7 +766,8 @@ int mpmg_create(const mpmg_config *cfg, size_t n, const double *m, const double 
         TRY(dalloc(&ctx->sorted_keys, n));
         TRY(dalloc(&ctx->perm, n));
         TRY(dalloc(&ctx->cell_start, ctx->ne + 1));
-        TRY(dalloc(&ctx->cell_sums, 20 * ctx->ne));
+        ctx->row.places = mpmg_sums_by_list(n, ctx->ne) ? n : ctx->ne;
+        TRY(dalloc(&ctx->cell_sums, 20 * ctx->row.places));
         double **nodes[] = {&ctx->node_m, &ctx->node_ax, &ctx->node_ay, &ctx->node_vx, &ctx->node_vy,
                             &ctx->node_gf};
         for (double **p : nodes) TRY(dalloc(p, ctx->nn));
@@ -772,7 +776,7 @@ int mpmg_create(const mpmg_config *cfg, size_t n, const double *m, const double 
             for (double **p : tn) TRY(dalloc(p, ctx->nn));
         }
         TRY(alloc_step_record(ctx, 1));
-        TRY(dalloc(&ctx->elem_coef, 16 * ctx->ne));
+        TRY(dalloc(&ctx->elem_coef, 16 * ctx->row.places));
         if (nonlocal) TRY(mpmg_nonlocal_init(ctx));
         if (cfg->material == MPMG_G_NONLOCAL_MU2) TRY(dalloc(&ctx->nl_trial, 5 * n));
 

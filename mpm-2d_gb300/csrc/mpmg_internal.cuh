@@ -133,6 +133,8 @@ struct RowBins {
     uint32_t *count[2];    // ne
     uint32_t *rows[2];     // ne x cap
     uint32_t *filled[2];   // min(ne, n): the elements with particles
+    uint32_t *pos[2];      // ne: their places on that list, or null (mpmg_sums_by_list)
+    size_t places;         // places of the corner sums and coefficients: those of the list, or ne
     uint32_t *n_filled;    // entries in filled[0], filled[1]
     uint32_t *cursor;      // entries taken from over_list
     size_t filled0;        // filled elements of the initial positions
@@ -178,8 +180,8 @@ struct mpmg_ctx {
     int *in_element;
     int *active;
 
-    // FP64 form: element rows, and per element the bilinear coefficients of
-    // the nodal acceleration and velocity (16 doubles, mpmg_step.cu).
+    // FP64 form: element rows, and per place the bilinear coefficients of the
+    // nodal acceleration and velocity (16 doubles, mpmg_step.cu).
     RowBins row;
     double *elem_coef;
     uint32_t *sort_keys;   // input of mpmg_fp64_sort, allocated last
@@ -194,8 +196,8 @@ struct mpmg_ctx {
     int *cell_start;       // num_elements + 1
     BinScratch bin;
 
-    // P2G corner sums: a run of 20 doubles per element (mpmg_step.cu; MUSL's
-    // and g_local_mu2_ext's own sums lie in it value-major).
+    // P2G corner sums: a run of 20 doubles a place (RowBins; MUSL's and
+    // g_local_mu2_ext's own sums lie in it value-major).
     double *cell_sums;
 
     // Grid.

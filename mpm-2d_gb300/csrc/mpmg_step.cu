@@ -58,7 +58,7 @@ inline int early_launch(const mpmg_ctx *ctx)
 // rows
 
 struct RowsOut {
-    uint32_t *count, *rows, *filled, *n_filled, *head, *next;
+    uint32_t *count, *rows, *filled, *pos, *n_filled, *head, *next;
     int cap;
 };
 
@@ -87,7 +87,11 @@ __device__ __forceinline__ void bin_particle(const RowsOut &R, int i, uint32_t k
         uint32_t at = 0;
         if (lane == 0) at = atomicAdd(R.n_filled, (uint32_t)__popc(firsts));
         at = __shfl_sync(0xffffffffu, at, 0);
-        if (start && base == 0) R.filled[at + __popc(firsts & ((1u << lane) - 1u))] = key;
+        if (start && base == 0) {
+            at += (uint32_t)__popc(firsts & ((1u << lane) - 1u));
+            R.filled[at] = key;
+            if (R.pos != nullptr) R.pos[key] = at;
+        }
     }
     base = __shfl_sync(0xffffffffu, base, leader);
     if (!valid) return;
@@ -136,8 +140,9 @@ __global__ void __launch_bounds__(256) keys_kernel(GridGeom g, float inv_hf, int
 // the sorted warps with the block index, so that no sub-partition gets the
 // full ones of every block.  SPLIT = 2 gives the two halves of an element's
 // moments to two threads in different warps, which shortens the serial chain
-// where there are too few elements to fill the chip.  The sums are stored per
-// element: 4 corners x (m, mx, my, h fx), then 4 x h fy.
+// where there are too few elements to fill the chip.  The sums are stored a run
+// an element, by element or in the list's order (RowBins::pos): 4 corners x (m,
+// mx, my, h fx), then 4 x h fy.
 
 constexpr int kCell = 20;                  // doubles an element
 constexpr int kStage = 16;                 // staged row entries an element, at most a row's slots
@@ -220,7 +225,7 @@ __device__ __noinline__ void order_long_lists(RowView rv, int lists, const int *
     }
 }
 
-template <int EB, int SPLIT>
+template <int EB, int SPLIT, bool LIST>
 __global__ void __launch_bounds__(EB * SPLIT) p2g_cells_kernel(
     GridGeom g, RowView rv, const uint32_t *__restrict__ filled, const uint32_t *__restrict__ n_filled,
     const uint32_t *__restrict__ head, const uint32_t *__restrict__ next, uint32_t *__restrict__ cursor,
@@ -427,7 +432,7 @@ __global__ void __launch_bounds__(EB * SPLIT) p2g_cells_kernel(
     const int here = min(EB, total - first);
     for (int q = tid; q < kCell * here; q += EB * SPLIT) {
         const int l = q / kCell, f = q - l * kCell;
-        cell_sums[(size_t)sh_elem[l] * kCell + f] = sh_sum[l * kSumStride + f];
+        cell_sums[(size_t)(LIST ? first + l : sh_elem[l]) * kCell + f] = sh_sum[l * kSumStride + f];
     }
     mpmg_pdl_trigger();
 }
@@ -457,9 +462,10 @@ __device__ __forceinline__ int c_corner(int c, int i, int j)
     return right ? (up ? 0 : 3) : (up ? 1 : 2);
 }
 
-template <int TX, int TY>
+template <int TX, int TY, bool LIST>
 __global__ void __launch_bounds__(TX * TY) grid_kernel(
-    GridGeom g, BcParams bc, int tiles_x, const uint32_t *__restrict__ count, uint32_t *__restrict__ count_next,
+    GridGeom g, BcParams bc, int tiles_x, const uint32_t *__restrict__ count, const uint32_t *__restrict__ pos,
+    uint32_t *__restrict__ count_next,
     uint32_t *__restrict__ n_filled_next, uint32_t *__restrict__ cursor,
     const double *__restrict__ cell_sums, const StepParams *__restrict__ sp, double dt,
     double *__restrict__ node_m, double *__restrict__ node_ax, double *__restrict__ node_ay,
@@ -483,6 +489,7 @@ __global__ void __launch_bounds__(TX * TY) grid_kernel(
     // The counts are the previous step's work: read before the wait.
     const double *src[4];
     bool filled = false;                   // the element whose BL node this is holds particles
+    uint32_t place = 0;                    // its place on the list
     if (node) {
 #pragma unroll
         for (int c = 0; c < 4; c++) {
@@ -492,9 +499,13 @@ __global__ void __launch_bounds__(TX * TY) grid_kernel(
             if (ci < 0 || cj < 0 || ci >= g.Ex || cj >= g.Ey) continue;
             const int e = cj * g.Ex + ci;
             if (count[e] == 0) continue;
+            const uint32_t at = LIST ? pos[e] : (uint32_t)e;
             const int corner = c_corner(c, i, j);
-            if (corner == 0) filled = true;
-            src[c] = cell_sums + (size_t)e * kCell + corner * 4;
+            if (corner == 0) {
+                filled = true;
+                place = at;
+            }
+            src[c] = cell_sums + (size_t)at * kCell + corner * 4;
         }
     }
     const bool own = node && (tx < TX - 1 || i == g.Nx - 1) && (ty < TY - 1 || j == g.Ny - 1);
@@ -582,7 +593,7 @@ __global__ void __launch_bounds__(TX * TY) grid_kernel(
     sh[3][ty][tx] = vyn;
     __syncthreads();
     if (filled && tx < TX - 1 && ty < TY - 1) {
-        double2 *out = coef + (size_t)(j * g.Ex + i) * 8;
+        double2 *out = coef + (size_t)place * 8;
 #pragma unroll
         for (int f = 0; f < 4; f++) {
             const double q0 = sh[f][ty][tx], q1 = sh[f][ty][tx + 1], q2 = sh[f][ty + 1][tx + 1], q3 = sh[f][ty + 1][tx];
@@ -599,8 +610,10 @@ cudaError_t launch_grid_t(mpmg_ctx *ctx, const GridGeom &g)
 {
     const RowBins &r = ctx->row;
     const int tiles_x = (g.Nx + TX - 2) / (TX - 1), tiles_y = (g.Ny + TY - 2) / (TY - 1);
-    return mpmg_launch_pdl(true, grid_kernel<TX, TY>, dim3(tiles_x * tiles_y), dim3(TX * TY), 0, ctx->stream, g,
-                           make_bc(ctx), tiles_x, (const uint32_t *)r.count[r.cur], r.count[1 - r.cur],
+    return mpmg_launch_pdl(true, r.pos[0] != nullptr ? grid_kernel<TX, TY, true> : grid_kernel<TX, TY, false>,
+                           dim3(tiles_x * tiles_y), dim3(TX * TY), 0, ctx->stream, g,
+                           make_bc(ctx), tiles_x, (const uint32_t *)r.count[r.cur], (const uint32_t *)r.pos[r.cur],
+                           r.count[1 - r.cur],
                            r.n_filled + (1 - r.cur), r.cursor, (const double *)ctx->cell_sums,
                            (const StepParams *)ctx->d_params, ctx->cfg.dt,
                            ctx->node_m, ctx->node_ax, ctx->node_ay, ctx->node_vx, ctx->node_vy, ctx->node_mx,
@@ -636,7 +649,7 @@ struct G2PArgs {
     RowsOut next;          // the next step's rows
     int *in_element;
     int *active;
-    const double2 *coef;   // element coefficients (grid_kernel)
+    const double2 *coef;   // element coefficients (grid_kernel) at their places (pos)
     const double *node_vx, *node_vy;
     double *x, *y, *vx, *vy, *ux, *uy, *v, *m;
     double *sxx, *sxy, *syy, *Tzz;
@@ -645,6 +658,7 @@ struct G2PArgs {
     // g_nonlocal_mu2: the trial stress the stress update reads after the
     // fluidity solve, 5 per particle, value-major (p_d, t0xx, t0xy, t0yy, tau)
     double *trial;
+    const uint32_t *pos;   // places of the filled elements (RowBins::pos)
 };
 
 // G2P phases.  USL (process_usl.c:465-592) runs them all in one pass; MUSL
@@ -774,10 +788,11 @@ __device__ __forceinline__ Field field_at(double2 c01, double2 c23, double x, do
     return f;
 }
 
-// One particle inside the grid, element e at the step's start; p.x, p.y leave
-// as the moved position.
+// One particle inside the grid, element e (its sums at `place`) at the step's
+// start; p.x, p.y leave as the moved position.
 template <class E, int MATERIAL, int PHASE>
-__device__ __forceinline__ void g2p_particle(const G2PArgs &A, const G2PConst &C, int i, int e, Particle &p)
+__device__ __forceinline__ void g2p_particle(const G2PArgs &A, const G2PConst &C, int i, int e, uint32_t place,
+                                             Particle &p)
 {
     const GridGeom &g = A.g;
     const E &u = C.el;
@@ -803,7 +818,7 @@ __device__ __forceinline__ void g2p_particle(const G2PArgs &A, const G2PConst &C
     } else {
         const double xl = mpmg_local_coord_fma(p.x, mat::small_int(ci), inv_h);
         const double yl = mpmg_local_coord_fma(p.y, mat::small_int(cj), inv_h);
-        const double2 *c = A.coef + (size_t)e * 8;
+        const double2 *c = A.coef + (size_t)place * 8;
         vx = field_at(c[4], c[5], xl, yl);
         vy = field_at(c[6], c[7], xl, yl);
         // move_particles_explicit_usl_split (process_usl.c:914-957); light
@@ -890,7 +905,7 @@ __device__ __forceinline__ void stage_const(G2PConst &C, const G2PConst &param)
 
 // The block's size and E are the launch's (g2p_pipe_bound).  Every thread stays to the
 // end: the binning is a warp's work.
-template <class E, int MATERIAL, int PHASE>
+template <class E, int MATERIAL, int PHASE, bool LIST>
 __global__ void __launch_bounds__(128) g2p_kernel(const __grid_constant__ G2PArgs A)
 {
     __shared__ G2PConst C;
@@ -899,14 +914,18 @@ __global__ void __launch_bounds__(128) g2p_kernel(const __grid_constant__ G2PArg
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t key = i < A.n ? A.keys[i] : A.sentinel;
     Particle p;
-    if (key != A.sentinel) p = load_particle<MATERIAL, PHASE>(A, i);
+    uint32_t place = 0;
+    if (key != A.sentinel) {
+        place = LIST ? A.pos[key] : key;
+        p = load_particle<MATERIAL, PHASE>(A, i);
+    }
     __syncthreads();
     mpmg_pdl_wait();
     if (A.early) mpmg_pdl_trigger();
     uint32_t next = A.sentinel;
     if (key != A.sentinel) {
         if (PHASE != G2P_STRAIN) A.in_element[i] = (int)key;
-        g2p_particle<E, MATERIAL, PHASE>(A, C, i, (int)key, p);
+        g2p_particle<E, MATERIAL, PHASE>(A, C, i, (int)key, place, p);
         if (PHASE != G2P_MOVE) {
             const int e = mpmg_which_element_fast(p.x, p.y, g.h, g.inv_h, A.inv_hf, g.xmax, g.ymax,
                                                   __double_as_longlong(g.xmax), __double_as_longlong(g.ymax), g.Ex,
@@ -926,14 +945,16 @@ __global__ void __launch_bounds__(128) g2p_kernel(const __grid_constant__ G2PArg
 // each particle's -v gflocal |grad N_j|^2 summed per corner in the binned
 // order of the step, with the start-of-step shape-function gradients.
 __global__ void __launch_bounds__(128) ext_cells_kernel(
-    int ne, double inv_h, RowView rv,
+    int ne, int most, double inv_h, RowView rv, const uint32_t *__restrict__ pos,
     const double *__restrict__ xl, const double *__restrict__ yl, const double *__restrict__ v,
     const double *__restrict__ gflocal, double *__restrict__ cell_sums)
 {
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= ne) return;
     const int cnt = (int)rv.count[e];
+    if (cnt == 0) return;
     const uint32_t *list = rv.list(e, cnt);
+    const uint32_t at = pos != nullptr ? pos[e] : (uint32_t)e;
     double acc[4] = {0, 0, 0, 0};
     for (int k = 0; k < cnt; k++) {
         const int i = (int)list[k];
@@ -946,11 +967,12 @@ __global__ void __launch_bounds__(128) ext_cells_kernel(
         }
     }
 #pragma unroll
-    for (int a = 0; a < 4; a++) cell_sums[(size_t)a * ne + e] = acc[a];
+    for (int a = 0; a < 4; a++) cell_sums[(size_t)a * most + at] = acc[a];
 }
 
 // The nodal sums of ext_cells_kernel's corners in colour order.
-__global__ void __launch_bounds__(256) ext_nodes_kernel(GridGeom g, int ne, const double *__restrict__ cell_sums,
+__global__ void __launch_bounds__(256) ext_nodes_kernel(GridGeom g, int most, const uint32_t *__restrict__ count,
+                                                        const uint32_t *__restrict__ pos, const double *__restrict__ cell_sums,
                                                         double *__restrict__ d2)
 {
     const int nn = g.Nx * g.Ny;
@@ -964,8 +986,9 @@ __global__ void __launch_bounds__(256) ext_nodes_kernel(GridGeom g, int ne, cons
         const int cj = ((j & 1) == (c >> 1)) ? j : j - 1;
         if (ci < 0 || cj < 0 || ci >= g.Ex || cj >= g.Ey) continue;
         const int e = cj * g.Ex + ci;
+        if (count[e] == 0) continue;
         const int corner = (ci == i) ? ((cj == j) ? 0 : 3) : ((cj == j) ? 1 : 2);
-        sum = mat::add(sum, cell_sums[(size_t)corner * ne + e]);
+        sum = mat::add(sum, cell_sums[(size_t)corner * most + (pos != nullptr ? pos[e] : (uint32_t)e)]);
     }
     d2[n] = sum;
 }
@@ -1007,9 +1030,11 @@ __global__ void __launch_bounds__(256) ext_stress_kernel(const __grid_constant__
 // MUSL's second projection (process_usl.c:424-431): per element, the moved
 // particles' mass and momentum with their start-of-step shape functions, in
 // the step's particle order, from the same moments as the P2G.
+template <bool LIST>
 __global__ void __launch_bounds__(128) p2g_momentum_kernel(
-    int ne, RowView rv, const double *__restrict__ xl, const double *__restrict__ yl, const double *__restrict__ m,
-    const double *__restrict__ vx, const double *__restrict__ vy, double *__restrict__ cell_sums)
+    int ne, int most, RowView rv, const uint32_t *__restrict__ pos, const double *__restrict__ xl,
+    const double *__restrict__ yl, const double *__restrict__ m, const double *__restrict__ vx, const double *__restrict__ vy,
+    double *__restrict__ cell_sums)
 {
     mpmg_pdl_wait();
     mpmg_pdl_trigger();
@@ -1018,6 +1043,7 @@ __global__ void __launch_bounds__(128) p2g_momentum_kernel(
     const int cnt = (int)rv.count[e];
     if (cnt == 0) return;
     const uint32_t *list = rv.list(e, cnt);
+    double *out = cell_sums + (LIST ? pos[e] : (uint32_t)e);
     double q[3][4];
 #pragma unroll
     for (int f = 0; f < 3; f++)
@@ -1037,10 +1063,10 @@ __global__ void __launch_bounds__(128) p2g_momentum_kernel(
     }
 #pragma unroll
     for (int f = 0; f < 3; f++) {
-        cell_sums[(size_t)(0 * 3 + f) * ne + e] = (q[f][0] - q[f][1]) - (q[f][2] - q[f][3]);
-        cell_sums[(size_t)(1 * 3 + f) * ne + e] = q[f][1] - q[f][3];
-        cell_sums[(size_t)(2 * 3 + f) * ne + e] = q[f][3];
-        cell_sums[(size_t)(3 * 3 + f) * ne + e] = q[f][2] - q[f][3];
+        out[(size_t)(0 * 3 + f) * most] = (q[f][0] - q[f][1]) - (q[f][2] - q[f][3]);
+        out[(size_t)(1 * 3 + f) * most] = q[f][1] - q[f][3];
+        out[(size_t)(2 * 3 + f) * most] = q[f][3];
+        out[(size_t)(3 * 3 + f) * most] = q[f][2] - q[f][3];
     }
 }
 
@@ -1048,8 +1074,10 @@ __global__ void __launch_bounds__(128) p2g_momentum_kernel(
 // v = p / m where m > 1e-10, else 0.  The reference zeroes the constrained
 // momenta only after forming v, so the boundary conditions do not reach v;
 // the zeroed momenta are what it keeps in the nodes (node_mx, node_my).
+template <bool LIST>
 __global__ void __launch_bounds__(256) node_velocity_kernel(
-    GridGeom g, BcParams bc, int ne, const uint32_t *__restrict__ count, const double *__restrict__ cell_sums,
+    GridGeom g, BcParams bc, int most, const uint32_t *__restrict__ count, const uint32_t *__restrict__ pos,
+    const double *__restrict__ cell_sums,
     const StepParams *__restrict__ sp, double *__restrict__ node_m, double *__restrict__ node_vx,
     double *__restrict__ node_vy, double *__restrict__ node_mx, double *__restrict__ node_my)
 {
@@ -1068,8 +1096,9 @@ __global__ void __launch_bounds__(256) node_velocity_kernel(
         const int e = cj * g.Ex + ci;
         if (count[e] == 0) continue;
         const int corner = (ci == i) ? ((cj == j) ? 0 : 3) : ((cj == j) ? 1 : 2);
+        const uint32_t at = LIST ? pos[e] : (uint32_t)e;
 #pragma unroll
-        for (int q = 0; q < 3; q++) sum[q] += cell_sums[(size_t)(corner * 3 + q) * ne + e];
+        for (int q = 0; q < 3; q++) sum[q] += cell_sums[(size_t)(corner * 3 + q) * most + at];
     }
     const double m = sum[0];
     double vxn = 0, vyn = 0;
@@ -1127,7 +1156,7 @@ __global__ void __launch_bounds__(256) map_keys_kernel(int n, const int *__restr
 RowsOut rows_out(const mpmg_ctx *ctx, int b)
 {
     const RowBins &r = ctx->row;
-    return RowsOut{r.count[b], r.rows[b], r.filled[b], r.n_filled + b, r.head, r.next, r.cap};
+    return RowsOut{r.count[b], r.rows[b], r.filled[b], r.pos[b], r.n_filled + b, r.head, r.next, r.cap};
 }
 
 RowView row_view(const mpmg_ctx *ctx)
@@ -1175,6 +1204,7 @@ G2PArgs make_g2p_args(mpmg_ctx *ctx)
     A.next = rows_out(ctx, 1 - ctx->row.cur);
     A.in_element = ctx->in_element;
     A.active = ctx->active;
+    A.pos = ctx->row.pos[ctx->row.cur];
     A.coef = (const double2 *)ctx->elem_coef;
     A.node_vx = ctx->node_vx;
     A.node_vy = ctx->node_vy;
@@ -1230,9 +1260,13 @@ static cudaError_t launch_g2p(mpmg_ctx *ctx, const G2PArgs &A)
     // two; 1 048 576: 253.8 and 255.6)
     const int t = !bound ? 32 : ctx->np <= (size_t)ctx->sms * 4 * 32 * 16 ? 64 : 128;
     ctx->launches += 1;
+    using E = typename BoundArith<PHASE>::E;
+    const bool list = PHASE != G2P_STRAIN && ctx->row.pos[0] != nullptr;
     return mpmg_launch_pdl(true,
-                           bound ? g2p_kernel<typename BoundArith<PHASE>::E, MATERIAL, PHASE>
-                                 : g2p_kernel<mat::Elastic, MATERIAL, PHASE>,
+                           list ? (bound ? g2p_kernel<E, MATERIAL, PHASE, PHASE != G2P_STRAIN>
+                                         : g2p_kernel<mat::Elastic, MATERIAL, PHASE, PHASE != G2P_STRAIN>)
+                                : (bound ? g2p_kernel<E, MATERIAL, PHASE, false>
+                                         : g2p_kernel<mat::Elastic, MATERIAL, PHASE, false>),
                            dim3(blocks_for(ctx->np, t)), dim3(t), 0, ctx->stream, A);
 }
 
@@ -1244,8 +1278,8 @@ static cudaError_t launch_p2g(mpmg_ctx *ctx, const GridGeom &g, bool keep_order)
     ctx->launches += 1;
     // blocks for the most elements that can be filled; the rest leave at once
     const size_t most = ctx->np < ctx->ne ? ctx->np : ctx->ne;
-    return mpmg_launch_pdl(true, p2g_cells_kernel<EB, SPLIT>, dim3(blocks_for(most, EB)), dim3(EB * SPLIT), 0,
-                           ctx->stream, g, row_view(ctx), (const uint32_t *)r.filled[r.cur],
+    return mpmg_launch_pdl(true, r.pos[0] != nullptr ? p2g_cells_kernel<EB, SPLIT, true> : p2g_cells_kernel<EB, SPLIT, false>,
+                           dim3(blocks_for(most, EB)), dim3(EB * SPLIT), 0, ctx->stream, g, row_view(ctx), (const uint32_t *)r.filled[r.cur],
                            (const uint32_t *)(r.n_filled + r.cur), (const uint32_t *)r.head,
                            (const uint32_t *)r.next, r.cursor, keep_order ? 1 : 0, early_launch(ctx),
                            (const double *)ctx->x, (const double *)ctx->y, (const double *)ctx->m, (const double *)ctx->vx,
@@ -1306,6 +1340,9 @@ int mpmg_launch_step(mpmg_ctx *ctx)
     const int n = (int)ctx->np;
     const int ne = (int)ctx->ne;
     const int nn = (int)ctx->nn;
+    const int most = (int)ctx->row.places;
+    const uint32_t *pos = ctx->row.pos[ctx->row.cur];   // null: sums by element
+    const bool list = pos != nullptr;
     const bool nonlocal = c.material == MPMG_G_NONLOCAL_MU2 || c.material == MPMG_G_NONLOCAL ||
                           c.material == MPMG_G_NONLOCAL_AVG;
     const bool musl = c.scheme == MPMG_SCHEME_MUSL;
@@ -1332,12 +1369,12 @@ int mpmg_launch_step(mpmg_ctx *ctx)
         // move, second projection of the moved momentum, then strain
         // the move phase does not depend on the material
         MPMG_CHECK((launch_g2p<MPMG_ISOLIN, G2P_MOVE>(ctx, A)));
-        MPMG_CHECK(mpmg_launch_pdl(true, p2g_momentum_kernel, dim3(blocks_for(ne, 128)), dim3(128), 0, s, ne,
-                                   row_view(ctx), (const double *)ctx->xl, (const double *)ctx->yl,
+        MPMG_CHECK(mpmg_launch_pdl(true, list ? p2g_momentum_kernel<true> : p2g_momentum_kernel<false>, dim3(blocks_for(ne, 128)), dim3(128), 0, s, ne, most,
+                                   row_view(ctx), pos, (const double *)ctx->xl, (const double *)ctx->yl,
                                    (const double *)ctx->m, (const double *)ctx->vx, (const double *)ctx->vy,
                                    ctx->cell_sums));
-        MPMG_CHECK(mpmg_launch_pdl(true, node_velocity_kernel, dim3(blocks_for(nn, 256)), dim3(256), 0, s, g,
-                                   make_bc(ctx), ne, (const uint32_t *)ctx->row.count[ctx->row.cur],
+        MPMG_CHECK(mpmg_launch_pdl(true, list ? node_velocity_kernel<true> : node_velocity_kernel<false>, dim3(blocks_for(nn, 256)), dim3(256), 0, s, g,
+                                   make_bc(ctx), most, (const uint32_t *)ctx->row.count[ctx->row.cur], pos,
                                    (const double *)ctx->cell_sums, (const StepParams *)ctx->d_params, ctx->node_m,
                                    ctx->node_vx, ctx->node_vy, ctx->node_mx, ctx->node_my));
         ctx->launches += 2;
@@ -1363,9 +1400,10 @@ int mpmg_launch_step(mpmg_ctx *ctx)
         case MPMG_G_LOCAL_MU2_REVERSE: MPMG_CHECK((launch_g2p<MPMG_G_LOCAL_MU2_REVERSE, G2P_FULL>(ctx, A))); break;
         case MPMG_G_LOCAL_MU2_EXT:
             MPMG_CHECK((launch_g2p<MPMG_G_LOCAL_MU2_EXT, G2P_FULL>(ctx, A)));
-            ext_cells_kernel<<<blocks_for(ne, 128), 128, 0, s>>>(ne, ctx->inv_h, row_view(ctx), ctx->xl, ctx->yl,
+            ext_cells_kernel<<<blocks_for(ne, 128), 128, 0, s>>>(ne, most, ctx->inv_h, row_view(ctx), pos, ctx->xl, ctx->yl,
                                                                 ctx->v, ctx->state[4], ctx->cell_sums);
-            ext_nodes_kernel<<<blocks_for(nn, 256), 256, 0, s>>>(g, ne, ctx->cell_sums, ctx->node_gf);
+            ext_nodes_kernel<<<blocks_for(nn, 256), 256, 0, s>>>(g, most, ctx->row.count[ctx->row.cur], pos,
+                                                                ctx->cell_sums, ctx->node_gf);
             ext_stress_kernel<<<blocks_for(n, 256), 256, 0, s>>>(A, ctx->node_gf);
             ctx->launches += 3;
             break;

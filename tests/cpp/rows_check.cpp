@@ -33,3 +33,8 @@ extern "C" int row_width(const int *emap, size_t n, size_t ne, int no_memory, in
     *cap = mpmg_row_slots(count.inside, *filled, n, ne);
     return 0;
 }
+
+extern "C" int sums_by_list(size_t n, size_t ne)
+{
+    return mpmg_sums_by_list(n, ne) ? 1 : 0;
+}

@@ -61,3 +61,10 @@ def test_crowd_on_a_large_grid_takes_narrow_rows(rows, ppc):
         rc, cap, filled = width(rows, emap, ne)
         assert rc == 0 and filled == crowded
         assert cap == 16 or cap * ne <= 128 * emap.size
+
+
+def test_sums_by_list_only_on_large_empty_grids(rows):
+    rows.sums_by_list.argtypes = [C.c_size_t, C.c_size_t]
+    for n, ne, want in ((0, 1, 0), (10, (1 << 24) - 1, 0), (10, 1 << 24, 1), (1 << 23, 1 << 24, 0), ((1 << 23) - 1, 1 << 24, 1),
+                        (1 << 28, 1 << 29, 0), (1 << 20, 1 << 30, 1)):
+        assert rows.sums_by_list(n, ne) == want, (n, ne)
