@@ -197,7 +197,7 @@ struct mpmg_ctx {
     BinScratch bin;
 
     // P2G corner sums: a run of 20 doubles a place (RowBins; MUSL's and
-    // g_local_mu2_ext's own sums lie in it value-major).
+    // g_local_mu2_ext's own sums lie in it by element value-major).
     double *cell_sums;
 
     // Grid.

@@ -62,7 +62,8 @@ inline int mpmg_row_slots(size_t inside, size_t filled, size_t n, size_t ne)
 // element of the grid.  By list, an element of an empty grid takes 200 bytes with
 // its node instead of 480, and the place is one more load (1 048 576 particles on
 // 262 144 elements 5570 us a pass of 20 steps, 5517 by element; 125k 2246 and
-// 2198): so only grids whose size is a matter of memory, 8 GB by element here.
+// 2198; 7 million on 2^24 3983 us a step and 3825): so only grids whose size is a
+// matter of memory, 8 GB by element here.
 inline bool mpmg_sums_by_list(size_t n, size_t ne)
 {
     return ne >= ((size_t)1 << 24) && ne > 2 * n;

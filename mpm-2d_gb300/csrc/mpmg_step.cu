@@ -945,7 +945,7 @@ __global__ void __launch_bounds__(128) g2p_kernel(const __grid_constant__ G2PArg
 // each particle's -v gflocal |grad N_j|^2 summed per corner in the binned
 // order of the step, with the start-of-step shape-function gradients.
 __global__ void __launch_bounds__(128) ext_cells_kernel(
-    int ne, int most, double inv_h, RowView rv, const uint32_t *__restrict__ pos,
+    int ne, double inv_h, RowView rv, const uint32_t *__restrict__ pos,
     const double *__restrict__ xl, const double *__restrict__ yl, const double *__restrict__ v,
     const double *__restrict__ gflocal, double *__restrict__ cell_sums)
 {
@@ -954,7 +954,8 @@ __global__ void __launch_bounds__(128) ext_cells_kernel(
     const int cnt = (int)rv.count[e];
     if (cnt == 0) return;
     const uint32_t *list = rv.list(e, cnt);
-    const uint32_t at = pos != nullptr ? pos[e] : (uint32_t)e;
+    double *out = pos != nullptr ? cell_sums + (size_t)pos[e] * 4 : cell_sums + e;
+    const size_t step = pos != nullptr ? 1 : (size_t)ne;
     double acc[4] = {0, 0, 0, 0};
     for (int k = 0; k < cnt; k++) {
         const int i = (int)list[k];
@@ -967,11 +968,11 @@ __global__ void __launch_bounds__(128) ext_cells_kernel(
         }
     }
 #pragma unroll
-    for (int a = 0; a < 4; a++) cell_sums[(size_t)a * most + at] = acc[a];
+    for (int a = 0; a < 4; a++) out[a * step] = acc[a];
 }
 
 // The nodal sums of ext_cells_kernel's corners in colour order.
-__global__ void __launch_bounds__(256) ext_nodes_kernel(GridGeom g, int most, const uint32_t *__restrict__ count,
+__global__ void __launch_bounds__(256) ext_nodes_kernel(GridGeom g, int ne, const uint32_t *__restrict__ count,
                                                         const uint32_t *__restrict__ pos, const double *__restrict__ cell_sums,
                                                         double *__restrict__ d2)
 {
@@ -988,7 +989,7 @@ __global__ void __launch_bounds__(256) ext_nodes_kernel(GridGeom g, int most, co
         const int e = cj * g.Ex + ci;
         if (count[e] == 0) continue;
         const int corner = (ci == i) ? ((cj == j) ? 0 : 3) : ((cj == j) ? 1 : 2);
-        sum = mat::add(sum, cell_sums[(size_t)corner * most + (pos != nullptr ? pos[e] : (uint32_t)e)]);
+        sum = mat::add(sum, cell_sums[pos != nullptr ? (size_t)pos[e] * 4 + corner : (size_t)corner * ne + e]);
     }
     d2[n] = sum;
 }
@@ -1032,7 +1033,7 @@ __global__ void __launch_bounds__(256) ext_stress_kernel(const __grid_constant__
 // the step's particle order, from the same moments as the P2G.
 template <bool LIST>
 __global__ void __launch_bounds__(128) p2g_momentum_kernel(
-    int ne, int most, RowView rv, const uint32_t *__restrict__ pos, const double *__restrict__ xl,
+    int ne, RowView rv, const uint32_t *__restrict__ pos, const double *__restrict__ xl,
     const double *__restrict__ yl, const double *__restrict__ m, const double *__restrict__ vx, const double *__restrict__ vy,
     double *__restrict__ cell_sums)
 {
@@ -1043,7 +1044,9 @@ __global__ void __launch_bounds__(128) p2g_momentum_kernel(
     const int cnt = (int)rv.count[e];
     if (cnt == 0) return;
     const uint32_t *list = rv.list(e, cnt);
-    double *out = cell_sums + (LIST ? pos[e] : (uint32_t)e);
+    // by element value-major, by list a run a place (they come in no order)
+    double *out = LIST ? cell_sums + (size_t)pos[e] * 12 : cell_sums + e;
+    const size_t step = LIST ? 1 : (size_t)ne;
     double q[3][4];
 #pragma unroll
     for (int f = 0; f < 3; f++)
@@ -1063,10 +1066,10 @@ __global__ void __launch_bounds__(128) p2g_momentum_kernel(
     }
 #pragma unroll
     for (int f = 0; f < 3; f++) {
-        out[(size_t)(0 * 3 + f) * most] = (q[f][0] - q[f][1]) - (q[f][2] - q[f][3]);
-        out[(size_t)(1 * 3 + f) * most] = q[f][1] - q[f][3];
-        out[(size_t)(2 * 3 + f) * most] = q[f][3];
-        out[(size_t)(3 * 3 + f) * most] = q[f][2] - q[f][3];
+        out[(0 * 3 + f) * step] = (q[f][0] - q[f][1]) - (q[f][2] - q[f][3]);
+        out[(1 * 3 + f) * step] = q[f][1] - q[f][3];
+        out[(2 * 3 + f) * step] = q[f][3];
+        out[(3 * 3 + f) * step] = q[f][2] - q[f][3];
     }
 }
 
@@ -1076,7 +1079,7 @@ __global__ void __launch_bounds__(128) p2g_momentum_kernel(
 // the zeroed momenta are what it keeps in the nodes (node_mx, node_my).
 template <bool LIST>
 __global__ void __launch_bounds__(256) node_velocity_kernel(
-    GridGeom g, BcParams bc, int most, const uint32_t *__restrict__ count, const uint32_t *__restrict__ pos,
+    GridGeom g, BcParams bc, int ne, const uint32_t *__restrict__ count, const uint32_t *__restrict__ pos,
     const double *__restrict__ cell_sums,
     const StepParams *__restrict__ sp, double *__restrict__ node_m, double *__restrict__ node_vx,
     double *__restrict__ node_vy, double *__restrict__ node_mx, double *__restrict__ node_my)
@@ -1096,9 +1099,9 @@ __global__ void __launch_bounds__(256) node_velocity_kernel(
         const int e = cj * g.Ex + ci;
         if (count[e] == 0) continue;
         const int corner = (ci == i) ? ((cj == j) ? 0 : 3) : ((cj == j) ? 1 : 2);
-        const uint32_t at = LIST ? pos[e] : (uint32_t)e;
+        const double *src = LIST ? cell_sums + (size_t)pos[e] * 12 + corner * 3 : cell_sums + (size_t)(corner * 3) * ne + e;
 #pragma unroll
-        for (int q = 0; q < 3; q++) sum[q] += cell_sums[(size_t)(corner * 3 + q) * most + at];
+        for (int q = 0; q < 3; q++) sum[q] += src[LIST ? q : (size_t)q * ne];
     }
     const double m = sum[0];
     double vxn = 0, vyn = 0;
@@ -1279,7 +1282,8 @@ static cudaError_t launch_p2g(mpmg_ctx *ctx, const GridGeom &g, bool keep_order)
     // blocks for the most elements that can be filled; the rest leave at once
     const size_t most = ctx->np < ctx->ne ? ctx->np : ctx->ne;
     return mpmg_launch_pdl(true, r.pos[0] != nullptr ? p2g_cells_kernel<EB, SPLIT, true> : p2g_cells_kernel<EB, SPLIT, false>,
-                           dim3(blocks_for(most, EB)), dim3(EB * SPLIT), 0, ctx->stream, g, row_view(ctx), (const uint32_t *)r.filled[r.cur],
+                           dim3(blocks_for(most, EB)), dim3(EB * SPLIT), 0, ctx->stream, g, row_view(ctx),
+                           (const uint32_t *)r.filled[r.cur],
                            (const uint32_t *)(r.n_filled + r.cur), (const uint32_t *)r.head,
                            (const uint32_t *)r.next, r.cursor, keep_order ? 1 : 0, early_launch(ctx),
                            (const double *)ctx->x, (const double *)ctx->y, (const double *)ctx->m, (const double *)ctx->vx,
@@ -1340,7 +1344,6 @@ int mpmg_launch_step(mpmg_ctx *ctx)
     const int n = (int)ctx->np;
     const int ne = (int)ctx->ne;
     const int nn = (int)ctx->nn;
-    const int most = (int)ctx->row.places;
     const uint32_t *pos = ctx->row.pos[ctx->row.cur];   // null: sums by element
     const bool list = pos != nullptr;
     const bool nonlocal = c.material == MPMG_G_NONLOCAL_MU2 || c.material == MPMG_G_NONLOCAL ||
@@ -1369,12 +1372,12 @@ int mpmg_launch_step(mpmg_ctx *ctx)
         // move, second projection of the moved momentum, then strain
         // the move phase does not depend on the material
         MPMG_CHECK((launch_g2p<MPMG_ISOLIN, G2P_MOVE>(ctx, A)));
-        MPMG_CHECK(mpmg_launch_pdl(true, list ? p2g_momentum_kernel<true> : p2g_momentum_kernel<false>, dim3(blocks_for(ne, 128)), dim3(128), 0, s, ne, most,
+        MPMG_CHECK(mpmg_launch_pdl(true, list ? p2g_momentum_kernel<true> : p2g_momentum_kernel<false>, dim3(blocks_for(ne, 128)), dim3(128), 0, s, ne,
                                    row_view(ctx), pos, (const double *)ctx->xl, (const double *)ctx->yl,
                                    (const double *)ctx->m, (const double *)ctx->vx, (const double *)ctx->vy,
                                    ctx->cell_sums));
         MPMG_CHECK(mpmg_launch_pdl(true, list ? node_velocity_kernel<true> : node_velocity_kernel<false>, dim3(blocks_for(nn, 256)), dim3(256), 0, s, g,
-                                   make_bc(ctx), most, (const uint32_t *)ctx->row.count[ctx->row.cur], pos,
+                                   make_bc(ctx), ne, (const uint32_t *)ctx->row.count[ctx->row.cur], pos,
                                    (const double *)ctx->cell_sums, (const StepParams *)ctx->d_params, ctx->node_m,
                                    ctx->node_vx, ctx->node_vy, ctx->node_mx, ctx->node_my));
         ctx->launches += 2;
@@ -1400,9 +1403,9 @@ int mpmg_launch_step(mpmg_ctx *ctx)
         case MPMG_G_LOCAL_MU2_REVERSE: MPMG_CHECK((launch_g2p<MPMG_G_LOCAL_MU2_REVERSE, G2P_FULL>(ctx, A))); break;
         case MPMG_G_LOCAL_MU2_EXT:
             MPMG_CHECK((launch_g2p<MPMG_G_LOCAL_MU2_EXT, G2P_FULL>(ctx, A)));
-            ext_cells_kernel<<<blocks_for(ne, 128), 128, 0, s>>>(ne, most, ctx->inv_h, row_view(ctx), pos, ctx->xl, ctx->yl,
+            ext_cells_kernel<<<blocks_for(ne, 128), 128, 0, s>>>(ne, ctx->inv_h, row_view(ctx), pos, ctx->xl, ctx->yl,
                                                                 ctx->v, ctx->state[4], ctx->cell_sums);
-            ext_nodes_kernel<<<blocks_for(nn, 256), 256, 0, s>>>(g, most, ctx->row.count[ctx->row.cur], pos,
+            ext_nodes_kernel<<<blocks_for(nn, 256), 256, 0, s>>>(g, ne, ctx->row.count[ctx->row.cur], pos,
                                                                 ctx->cell_sums, ctx->node_gf);
             ext_stress_kernel<<<blocks_for(n, 256), 256, 0, s>>>(A, ctx->node_gf);
             ctx->launches += 3;
