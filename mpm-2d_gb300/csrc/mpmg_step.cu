@@ -1037,11 +1037,15 @@ __global__ void __launch_bounds__(128) p2g_momentum_kernel(
     const double *__restrict__ yl, const double *__restrict__ m, const double *__restrict__ vx, const double *__restrict__ vy,
     double *__restrict__ cell_sums)
 {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    // The counts are the previous step's work.  A warp of empty elements leaves
+    // without waiting; block 0 waits always, so that this kernel ends after the
+    // one before it (4000 particles on 2048^2 elements: 187 us a step, 206 with a
+    // wait in every warp).
+    const int cnt = e < ne ? (int)rv.count[e] : 0;
+    if (!__any_sync(0xffffffffu, cnt != 0) && blockIdx.x != 0) return;
     mpmg_pdl_wait();
     mpmg_pdl_trigger();
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= ne) return;
-    const int cnt = (int)rv.count[e];
     if (cnt == 0) return;
     const uint32_t *list = rv.list(e, cnt);
     // by element value-major, by list a run a place (they come in no order)
