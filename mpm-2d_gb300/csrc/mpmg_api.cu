@@ -365,17 +365,24 @@ double *mpmg_device_view(const void *p, size_t bytes)
 
 namespace {
 
-// Has the pages of [dst, dst + bytes) mapped where its last one is not: an array
-// fresh from the allocator, which is about to be written.
+// Has the pages of [dst, dst + bytes) mapped, from the first that is not (an array
+// fresh from the allocator, or grown by it), since they are about to be written.
 void map_pages(void *dst, size_t bytes)
 {
 #ifndef MADV_POPULATE_WRITE
 #define MADV_POPULATE_WRITE 23
 #endif
-    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), begin = (uintptr_t)dst, end = begin + bytes;
-    unsigned char there = 0;
-    if (mincore((void *)((end - 1) / page * page), 1, &there) == 0 && (there & 1)) return;
-    madvise((void *)(begin / page * page), end - begin / page * page, MADV_POPULATE_WRITE);   // a hint: may fail
+    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), end = (uintptr_t)dst + bytes;
+    unsigned char there[1024];
+    for (uintptr_t p = (uintptr_t)dst / page * page; p < end;) {
+        const size_t pages = std::min((size_t)((end - p + page - 1) / page), sizeof(there));
+        if (mincore((void *)p, pages * page, there) != 0) return;
+        for (size_t k = 0; k < pages; k++, p += page) {
+            if (there[k] & 1) continue;
+            madvise((void *)p, end - p, MADV_POPULATE_WRITE);   // a hint: may fail
+            return;
+        }
+    }
 }
 
 }  // namespace

@@ -49,6 +49,28 @@ def test_reads_into_fresh_and_partly_mapped_pages():
     sim.close()
 
 
+def test_partly_mapped_arrays_cost_no_more_than_fresh_ones():
+    """An array grown by its allocator: some pages mapped, the rest not (twice the fresh array's time at most)."""
+    sim = mpm2d.Simulation(scenes.box_fill(cells=128, material="isolin"))
+    sim.step(1)
+
+    def best(touched):
+        t = np.inf
+        for _ in range(15):
+            a = np.frombuffer(mmap.mmap(-1, 8 * sim.n), dtype=np.float64)
+            a[touched] = 1.0
+            start = time.perf_counter()
+            sim.get_frame(["x"], out={"x": a})
+            t = min(t, time.perf_counter() - start)
+        return t
+
+    best([])
+    fresh = best([])
+    for touched in ([0], [-1], [0, -1]):
+        assert best(touched) <= 2 * fresh, (touched, best(touched), fresh)
+    sim.close()
+
+
 def test_a_mixed_field_is_one_launch():
     """No permutation formed for a single field, and the values of the frame export (bit for bit)."""
     for members in (None, 3):
