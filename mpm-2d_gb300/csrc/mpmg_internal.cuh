@@ -186,6 +186,7 @@ struct mpmg_ctx {
     double *elem_coef;
     uint32_t *sort_keys;   // input of mpmg_fp64_sort, allocated last
     SortScratch sort_scratch;
+    void *out_small;       // pinned, 32 KB: mpmg_copy_out
     std::recursive_mutex read_lock;   // held by a read that goes through the context's own buffers
     int sms;
 
