@@ -1327,16 +1327,18 @@ size_t p2g_tiles(const mpmg_config &c, int v)
     return (size_t)mpmg_tiles_along((uint32_t)c.Nx, kTileX[v]) * mpmg_tiles_along((uint32_t)c.Ny, kTileY[v]);
 }
 
-// The shape that stands for variant 0: rows of 32 elements, or the square where
-// it leaves at most 7/8 of the tiles (us a step with rows and squares: 3 x 20001
-// nodes 40.0 and 26.3, 33 x 4001 33.6 and 31.7, 129 x 1001 30.4 and 28.6; 48 x
-// 3001, at 0.94 of the tiles, 31.9 and 33.0); in a batch the half tile where it
+// The shape that stands for variant 0: rows of 32 elements.  Where those are more
+// tiles than a wave (four blocks an SM), the square if it leaves at most 7/8 of
+// them (us a step with rows and squares: 3 x 20001 nodes 40.0 and 26.3, 33 x 4001
+// 33.6 and 31.7, 129 x 1001 30.4 and 28.6; 48 x 3001, at 0.94 of the tiles, 31.9
+// and 33.0; within a wave, 70 x 70, 17.6 and 18.5); in a batch the half tile if it
 // takes no more tiles than the square (2000 members of 5 x 5 nodes 38.7 and 32.0).
-int p2g_default_shape(const mpmg_config *cfg, int count, bool batch)
+int p2g_default_shape(const mpmg_config *cfg, int count, bool batch, int sms)
 {
     size_t tiles[kP2GShapes] = {0, 0, 0, 0};
     for (int k = 0; k < count; k++)
         for (int v = 0; v < kP2GShapes; v++) tiles[v] += p2g_tiles(cfg[k], v);
+    if (tiles[0] <= (size_t)sms * 4) return 0;
     if (batch && tiles[1] <= tiles[3] && tiles[1] <= tiles[0]) return 1;
     return 8 * tiles[3] <= 7 * tiles[0] ? 3 : 0;
 }
@@ -1382,7 +1384,9 @@ int mpmg_mixed_init(mpmg_ctx *ctx, const double *m, const double *v, const doubl
     // members: one, or the batch's (their constants and first-index tables)
     BatchInfo *bt = ctx->batch;
     const int count = bt ? bt->count : 1;
-    s->p2g_default = p2g_default_shape(bt ? bt->cfg.data() : &ctx->cfg, count, bt != nullptr);
+    int sms = 0;
+    MPMG_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->dev));
+    s->p2g_default = p2g_default_shape(bt ? bt->cfg.data() : &ctx->cfg, count, bt != nullptr, sms);
     if (bt) {
         std::vector<MemberM> hm(count);
         std::vector<int> eo(count + 1);
@@ -1473,8 +1477,6 @@ int mpmg_mixed_init(mpmg_ctx *ctx, const double *m, const double *v, const doubl
     s->cur = 0;
     // persistent G2P grid: as many blocks as fit on the device at once, at
     // most one per tile
-    int sms = 0;
-    MPMG_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->dev));
     for (int t = 0; t < kG2PTiles; t++) {
         const int tile = kG2PTileSizes[t];
         MPMG_CHECK(cudaFuncSetAttribute(g2p_variant(ctx->cfg.material, bt != nullptr, tile),

@@ -1,7 +1,7 @@
-"""The mixed P2G's tile shapes, by the grids they are chosen for: thin and small ones
-(square tiles), tiny batch members (half tiles) and wide ones (rows).  Batches equal
-their members run alone bit for bit, whatever shape either takes, and those the FP64
-form: FP32 state, a few steps, 1e-5 of the field's norm."""
+"""The mixed P2G's tile shapes, by the grids they are chosen for: more tiles than a wave
+on thin and small ones (square tiles) and tiny batch members (half tiles), rows else.
+Batches equal their members run alone bit for bit, whatever shape either takes, and
+those the FP64 form: FP32 state, a few steps, 1e-5 of the field's norm."""
 import time
 
 import numpy as np
@@ -15,7 +15,9 @@ pytestmark = pytest.mark.gpu
 
 FIELDS = ("x", "y", "vx", "vy", "v", "sxx", "sxy", "syy", "node_m", "node_vx", "node_vy")
 GRIDS = {"tiny": [(2, 2), (3, 3), (5, 5), (5, 4), (3, 6)], "small": [(9, 9), (13, 13), (16, 9)],
-         "thin": [(3, 301), (9, 200), (33, 130), (16, 100)], "wide": [(300, 3), (200, 33)]}
+         "thin": [(3, 301), (9, 200), (33, 130), (16, 100)], "wide": [(300, 3), (200, 33)],
+         "many tiny": [(2, 2), (3, 3), (5, 5), (5, 4), (3, 6)] * 160, "many small": [(9, 9), (13, 13), (16, 9)] * 160,
+         "long": [(3, 9200), (9, 6001), (33, 3001)]}
 
 
 @pytest.mark.parametrize("precision", ["mixed", "mixed_f64node"])
@@ -24,7 +26,7 @@ def test_shapes(kind, precision):
     members = [small_grid(nx, ny, k) for k, (nx, ny) in enumerate(GRIDS[kind])]
     batch = mpm2d.Batch(members, precision=precision)
     batch.step(5)
-    for k, sc in enumerate(members):
+    for k, sc in list(enumerate(members))[-8:]:
         one = mpm2d.Simulation(sc, precision=precision)
         ref = mpm2d.Simulation(sc, precision="fp64")
         one.step(5)
